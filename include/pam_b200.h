@@ -72,6 +72,16 @@ int pamk_pam_bwd(const float* a, int a_kind, float a_imm, const float* b, int b_
 int pamk_pad_bwd(const float* a, int a_kind, float a_imm, const float* b, int b_kind, float b_imm,
                  const float* dc, int dc_kind, float dc_imm,
                  float* out, int64_t n, int64_t inner, float offset, void* stream);
+/* Both gradients of c = pam(a, b) (pamk_pam_grad) or c = pad(a, b) (pamk_pad_grad) in one pass over a, b and dc:
+ * da[i] and db[i] (either may be NULL), by the approximate rule of pam/cuda_bindings.py:39-57, 79-97 where
+ * approx_a / approx_b is set and by the exact one (pam_bwd / pad_bwd) where not.  Bit for bit what the chain of
+ * launches above gives. */
+int pamk_pam_grad(const float* a, int a_kind, float a_imm, const float* b, int b_kind, float b_imm,
+                  const float* dc, int dc_kind, float dc_imm,
+                  float* da, float* db, int64_t n, int64_t inner, float offset, int approx_a, int approx_b, void* stream);
+int pamk_pad_grad(const float* a, int a_kind, float a_imm, const float* b, int b_kind, float b_imm,
+                  const float* dc, int dc_kind, float dc_imm,
+                  float* da, float* db, int64_t n, int64_t inner, float offset, int approx_a, int approx_b, void* stream);
 /* y = base^x                    replaces pa_exp_fwd — elementwise_pa_exp_caller, cuda_kernels.cu:348-373 */
 int pamk_pa_exp_fwd(const float* x, float* y, int64_t n, float base, float offset, void* stream);
 /* exact backward of base^x      replaces pa_exp_bwd — cuda_kernels.cu:395-423 */

@@ -13,6 +13,7 @@ import torch
 _PKG = pathlib.Path(__file__).resolve().parent
 # PAM_B200_LIBRARY points at another build of the same library (A/B comparisons of kernel variants).
 LIB_PATH = pathlib.Path(os.environ.get("PAM_B200_LIBRARY") or _PKG / "libpam_b200.so")
+HOST_PATH = _PKG / "_host.so"
 
 FULL, SCALAR, ROW, COL, IMM = 0, 1, 2, 3, 4
 MUL_PAM, MUL_STANDARD = 0, 1
@@ -29,6 +30,8 @@ _SIGNATURES = {
     "pamk_pad_fwd": (_i, _operand * 2 + [_p, _i64, _i64, _f, _p]),
     "pamk_pam_bwd": (_i, _operand * 3 + [_p, _i64, _i64, _f, _p]),
     "pamk_pad_bwd": (_i, _operand * 3 + [_p, _i64, _i64, _f, _p]),
+    "pamk_pam_grad": (_i, _operand * 3 + [_p, _p, _i64, _i64, _f, _i, _i, _p]),
+    "pamk_pad_grad": (_i, _operand * 3 + [_p, _p, _i64, _i64, _f, _i, _i, _p]),
     "pamk_pa_exp_fwd": (_i, [_p, _p, _i64, _f, _f, _p]),
     "pamk_pa_exp_bwd": (_i, [_p, _p, _p, _i64, _f, _f, _p]),
     "pamk_pa_log_fwd": (_i, [_p, _p, _i64, _f, _f, _p]),
@@ -124,6 +127,31 @@ def lib():
             fn.restype, fn.argtypes = res, args
         _lib = handle
     return lib() if _nvtx else _lib
+
+
+_host = None
+
+
+def host():
+    """The native host path (csrc/host.cpp) bound to the loaded library, or None while NVTX ranges are on (the
+    Python layer then runs, whose library calls carry them).  Raises if it was never built."""
+    global _host
+    if _nvtx:
+        return None
+    if _host is None:
+        if not HOST_PATH.exists():
+            raise RuntimeError(f"{HOST_PATH} is missing: build it with `python -m pam_b200.build`")
+        lib()
+        import importlib.machinery
+        import importlib.util
+        loader = importlib.machinery.ExtensionFileLoader("pam_b200._host", str(HOST_PATH))
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader(loader.name, loader))
+        loader.exec_module(module)
+        module.setup(str(LIB_PATH), PamKernelError)
+        from . import cuda_bindings
+        module.set_strict(cuda_bindings.strict_k_order())
+        _host = module
+    return _host
 
 
 def exported_names():

@@ -1,9 +1,11 @@
 """Builds ``pam_b200/libpam_b200.so`` — every CUDA source under ``pam_b200/csrc`` compiled for
-sm_100a with nvcc and linked into one C-ABI shared library (declared in ``include/pam_b200.h``).
+sm_100a with nvcc and linked into one C-ABI shared library (declared in ``include/pam_b200.h``) —
+and ``pam_b200/_host.so``, the host path of the operators (``csrc/host.cpp``, a CPython module over
+torch's C++ headers that calls that library).
 
     python -m pam_b200.build [--force] [--verbose]
 
-The library does not depend on torch.  ``-fmad=false`` keeps nvcc from fusing a multiply into a
+The kernel library does not depend on torch.  ``-fmad=false`` keeps nvcc from fusing a multiply into a
 following add: the PAM kernels reproduce the reference's roundings operation by operation and
 use explicit fused multiply-adds only where the reference's build does.
 """
@@ -17,6 +19,7 @@ PKG = pathlib.Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 OBJ = PKG / "build"
 LIB = PKG / "libpam_b200.so"
+HOST = PKG / "_host.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -33,6 +36,28 @@ def _nvcc():
 
 def _stale(target, deps):
     return not target.exists() or any(d.stat().st_mtime > target.stat().st_mtime for d in deps)
+
+
+def build_host(force=False, verbose=False):
+    """The CPython module with the operators' host path: plain C++, no device code."""
+    import sysconfig
+
+    import torch
+    src = CSRC / "host.cpp"
+    if not force and not _stale(HOST, [src, PKG.parent / "include" / "pam_b200.h", pathlib.Path(__file__)]):
+        return HOST
+    root = pathlib.Path(torch.__file__).resolve().parent
+    cuda = pathlib.Path(_nvcc()).resolve().parents[1] / "include"
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *(f"-isystem{d}" for d in (root / "include", root / "include/torch/csrc/api/include", cuda, sysconfig.get_paths()["include"])),
+           str(src), "-o", str(HOST), f"-L{root / 'lib'}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda",
+           "-lc10", "-lc10_cuda", "-ldl"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if verbose or res.returncode:
+        sys.stderr.write(res.stdout + res.stderr)
+    if res.returncode:
+        raise RuntimeError("g++ failed: " + " ".join(cmd))
+    return HOST
 
 
 def build(force=False, verbose=False):
@@ -59,6 +84,7 @@ def build(force=False, verbose=False):
     if force or jobs or _stale(LIB, objs):
         subprocess.check_call([nvcc, "-shared", "-o", str(LIB), *map(str, objs), "-gencode",
                                "arch=compute_100a,code=sm_100a"])
+    build_host(force, verbose)
     return LIB
 
 

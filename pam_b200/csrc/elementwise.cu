@@ -101,6 +101,26 @@ struct LogBwd {
     }
 };
 
+// Both gradients of a product / quotient from one read of the operands and of dc.  AA / AB: the approximate
+// rule for the first / second operand (PAM products, pam/cuda_bindings.py:39-57, 79-97), else the exact one.
+template <bool AA, bool AB>
+struct PamGrad {
+    int32_t off;
+    __device__ float first(float a, float b, float dc) const { return AA ? mul(dc, b, off) : mul_bwd(a, b, dc, off); }
+    __device__ float second(float a, float b, float dc) const { return AB ? mul(dc, a, off) : mul_bwd(b, a, dc, off); }
+};
+template <bool AA, bool AB>
+struct PadGrad {
+    int32_t off;
+    __device__ float first(float a, float b, float dc) const {
+        const float recip = div(1.0f, b, off);
+        return AA ? mul(recip, dc, off) : mul_bwd(a, recip, dc, 0);
+    }
+    __device__ float second(float a, float b, float dc) const {
+        return AB ? -mul(div(div(a, b, off), b, off), dc, off) : div_bwd(a, b, dc, off);
+    }
+};
+
 constexpr int kThreads = 256;
 constexpr int kPerThread = 8;                       // two 128-bit vectors per operand per thread
 constexpr int kPerBlock = kThreads * kPerThread;
@@ -159,6 +179,62 @@ __global__ void __launch_bounds__(kThreads, NIN > 2 ? 6 : 8) ew_kernel(Op op, Op
     }
 }
 
+// Bound by DRAM: a, b and dc are read once for both gradients (20 bytes per element; a launch for each gradient
+// moved 24, and the approximate quotient's chain of five 52).  A launch covers what ew_kernel's does; da or db
+// may be null.
+template <class Op, bool VEC>
+__global__ void __launch_bounds__(kThreads, 4) ew_grad_kernel(Op op, Operand o0, Operand o1, Operand o2, float* __restrict__ da,
+                                                              float* __restrict__ db, Shape s) {
+    const float s0 = splat_value(o0), s1 = splat_value(o1), s2 = splat_value(o2);
+    const int64_t base = (int64_t)blockIdx.x * kPerBlock;
+    if (VEC) {
+        const int64_t n4 = s.n & ~(int64_t)3;
+        float4 a[2], b[2], c[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int64_t i = base + threadIdx.x * 4 + u * kThreads * 4;
+            if (i < n4) {
+                a[u] = load4(o0, i, s, s0);
+                b[u] = load4(o1, i, s, s1);
+                c[u] = load4(o2, i, s, s2);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int64_t i = base + threadIdx.x * 4 + u * kThreads * 4;
+            if (i < n4) {
+                if (da)
+                    *reinterpret_cast<float4*>(da + i) =
+                        make_float4(op.first(a[u].x, b[u].x, c[u].x), op.first(a[u].y, b[u].y, c[u].y),
+                                    op.first(a[u].z, b[u].z, c[u].z), op.first(a[u].w, b[u].w, c[u].w));
+                if (db)
+                    *reinterpret_cast<float4*>(db + i) =
+                        make_float4(op.second(a[u].x, b[u].x, c[u].x), op.second(a[u].y, b[u].y, c[u].y),
+                                    op.second(a[u].z, b[u].z, c[u].z), op.second(a[u].w, b[u].w, c[u].w));
+            }
+        }
+        // ragged tail (fewer than four elements), done by the last CTA
+        if (blockIdx.x == gridDim.x - 1) {
+            const int64_t t = n4 + threadIdx.x;
+            if (t < s.n) {
+                const float x = load1(o0, t, s, s0), y = load1(o1, t, s, s1), z = load1(o2, t, s, s2);
+                if (da) da[t] = op.first(x, y, z);
+                if (db) db[t] = op.second(x, y, z);
+            }
+        }
+    } else {
+#pragma unroll 2
+        for (int u = 0; u < kPerThread; ++u) {
+            const int64_t i = base + threadIdx.x + u * kThreads;
+            if (i < s.n) {
+                const float x = load1(o0, i, s, s0), y = load1(o1, i, s, s1), z = load1(o2, i, s, s2);
+                if (da) da[i] = op.first(x, y, z);
+                if (db) db[i] = op.second(x, y, z);
+            }
+        }
+    }
+}
+
 // An empty launch (n == 0) may carry null pointers: an empty tensor has no storage.
 bool operand_ok(const Operand& o, int64_t n) {
     if (o.kind < PAMK_FULL || o.kind > PAMK_IMM) return false;
@@ -196,6 +272,35 @@ int launch(Op op, Operand o0, Operand o1, Operand o2, float* out, int64_t n, int
     return check_launch();
 }
 
+template <template <bool, bool> class Op>
+int launch_grad(Operand o0, Operand o1, Operand o2, float* da, float* db, int64_t n, int64_t inner, float offset, int approx_a,
+                int approx_b, void* stream) {
+    if (n < 0 || (da == nullptr && db == nullptr && n > 0)) return PAMK_ERR_ARG;
+    if (!operand_ok(o0, n) || !operand_ok(o1, n) || !operand_ok(o2, n)) return PAMK_ERR_ARG;
+    bool needs_inner = false;
+    for (const Operand* o : {&o0, &o1, &o2}) needs_inner |= o->kind == PAMK_ROW || o->kind == PAMK_COL;
+    if (needs_inner && (inner <= 0 || n % inner != 0)) return PAMK_ERR_ARG;
+    if (n == 0) return PAMK_OK;
+    if (inner <= 0) inner = n;
+    const bool vec = aligned16(da) && aligned16(db) && operand_vectorisable(o0, inner) && operand_vectorisable(o1, inner) &&
+                     operand_vectorisable(o2, inner);
+    const Shape s{n, inner};
+    const int64_t blocks = (n + kPerBlock - 1) / kPerBlock;
+    if (blocks > 0x7fffffff) return PAMK_ERR_SIZE;
+    const unsigned grid = (unsigned)blocks;
+    const int32_t off = offset_bits(offset);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+#define PAMK_GRAD(AA, AB)                                                                                       \
+    do {                                                                                                        \
+        if (vec) ew_grad_kernel<Op<AA, AB>, true><<<grid, kThreads, 0, st>>>(Op<AA, AB>{off}, o0, o1, o2, da, db, s);  \
+        else ew_grad_kernel<Op<AA, AB>, false><<<grid, kThreads, 0, st>>>(Op<AA, AB>{off}, o0, o1, o2, da, db, s);     \
+    } while (0)
+    if (approx_a) { if (approx_b) PAMK_GRAD(true, true); else PAMK_GRAD(true, false); }
+    else          { if (approx_b) PAMK_GRAD(false, true); else PAMK_GRAD(false, false); }
+#undef PAMK_GRAD
+    return check_launch();
+}
+
 const Operand kNone{nullptr, PAMK_IMM, 0.0f};
 
 }  // namespace
@@ -229,6 +334,18 @@ int pamk_pad_bwd(const float* a, int a_kind, float a_imm, const float* b, int b_
                  float* out, int64_t n, int64_t inner, float offset, void* stream) {
     return launch<PadBwd, 3>(PadBwd{offset_bits(offset)}, {a, a_kind, a_imm}, {b, b_kind, b_imm},
                              {dc, dc_kind, dc_imm}, out, n, inner, stream);
+}
+
+int pamk_pam_grad(const float* a, int a_kind, float a_imm, const float* b, int b_kind, float b_imm,
+                  const float* dc, int dc_kind, float dc_imm,
+                  float* da, float* db, int64_t n, int64_t inner, float offset, int approx_a, int approx_b, void* stream) {
+    return launch_grad<PamGrad>({a, a_kind, a_imm}, {b, b_kind, b_imm}, {dc, dc_kind, dc_imm}, da, db, n, inner, offset, approx_a, approx_b, stream);
+}
+
+int pamk_pad_grad(const float* a, int a_kind, float a_imm, const float* b, int b_kind, float b_imm,
+                  const float* dc, int dc_kind, float dc_imm,
+                  float* da, float* db, int64_t n, int64_t inner, float offset, int approx_a, int approx_b, void* stream) {
+    return launch_grad<PadGrad>({a, a_kind, a_imm}, {b, b_kind, b_imm}, {dc, dc_kind, dc_imm}, da, db, n, inner, offset, approx_a, approx_b, stream);
 }
 
 int pamk_pa_exp_fwd(const float* x, float* y, int64_t n, float base, float offset, void* stream) {

@@ -28,6 +28,8 @@ _strict_k_order = False
 def set_strict_k_order(flag=True):
     global _strict_k_order
     _strict_k_order = bool(flag)
+    if _lib._host is not None:
+        _lib._host.set_strict(_strict_k_order)
 
 
 def strict_k_order():
@@ -478,6 +480,9 @@ class _StandardMatMul(torch.autograd.Function):
 
 
 # ---- public functions (names and keyword arguments of pam/cuda_bindings.py) ----------------------
+#
+# fp32 CUDA tensors take the native host path (csrc/host.cpp: the same kernels and gradient pairing without
+# the interpreter in between); it declines what it does not cover with None, and the call goes on here.
 
 def _as_operand(v, device):
     """Tensors pass through; Python numbers stay numbers (passed by value to the kernel)."""
@@ -488,12 +493,24 @@ def _as_operand(v, device):
     raise TypeError(f"unsupported operand type {type(v)}")
 
 
+def _on_cuda(t):
+    return isinstance(t, torch.Tensor) and t.is_cuda
+
+
 def pam(A, B, *, offset=None, approx_bwd=False):
+    if (_on_cuda(A) or _on_cuda(B)) and (host := _lib.host()) is not None:
+        out = host.mul(A, B, offset, approx_bwd)
+        if out is not None:
+            return out
     _lib.require_cuda(A, B)
     return _Mul.apply(_as_operand(A, None), _as_operand(B, None), _offset(offset), _pair(approx_bwd))
 
 
 def pad(A, B, *, offset=None, approx_bwd=False):
+    if (_on_cuda(A) or _on_cuda(B)) and (host := _lib.host()) is not None:
+        out = host.div(A, B, offset, approx_bwd)
+        if out is not None:
+            return out
     _lib.require_cuda(A, B)
     if not isinstance(A, torch.Tensor):          # number / tensor: give the kernel a tensor dividend
         A = torch.full((1,), float(A), dtype=torch.float32, device=B.device)
@@ -501,16 +518,28 @@ def pad(A, B, *, offset=None, approx_bwd=False):
 
 
 def pam_matmul(A, B, *, offset=None, approx_bwd=False):
+    if _on_cuda(A) and (host := _lib.host()) is not None:
+        out = host.matmul(A, B, offset, approx_bwd, 2)
+        if out is not None:
+            return out
     return _MatMul.apply(A, B, _offset(offset), _pair(approx_bwd), False)
 
 
 def pam_linear(X, W, bias, *, offset=None, approx_bwd=False):
     """[rows, in] x [out, in] + [out] (no counterpart in the reference's bindings: its `linear` is
     pam_matmul followed by a torch add)."""
+    if _on_cuda(X) and (host := _lib.host()) is not None:
+        out = host.linear(X, W, bias, offset, approx_bwd)
+        if out is not None:
+            return out
     return _Linear.apply(X, W, bias, _offset(offset), _pair(approx_bwd))
 
 
 def pam_bmm(A, B, *, offset=None, approx_bwd=False):
+    if _on_cuda(A) and (host := _lib.host()) is not None:
+        out = host.matmul(A, B, offset, approx_bwd, 3)
+        if out is not None:
+            return out
     return _MatMul.apply(A, B, _offset(offset), _pair(approx_bwd), True)
 
 

@@ -389,10 +389,18 @@ class _AttentionHeads(torch.autograd.Function):
 
 
 def attention_heads(q, k, v, num_heads, mask=None, *, offset=None):
+    if q.is_cuda and (host := _lib.host()) is not None:
+        out = host.attention_heads(q, k, v, mask, int(num_heads), offset)
+        if out is not None:
+            return out
     return _AttentionHeads.apply(q, k, v, mask, int(num_heads), _offset(offset))
 
 
 def attention_qkv(qkv, num_heads, scale, *, offset=None):
+    if qkv.is_cuda and (host := _lib.host()) is not None:
+        out = host.attention_qkv(qkv, int(num_heads), float(scale), offset)
+        if out is not None:
+            return out
     return _AttentionQKV.apply(qkv, int(num_heads), float(scale), _offset(offset))
 
 

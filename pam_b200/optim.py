@@ -14,7 +14,7 @@ import math
 
 import torch
 
-from . import factories, fused
+from . import _lib, factories, fused
 
 
 class Adam(torch.optim.Optimizer):
@@ -45,6 +45,22 @@ class Adam(torch.optim.Optimizer):
         step_size = group["lr"] * math.sqrt(1 - beta2 ** step) / (1 - beta1 ** step)
         return step_size, group["weight_decay"] * group["lr"]
 
+    def _native_step(self, group):
+        """The fused update of a whole group whose parameters, gradients and state are all in the form the kernel
+        takes (fp32, contiguous, on a GPU), collected natively; False leaves the group as it was."""
+        params = group["params"]
+        if not params or not params[0].is_cuda or (host := _lib.host()) is None:
+            return False
+        batches = host.adam_collect(params, self.state)
+        if batches is None:
+            return False
+        beta1, beta2 = group["betas"]
+        for step, tensors in batches:
+            step_size, decay = self._scalars(group, step)
+            host.adam_apply(tensors, beta1, 1 - beta1, beta2, 1 - beta2, group["eps"],
+                            decay if group["weight_decay"] != 0 else 0.0, step_size)
+        return True
+
     @torch.no_grad()
     def step(self, closure=None):
         loss = None
@@ -54,6 +70,8 @@ class Adam(torch.optim.Optimizer):
         ops = self.op_dict
         for group in self.param_groups:
             beta1, beta2 = group["betas"]
+            if self._fusable and fused.enabled and self._native_step(group):
+                continue
             batches = {}             # step count -> tensors that share every scalar of the rule
             for p in group["params"]:
                 if p.grad is None:

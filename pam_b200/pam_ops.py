@@ -10,7 +10,7 @@ import math
 
 import torch
 
-from . import cuda_bindings, fused, utils
+from . import _lib, cuda_bindings, fused, utils
 from .utils import is_number
 
 __all__ = [
@@ -36,12 +36,16 @@ def _lift(*values):
 
 def mul(A, B, *, offset=None, approx_bwd=False, use_kernel=True):
     # pam/pam_ops.py:16-22
+    if isinstance(A, torch.Tensor) or isinstance(B, torch.Tensor):
+        return cuda_bindings.pam(A, B, offset=offset, approx_bwd=approx_bwd)
     tA, tB = _lift(A, B)
     return utils.demote_tensor(cuda_bindings.pam(tA, tB, offset=offset, approx_bwd=approx_bwd), (A, B))
 
 
 def div(A, B, *, offset=None, approx_bwd=False, use_kernel=True):
     # pam/pam_ops.py:25-31
+    if isinstance(A, torch.Tensor) or isinstance(B, torch.Tensor):
+        return cuda_bindings.pad(A, B, offset=offset, approx_bwd=approx_bwd)
     tA, tB = _lift(A, B)
     return utils.demote_tensor(cuda_bindings.pad(tA, tB, offset=offset, approx_bwd=approx_bwd), (A, B))
 
@@ -88,6 +92,10 @@ def bmm(A, B, *, offset=None, approx_bwd=False, use_kernel=True):
 def linear(X, W, bias=None, *, offset=None, approx_bwd=False, use_kernel=True):
     """X @ W.T (+ bias with an ordinary add) over the flattened leading dimensions
     (pam/pam_ops.py:107-115).  W is [out, in]: both operands are contiguous along K."""
+    if fused.enabled and X.is_cuda and (host := _lib.host()) is not None:
+        out = host.linear(X, W, bias, offset, approx_bwd)
+        if out is not None:
+            return out
     lead = X.shape[:-1]
     X2 = X.reshape(-1, X.shape[-1])
     if fused.linear_bias_supported(X2, W, bias):
@@ -226,6 +234,10 @@ def softmax(x, dim=None, *, offset=None, approx_bwd=False, use_kernel=True):
     """PAM softmax (pam/pam_ops.py:305-328): x*log2(e) by PAM, exp2 by the piecewise affine
     exponential after subtracting floor(max) of the WHOLE tensor, -inf entries (attention masks)
     forced to probability 0, ordinary sum, PAM division."""
+    if fused.enabled and x.is_cuda and fused._last_dim(x, dim) and (host := _lib.host()) is not None:
+        out = host.softmax(x, offset, approx_bwd)
+        if out is not None:
+            return out
     if fused.softmax_supported(x, dim, approx_bwd):
         return fused.softmax(x, dim, offset=offset, approx_bwd=approx_bwd)
     if x.numel() == 0:              # (the reference fails here: torch.max of an empty tensor)
@@ -267,6 +279,10 @@ def layer_norm(x, normalized_shape, weight=None, bias=None, eps=1e-05, *,
         normalized_shape = (normalized_shape,)
     normalized_shape = tuple(normalized_shape)
     assert tuple(x.shape[-len(normalized_shape):]) == normalized_shape
+    if fused.enabled and x.is_cuda and (host := _lib.host()) is not None:
+        out = host.layer_norm(x, math.prod(normalized_shape), weight, bias, eps, offset, approx_bwd)
+        if out is not None:
+            return out
     if fused.layer_norm_supported(x, normalized_shape, weight, bias, approx_bwd):
         return fused.layer_norm(x, normalized_shape, weight, bias, eps, offset=offset, approx_bwd=approx_bwd)
     kw = dict(offset=offset, approx_bwd=approx_bwd)
