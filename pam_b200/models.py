@@ -191,13 +191,29 @@ class _Stack(nn.Module):
     def __init__(self, cfg, layers, cross, linear_factory, norm_layer, op_dict):
         super().__init__()
         self.cfg, self.op_dict = cfg, op_dict
+        self._tables = {}
         self.embed_tokens = nn.Embedding(cfg.vocab, cfg.dim, padding_idx=cfg.pad)
         self.embed_scale = math.sqrt(cfg.dim)
         self.layers = nn.ModuleList([TransformerLayer(cfg, cross, linear_factory, norm_layer, op_dict) for _ in range(layers)])
 
+    def _kept(self, name, length, device, make):
+        """A constant table of `length`, made on the host and copied to the device when the length or the device
+        changes (the copy is complete before it is used, on whatever stream), and kept in between."""
+        key, table = self._tables.get(name, (None, None))
+        if key != (length, device):
+            with torch.inference_mode(False):
+                table = make().to(device)
+            self._tables[name] = ((length, device), table)
+        return table
+
     def embed(self, tokens):
         x = self.op_dict["mul"](self.embed_scale, self.embed_tokens(tokens))
-        return x + sinusoidal_positions(tokens.shape[1], self.cfg.dim, self.cfg.pad, tokens.device)
+        length = tokens.shape[1]
+        return x + self._kept("positions", length, tokens.device,
+                              lambda: sinusoidal_positions(length, self.cfg.dim, self.cfg.pad, torch.device("cpu")))
+
+    def future_mask(self, length, device):
+        return self._kept("future", length, device, lambda: torch.full((length, length), float("-inf")).triu(1))
 
 
 class Transformer(nn.Module):
@@ -221,8 +237,7 @@ class Transformer(nn.Module):
         x = self.encoder.embed(src)
         for layer in self.encoder.layers:
             x = layer(x)
-        T = prev_out.shape[1]
-        future = torch.full((T, T), float("-inf"), device=src.device).triu(1)
+        future = self.decoder.future_mask(prev_out.shape[1], src.device)
         y = self.decoder.embed(prev_out)
         for layer in self.decoder.layers:
             y = layer(y, x, future)

@@ -1,17 +1,16 @@
 """Cross entropy with a PAM backward — the counterpart of the reference's ``pam/pam_opt.py`` — and the
 label-smoothed loss of the reference's fairseq criterion computed straight from the logits."""
+import functools
+
 import torch
 
 from . import fused, pam_ops
 
 
-def _pam_binding(ops, names):
-    """If the entries `names` of an operator dictionary are this package's PAM functions, bound (by the
-    factories' dict-form configuration) to one common set of keyword arguments, those arguments; else
-    None.  Lets a chain of dictionary calls be replaced by one fused kernel without changing results."""
+@functools.lru_cache(maxsize=64)
+def _common_binding(names, ops):
     common = None
-    for name in names:
-        op = ops.get(name)
+    for name, op in zip(names, ops):
         func, kwargs = getattr(op, "pam_function", op), getattr(op, "pam_kwargs", {})
         if func is not getattr(pam_ops, name):
             return None
@@ -20,6 +19,14 @@ def _pam_binding(ops, names):
             return None
         common = kwargs
     return common
+
+
+def _pam_binding(ops, names):
+    """If the entries `names` of an operator dictionary are this package's PAM functions, bound (by the
+    factories' dict-form configuration) to one common set of keyword arguments, those arguments; else
+    None.  Lets a chain of dictionary calls be replaced by one fused kernel without changing results.
+    (Remembered per set of functions: a model asks on every forward pass.)"""
+    return _common_binding(names, tuple(ops.get(name) for name in names))
 
 
 class cross_entropy_autograd(torch.autograd.Function):
