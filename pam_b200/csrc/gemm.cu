@@ -18,7 +18,8 @@
 //     every element's exponent is tested against the safe band;
 //   * the reference's per-product range rule (flush below 1e-37, NaN above 1e37 or for
 //     inf/NaN; epfml/pam pam/cuda_kernels.cu:24-37) is hoisted.  A slab whose elements all have their
-//     exponent in a band that keeps every product in range runs the two-instruction loop.  In any other
+//     exponent in a band that keeps every product in range runs the two-instruction loop, and so does one
+//     whose other elements are all zeros (their products get weight 0).  In any other
 //     slab the choice is made per k line: a line without out-of-band elements still costs two
 //     instructions per product; a line whose largest magnitudes cannot multiply beyond the pass range
 //     evaluates the true product only to decide "flush or add" (four instructions); only a line
@@ -206,7 +207,9 @@ __device__ __forceinline__ void store_slab(float* s, const float (&r)[NT * 4], i
 //   * Otherwise the staging threads that hold out-of-band elements record, per k line, that the line
 //     is dirty and whether it holds an element above the band.  A clean line of a dirty slab still
 //     costs two instructions per product.
-//   * A dirty line evaluates the true fp32 product.  It can skip the overflow test when the largest
+//   * A slab whose out-of-band elements are all zeros gives them weight 0 in a fused multiply-add and stays
+//     at two instructions per product (see the loop).
+//   * Any other dirty line evaluates the true fp32 product.  It can skip the overflow test when the largest
 //     magnitudes of its two operand lines cannot multiply beyond 1e37 and neither holds an inf / NaN
 //     (|a * b| rounded grows with |a| and |b|, so the two maxima bound every product of the line):
 //     four instructions per product, "flush or add".  Only the remaining lines apply the full rule.
@@ -251,6 +254,21 @@ __device__ __forceinline__ unsigned dirty_lines(const float (&r)[NT * 4], int ti
     return lines;
 }
 
+// Sorts of out-of-band elements in four consecutive words of a staged slab row (`bias` undoes the A side's
+// pre-bias): `zero_kind` for zeros, kOther for the rest.
+enum Kind { kZerosA = 1, kZerosB = 2, kOther = 4 };
+
+__device__ __forceinline__ unsigned kinds_of(const int4& v, int bias, unsigned zero_kind) {
+    unsigned kinds = 0;
+    const int e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const uint32_t b = (uint32_t)iadd(e[c], bias), m2 = b + b;
+        if (m2 - kBandLo2 >= kBandSpan2) kinds |= m2 == 0 ? zero_kind : (unsigned)kOther;
+    }
+    return kinds;
+}
+
 template <int MODE, class T, bool A_KC, bool B_KC, bool VEC>
 __global__ void __launch_bounds__(T::kThreads, MODE == kPam || MODE == kStd ? T::kCtasPerSm : T::kCtasPerSm / 2)
 gemm_kernel(const GemmParams p) {
@@ -259,6 +277,8 @@ gemm_kernel(const GemmParams p) {
     constexpr int kFastUnroll = (!A_KC && !B_KC) || 8 > BK ? BK : 8;
     __shared__ __align__(16) float As[2][BK * row_stride(BM)];
     __shared__ __align__(16) float Bs[2][BK * row_stride(BN)];
+    __shared__ __align__(16) float weights[MODE == kPam ? BK * row_stride(BM) : 1];   // of the side that holds zeros
+    __shared__ unsigned kinds[3];   // per slab: the sorts of out-of-band elements it holds (Kind), filled where a loop below asks
     __shared__ unsigned lines[3];   // per slab: bit k = k line holds an out-of-band element, bit 16 + k = one above the band
     __shared__ unsigned overflow_lines;   // bit k = some product of k line may leave the pass range
 
@@ -301,7 +321,7 @@ gemm_kernel(const GemmParams p) {
         }
     }
 
-    if (MODE == kPam && tid < 3) lines[tid] = 0;
+    if (MODE == kPam && tid < 3) lines[tid] = kinds[tid] = 0;
 
     float ra[T::kTasksA * 4], rb[T::kTasksB * 4];
     SlabWalker<T, BM, T::kTasksA, A_KC> walk_a;
@@ -352,8 +372,8 @@ gemm_kernel(const GemmParams p) {
         unsigned dirty = 0;
         if (MODE == kPam) {
             dirty = lines[s % 3];
-            // the word two slabs ahead was last read before the previous barrier: reset it now
-            if (tid == 0) lines[(s + 2) % 3] = 0;
+            // the words two slabs ahead were last read before the previous barrier: reset them now
+            if (tid == 0) lines[(s + 2) % 3] = kinds[(s + 2) % 3] = 0;
         }
         const float* as = As[buf];
         const float* bs = Bs[buf];
@@ -366,6 +386,11 @@ gemm_kernel(const GemmParams p) {
         const int a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};                              \
         const int b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
 
+#define PAMK_WEIGHTS(kk, at)                                                                            \
+        const float4 w0 = *reinterpret_cast<const float4*>(weights + (kk) * row_stride(BM) + (at) * 4); \
+        const float4 w1 = MT == 8 ? *reinterpret_cast<const float4*>(weights + (kk) * row_stride(BM) + (at) * 4 + BM / 2) : w0; \
+        const float w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+
         if (MODE == kPam && dirty == 0) {
 #pragma unroll kFastUnroll
             for (int kk = 0; kk < BK; ++kk) {
@@ -376,57 +401,121 @@ gemm_kernel(const GemmParams p) {
                     for (int j = 0; j < MT; ++j) acc[i][j] = fadd(acc[i][j], i2f(iadd(a[i], b[j])));
             }
         } else if constexpr (MODE == kPam) {
-            // lines that hold an element above the band: can a product leave the pass range?
-            unsigned full = 0;
-            if (dirty >> 16) {                                  // (uniform: read from shared memory after a barrier)
-                constexpr int kLanes = T::kThreads / BK;        // threads that share one k line
-                const int line = tid / kLanes, lane = tid % kLanes;
-                if (tid == 0) overflow_lines = 0;
-                __syncthreads();
-                // (every thread takes part, whatever its line: the shuffles below name all 32 lanes)
-                uint32_t hi_a = 0, hi_b = 0;                    // magnitudes compare like their bit patterns; inf / NaN are largest
-                for (int q = lane; q < BM; q += kLanes) {
-                    hi_a = max(hi_a, (uint32_t)iadd(f2i(as[line * row_stride(BM) + q]), p.bias_sub) & 0x7fffffffu);
-                    hi_b = max(hi_b, (uint32_t)f2i(bs[line * row_stride(BN) + q]) & 0x7fffffffu);
-                }
+            constexpr unsigned all_lines = (1u << BK) - 1u;
+            // Is everything out of the band a zero?  Looked up here and not while staging, where the registers
+            // for it spilled and every dirty slab slowed down by 3 to 7 %.  A slab with elements above the band need
+            // not be asked, one with few dirty lines is better off in the runs below (0.1 % zeros: 261 us with
+            // them, 283 us when asked).  The zero-filled lines past the end of K count on both sides.
+            unsigned kind = kOther;
+            if (dirty >> 16 == 0 && __popc(dirty) * 4 >= BK * 3) {
+                unsigned seen = 0;
 #pragma unroll
-                for (int d = 1; d < kLanes; d <<= 1) {
-                    hi_a = max(hi_a, __shfl_xor_sync(0xffffffffu, hi_a, d));
-                    hi_b = max(hi_b, __shfl_xor_sync(0xffffffffu, hi_b, d));
+                for (int t = 0; t < T::kTasksA; ++t) {
+                    const int id = tid + t * T::kThreads;
+                    const int at = id / (BM / 4) * row_stride(BM) + id % (BM / 4) * 4;
+                    seen |= kinds_of(*reinterpret_cast<const int4*>(as + at), p.bias_sub, kZerosA);
+                    seen |= kinds_of(*reinterpret_cast<const int4*>(bs + at), 0, kZerosB);
                 }
-                // (an inf or NaN maximum makes the product inf or NaN: not <= the pass bound)
-                if (lane == 0 && !(fmul(i2f((int32_t)hi_a), i2f((int32_t)hi_b)) <= i2f(kPassBits))) atomicOr(&overflow_lines, 1u << line);
+                seen = __reduce_or_sync(0xffffffffu, seen);
+                if ((tid & 31) == 0) atomicOr(&kinds[s % 3], seen);
                 __syncthreads();
-                full = overflow_lines;
+                kind = kinds[s % 3];
             }
-            const unsigned all_lines = (1u << BK) - 1u;
-            if (__popc(dirty & all_lines) * 4 >= BK * 3 && full == 0) {
-                // most lines dirty, none can overflow (e.g. an operand that is half zeros): "flush or add"
-                // for the whole slab in one unrolled loop (it is exact for clean lines too)
-#pragma unroll 2
-                for (int kk = 0; kk < BK; ++kk) {
-                    PAMK_FRAGMENTS(kk)
-                    float araw[MT];          // a[] holds pre-biased patterns; the rule needs the values
+            if (kind < kOther) {                                // (not 0: the slab is dirty)
+                // Zeros, and everything else in the band (an operand that went through a ReLU).  A pass over one
+                // side's slab replaces each zero by a value that makes the product in-band and writes a weight beside
+                // it, 0 for a zero and 1 for anything else; the sum then is acc = fma(product, weight, acc), which
+                // is the plain sum for weight 1 and leaves acc alone for weight 0 (the products are finite, and a
+                // sum is never -0).  Two instructions per product, no compare and no predicate, against the four of
+                // "flush or add": 4096x1024x512 with one operand half zeros 387 -> 252 us (clean: 188),
+                // 1024x512x4096 359 -> 237 us, both operands half zeros 387 -> 346 us.  (Unrolling these loops by
+                // two spilled up to 160 bytes in the 128x128 kernels and cost clean slabs 7 %; predicated adds
+                // without weights took 249 and 294 us, and 376 us instead of 288 where an SM holds eight warps.)
+                const bool side_b = kind == kZerosB;
+                float* side = side_b ? Bs[buf] : As[buf];
+                // (the stand-in makes the product the other operand's own pattern, whatever the offset)
+                const int zero_bits = side_b ? 0 : -p.bias_sub, stand_in = side_b ? p.bias_sub : 0;
+                static_assert(BM == BN, "one loop serves both sides");
 #pragma unroll
-                    for (int i = 0; i < MT; ++i) araw[i] = i2f(iadd(a[i], p.bias_sub));
-#pragma unroll
-                    for (int i = 0; i < MT; ++i)
+                for (int t = 0; t < T::kTasksA; ++t) {
+                    const int id = tid + t * T::kThreads;
+                    const int at = id / (BM / 4) * row_stride(BM) + id % (BM / 4) * 4;
+                    int4 v = *reinterpret_cast<const int4*>(side + at);
+                    float4 w;
+                    w.x = 2u * (uint32_t)isub(v.x, zero_bits) == 0 ? 0.0f : 1.0f; v.x = 2u * (uint32_t)isub(v.x, zero_bits) == 0 ? stand_in : v.x;
+                    w.y = 2u * (uint32_t)isub(v.y, zero_bits) == 0 ? 0.0f : 1.0f; v.y = 2u * (uint32_t)isub(v.y, zero_bits) == 0 ? stand_in : v.y;
+                    w.z = 2u * (uint32_t)isub(v.z, zero_bits) == 0 ? 0.0f : 1.0f; v.z = 2u * (uint32_t)isub(v.z, zero_bits) == 0 ? stand_in : v.z;
+                    w.w = 2u * (uint32_t)isub(v.w, zero_bits) == 0 ? 0.0f : 1.0f; v.w = 2u * (uint32_t)isub(v.w, zero_bits) == 0 ? stand_in : v.w;
+                    *reinterpret_cast<int4*>(side + at) = v;
+                    *reinterpret_cast<float4*>(weights + at) = w;
+                }
+                __syncthreads();
+                if (kind == (kZerosA | kZerosB)) {
+                    // (weights for A's zeros, a predicate for B's)
+#pragma unroll 1
+                    for (int kk = 0; kk < BK; ++kk) {
+                        PAMK_FRAGMENTS(kk)
+                        PAMK_WEIGHTS(kk, ty)
 #pragma unroll
                         for (int j = 0; j < MT; ++j) {
-                            const float mag = fabsf(fmul(araw[i], i2f(b[j])));
-                            if (mag > i2f(kFlushBits)) acc[i][j] = fadd(acc[i][j], i2f(iadd(a[i], b[j])));
+                            const bool on = 2u * (uint32_t)b[j] != 0;
+#pragma unroll
+                            for (int i = 0; i < MT; ++i)
+                                if (on) acc[i][j] = __fmaf_rn(i2f(iadd(a[i], b[j])), w[i], acc[i][j]);
                         }
+                    }
+                } else if (!side_b) {
+#pragma unroll 1
+                    for (int kk = 0; kk < BK; ++kk) {
+                        PAMK_FRAGMENTS(kk)
+                        PAMK_WEIGHTS(kk, ty)
+#pragma unroll
+                        for (int i = 0; i < MT; ++i)
+#pragma unroll
+                            for (int j = 0; j < MT; ++j) acc[i][j] = __fmaf_rn(i2f(iadd(a[i], b[j])), w[i], acc[i][j]);
+                    }
+                } else {
+#pragma unroll 1
+                    for (int kk = 0; kk < BK; ++kk) {
+                        PAMK_FRAGMENTS(kk)
+                        PAMK_WEIGHTS(kk, tx)
+#pragma unroll
+                        for (int i = 0; i < MT; ++i)
+#pragma unroll
+                            for (int j = 0; j < MT; ++j) acc[i][j] = __fmaf_rn(i2f(iadd(a[i], b[j])), w[j], acc[i][j]);
+                    }
                 }
             } else {
-                // The lines are walked in runs of one kind, each run by a loop of its own with one copy of
-                // its body (with the three bodies side by side in one loop the schedule cost 12 %).
-                const unsigned flush = dirty & ~full & all_lines;
-                int kk = 0;
-                while (kk < BK) {
-                    const unsigned here = 1u << kk;
-                    if (full & here) {
+                // lines that hold an element above the band: can a product leave the pass range?
+                unsigned full = 0;
+                if (dirty >> 16) {                                  // (uniform: read from shared memory after a barrier)
+                    constexpr int kLanes = T::kThreads / BK;        // threads that share one k line
+                    const int line = tid / kLanes, lane = tid % kLanes;
+                    if (tid == 0) overflow_lines = 0;
+                    __syncthreads();
+                    // (every thread takes part, whatever its line: the shuffles below name all 32 lanes)
+                    uint32_t hi_a = 0, hi_b = 0;                    // magnitudes compare like their bit patterns; inf / NaN are largest
+                    for (int q = lane; q < BM; q += kLanes) {
+                        hi_a = max(hi_a, (uint32_t)iadd(f2i(as[line * row_stride(BM) + q]), p.bias_sub) & 0x7fffffffu);
+                        hi_b = max(hi_b, (uint32_t)f2i(bs[line * row_stride(BN) + q]) & 0x7fffffffu);
+                    }
+#pragma unroll
+                    for (int d = 1; d < kLanes; d <<= 1) {
+                        hi_a = max(hi_a, __shfl_xor_sync(0xffffffffu, hi_a, d));
+                        hi_b = max(hi_b, __shfl_xor_sync(0xffffffffu, hi_b, d));
+                    }
+                    // (an inf or NaN maximum makes the product inf or NaN: not <= the pass bound)
+                    if (lane == 0 && !(fmul(i2f((int32_t)hi_a), i2f((int32_t)hi_b)) <= i2f(kPassBits))) atomicOr(&overflow_lines, 1u << line);
+                    __syncthreads();
+                    full = overflow_lines;
+                }
+                if (__popc(dirty & all_lines) * 4 >= BK * 3 && full == 0) {
+                    // most lines dirty, none can overflow (e.g. an operand that is half zeros): "flush or add"
+                    // for the whole slab in one unrolled loop (it is exact for clean lines too)
+#pragma unroll 2
+                    for (int kk = 0; kk < BK; ++kk) {
                         PAMK_FRAGMENTS(kk)
-                        float araw[MT];
+                        float araw[MT];          // a[] holds pre-biased patterns; the rule needs the values
 #pragma unroll
                         for (int i = 0; i < MT; ++i) araw[i] = i2f(iadd(a[i], p.bias_sub));
 #pragma unroll
@@ -434,15 +523,17 @@ gemm_kernel(const GemmParams p) {
 #pragma unroll
                             for (int j = 0; j < MT; ++j) {
                                 const float mag = fabsf(fmul(araw[i], i2f(b[j])));
-                                const float prod = mag <= i2f(kPassBits) ? i2f(iadd(a[i], b[j])) : quiet_nan();
-                                if (!(mag <= i2f(kFlushBits))) acc[i][j] = fadd(acc[i][j], prod);
+                                if (mag > i2f(kFlushBits)) acc[i][j] = fadd(acc[i][j], i2f(iadd(a[i], b[j])));
                             }
-                        ++kk;
-                    } else if (flush & here) {
-                        const unsigned others = ~flush >> kk;
-                        const int end = min(BK, kk + __ffs((int)others) - 1);
-#pragma unroll 1
-                        for (; kk < end; ++kk) {
+                    }
+                } else {
+                    // The lines are walked in runs of one kind, each run by a loop of its own with one copy of
+                    // its body (with the three bodies side by side in one loop the schedule cost 12 %).
+                    const unsigned flush = dirty & ~full & all_lines;
+                    int kk = 0;
+                    while (kk < BK) {
+                        const unsigned here = 1u << kk;
+                        if (full & here) {
                             PAMK_FRAGMENTS(kk)
                             float araw[MT];
 #pragma unroll
@@ -452,19 +543,38 @@ gemm_kernel(const GemmParams p) {
 #pragma unroll
                                 for (int j = 0; j < MT; ++j) {
                                     const float mag = fabsf(fmul(araw[i], i2f(b[j])));
-                                    if (mag > i2f(kFlushBits)) acc[i][j] = fadd(acc[i][j], i2f(iadd(a[i], b[j])));
+                                    const float prod = mag <= i2f(kPassBits) ? i2f(iadd(a[i], b[j])) : quiet_nan();
+                                    if (!(mag <= i2f(kFlushBits))) acc[i][j] = fadd(acc[i][j], prod);
                                 }
-                        }
-                    } else {
-                        const unsigned others = (dirty & all_lines) >> kk;
-                        const int end = others ? kk + __ffs((int)others) - 1 : BK;
+                            ++kk;
+                        } else if (flush & here) {
+                            const unsigned others = ~flush >> kk;
+                            const int end = min(BK, kk + __ffs((int)others) - 1);
 #pragma unroll 1
-                        for (; kk < end; ++kk) {
-                            PAMK_FRAGMENTS(kk)
+                            for (; kk < end; ++kk) {
+                                PAMK_FRAGMENTS(kk)
+                                float araw[MT];
 #pragma unroll
-                            for (int i = 0; i < MT; ++i)
+                                for (int i = 0; i < MT; ++i) araw[i] = i2f(iadd(a[i], p.bias_sub));
 #pragma unroll
-                                for (int j = 0; j < MT; ++j) acc[i][j] = fadd(acc[i][j], i2f(iadd(a[i], b[j])));
+                                for (int i = 0; i < MT; ++i)
+#pragma unroll
+                                    for (int j = 0; j < MT; ++j) {
+                                        const float mag = fabsf(fmul(araw[i], i2f(b[j])));
+                                        if (mag > i2f(kFlushBits)) acc[i][j] = fadd(acc[i][j], i2f(iadd(a[i], b[j])));
+                                    }
+                            }
+                        } else {
+                            const unsigned others = (dirty & all_lines) >> kk;
+                            const int end = others ? kk + __ffs((int)others) - 1 : BK;
+#pragma unroll 1
+                            for (; kk < end; ++kk) {
+                                PAMK_FRAGMENTS(kk)
+#pragma unroll
+                                for (int i = 0; i < MT; ++i)
+#pragma unroll
+                                    for (int j = 0; j < MT; ++j) acc[i][j] = fadd(acc[i][j], i2f(iadd(a[i], b[j])));
+                            }
                         }
                     }
                 }
@@ -492,6 +602,7 @@ gemm_kernel(const GemmParams p) {
             }
         }
 #undef PAMK_FRAGMENTS
+#undef PAMK_WEIGHTS
 
         if (more) stage_store(buf ^ 1, (s + 1) % 3);
         __syncthreads();
