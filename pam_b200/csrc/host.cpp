@@ -23,6 +23,7 @@
 #include <ATen/ATen.h>
 #include <ATen/ExpandUtils.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
@@ -773,6 +774,13 @@ PyObject* none() { Py_RETURN_NONE; }
 
 PyObject* wrap(std::optional<Tensor>&& t) { return t ? THPVariable_Wrap(std::move(*t)) : none(); }
 
+// Whether nothing watches the operators that run.  A trace would keep an answer of this path as a constant, so
+// the Python layer's autograd functions, which it records, take the call.
+bool unwatched() {
+    constexpr c10::DispatchKeySet watching({c10::DispatchKey::Tracer});
+    return !c10::impl::tls_local_dispatch_key_set().included_.has_any(watching);
+}
+
 template <class F>
 PyObject* guarded(F&& body) {
     try {
@@ -785,6 +793,12 @@ PyObject* guarded(F&& body) {
     return nullptr;
 }
 
+// An operator's entry: `body`, or None where the call is for the Python layer.
+template <class F>
+PyObject* operator_call(F&& body) {
+    return unwatched() ? guarded(std::forward<F>(body)) : none();
+}
+
 #define PAMK_ARGS(count)                                                                            \
     if (nargs != (count)) {                                                                         \
         PyErr_SetString(PyExc_TypeError, "wrong number of arguments");                              \
@@ -794,7 +808,7 @@ PyObject* guarded(F&& body) {
 // linear(x, weight, bias | None, offset, approx_bwd)
 PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     PAMK_ARGS(5)
-    return guarded([&]() -> PyObject* {
+    return operator_call([&]() -> PyObject* {
         Tensor x, w, b;
         double off;
         bool p, q;
@@ -806,7 +820,7 @@ PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
 // matmul(a, b, offset, approx_bwd, dims)
 PyObject* py_matmul(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     PAMK_ARGS(5)
-    return guarded([&]() -> PyObject* {
+    return operator_call([&]() -> PyObject* {
         Tensor x, y;
         double off;
         bool p, q;
@@ -819,7 +833,7 @@ PyObject* py_matmul(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
 template <Ew OP>
 PyObject* py_elementwise(PyObject*, PyObject* const* a, Py_ssize_t nargs) {   // (a, b, offset, approx_bwd)
     PAMK_ARGS(4)
-    return guarded([&]() -> PyObject* {
+    return operator_call([&]() -> PyObject* {
         Tensor x, y;
         double nx = 0.0, ny = 0.0, off;
         bool p, q;
@@ -833,7 +847,7 @@ PyObject* py_elementwise(PyObject*, PyObject* const* a, Py_ssize_t nargs) {   //
 // layer_norm(x, width, weight | None, bias | None, eps, offset, approx_bwd)
 PyObject* py_layer_norm(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     PAMK_ARGS(7)
-    return guarded([&]() -> PyObject* {
+    return operator_call([&]() -> PyObject* {
         Tensor x, w, b;
         int64_t width;
         double eps, off;
@@ -848,7 +862,7 @@ PyObject* py_layer_norm(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
 // softmax(x, offset, approx_bwd) over the last dimension
 PyObject* py_softmax(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     PAMK_ARGS(3)
-    return guarded([&]() -> PyObject* {
+    return operator_call([&]() -> PyObject* {
         Tensor x;
         double off;
         bool p, q;
@@ -860,7 +874,7 @@ PyObject* py_softmax(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
 // attention_qkv(qkv, heads, scale, offset)
 PyObject* py_attention_qkv(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     PAMK_ARGS(4)
-    return guarded([&]() -> PyObject* {
+    return operator_call([&]() -> PyObject* {
         Tensor x;
         int64_t heads;
         double scale, off;
@@ -872,7 +886,7 @@ PyObject* py_attention_qkv(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
 // attention_heads(q, k, v, mask | None, heads, offset)
 PyObject* py_attention_heads(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     PAMK_ARGS(6)
-    return guarded([&]() -> PyObject* {
+    return operator_call([&]() -> PyObject* {
         Tensor q, k, v, m;
         int64_t heads;
         double off;

@@ -1,0 +1,48 @@
+"""What torch.autograd.Function promises and the native host path has to keep: tracing records the operator, forward-mode
+AD and functorch transforms are refused, exceptions keep their type, missing gradients count as zeros, a compiled
+backward pass runs.  Each test failed on a host path that went past one of these."""
+import pytest
+import torch
+
+import pam_b200 as pam
+from conftest import assert_bits_equal
+from pam_b200 import fused
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def randn(*shape, seed=1):
+    return torch.randn(*shape, generator=torch.Generator(DEV).manual_seed(seed), device=DEV)
+
+
+# every operator of the host path as a function of one [2, 4, 12] tensor
+W = GAIN = None
+OPERATORS = {
+    "mul": lambda t: pam.mul(t, GAIN, approx_bwd=True),
+    "mul_number": lambda t: pam.mul(2.5, t, approx_bwd=True),
+    "div": lambda t: pam.div(t, 3.0, approx_bwd=True),
+    "linear": lambda t: pam.linear(t, W, GAIN[:6].contiguous(), approx_bwd=True),
+    "matmul": lambda t: pam.matmul(t[0], W.T, approx_bwd=True),
+    "bmm": lambda t: pam.bmm(t, t.mT, approx_bwd=True),
+    "layer_norm": lambda t: pam.layer_norm(t, (12,), GAIN, GAIN, approx_bwd=True),
+    "softmax": lambda t: pam.softmax(t, dim=-1, approx_bwd=True),
+    "attention_qkv": lambda t: fused.attention_qkv(t, 2, 0.5),
+    "attention_heads": lambda t: fused.attention_heads(t, t, t, 2),
+}
+each_operator = pytest.mark.parametrize("name", OPERATORS)
+
+
+@pytest.fixture(autouse=True, scope="module")
+def constants():
+    global W, GAIN
+    W, GAIN = randn(6, 12, seed=2), randn(12, seed=3)
+
+
+@each_operator
+def test_a_trace_holds_the_operator_and_not_its_result(name):
+    op = OPERATORS[name]
+    with torch.no_grad():
+        traced = torch.jit.trace(lambda t: op(t) + 1, randn(2, 4, 12), check_trace=False)
+        x = randn(2, 4, 12, seed=9)
+        assert_bits_equal(traced(x), op(x) + 1, name)
