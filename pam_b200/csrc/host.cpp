@@ -94,8 +94,11 @@ Tensor scratch_bytes(size_t bytes, const Tensor& like) {
 
 float* ptr(const Tensor& t) { return t.defined() ? static_cast<float*>(t.data_ptr()) : nullptr; }
 
-// fp32 CUDA data that the kernels may read in place
-bool usable(const Tensor& t) { return t.defined() && t.is_cuda() && t.scalar_type() == at::kFloat && !t.is_sparse(); }
+// fp32 CUDA data that the kernels may read in place.  A tensor with a tangent (forward-mode AD) is for the Python layer,
+// which refuses it: here the tangent would be lost without a word.
+bool usable(const Tensor& t) {
+    return t.defined() && t.is_cuda() && t.scalar_type() == at::kFloat && !t.is_sparse() && !t._fw_grad(0).defined();
+}
 
 bool wants_grad(const Tensor& t) { return t.defined() && t.requires_grad(); }
 

@@ -3,6 +3,7 @@ AD and functorch transforms are refused, exceptions keep their type, missing gra
 backward pass runs.  Each test failed on a host path that went past one of these."""
 import pytest
 import torch
+import torch.autograd.forward_ad as fwAD
 
 import pam_b200 as pam
 from conftest import assert_bits_equal
@@ -46,3 +47,15 @@ def test_a_trace_holds_the_operator_and_not_its_result(name):
         traced = torch.jit.trace(lambda t: op(t) + 1, randn(2, 4, 12), check_trace=False)
         x = randn(2, 4, 12, seed=9)
         assert_bits_equal(traced(x), op(x) + 1, name)
+
+
+@each_operator
+def test_forward_mode_is_refused(name):
+    with fwAD.dual_level():
+        dual = fwAD.make_dual(randn(2, 4, 12), randn(2, 4, 12, seed=4))
+        with pytest.raises(NotImplementedError, match="jvp"):
+            OPERATORS[name](dual)
+    with torch.no_grad(), fwAD.dual_level():
+        dual = fwAD.make_dual(randn(2, 4, 12), randn(2, 4, 12, seed=4))
+        with pytest.raises(NotImplementedError, match="jvp"):
+            OPERATORS[name](dual)
