@@ -94,10 +94,15 @@ Tensor scratch_bytes(size_t bytes, const Tensor& like) {
 
 float* ptr(const Tensor& t) { return t.defined() ? static_cast<float*>(t.data_ptr()) : nullptr; }
 
-// fp32 CUDA data that the kernels may read in place.  A tensor with a tangent (forward-mode AD) is for the Python layer,
+// fp32 CUDA data that the kernels may read in place: no wrapper of other tensors (functorch, fake, functional), no lazy
+// negation or zero.  A tensor with a tangent (forward-mode AD) is for the Python layer,
 // which refuses it: here the tangent would be lost without a word.
 bool usable(const Tensor& t) {
-    return t.defined() && t.is_cuda() && t.scalar_type() == at::kFloat && !t.is_sparse() && !t._fw_grad(0).defined();
+    using K = c10::DispatchKey;
+    constexpr c10::DispatchKeySet special({K::Python, K::PythonTLSSnapshot, K::FuncTorchBatched, K::FuncTorchGradWrapper, K::Batched,
+                                           K::Functionalize, K::Conjugate, K::Negative, K::ZeroTensor});
+    return t.defined() && t.is_cuda() && t.scalar_type() == at::kFloat && t.layout() == at::kStrided && !t.key_set().has_any(special) &&
+           !t._fw_grad(0).defined();
 }
 
 bool wants_grad(const Tensor& t) { return t.defined() && t.requires_grad(); }
@@ -729,10 +734,11 @@ std::optional<Tensor> op_attention_heads(const Tensor& gq, const Tensor& gk, con
 
 // ---- Python entry points -----------------------------------------------------------------------------------------
 
-// Reads a tensor argument: undefined for None, false for anything that is neither.
+// Reads a tensor argument: undefined for None, false for anything that is neither (a subclass other than
+// Parameter included: it may override operators that the Python layer calls).
 bool as_tensor(PyObject* o, Tensor& t) {
     if (o == Py_None) return true;
-    if (!THPVariable_Check(o)) return false;
+    if (!THPVariable_CheckExact(o)) return false;
     t = THPVariable_Unpack(o);
     return true;
 }
@@ -777,10 +783,13 @@ PyObject* none() { Py_RETURN_NONE; }
 
 PyObject* wrap(std::optional<Tensor>&& t) { return t ? THPVariable_Wrap(std::move(*t)) : none(); }
 
-// Whether nothing watches the operators that run.  A trace would keep an answer of this path as a constant, so
-// the Python layer's autograd functions, which it records, take the call.
+// Whether nothing watches or transforms the operators that run.  A trace would keep an answer of this path as a constant,
+// a dispatch mode would not see its allocations, and functorch's transforms refuse autograd functions like
+// these whether or not an operand is wrapped: the Python layer's functions take such a call.
 bool unwatched() {
-    constexpr c10::DispatchKeySet watching({c10::DispatchKey::Tracer});
+    using K = c10::DispatchKey;
+    constexpr c10::DispatchKeySet watching({K::Tracer, K::Python, K::PythonTLSSnapshot, K::FuncTorchDynamicLayerFrontMode,
+                                            K::Functionalize});
     return !c10::impl::tls_local_dispatch_key_set().included_.has_any(watching);
 }
 

@@ -59,3 +59,33 @@ def test_forward_mode_is_refused(name):
         dual = fwAD.make_dual(randn(2, 4, 12), randn(2, 4, 12, seed=4))
         with pytest.raises(NotImplementedError, match="jvp"):
             OPERATORS[name](dual)
+
+
+@each_operator
+def test_functorch_transforms_are_refused(name):
+    x, op = randn(2, 4, 12), OPERATORS[name]
+    for call in (lambda: torch.func.grad(lambda t: op(t).sum())(x), lambda: torch.func.vmap(op)(x[None]),
+                 lambda: torch.func.vmap(lambda s: op(x) * s)(torch.ones(2, device=DEV))):     # (x is no wrapper here)
+        with pytest.raises(RuntimeError, match="setup_context"):
+            call()
+
+
+def test_dispatch_modes_and_subclasses_take_the_python_layer():
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Count(TorchDispatchMode):
+        seen = 0
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            Count.seen += 1
+            return func(*args, **(kwargs or {}))
+
+    class Sub(torch.Tensor):
+        pass
+
+    x = randn(5)
+    with Count():
+        y = pam.mul(x, 2.0)
+    assert Count.seen > 0
+    assert_bits_equal(y, pam.mul(x, 2.0))
+    assert_bits_equal(pam.mul(x.as_subclass(Sub), 2.0), y)
