@@ -14,6 +14,7 @@
 //
 // Scratch is allocated per call: the caching allocator orders its reuse on the stream, keeps calls
 // from several threads and streams apart, and takes it back.
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -34,7 +35,6 @@
 #include <map>
 #include <mutex>
 #include <optional>
-#include <stdexcept>
 #include <string>
 #include <vector>
 
@@ -71,8 +71,10 @@ Library lib;
 PyObject* g_kernel_error = nullptr;      // the Python layer's PamKernelError
 std::atomic<bool> g_strict{false};       // set_strict_k_order
 
-struct KernelError : std::runtime_error {
-    using std::runtime_error::runtime_error;
+// (a PyTorchError is what torch's own handlers, the autograd engine's included, turn into an exception of its Python type)
+struct KernelError : torch::PyTorchError {
+    using torch::PyTorchError::PyTorchError;
+    PyObject* python_type() override { return g_kernel_error ? g_kernel_error : PyExc_RuntimeError; }
 };
 
 void check(int status, const char* what) {
@@ -793,16 +795,13 @@ bool unwatched() {
     return !c10::impl::tls_local_dispatch_key_set().included_.has_any(watching);
 }
 
+// Torch's translation of exceptions: one raised by Python code further down (a saved-tensor hook) goes on as it
+// is, an allocation that fails is an OutOfMemoryError.
 template <class F>
 PyObject* guarded(F&& body) {
-    try {
-        return body();
-    } catch (const KernelError& e) {
-        PyErr_SetString(g_kernel_error ? g_kernel_error : PyExc_RuntimeError, e.what());
-    } catch (const std::exception& e) {
-        PyErr_SetString(PyExc_RuntimeError, e.what());
-    }
-    return nullptr;
+    HANDLE_TH_ERRORS
+    return body();
+    END_HANDLE_TH_ERRORS
 }
 
 // An operator's entry: `body`, or None where the call is for the Python layer.

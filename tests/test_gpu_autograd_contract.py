@@ -4,10 +4,11 @@ backward pass runs.  Each test failed on a host path that went past one of these
 import pytest
 import torch
 import torch.autograd.forward_ad as fwAD
+from torch.utils.checkpoint import checkpoint
 
 import pam_b200 as pam
 from conftest import assert_bits_equal
-from pam_b200 import fused
+from pam_b200 import _lib, fused
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -89,3 +90,42 @@ def test_dispatch_modes_and_subclasses_take_the_python_layer():
     assert Count.seen > 0
     assert_bits_equal(y, pam.mul(x, 2.0))
     assert_bits_equal(pam.mul(x.as_subclass(Sub), 2.0), y)
+
+
+@each_operator
+def test_checkpointed_block_ending_in_an_operator(name):
+    op = OPERATORS[name]
+    grads = []
+    for run in (lambda t: op(torch.tanh(t)), lambda t: checkpoint(lambda u: op(torch.tanh(u)), t, use_reentrant=False)):
+        x = randn(2, 4, 12).requires_grad_()
+        y = run(x)
+        grads.append(torch.autograd.grad(y, x, randn(*y.shape, seed=5))[0])
+    assert_bits_equal(*grads)
+
+
+class _Mine(Exception):
+    pass
+
+
+def _raise(message):
+    raise _Mine(message)
+
+
+def test_exceptions_keep_their_type():
+    x = randn(3).requires_grad_()
+    with pytest.raises(_Mine, match="pack"):
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: _raise("pack"), lambda t: t):
+            pam.mul(x, 2.0)
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: _raise("unpack")):
+        y = pam.mul(x, 2.0)
+    with pytest.raises(_Mine, match="unpack"):
+        y.sum().backward()
+    with pytest.raises(torch.cuda.OutOfMemoryError):                      # (4 TiB of output: refused by the allocator)
+        pam.mul(torch.ones(1, device=DEV).expand(1 << 40), 2.0)
+    # a product of more row tiles than a grid holds is refused by the kernel library: here only the gradient's is one
+    a, b = torch.ones(1, 65535 * 128 + 1, device=DEV), torch.ones(65535 * 128 + 1, 1, device=DEV, requires_grad=True)
+    with pytest.raises(_lib.PamKernelError):
+        pam.matmul(b.detach(), a[:, :1].contiguous(), approx_bwd=True)
+    y = pam.matmul(a, b, approx_bwd=True)
+    with pytest.raises(_lib.PamKernelError):
+        y.sum().backward()
