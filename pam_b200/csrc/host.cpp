@@ -300,10 +300,11 @@ struct PamNode : Node {
     virtual variable_list grads(const Tensor& g) = 0;
     variable_list apply(variable_list&& in) override {
         std::lock_guard<std::mutex> lock(mutex_);
-        if (!in[0].defined()) return variable_list(num_outputs());
         at::AutoGradMode no_grad(false);
-        c10::cuda::CUDAGuard guard(in[0].device());
-        Tensor g = in[0].scalar_type() == at::kFloat ? in[0] : in[0].to(at::kFloat);
+        // (a gradient that never came counts as zeros, as autograd.Function has it: the inputs get theirs)
+        Tensor g = in[0].defined() ? in[0] : input_metadata(0).zeros_like();
+        c10::cuda::CUDAGuard guard(g.device());
+        if (g.scalar_type() != at::kFloat) g = g.to(at::kFloat);
         return grads(g);
     }
 };

@@ -129,3 +129,20 @@ def test_exceptions_keep_their_type():
     y = pam.matmul(a, b, approx_bwd=True)
     with pytest.raises(_lib.PamKernelError):
         y.sum().backward()
+
+
+class _NoGradient(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, t):
+        return t.clone()
+
+    @staticmethod
+    def backward(ctx, g):
+        return None
+
+
+@each_operator
+def test_a_missing_gradient_counts_as_zeros(name):
+    x = randn(2, 4, 12).requires_grad_()
+    (grad,) = torch.autograd.grad(_NoGradient.apply(OPERATORS[name](x)).sum(), x)
+    assert grad.shape == x.shape and bool((grad == 0).all())
