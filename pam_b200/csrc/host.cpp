@@ -291,21 +291,23 @@ struct PamNode : Node {
     void keep(std::initializer_list<Tensor> ts) {
         for (const Tensor& t : ts) saved.emplace_back(t, false);
     }
-    Tensor get(size_t k) { return saved[k].unpack(); }
     void release_variables() override {
         std::lock_guard<std::mutex> lock(mutex_);
         for (auto& s : saved) s.reset_data();
     }
     bool needs(size_t k) const { return task_should_compute_output(k); }
-    virtual variable_list grads(const Tensor& g) = 0;
+    virtual variable_list grads(const variable_list& kept, const Tensor& g) = 0;
     variable_list apply(variable_list&& in) override {
         std::lock_guard<std::mutex> lock(mutex_);
+        variable_list kept;                   // (unpack hooks run in the grad mode of the backward pass)
+        kept.reserve(saved.size());
+        for (SavedVariable& s : saved) kept.push_back(s.unpack());
         at::AutoGradMode no_grad(false);
         // (a gradient that never came counts as zeros, as autograd.Function has it: the inputs get theirs)
         Tensor g = in[0].defined() ? in[0] : input_metadata(0).zeros_like();
         c10::cuda::CUDAGuard guard(g.device());
         if (g.scalar_type() != at::kFloat) g = g.to(at::kFloat);
-        return grads(g);
+        return grads(kept, g);
     }
 };
 
@@ -324,11 +326,11 @@ struct EwNode : PamNode {
     bool approx_a, approx_b, has_a, has_b;
     double num_a = 0.0, num_b = 0.0;
     std::string name() const override { return op == Ew::kMul ? "PamMulBackward" : "PamDivBackward"; }
-    variable_list grads(const Tensor& g) override {
+    variable_list grads(const variable_list& kept, const Tensor& g) override {
         Tensor a, b;
         size_t k = 0;
-        if (has_a) a = get(k++);
-        if (has_b) b = get(k++);
+        if (has_a) a = kept[k++];
+        if (has_b) b = kept[k++];
         variable_list out(2);
         const bool na = has_a && needs(0), nb = has_b && needs(1);
         if (!na && !nb) return out;
@@ -353,8 +355,8 @@ struct LinearNode : PamNode {
     double offset;
     bool approx_x, approx_w, has_bias;
     std::string name() const override { return "PamLinearBackward"; }
-    variable_list grads(const Tensor& grad) override {
-        Tensor x = get(0), w = get(1);
+    variable_list grads(const variable_list& kept, const Tensor& grad) override {
+        Tensor x = kept[0], w = kept[1];
         const int64_t in = w.size(1), out_f = w.size(0), rows = x.numel() / in;
         Tensor g2 = grad.reshape({rows, out_f}), x2 = x.reshape({rows, in});
         const Mat g = matrix(g2), mx = matrix(x2), mw = matrix(w);
@@ -374,8 +376,8 @@ struct MatMulNode : PamNode {
     double offset;
     bool approx_a, approx_b;
     std::string name() const override { return "PamMatMulBackward"; }
-    variable_list grads(const Tensor& grad) override {
-        Tensor a = get(0), b = get(1), g2 = grad;
+    variable_list grads(const variable_list& kept, const Tensor& grad) override {
+        Tensor a = kept[0], b = kept[1], g2 = grad;
         const int64_t d = a.dim(), batch = d == 3 ? a.size(0) : 1, M = a.size(d - 2), K = a.size(d - 1), N = b.size(d - 1);
         const Mat ma = matrix(a), mb = matrix(b), g = matrix(g2);
         variable_list out(2);
@@ -396,11 +398,11 @@ struct LayerNormNode : PamNode {
     int64_t width;
     std::vector<int64_t> x_shape, w_shape, b_shape;
     std::string name() const override { return "PamLayerNormBackward"; }
-    variable_list grads(const Tensor& grad) override {
+    variable_list grads(const variable_list& kept, const Tensor& grad) override {
         size_t k = 0;
-        Tensor x = get(k++), w, stats;
-        if (has_w) w = get(k++);
-        if (approx) stats = get(k++);
+        Tensor x = kept[k++], w, stats;
+        if (has_w) w = kept[k++];
+        if (approx) stats = kept[k++];
         const Tensor g = grad.contiguous();
         const int64_t rows = x.numel() / width;
         Tensor dx = empty_on(x_shape, x);
@@ -448,14 +450,14 @@ struct SoftmaxNode : PamNode {
     double offset;
     bool approx;
     std::string name() const override { return "PamSoftmaxBackward"; }
-    variable_list grads(const Tensor& grad) override {
-        const Tensor kept = get(0), g = grad.contiguous();
-        const int64_t len = kept.size(-1), rows = kept.numel() / len;
-        if (approx) return {softmax_backward_saved(kept, g, rows, len, offset, std::nullopt, kept.sizes())};
-        Tensor dx = empty_on(kept.sizes(), kept);
+    variable_list grads(const variable_list& kept, const Tensor& grad) override {
+        const Tensor &from = kept[0], g = grad.contiguous();
+        const int64_t len = from.size(-1), rows = from.numel() / len;
+        if (approx) return {softmax_backward_saved(from, g, rows, len, offset, std::nullopt, from.sizes())};
+        Tensor dx = empty_on(from.sizes(), from);
         const size_t bytes = lib.pamk_softmax_workspace_bytes(rows, len);
-        Tensor ws = scratch_bytes(bytes, kept);
-        check(lib.pamk_softmax_bwd(ptr(kept), ptr(g), ptr(dx), rows, len, (float)offset, 0, ws.data_ptr(), bytes, stream_of(kept)),
+        Tensor ws = scratch_bytes(bytes, from);
+        check(lib.pamk_softmax_bwd(ptr(from), ptr(g), ptr(dx), rows, len, (float)offset, 0, ws.data_ptr(), bytes, stream_of(from)),
               "pamk_softmax_bwd");
         return {dx};
     }
@@ -467,8 +469,8 @@ struct AttentionQkvNode : PamNode {
     int64_t heads;
     double scale, offset;
     std::string name() const override { return "PamAttentionQkvBackward"; }
-    variable_list grads(const Tensor& grad) override {
-        const Tensor qkv = get(0), expo = get(1), probs = get(2), g = grad.contiguous();
+    variable_list grads(const variable_list& kept, const Tensor& grad) override {
+        const Tensor qkv = kept[0], expo = kept[1], probs = kept[2], g = grad.contiguous();
         const int64_t B = qkv.size(0), N = qkv.size(1), C3 = qkv.size(2), C = C3 / 3, hd = C / heads;
         const float *q = ptr(qkv), *k = q + C, *v = q + 2 * C;
         Tensor dqkv = empty_on(qkv.sizes(), qkv);
@@ -490,8 +492,8 @@ struct AttentionHeadsNode : PamNode {
     int64_t heads;
     double offset;
     std::string name() const override { return "PamAttentionHeadsBackward"; }
-    variable_list grads(const Tensor& grad) override {
-        const Tensor q = get(0), k = get(1), v = get(2), expo = get(3), probs = get(4), g = grad.contiguous();
+    variable_list grads(const variable_list& kept, const Tensor& grad) override {
+        const Tensor q = kept[0], k = kept[1], v = kept[2], expo = kept[3], probs = kept[4], g = grad.contiguous();
         const int64_t B = q.size(0), T = q.size(1), d = q.size(2), S = k.size(1), hd = d / heads;
         const int64_t H = heads * T * S, TS = T * S;
         variable_list out(3);

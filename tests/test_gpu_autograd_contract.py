@@ -131,6 +131,19 @@ def test_exceptions_keep_their_type():
         y.sum().backward()
 
 
+def test_unpack_hooks_run_in_the_grad_mode_of_the_backward_pass():
+    x, seen = randn(3).requires_grad_(), []
+
+    def unpack(t):
+        seen.append(torch.is_grad_enabled())
+        return t
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, unpack):
+        y = pam.mul(x, 2.0, approx_bwd=True)
+    torch.autograd.grad(y.sum(), x, retain_graph=True)
+    torch.autograd.grad(y.sum(), x, create_graph=True)
+    assert seen == [False, True]
+
+
 class _NoGradient(torch.autograd.Function):
     @staticmethod
     def forward(ctx, t):
