@@ -20,6 +20,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/autograd/variable.h>
+#include <torch/csrc/dynamo/compiled_autograd.h>
 
 #include <ATen/ATen.h>
 #include <ATen/ExpandUtils.h>
@@ -284,10 +285,39 @@ Tensor ew_forward(Ew op, const Operand& a, const Operand& b, int64_t inner, at::
 
 // ---- gradients ------------------------------------------------------------------------------------------------
 
+// Which of its inputs' gradients a backward pass asks a rule for.
+struct Wanted {
+    uint32_t bits = 0;
+    bool operator()(size_t k) const { return bits >> k & 1; }
+};
+
+// The backward pass of one operator: a rule holds the settings of the call, `kept` is what the forward pass kept.
+template <class Rule>
+variable_list backward_pass(const Rule& rule, const variable_list& kept, const Tensor& grad, const Wanted& wanted) {
+    at::AutoGradMode no_grad(false);
+    c10::cuda::CUDAGuard guard(grad.device());
+    return rule.grads(kept, grad.scalar_type() == at::kFloat ? grad : grad.to(at::kFloat), wanted);
+}
+
+// The bytes of a rule's settings, which tell one compiled backward pass from another.
+template <class... T>
+std::string bytes_of(const T&... v) {
+    std::string out;
+    (out.append(reinterpret_cast<const char*>(&v), sizeof v), ...);
+    return out;
+}
+
+std::string bytes_of_list(at::IntArrayRef v) { return bytes_of(v.size()).append(reinterpret_cast<const char*>(v.data()), v.size() * sizeof(int64_t)); }
+
 // A node keeps its saved tensors until the engine releases them; apply() runs on an engine thread, without
 // the interpreter, on the stream of the forward pass.
-struct PamNode : Node {
+template <class Rule>
+struct RuleNode : Node {
+    Rule rule;
     std::vector<SavedVariable> saved;
+
+    explicit RuleNode(Rule r) : rule(std::move(r)) {}
+    std::string name() const override { return rule.name(); }
     void keep(std::initializer_list<Tensor> ts) {
         for (const Tensor& t : ts) saved.emplace_back(t, false);
     }
@@ -295,44 +325,79 @@ struct PamNode : Node {
         std::lock_guard<std::mutex> lock(mutex_);
         for (auto& s : saved) s.reset_data();
     }
-    bool needs(size_t k) const { return task_should_compute_output(k); }
-    virtual variable_list grads(const variable_list& kept, const Tensor& g) = 0;
-    variable_list apply(variable_list&& in) override {
-        std::lock_guard<std::mutex> lock(mutex_);
-        variable_list kept;                   // (unpack hooks run in the grad mode of the backward pass)
+    variable_list unpacked() {
+        variable_list kept;
         kept.reserve(saved.size());
         for (SavedVariable& s : saved) kept.push_back(s.unpack());
-        at::AutoGradMode no_grad(false);
+        return kept;
+    }
+    variable_list apply(variable_list&& in) override {
+        std::lock_guard<std::mutex> lock(mutex_);
+        const variable_list kept = unpacked();            // (unpack hooks run in the grad mode of the backward pass)
+        Wanted wanted;
+        for (size_t k = 0; k < num_outputs(); ++k) wanted.bits |= (uint32_t)task_should_compute_output(k) << k;
         // (a gradient that never came counts as zeros, as autograd.Function has it: the inputs get theirs)
-        Tensor g = in[0].defined() ? in[0] : input_metadata(0).zeros_like();
-        c10::cuda::CUDAGuard guard(g.device());
-        if (g.scalar_type() != at::kFloat) g = g.to(at::kFloat);
-        return grads(kept, g);
+        return backward_pass(rule, kept, in[0].defined() ? in[0] : input_metadata(0).zeros_like(), wanted);
+    }
+
+    // Compiled autograd: the backward pass becomes one opaque call in the graph, bound to the rule's settings.
+    std::vector<int64_t> output_shape() const {
+        std::vector<int64_t> shape;
+        for (const c10::SymInt& n : input_metadata(0).shape_as_dim_vector()) shape.push_back(n.guard_int(__FILE__, __LINE__));
+        return shape;
+    }
+    Wanted reachable() const {
+        Wanted wanted;
+        for (size_t k = 0; k < num_outputs(); ++k) wanted.bits |= (uint32_t)should_compute_output(k) << k;
+        return wanted;
+    }
+    void compiled_args(torch::dynamo::autograd::CompiledNodeArgs& args) const override {
+        args.collect(rule.name() + rule.key() + bytes_of_list(output_shape()) + bytes_of(reachable().bits));
+        args.collect(saved, false);
+    }
+    variable_list apply_with_saved(const variable_list& inputs, torch::dynamo::autograd::SwapSavedVariables& swap) override {
+        namespace ca = torch::dynamo::autograd;
+        swap.before(saved);
+        ca::PackedArgs args;
+        args.pack(unpacked());
+        const auto call = [rule = rule, wanted = reachable(), shape = output_shape(), options = input_metadata(0).options()](
+                              const variable_list& in, const std::vector<c10::IValue>& packed) {
+            const variable_list kept = ca::PackedArgs(packed).template unpack<variable_list>();
+            return backward_pass(rule, kept, in[0].defined() ? in[0] : at::zeros(shape, options), wanted);
+        };
+        const auto& compiler = ca::getPyCompilerInterface();
+        const std::string fn = compiler->bind_function(swap.get_py_compiler(), rule.name(), call, {c10::ListType::ofTensors()},
+                                                       /*is_custom_function*/ true, /*is_traceable*/ false);
+        const auto metadata = ca::IValuePacker<std::vector<std::optional<ca::InputMetadata>>>::pack(ca::get_input_metadata(next_edges()));
+        variable_list out = compiler->call_function(swap.get_py_compiler(), "apply_functional", fn, inputs, args.vec(), metadata);
+        swap.after(saved);
+        return out;
     }
 };
 
-template <class N, class... Inputs>
-std::shared_ptr<N> node(const Inputs&... inputs) {
-    std::shared_ptr<N> fn(new N(), torch::autograd::deleteNode);
+template <class Rule, class... Inputs>
+std::shared_ptr<RuleNode<Rule>> node(Rule rule, const Inputs&... inputs) {
+    std::shared_ptr<RuleNode<Rule>> fn(new RuleNode<Rule>(std::move(rule)), torch::autograd::deleteNode);
     fn->set_next_edges(torch::autograd::collect_next_edges(inputs...));
     return fn;
 }
 
 bool recording() { return at::GradMode::is_enabled(); }
 
-struct EwNode : PamNode {
+struct EwRule {
     Ew op;
     double offset;
     bool approx_a, approx_b, has_a, has_b;
     double num_a = 0.0, num_b = 0.0;
-    std::string name() const override { return op == Ew::kMul ? "PamMulBackward" : "PamDivBackward"; }
-    variable_list grads(const variable_list& kept, const Tensor& g) override {
+    std::string name() const { return op == Ew::kMul ? "PamMulBackward" : "PamDivBackward"; }
+    std::string key() const { return bytes_of(op, offset, approx_a, approx_b, has_a, has_b, num_a, num_b); }
+    variable_list grads(const variable_list& kept, const Tensor& g, const Wanted& wanted) const {
         Tensor a, b;
         size_t k = 0;
         if (has_a) a = kept[k++];
         if (has_b) b = kept[k++];
         variable_list out(2);
-        const bool na = has_a && needs(0), nb = has_b && needs(1);
+        const bool na = has_a && wanted(0), nb = has_b && wanted(1);
         if (!na && !nb) return out;
         const auto shape = g.sizes();
         Operand oa = has_a ? describe(a, shape) : number(num_a), ob = has_b ? describe(b, shape) : number(num_b);
@@ -351,40 +416,42 @@ struct EwNode : PamNode {
 
 // X [.., in] x W [out, in] (+ bias).  The weight gradient is formed as [out, in] like the weight itself (g^T X:
 // the terms and the order over the tokens of X^T g), so nothing transposes it afterwards.
-struct LinearNode : PamNode {
+struct LinearRule {
     double offset;
     bool approx_x, approx_w, has_bias;
-    std::string name() const override { return "PamLinearBackward"; }
-    variable_list grads(const variable_list& kept, const Tensor& grad) override {
+    std::string name() const { return "PamLinearBackward"; }
+    std::string key() const { return bytes_of(offset, approx_x, approx_w, has_bias); }
+    variable_list grads(const variable_list& kept, const Tensor& grad, const Wanted& wanted) const {
         Tensor x = kept[0], w = kept[1];
         const int64_t in = w.size(1), out_f = w.size(0), rows = x.numel() / in;
         Tensor g2 = grad.reshape({rows, out_f}), x2 = x.reshape({rows, in});
         const Mat g = matrix(g2), mx = matrix(x2), mw = matrix(w);
         variable_list out(has_bias ? 3 : 2);
-        if (needs(0))
+        if (wanted(0))
             out[0] = approx_x ? product(g, mw, Tensor(), 1, rows, in, out_f, offset, x.sizes(), x)
                               : product_bwd(g, mw, mx, true, 1, rows, in, out_f, offset, x.sizes(), x);
-        if (needs(1))
+        if (wanted(1))
             out[1] = approx_w ? product(g.t(), mx, Tensor(), 1, out_f, in, rows, offset, w.sizes(), x)
                               : product_bwd(g.t(), mx, mw, true, 1, out_f, in, rows, offset, w.sizes(), x);
-        if (has_bias && needs(2)) out[2] = column_sum(g2.contiguous(), rows, out_f);
+        if (has_bias && wanted(2)) out[2] = column_sum(g2.contiguous(), rows, out_f);
         return out;
     }
 };
 
-struct MatMulNode : PamNode {
+struct MatMulRule {
     double offset;
     bool approx_a, approx_b;
-    std::string name() const override { return "PamMatMulBackward"; }
-    variable_list grads(const variable_list& kept, const Tensor& grad) override {
+    std::string name() const { return "PamMatMulBackward"; }
+    std::string key() const { return bytes_of(offset, approx_a, approx_b); }
+    variable_list grads(const variable_list& kept, const Tensor& grad, const Wanted& wanted) const {
         Tensor a = kept[0], b = kept[1], g2 = grad;
         const int64_t d = a.dim(), batch = d == 3 ? a.size(0) : 1, M = a.size(d - 2), K = a.size(d - 1), N = b.size(d - 1);
         const Mat ma = matrix(a), mb = matrix(b), g = matrix(g2);
         variable_list out(2);
-        if (needs(0))
+        if (wanted(0))
             out[0] = approx_a ? product(g, mb.t(), Tensor(), batch, M, K, N, offset, a.sizes(), a)
                               : product_bwd(g, mb.t(), ma, true, batch, M, K, N, offset, a.sizes(), a);
-        if (needs(1))
+        if (wanted(1))
             out[1] = approx_b ? product(ma.t(), g, Tensor(), batch, K, N, M, offset, b.sizes(), a)
                               : product_bwd(ma.t(), g, mb, false, batch, K, N, M, offset, b.sizes(), a);
         return out;
@@ -392,22 +459,23 @@ struct MatMulNode : PamNode {
 };
 
 // The approximate backward pass works from eight scalars per row that the forward pass kept.
-struct LayerNormNode : PamNode {
+struct LayerNormRule {
     double eps, offset;
     bool approx, has_w, has_b;
     int64_t width;
-    std::vector<int64_t> x_shape, w_shape, b_shape;
-    std::string name() const override { return "PamLayerNormBackward"; }
-    variable_list grads(const variable_list& kept, const Tensor& grad) override {
+    std::vector<int64_t> b_shape;
+    std::string name() const { return "PamLayerNormBackward"; }
+    std::string key() const { return bytes_of(eps, offset, approx, has_w, has_b, width) + bytes_of_list(b_shape); }
+    variable_list grads(const variable_list& kept, const Tensor& grad, const Wanted& wanted) const {
         size_t k = 0;
         Tensor x = kept[k++], w, stats;
         if (has_w) w = kept[k++];
         if (approx) stats = kept[k++];
         const Tensor g = grad.contiguous();
         const int64_t rows = x.numel() / width;
-        Tensor dx = empty_on(x_shape, x);
-        const bool nw = has_w && needs(1), nb = has_b && needs(has_w ? 2 : 1);
-        Tensor dw = nw ? empty_on(w_shape, x) : Tensor(), db = nb ? empty_on(b_shape, x) : Tensor();
+        Tensor dx = empty_on(x.sizes(), x);
+        const bool nw = has_w && wanted(1), nb = has_b && wanted(has_w ? 2 : 1);
+        Tensor dw = nw ? empty_on(w.sizes(), x) : Tensor(), db = nb ? empty_on(b_shape, x) : Tensor();
         Tensor ws;
         size_t bytes = 0;
         if (nw || nb) {
@@ -446,11 +514,12 @@ Tensor softmax_backward_saved(const Tensor& e, const Tensor& g, int64_t rows, in
 }
 
 // With the approximate backward the forward pass keeps its exponentials instead of its input.
-struct SoftmaxNode : PamNode {
+struct SoftmaxRule {
     double offset;
     bool approx;
-    std::string name() const override { return "PamSoftmaxBackward"; }
-    variable_list grads(const variable_list& kept, const Tensor& grad) override {
+    std::string name() const { return "PamSoftmaxBackward"; }
+    std::string key() const { return bytes_of(offset, approx); }
+    variable_list grads(const variable_list& kept, const Tensor& grad, const Wanted& wanted) const {
         const Tensor &from = kept[0], g = grad.contiguous();
         const int64_t len = from.size(-1), rows = from.numel() / len;
         if (approx) return {softmax_backward_saved(from, g, rows, len, offset, std::nullopt, from.sizes())};
@@ -465,11 +534,12 @@ struct SoftmaxNode : PamNode {
 
 // softmax(pam(q k^T, scale)) v on the heads of a fused projection [B, N, 3, heads, head_dim] read in place, the
 // context written token-major; the approximate gradients (see fused.py for the correspondence with the chain).
-struct AttentionQkvNode : PamNode {
+struct AttentionQkvRule {
     int64_t heads;
     double scale, offset;
-    std::string name() const override { return "PamAttentionQkvBackward"; }
-    variable_list grads(const variable_list& kept, const Tensor& grad) override {
+    std::string name() const { return "PamAttentionQkvBackward"; }
+    std::string key() const { return bytes_of(heads, scale, offset); }
+    variable_list grads(const variable_list& kept, const Tensor& grad, const Wanted& wanted) const {
         const Tensor qkv = kept[0], expo = kept[1], probs = kept[2], g = grad.contiguous();
         const int64_t B = qkv.size(0), N = qkv.size(1), C3 = qkv.size(2), C = C3 / 3, hd = C / heads;
         const float *q = ptr(qkv), *k = q + C, *v = q + 2 * C;
@@ -488,11 +558,12 @@ struct AttentionQkvNode : PamNode {
 };
 
 // The same for separate projections q [B, T, d], k, v [B, S, d] and an additive mask.
-struct AttentionHeadsNode : PamNode {
+struct AttentionHeadsRule {
     int64_t heads;
     double offset;
-    std::string name() const override { return "PamAttentionHeadsBackward"; }
-    variable_list grads(const variable_list& kept, const Tensor& grad) override {
+    std::string name() const { return "PamAttentionHeadsBackward"; }
+    std::string key() const { return bytes_of(heads, offset); }
+    variable_list grads(const variable_list& kept, const Tensor& grad, const Wanted& wanted) const {
         const Tensor q = kept[0], k = kept[1], v = kept[2], expo = kept[3], probs = kept[4], g = grad.contiguous();
         const int64_t B = q.size(0), T = q.size(1), d = q.size(2), S = k.size(1), hd = d / heads;
         const int64_t H = heads * T * S, TS = T * S;
@@ -529,11 +600,8 @@ std::optional<Tensor> op_linear(const Tensor& x, const Tensor& w, const Tensor& 
         y = product(mx, mw.t(), bias, 1, rows, out_f, in, offset, shape, x);
     }
     if (recording() && (wants_grad(x) || wants_grad(w) || wants_grad(bias))) {
-        auto fn = bias.defined() ? node<LinearNode>(x, w, bias) : node<LinearNode>(x, w);
-        fn->offset = offset;
-        fn->approx_x = approx_x;
-        fn->approx_w = approx_w;
-        fn->has_bias = bias.defined();
+        const LinearRule rule{offset, approx_x, approx_w, bias.defined()};
+        auto fn = bias.defined() ? node(rule, x, w, bias) : node(rule, x, w);
         fn->keep({x, w});
         torch::autograd::set_history(y, fn);
     }
@@ -554,10 +622,7 @@ std::optional<Tensor> op_matmul(const Tensor& a, const Tensor& b, double offset,
         y = product(ma, mb, Tensor(), batch, M, N, K, offset, at::IntArrayRef(shape + (3 - dims), dims), a);
     }
     if (recording() && (wants_grad(a) || wants_grad(b))) {
-        auto fn = node<MatMulNode>(a, b);
-        fn->offset = offset;
-        fn->approx_a = approx_a;
-        fn->approx_b = approx_b;
+        auto fn = node(MatMulRule{offset, approx_a, approx_b}, a, b);
         fn->keep({a, b});
         torch::autograd::set_history(y, fn);
     }
@@ -593,15 +658,7 @@ std::optional<Tensor> op_elementwise(Ew op, const Tensor& a, double num_a, const
         y = ew_forward(op, oa, ob, inner, shape, offset, like);
     }
     if (recording() && (wants_grad(a) || wants_grad(b))) {
-        auto fn = node<EwNode>(a, b);
-        fn->op = op;
-        fn->offset = offset;
-        fn->approx_a = approx_a;
-        fn->approx_b = approx_b;
-        fn->has_a = has_a;
-        fn->has_b = has_b;
-        fn->num_a = num_a;
-        fn->num_b = num_b;
+        auto fn = node(EwRule{op, offset, approx_a, approx_b, has_a, has_b, num_a, num_b}, a, b);
         if (has_a) fn->keep({a});
         if (has_b) fn->keep({b});
         torch::autograd::set_history(y, fn);
@@ -628,17 +685,9 @@ std::optional<Tensor> op_layer_norm(const Tensor& x, int64_t width, const Tensor
               "pamk_layer_norm_fwd");
     }
     if (keep) {
-        std::shared_ptr<LayerNormNode> fn = w.defined() ? (b.defined() ? node<LayerNormNode>(x, w, b) : node<LayerNormNode>(x, w))
-                                                        : (b.defined() ? node<LayerNormNode>(x, b) : node<LayerNormNode>(x));
-        fn->eps = eps;
-        fn->offset = offset;
-        fn->approx = approx;
-        fn->has_w = w.defined();
-        fn->has_b = b.defined();
-        fn->width = width;
-        fn->x_shape = x.sizes().vec();
-        if (w.defined()) fn->w_shape = w.sizes().vec();
-        if (b.defined()) fn->b_shape = b.sizes().vec();
+        LayerNormRule rule{eps, offset, approx, w.defined(), b.defined(), width, {}};
+        if (b.defined()) rule.b_shape = b.sizes().vec();
+        auto fn = w.defined() ? (b.defined() ? node(rule, x, w, b) : node(rule, x, w)) : (b.defined() ? node(rule, x, b) : node(rule, x));
         fn->keep({xc});
         if (w.defined()) fn->keep({w});
         if (approx) fn->keep({stats});
@@ -661,9 +710,7 @@ std::optional<Tensor> op_softmax(const Tensor& x, double offset, bool approx) {
         softmax_forward(xc, y, e, rows, len, offset);
     }
     if (keep) {
-        auto fn = node<SoftmaxNode>(x);
-        fn->offset = offset;
-        fn->approx = approx;
+        auto fn = node(SoftmaxRule{offset, approx}, x);
         fn->keep({approx ? e : xc});
         torch::autograd::set_history(y, fn);
     }
@@ -691,10 +738,7 @@ std::optional<Tensor> op_attention_qkv(const Tensor& given, int64_t heads, doubl
                 std::nullopt, qkv);
     }
     if (keep) {
-        auto fn = node<AttentionQkvNode>(given);
-        fn->heads = heads;
-        fn->scale = scale;
-        fn->offset = offset;
+        auto fn = node(AttentionQkvRule{heads, scale, offset}, given);
         fn->keep({qkv, expo, probs});
         torch::autograd::set_history(out, fn);
     }
@@ -728,9 +772,7 @@ std::optional<Tensor> op_attention_heads(const Tensor& gq, const Tensor& gk, con
                 std::nullopt, q);
     }
     if (keep) {
-        auto fn = node<AttentionHeadsNode>(gq, gk, gv);
-        fn->heads = heads;
-        fn->offset = offset;
+        auto fn = node(AttentionHeadsRule{heads, offset}, gq, gk, gv);
         fn->keep({q, k, v, expo, probs});
         torch::autograd::set_history(out, fn);
     }

@@ -159,3 +159,33 @@ def test_a_missing_gradient_counts_as_zeros(name):
     x = randn(2, 4, 12).requires_grad_()
     (grad,) = torch.autograd.grad(_NoGradient.apply(OPERATORS[name](x)).sum(), x)
     assert grad.shape == x.shape and bool((grad == 0).all())
+
+
+@each_operator
+def test_compiled_autograd(name):
+    from torch._dynamo import compiled_autograd
+    op = OPERATORS[name]
+    for seed, scale in ((1, 1.0), (2, 3.0)):
+        x = randn(2, 4, 12, seed=seed).requires_grad_()
+        y = op(x * scale)
+        gy = randn(*y.shape, seed=5)
+        (want,) = torch.autograd.grad(y, x, gy, retain_graph=True)
+        with compiled_autograd._enable(lambda gm: torch.compile(gm, backend="eager")):
+            y.backward(gy)
+        assert_bits_equal(x.grad, want, name)
+
+
+def test_compiled_autograd_tells_settings_apart():
+    """The same graph with another number, offset or gradient mode must not run an earlier one's compiled backward pass."""
+    from torch._dynamo import compiled_autograd
+    for approx in (True, False):
+        for offset in (None, 1.0552):
+            for number in (2.0, 3.3):
+                x = randn(2, 4, 12).requires_grad_()
+                y = pam.softmax(pam.mul(pam.layer_norm(x, (12,), GAIN, GAIN, offset=offset, approx_bwd=approx), number, offset=offset, approx_bwd=approx),
+                                dim=-1, offset=offset, approx_bwd=approx)
+                gy = randn(*y.shape, seed=5)
+                (want,) = torch.autograd.grad(y, x, gy, retain_graph=True)
+                with compiled_autograd._enable(lambda gm: torch.compile(gm, backend="eager")):
+                    y.backward(gy)
+                assert_bits_equal(x.grad, want, f"{approx} {offset} {number}")
