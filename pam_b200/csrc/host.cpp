@@ -961,20 +961,32 @@ struct AdamEntry {
 };
 
 // adam_collect(params, state): for one parameter group, whether every parameter with a gradient is in the form that
-// the fused update takes and has its state; then the steps are counted up and [(step, capsule of tensors)] comes
-// back, one entry for each distinct step count and device.  None leaves everything as it was.
+// the fused update takes and has its state; then [(step, capsule of tensors)] comes back, one entry for each
+// distinct step count and device.  Nothing is changed: adam_apply counts the steps, once they are taken.
 struct AdamBatch {
     std::vector<Tensor> keep;
+    std::vector<PyObject*> states;      // the optimizer's dicts, held
+    PyObject* step = nullptr;           // the count that they get
+    AdamBatch() = default;
+    AdamBatch(const AdamBatch&) = delete;
+    ~AdamBatch() {
+        for (PyObject* st : states) Py_DECREF(st);
+        Py_XDECREF(step);
+    }
     std::vector<float*> p, m, v;
     std::vector<const float*> g;
     std::vector<int64_t> n;
 };
 const char* kAdamCapsule = "pam_b200.adam_batch";
 
+PyObject* step_key() {
+    static PyObject* key = PyUnicode_InternFromString("step");
+    return key;
+}
+
 PyObject* py_adam_collect(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     PAMK_ARGS(2)
-    static PyObject *k_step = PyUnicode_InternFromString("step"), *k_m = PyUnicode_InternFromString("exp_avg"),
-                    *k_v = PyUnicode_InternFromString("exp_avg_sq");
+    static PyObject *k_m = PyUnicode_InternFromString("exp_avg"), *k_v = PyUnicode_InternFromString("exp_avg_sq");
     return guarded([&]() -> PyObject* {
         if (!PyList_Check(a[0]) || !PyDict_Check(a[1])) return none();
         std::vector<AdamEntry> found;
@@ -993,7 +1005,7 @@ PyObject* py_adam_collect(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
                 return none();
             }
             if (!PyDict_Check(st)) return none();
-            PyObject *step = PyDict_GetItem(st, k_step), *m = PyDict_GetItem(st, k_m), *v = PyDict_GetItem(st, k_v);
+            PyObject *step = PyDict_GetItem(st, step_key()), *m = PyDict_GetItem(st, k_m), *v = PyDict_GetItem(st, k_v);
             if (step == nullptr || m == nullptr || v == nullptr || !PyLong_CheckExact(step) || !THPVariable_Check(m) || !THPVariable_Check(v)) return none();
             e.m = THPVariable_Unpack(m);
             e.v = THPVariable_Unpack(v);
@@ -1005,14 +1017,14 @@ PyObject* py_adam_collect(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
         }
         std::map<std::pair<int64_t, int>, std::unique_ptr<AdamBatch>> batches;
         for (AdamEntry& e : found) {
-            PyObject* next = PyLong_FromLongLong(e.step + 1);
-            if (next == nullptr || PyDict_SetItem(e.state, k_step, next) < 0) {
-                Py_XDECREF(next);
-                return nullptr;
-            }
-            Py_DECREF(next);
             auto& b = batches[{e.step + 1, e.p.device().index()}];
-            if (!b) b = std::make_unique<AdamBatch>();
+            if (!b) {
+                b = std::make_unique<AdamBatch>();
+                b->step = PyLong_FromLongLong(e.step + 1);
+                if (b->step == nullptr) return nullptr;
+            }
+            Py_INCREF(e.state);
+            b->states.push_back(e.state);
             b->p.push_back(ptr(e.p));
             b->g.push_back(ptr(e.g));
             b->m.push_back(ptr(e.m));
@@ -1039,14 +1051,18 @@ PyObject* py_adam_apply(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     return guarded([&]() -> PyObject* {
         auto* b = static_cast<AdamBatch*>(PyCapsule_GetPointer(a[0], kAdamCapsule));
         if (b == nullptr) return nullptr;
-        double s[7];
-        for (int i = 0; i < 7; ++i)
-            if (!as_number(a[i + 1], s[i])) { PyErr_SetString(PyExc_TypeError, "adam_apply: numbers expected"); return nullptr; }
+        double s[7];                    // (anything that converts: a learning rate may be a NumPy scalar or a tensor)
+        for (int i = 0; i < 7; ++i) {
+            s[i] = PyFloat_AsDouble(a[i + 1]);
+            if (s[i] == -1.0 && PyErr_Occurred()) return nullptr;
+        }
         const Tensor& like = b->keep[0];
         c10::cuda::CUDAGuard guard(like.device());
         check(lib.pamk_adam_step(b->p.data(), b->g.data(), b->m.data(), b->v.data(), b->n.data(), (int)b->n.size(), (float)s[0], (float)s[1],
                                  (float)s[2], (float)s[3], (float)s[4], (float)s[5], (float)s[6], 1.0f, stream_of(like)),
               "pamk_adam_step");
+        for (PyObject* st : b->states)
+            if (PyDict_SetItem(st, step_key(), b->step) < 0) return nullptr;
         return none();
     });
 }

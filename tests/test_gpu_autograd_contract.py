@@ -1,6 +1,7 @@
 """What torch.autograd.Function promises and the native host path has to keep: tracing records the operator, forward-mode
 AD and functorch transforms are refused, exceptions keep their type, missing gradients count as zeros, a compiled
 backward pass runs.  Each test failed on a host path that went past one of these."""
+import numpy as np
 import pytest
 import torch
 import torch.autograd.forward_ad as fwAD
@@ -8,7 +9,7 @@ from torch.utils.checkpoint import checkpoint
 
 import pam_b200 as pam
 from conftest import assert_bits_equal
-from pam_b200 import _lib, fused
+from pam_b200 import _lib, fused, optim
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -189,3 +190,39 @@ def test_compiled_autograd_tells_settings_apart():
                 with compiled_autograd._enable(lambda gm: torch.compile(gm, backend="eager")):
                     y.backward(gy)
                 assert_bits_equal(x.grad, want, f"{approx} {offset} {number}")
+
+
+# ---- Adam -------------------------------------------------------------------------------------------------------
+
+def _adam(**kw):
+    ps = [torch.nn.Parameter(randn(n, seed=n)) for n in (5, 1024, 33)]
+    opt = optim.Adam(ps, opt_functional_cfg="pam", **kw)
+    for p in ps:
+        p.grad = randn(p.numel(), seed=p.numel() + 1)
+        opt.state[p] = {"step": 3, "exp_avg": 0.1 * p.grad, "exp_avg_sq": 0.01 * p.grad.square()}
+    return ps, opt
+
+
+@pytest.mark.parametrize("number", [np.float32, np.float64, torch.tensor, lambda v: torch.tensor(v, device=DEV)])
+def test_adam_takes_any_number(number, monkeypatch):
+    """The native collection against the Python layer's, whose ctypes call converts whatever has a float value."""
+    results = []
+    for python in (False, True):
+        with monkeypatch.context() as m:
+            if python:
+                m.setattr(_lib, "host", lambda: None)
+            ps, opt = _adam(lr=number(1e-3), eps=number(1e-8), weight_decay=number(0.1))
+            opt.step()
+            results.append([t for p in ps for t in (p.detach(), opt.state[p]["exp_avg"], opt.state[p]["exp_avg_sq"])])
+    for got, want in zip(*results):
+        assert_bits_equal(got, want)
+
+
+def test_adam_counts_a_step_when_it_was_taken():
+    ps, opt = _adam(lr=1e-3, eps="1e-8")
+    with pytest.raises(TypeError):
+        opt.step()
+    assert [opt.state[p]["step"] for p in ps] == [3, 3, 3]
+    opt.param_groups[0]["eps"] = 1e-8
+    opt.step()
+    assert [opt.state[p]["step"] for p in ps] == [4, 4, 4]
