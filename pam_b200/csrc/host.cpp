@@ -31,6 +31,7 @@
 
 #include <dlfcn.h>
 
+#include <algorithm>
 #include <array>
 #include <atomic>
 #include <map>
@@ -1015,6 +1016,12 @@ PyObject* py_adam_collect(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
             if (!as_int(step, e.step)) return none();
             found.push_back(std::move(e));
         }
+        // A parameter that is listed twice takes two steps, one after the other: one launch would run both at once.
+        std::vector<PyObject*> once;
+        once.reserve(found.size());
+        for (const AdamEntry& e : found) once.push_back(e.state);
+        std::sort(once.begin(), once.end());
+        if (std::adjacent_find(once.begin(), once.end()) != once.end()) return none();
         std::map<std::pair<int64_t, int>, std::unique_ptr<AdamBatch>> batches;
         for (AdamEntry& e : found) {
             auto& b = batches[{e.step + 1, e.p.device().index()}];

@@ -226,3 +226,19 @@ def test_adam_counts_a_step_when_it_was_taken():
     opt.param_groups[0]["eps"] = 1e-8
     opt.step()
     assert [opt.state[p]["step"] for p in ps] == [4, 4, 4]
+
+
+@pytest.mark.filterwarnings("ignore:optimizer contains a parameter group with duplicate")
+def test_adam_takes_a_parameter_listed_twice_in_turn():
+    def run(twice):
+        p = torch.nn.Parameter(randn(1 << 20))
+        opt = optim.Adam([p, p] if twice else [p], lr=1e-2, opt_functional_cfg="pam")
+        p.grad = randn(1 << 20, seed=2)
+        opt.state[p] = {"step": 0, "exp_avg": torch.zeros_like(p), "exp_avg_sq": torch.zeros_like(p)}
+        for _ in range(1 if twice else 2):
+            opt.step()
+        return p.detach(), opt.state[p]
+    (got, s), (want, t) = run(True), run(False)
+    assert s["step"] == t["step"] == 2
+    assert_bits_equal(got, want)
+    assert_bits_equal(s["exp_avg"], t["exp_avg"])
