@@ -528,7 +528,7 @@ def pam_matmul(A, B, *, offset=None, approx_bwd=False):
 def pam_linear(X, W, bias, *, offset=None, approx_bwd=False):
     """[rows, in] x [out, in] + [out] (no counterpart in the reference's bindings: its `linear` is
     pam_matmul followed by a torch add)."""
-    if _on_cuda(X) and (host := _lib.host()) is not None:
+    if _on_cuda(X) and X.dim() == 2 and (host := _lib.host()) is not None:
         out = host.linear(X, W, bias, offset, approx_bwd)
         if out is not None:
             return out

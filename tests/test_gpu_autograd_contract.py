@@ -9,7 +9,7 @@ from torch.utils.checkpoint import checkpoint
 
 import pam_b200 as pam
 from conftest import assert_bits_equal
-from pam_b200 import _lib, fused, optim
+from pam_b200 import _lib, cuda_bindings, fused, optim
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -190,6 +190,11 @@ def test_compiled_autograd_tells_settings_apart():
                 with compiled_autograd._enable(lambda gm: torch.compile(gm, backend="eager")):
                     y.backward(gy)
                 assert_bits_equal(x.grad, want, f"{approx} {offset} {number}")
+
+
+def test_pam_linear_binding_takes_matrices_only():
+    with pytest.raises(ValueError, match="target_dim=2"):
+        cuda_bindings.pam_linear(randn(2, 4, 12), W, GAIN[:6].contiguous())
 
 
 # ---- Adam -------------------------------------------------------------------------------------------------------
