@@ -107,6 +107,8 @@ def set_nvtx(on):
     """Turns the NVTX ranges around the library's launches on or off (also: PAM_B200_NVTX=1)."""
     global _nvtx
     _nvtx = bool(on)
+    if _host is not None:
+        _host.set_nvtx(_nvtx)
 
 
 def lib():
@@ -133,11 +135,8 @@ _host = None
 
 
 def host():
-    """The native host path (csrc/host.cpp) bound to the loaded library, or None while NVTX ranges are on (the
-    Python layer then runs, whose library calls carry them).  Raises if it was never built."""
+    """The native host path (csrc/host.cpp) bound to the loaded library.  Raises if it was never built."""
     global _host
-    if _nvtx:
-        return None
     if _host is None:
         if not HOST_PATH.exists():
             raise RuntimeError(f"{HOST_PATH} is missing: build it with `python -m pam_b200.build`")
@@ -150,6 +149,7 @@ def host():
         module.setup(str(LIB_PATH), PamKernelError)
         from . import cuda_bindings
         module.set_strict(cuda_bindings.strict_k_order())
+        module.set_nvtx(_nvtx)
         _host = module
     return _host
 

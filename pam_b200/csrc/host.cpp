@@ -30,6 +30,7 @@
 #include <c10/cuda/CUDAStream.h>
 
 #include <dlfcn.h>
+#include <nvtx3/nvToolsExt.h>
 
 #include <algorithm>
 #include <array>
@@ -52,20 +53,41 @@ using torch::autograd::variable_list;
 
 // ---- the kernel library ---------------------------------------------------------------------------
 
-// Entry points used here, bound by name from the library that the Python layer loaded.
-#define PAMK_ENTRIES(X)                                                                                   \
-    X(pamk_status_string) X(pamk_last_cuda_error) X(pamk_pam_fwd) X(pamk_pad_fwd) X(pamk_pam_grad)        \
-    X(pamk_pad_grad) X(pamk_matmul_bias) X(pamk_matmul_strided) X(pamk_matmul_bwd)                        \
-    X(pamk_matmul_auto_split) X(pamk_matmul_bwd_auto_split) X(pamk_column_sum_workspace_bytes)            \
-    X(pamk_column_sum) X(pamk_layer_norm_max_width) X(pamk_layer_norm_stats_per_row)                      \
-    X(pamk_layer_norm_fwd) X(pamk_layer_norm_fwd_save) X(pamk_layer_norm_bwd)                             \
-    X(pamk_layer_norm_bwd_saved) X(pamk_layer_norm_bwd_workspace_bytes) X(pamk_softmax_max_len)           \
-    X(pamk_softmax_workspace_bytes) X(pamk_softmax_fwd) X(pamk_softmax_fwd_save) X(pamk_softmax_bwd)      \
-    X(pamk_softmax_bwd_saved) X(pamk_adam_step)
+// Entry points used here, bound by name from the library that the Python layer loaded: those that only answer, and
+// those that launch.
+#define PAMK_QUERIES(X)                                                                                   \
+    X(pamk_status_string) X(pamk_last_cuda_error) X(pamk_matmul_auto_split) X(pamk_matmul_bwd_auto_split) \
+    X(pamk_column_sum_workspace_bytes) X(pamk_layer_norm_max_width) X(pamk_layer_norm_stats_per_row)      \
+    X(pamk_layer_norm_bwd_workspace_bytes) X(pamk_softmax_max_len) X(pamk_softmax_workspace_bytes)
+#define PAMK_LAUNCHES(X)                                                                                  \
+    X(pamk_pam_fwd) X(pamk_pad_fwd) X(pamk_pam_grad) X(pamk_pad_grad) X(pamk_matmul_bias)                 \
+    X(pamk_matmul_strided) X(pamk_matmul_bwd) X(pamk_column_sum) X(pamk_layer_norm_fwd)                   \
+    X(pamk_layer_norm_fwd_save) X(pamk_layer_norm_bwd) X(pamk_layer_norm_bwd_saved) X(pamk_softmax_fwd)   \
+    X(pamk_softmax_fwd_save) X(pamk_softmax_bwd) X(pamk_softmax_bwd_saved) X(pamk_adam_step)
+
+std::atomic<bool> g_nvtx{false};         // set_nvtx
+
+// A launching entry point, inside an NVTX range of its name while those are on.
+template <class F>
+struct Launch {
+    F* fn = nullptr;
+    const char* label = "";
+    template <class... A>
+    int operator()(A&&... a) const {
+        if (!g_nvtx.load(std::memory_order_relaxed)) return fn(std::forward<A>(a)...);
+        nvtxRangePushA(label);
+        const int status = fn(std::forward<A>(a)...);
+        nvtxRangePop();
+        return status;
+    }
+};
 
 struct Library {
 #define PAMK_MEMBER(name) decltype(&::name) name = nullptr;
-    PAMK_ENTRIES(PAMK_MEMBER)
+    PAMK_QUERIES(PAMK_MEMBER)
+#undef PAMK_MEMBER
+#define PAMK_MEMBER(name) Launch<decltype(::name)> name;
+    PAMK_LAUNCHES(PAMK_MEMBER)
 #undef PAMK_MEMBER
 };
 
@@ -1081,6 +1103,13 @@ PyObject* py_set_strict(PyObject*, PyObject* flag) {
     return none();
 }
 
+PyObject* py_set_nvtx(PyObject*, PyObject* flag) {
+    const int v = PyObject_IsTrue(flag);
+    if (v < 0) return nullptr;
+    g_nvtx.store(v != 0, std::memory_order_relaxed);
+    return none();
+}
+
 // setup(library path, error class)
 PyObject* py_setup(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     PAMK_ARGS(2)
@@ -1091,13 +1120,18 @@ PyObject* py_setup(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
         PyErr_Format(PyExc_RuntimeError, "cannot load %s: %s", path, dlerror());
         return nullptr;
     }
-#define PAMK_BIND(name)                                                                      \
-    lib.name = reinterpret_cast<decltype(lib.name)>(dlsym(h, #name));                        \
-    if (lib.name == nullptr) {                                                               \
+#define PAMK_BIND(name, to)                                                                  \
+    to = reinterpret_cast<decltype(to)>(dlsym(h, #name));                                    \
+    if (to == nullptr) {                                                                     \
         PyErr_Format(PyExc_RuntimeError, "%s does not export " #name, path);                 \
         return nullptr;                                                                      \
     }
-    PAMK_ENTRIES(PAMK_BIND)
+#define PAMK_BIND_QUERY(name) PAMK_BIND(name, lib.name)
+#define PAMK_BIND_LAUNCH(name) PAMK_BIND(name, lib.name.fn) lib.name.label = #name;
+    PAMK_QUERIES(PAMK_BIND_QUERY)
+    PAMK_LAUNCHES(PAMK_BIND_LAUNCH)
+#undef PAMK_BIND_QUERY
+#undef PAMK_BIND_LAUNCH
 #undef PAMK_BIND
     Py_INCREF(a[1]);
     Py_XDECREF(g_kernel_error);
@@ -1109,6 +1143,7 @@ PyObject* py_setup(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
 PyMethodDef methods[] = {
     PAMK_FAST("setup", py_setup),
     {"set_strict", py_set_strict, METH_O, nullptr},
+    {"set_nvtx", py_set_nvtx, METH_O, nullptr},
     PAMK_FAST("linear", py_linear),
     PAMK_FAST("matmul", py_matmul),
     PAMK_FAST("mul", py_elementwise<Ew::kMul>),

@@ -1,6 +1,7 @@
 """The native host path (csrc/host.cpp) against the Python layer on the same kernels: results and gradients
-bit for bit, over operand forms, sizes at the edges of a vector and of a block, and layouts.  With NVTX ranges
-on every operator runs through the Python layer, which is how the second route is taken here."""
+bit for bit, over operand forms, sizes at the edges of a vector and of a block, and layouts."""
+import contextlib
+
 import pytest
 import torch
 
@@ -12,18 +13,24 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda"
 
 
+@contextlib.contextmanager
+def route(python):
+    """The native host path, or the Python layer as if the native one declined every call."""
+    with pytest.MonkeyPatch.context() as m:
+        if python:
+            m.setattr(_lib, "host", lambda: None)
+        yield
+
+
 def both(fn, *inputs, gy_seed=5):
     """fn on copies of `inputs` through each route: outputs and the gradients of the tensor inputs."""
     results = []
     for python in (False, True):
-        _lib.set_nvtx(python)
-        try:
+        with route(python):
             ins = [t.detach().clone(memory_format=torch.preserve_format).requires_grad_() if isinstance(t, torch.Tensor) else t for t in inputs]
             y = fn(*ins)
             gy = torch.randn(y.shape, generator=torch.Generator(DEV).manual_seed(gy_seed), device=DEV)
             results.append([y.detach(), *torch.autograd.grad(y, [t for t in ins if isinstance(t, torch.Tensor)], gy)])
-        finally:
-            _lib.set_nvtx(False)
     for k, (got, want) in enumerate(zip(*results)):
         assert_bits_equal(got, want, f"output {k}")
 
@@ -92,8 +99,7 @@ def test_adam_groups_and_fallbacks():
     """Two groups, a parameter without a gradient, unequal step counts; then a group that the native collection
     declines (a half-precision parameter), which steps through the dictionary of operators."""
     def run(python, half):
-        _lib.set_nvtx(python)
-        try:
+        with route(python):
             g = torch.Generator(DEV).manual_seed(3)
             ps = [torch.nn.Parameter(torch.randn(n, generator=g, device=DEV)) for n in (1, 5, 1024, 4099)]
             if half:
@@ -105,8 +111,6 @@ def test_adam_groups_and_fallbacks():
                 opt.step()
             steps = [opt.state[p]["step"] for p in ps]
             return [t for p in ps for t in (p.detach().float(), opt.state[p]["exp_avg"], opt.state[p]["exp_avg_sq"])], steps
-        finally:
-            _lib.set_nvtx(False)
 
     for half in (False, True):
         (got, steps), (want, want_steps) = run(False, half), run(True, half)
@@ -127,3 +131,17 @@ def test_errors_are_those_of_the_python_layer():
     y.sum().backward()
     with pytest.raises(RuntimeError, match="second time"):
         y.sum().backward()
+
+
+def test_nvtx_ranges_are_around_the_path_that_runs_without_them():
+    x, w = randn(70, 50, specials=False).requires_grad_(), randn(30, 50, seed=2, specials=False).requires_grad_()
+    plain = pam.linear(x, w, approx_bwd=True)
+    pam.set_nvtx(True)
+    try:
+        traced = pam.linear(x, w, approx_bwd=True)
+        grads = torch.autograd.grad(traced.sum(), [x, w])
+    finally:
+        pam.set_nvtx(False)
+    assert traced.grad_fn.name() == plain.grad_fn.name() == "PamLinearBackward"
+    for got, want in zip((traced, *grads), (plain, *torch.autograd.grad(plain.sum(), [x, w]))):
+        assert_bits_equal(got.detach(), want.detach())
