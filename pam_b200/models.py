@@ -187,33 +187,40 @@ class TransformerLayer(nn.Module):
         return self.final_layer_norm(x + self.fc2(torch.relu(self.fc1(x))))
 
 
+def _ordinary_call(device):
+    """Whether a tensor made now may be kept: not one that belongs to a trace, a transform, a dispatch mode or a compiler,
+    nor one that a captured graph would go on reading after it was replaced."""
+    return not (torch.jit.is_tracing() or torch.compiler.is_compiling() or torch._C._are_functorch_transforms_active()
+                or torch._C._len_torch_dispatch_stack() or (device.type == "cuda" and torch.cuda.is_current_stream_capturing()))
+
+
 class _Stack(nn.Module):
     def __init__(self, cfg, layers, cross, linear_factory, norm_layer, op_dict):
         super().__init__()
         self.cfg, self.op_dict = cfg, op_dict
-        self._tables = {}
         self.embed_tokens = nn.Embedding(cfg.vocab, cfg.dim, padding_idx=cfg.pad)
         self.embed_scale = math.sqrt(cfg.dim)
         self.layers = nn.ModuleList([TransformerLayer(cfg, cross, linear_factory, norm_layer, op_dict) for _ in range(layers)])
 
-    def _kept(self, name, length, device, make):
-        """A constant table of `length`, made on the host and copied to the device when the length or the device
-        changes (the copy is complete before it is used, on whatever stream), and kept in between."""
-        key, table = self._tables.get(name, (None, None))
-        if key != (length, device):
+    def _positions(self, length, device):
+        """The first `length` rows of the sinusoidal table.  Making them takes the host and a copy that waits, so the
+        table is kept, on each device, for the longest sequence so far (to the next power of two)."""
+        if not _ordinary_call(device):
+            return sinusoidal_positions(length, self.cfg.dim, self.cfg.pad, device)
+        tables = self.__dict__.setdefault("_position_tables", {})
+        stream = torch.cuda.current_stream(device) if device.type == "cuda" else None
+        owner, table = tables.get(device, (None, None))
+        if table is None or table.shape[0] < length or table.device != device:
             with torch.inference_mode(False):
-                table = make().to(device)
-            self._tables[name] = ((length, device), table)
-        return table
+                table = sinusoidal_positions(1 << (length - 1).bit_length(), self.cfg.dim, self.cfg.pad, device)
+            tables[device] = (stream and stream.cuda_stream, table)
+        elif stream and stream.cuda_stream != owner:
+            table.record_stream(stream)          # (a longer table may replace this one while the stream still reads it)
+        return table[:length]
 
     def embed(self, tokens):
         x = self.op_dict["mul"](self.embed_scale, self.embed_tokens(tokens))
-        length = tokens.shape[1]
-        return x + self._kept("positions", length, tokens.device,
-                              lambda: sinusoidal_positions(length, self.cfg.dim, self.cfg.pad, torch.device("cpu")))
-
-    def future_mask(self, length, device):
-        return self._kept("future", length, device, lambda: torch.full((length, length), float("-inf")).triu(1))
+        return x + self._positions(tokens.shape[1], tokens.device)
 
 
 class Transformer(nn.Module):
@@ -237,7 +244,8 @@ class Transformer(nn.Module):
         x = self.encoder.embed(src)
         for layer in self.encoder.layers:
             x = layer(x)
-        future = self.decoder.future_mask(prev_out.shape[1], src.device)
+        T = prev_out.shape[1]
+        future = torch.full((T, T), float("-inf"), device=src.device).triu(1)
         y = self.decoder.embed(prev_out)
         for layer in self.decoder.layers:
             y = layer(y, x, future)

@@ -59,3 +59,33 @@ def test_module_form_equals_functional_graph(oracle, monkeypatch, name):
         assert_bits_equal(grads[dotted].reshape(leaves[flat].shape), leaves[flat].grad, f"gradient of {flat}")
     assert list(model.state_dict().keys()) == list(stock.state_dict().keys())
     assert isinstance(dict(model.named_modules())["blocks.0.attn.qkv" if name == "deit" else "encoder.layers.0.fc1"], pam.Linear)
+
+
+def test_kept_position_table(monkeypatch):
+    """One table serves every length, is rebuilt only for a longer one, and holds nothing that a transform or a mode made."""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+
+    from pam_b200 import models, steps
+    made = []
+
+    def counted(length, *rest):
+        made.append(length)
+        return steps.sinusoidal_positions(length, *rest)
+    monkeypatch.setattr(models, "sinusoidal_positions", counted)
+    cpu = torch.device("cpu")
+    stack = models.Transformer(TRANSFORMER).encoder
+    with torch.inference_mode():
+        stack._positions(3, cpu)
+    for length in (5, 8, 1, 7, 16, 2, 9, 16):
+        got = stack._positions(length, cpu)
+        assert not got.is_inference()
+        assert_bits_equal(got, steps.sinusoidal_positions(length, TRANSFORMER.dim, TRANSFORMER.pad, cpu), str(length))
+    assert made == [4, 8, 16]
+
+    torch.func.grad(lambda t: (t * stack._positions(20, cpu)[0, 0]).sum())(torch.ones(2))
+    with FakeTensorMode():
+        stack._positions(21, cpu)
+    assert made == [4, 8, 16, 20, 21] and type(stack._positions(16, cpu)) is torch.Tensor and len(made) == 5
+
+    del stack.__dict__["_position_tables"]                        # a model that was saved before there was one
+    assert stack._positions(2, cpu).shape[0] == 2
