@@ -14,7 +14,6 @@ Configuration grammar (unchanged):
   with the keys ``mean mul div softmax bmm logsumexp log_softmax pow``.
 """
 import copy
-import functools
 import inspect
 import warnings
 
@@ -105,24 +104,29 @@ class LazyGain(_LazyPerChannel, Gain):
     cls_to_become = Gain
 
 
-@functools.lru_cache(maxsize=256)
 def _accepted(func):
-    """Names of the parameters of `func`, or None if it takes any keyword.  (Inspecting the signature costs 15 us:
-    more than the operators that the bound dictionaries call through here.)"""
+    """Names of the parameters of `func`, or None if it takes any keyword."""
     params = inspect.signature(func).parameters
     return None if any(p.kind == p.VAR_KEYWORD for p in params.values()) else frozenset(params)
 
 
-def get_valid_kwargs(func, argdict):
-    names = _accepted(func)
+def _valid_kwargs(names, argdict):
     return argdict if names is None else {k: v for k, v in argdict.items() if k in names}
 
 
-def call_valid_kwargs(func, kwargs_dict, args_tuple=tuple()):
-    kwargs = get_valid_kwargs(func, kwargs_dict)
+def get_valid_kwargs(func, argdict):
+    return _valid_kwargs(_accepted(func), argdict)
+
+
+def _call_accepted(func, names, kwargs_dict, args_tuple):
+    kwargs = _valid_kwargs(names, kwargs_dict)
     if extra := sorted(set(kwargs_dict) - set(kwargs)):
         warnings.warn(f"Function {func} ignored extra arguments {extra}")
     return func(*args_tuple, **kwargs)
+
+
+def call_valid_kwargs(func, kwargs_dict, args_tuple=tuple()):
+    return _call_accepted(func, _accepted(func), kwargs_dict, args_tuple)
 
 
 def get_module_factory(desc, factories):
@@ -227,8 +231,9 @@ def get_function_dict(desc):
     # as in the reference (factories.py:291-298) the dict form wraps the full PAM dictionary
     # whatever `type` says
     def bind(func):
+        names = _accepted(func)      # (once: inspecting a signature costs 15 us, more than the operators called through here)
         def bound(*a, **ka):
-            return call_valid_kwargs(func, {**defaults, **ka, **overrides}, a)
+            return _call_accepted(func, names, {**defaults, **ka, **overrides}, a)
         # what the wrapper binds, for callers that can fuse a chain of these operators into one kernel
         bound.pam_function, bound.pam_kwargs = func, {**defaults, **overrides}
         return bound

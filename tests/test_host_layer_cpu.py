@@ -146,3 +146,25 @@ def test_linear_with_bias_in_the_epilogue_equals_product_plus_add(backend, appro
     for name, got, want in zip(("y", "dx", "dw", "db"), *outs):
         assert torch.equal(got, want), name
     assert any(c[0] == "matmul" for c in backend.calls)
+
+
+def test_factories_take_any_callable_and_keep_none():
+    import gc
+    import weakref
+
+    class Unhashable:
+        __hash__ = None
+
+        def __call__(self, a, b=1):
+            return a + b
+    assert factories.call_valid_kwargs(Unhashable(), {"b": 5}, (2,)) == 7
+
+    class Owner:
+        def method(self, a, b=1):
+            return a * b
+    owner = Owner()
+    assert factories.call_valid_kwargs(owner.method, {"b": 5}, (2,)) == 10
+    gone = weakref.ref(owner)
+    del owner
+    gc.collect()
+    assert gone() is None
