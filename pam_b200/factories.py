@@ -228,6 +228,7 @@ def get_function_dict(desc):
     assert isinstance(desc, dict), f"Unknown function cfg {desc=}"
     assert desc["type"] in ("pam", "pam_bmm_only", "pam_softmax_only"), "Only support custom cfg for pam"
     defaults, overrides = desc.get("dkwargs", {}), desc.get("okwargs", {})
+    settings = {k: v for k, v in {**defaults, **overrides}.items() if k in ("offset", "approx_bwd")}
     # as in the reference (factories.py:291-298) the dict form wraps the full PAM dictionary
     # whatever `type` says
     def bind(func):
@@ -235,6 +236,6 @@ def get_function_dict(desc):
         def bound(*a, **ka):
             return _call_accepted(func, names, {**defaults, **ka, **overrides}, a)
         # what the wrapper binds, for callers that can fuse a chain of these operators into one kernel
-        bound.pam_function, bound.pam_kwargs = func, {**defaults, **overrides}
+        bound.pam_function, bound.pam_kwargs, bound.pam_settings = func, {**defaults, **overrides}, settings
         return bound
     return {name: bind(func) for name, func in _pam_dict().items()}

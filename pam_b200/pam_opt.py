@@ -1,32 +1,28 @@
 """Cross entropy with a PAM backward — the counterpart of the reference's ``pam/pam_opt.py`` — and the
 label-smoothed loss of the reference's fairseq criterion computed straight from the logits."""
-import functools
-
 import torch
 
 from . import fused, pam_ops
-
-
-@functools.lru_cache(maxsize=64)
-def _common_binding(names, ops):
-    common = None
-    for name, op in zip(names, ops):
-        func, kwargs = getattr(op, "pam_function", op), getattr(op, "pam_kwargs", {})
-        if func is not getattr(pam_ops, name):
-            return None
-        kwargs = {k: v for k, v in kwargs.items() if k in ("offset", "approx_bwd")}
-        if common is not None and kwargs != common:
-            return None
-        common = kwargs
-    return common
 
 
 def _pam_binding(ops, names):
     """If the entries `names` of an operator dictionary are this package's PAM functions, bound (by the
     factories' dict-form configuration) to one common set of keyword arguments, those arguments; else
     None.  Lets a chain of dictionary calls be replaced by one fused kernel without changing results.
-    (Remembered per set of functions: a model asks on every forward pass.)"""
-    return _common_binding(names, tuple(ops.get(name) for name in names))
+    (Looked up on every call, as an entry may have been replaced; the functions of one dictionary share their
+    `pam_settings`, so this costs half a microsecond.)"""
+    common = None
+    for name in names:
+        op = ops.get(name)
+        if getattr(op, "pam_function", op) is not getattr(pam_ops, name):
+            return None
+        kwargs = getattr(op, "pam_settings", None)
+        if kwargs is None:
+            kwargs = {k: v for k, v in getattr(op, "pam_kwargs", {}).items() if k in ("offset", "approx_bwd")}
+        if common is not None and kwargs is not common and kwargs != common:
+            return None
+        common = kwargs
+    return dict(common)
 
 
 class cross_entropy_autograd(torch.autograd.Function):

@@ -168,3 +168,27 @@ def test_factories_take_any_callable_and_keep_none():
     del owner
     gc.collect()
     assert gone() is None
+
+
+def test_common_settings_of_an_operator_dictionary():
+    """Read from the entries as they are: any callable may be one, a replaced entry counts, an answer is the caller's own."""
+    from pam_b200.pam_opt import _pam_binding
+    names = ("bmm", "softmax", "mul")
+    ops = factories.get_function_dict('{"type": "pam", "dkwargs": {"approx_bwd": true, "use_kernel": true}}')
+    assert _pam_binding(ops, names) == {"approx_bwd": True}
+    _pam_binding(ops, names)["approx_bwd"] = False
+    assert _pam_binding(ops, names) == {"approx_bwd": True}
+    other = factories.get_function_dict('{"type": "pam", "dkwargs": {"approx_bwd": false}}')
+    assert _pam_binding({**ops, "mul": other["mul"]}, names) is None
+
+    def own(*args):
+        return pam.mul(*args)
+    own.pam_function, own.pam_kwargs = pam.mul, {"approx_bwd": True}
+    assert _pam_binding({**ops, "mul": own}, names) == {"approx_bwd": True}
+    own.pam_kwargs["approx_bwd"] = False
+    assert _pam_binding({**ops, "mul": own}, names) is None
+
+    class Unhashable:
+        __hash__ = None
+    assert _pam_binding({**ops, "mul": Unhashable()}, names) is None
+    assert _pam_binding(factories.get_function_dict("pam"), names) == {}
