@@ -32,7 +32,6 @@
 #include <dlfcn.h>
 #include <nvtx3/nvToolsExt.h>
 
-#include <algorithm>
 #include <array>
 #include <atomic>
 #include <map>
@@ -120,15 +119,21 @@ Tensor scratch_bytes(size_t bytes, const Tensor& like) {
 
 float* ptr(const Tensor& t) { return t.defined() ? static_cast<float*>(t.data_ptr()) : nullptr; }
 
-// fp32 CUDA data that the kernels may read in place: no wrapper of other tensors (functorch, fake, functional), no lazy
-// negation or zero.  A tensor with a tangent (forward-mode AD) is for the Python layer,
-// which refuses it: here the tangent would be lost without a word.
+// Whether forward-mode AD gave the tensor a tangent.  (Almost none ever had one: that is read from the tensor without a call,
+// which an Adam step over 250 parameters asks a thousand times.)
+bool has_tangent(const Tensor& t) {
+    const auto* meta = static_cast<const torch::autograd::AutogradMeta*>(t.unsafeGetTensorImpl()->autograd_meta());
+    return meta != nullptr && meta->fw_grad_ != nullptr && t._fw_grad(0).defined();
+}
+
+// fp32 CUDA data that the kernels may read in place: strided, no wrapper of other tensors (functorch, fake, functional), no
+// lazy negation or zero.  A tensor with a tangent is for the Python layer, which refuses it: here the tangent
+// would be lost without a word.
 bool usable(const Tensor& t) {
     using K = c10::DispatchKey;
     constexpr c10::DispatchKeySet special({K::Python, K::PythonTLSSnapshot, K::FuncTorchBatched, K::FuncTorchGradWrapper, K::Batched,
-                                           K::Functionalize, K::Conjugate, K::Negative, K::ZeroTensor});
-    return t.defined() && t.is_cuda() && t.scalar_type() == at::kFloat && t.layout() == at::kStrided && !t.key_set().has_any(special) &&
-           !t._fw_grad(0).defined();
+                                           K::Functionalize, K::Conjugate, K::Negative, K::ZeroTensor, K::Sparse, K::SparseCsr, K::NestedTensor});
+    return t.defined() && t.is_cuda() && t.scalar_type() == at::kFloat && !t.key_set().has_any(special) && !has_tangent(t);
 }
 
 bool wants_grad(const Tensor& t) { return t.defined() && t.requires_grad(); }
@@ -867,9 +872,12 @@ bool unwatched() {
 // is, an allocation that fails is an OutOfMemoryError.
 template <class F>
 PyObject* guarded(F&& body) {
-    HANDLE_TH_ERRORS
-    return body();
-    END_HANDLE_TH_ERRORS
+    try {
+        return body();
+    } catch (...) {
+        torch::translate_exception_to_python(std::current_exception());
+        return nullptr;
+    }
 }
 
 // An operator's entry: `body`, or None where the call is for the Python layer.
@@ -1039,11 +1047,16 @@ PyObject* py_adam_collect(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
             found.push_back(std::move(e));
         }
         // A parameter that is listed twice takes two steps, one after the other: one launch would run both at once.
-        std::vector<PyObject*> once;
-        once.reserve(found.size());
-        for (const AdamEntry& e : found) once.push_back(e.state);
-        std::sort(once.begin(), once.end());
-        if (std::adjacent_find(once.begin(), once.end()) != once.end()) return none();
+        // (a hash table of the states: sorting them took a tenth of the collection)
+        size_t slots = 16;
+        while (slots < 2 * found.size()) slots *= 2;
+        std::vector<PyObject*> seen(slots, nullptr);
+        for (const AdamEntry& e : found) {
+            size_t at = (reinterpret_cast<uintptr_t>(e.state) >> 4) * 0x9e3779b97f4a7c15ull >> 32 & (slots - 1);
+            while (seen[at] != nullptr && seen[at] != e.state) at = (at + 1) & (slots - 1);
+            if (seen[at] == e.state) return none();
+            seen[at] = e.state;
+        }
         std::map<std::pair<int64_t, int>, std::unique_ptr<AdamBatch>> batches;
         for (AdamEntry& e : found) {
             auto& b = batches[{e.step + 1, e.p.device().index()}];
