@@ -856,7 +856,17 @@ bool as_int(PyObject* o, int64_t& v) {
 
 PyObject* none() { Py_RETURN_NONE; }
 
-PyObject* wrap(std::optional<Tensor>&& t) { return t ? THPVariable_Wrap(std::move(*t)) : none(); }
+// The operator itself runs without the interpreter's lock, as torch's own operators do: an allocation or a launch may wait
+// for the GPU, and Python's other threads go on meanwhile.
+template <class F>
+PyObject* wrapped(F&& op) {
+    std::optional<Tensor> t;
+    {
+        pybind11::gil_scoped_release unlocked;
+        t = op();
+    }
+    return t ? THPVariable_Wrap(std::move(*t)) : none();
+}
 
 // Whether nothing watches or transforms the operators that run.  A trace would keep an answer of this path as a constant,
 // a dispatch mode would not see its allocations, and functorch's transforms refuse autograd functions like
@@ -900,7 +910,7 @@ PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
         double off;
         bool p, q;
         if (!as_tensor(a[0], x) || !as_tensor(a[1], w) || !as_tensor(a[2], b) || !as_offset(a[3], off) || !as_pair(a[4], p, q)) return none();
-        return wrap(op_linear(x, w, b, off, p, q));
+        return wrapped([&] { return op_linear(x, w, b, off, p, q); });
     });
 }
 
@@ -913,7 +923,7 @@ PyObject* py_matmul(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
         bool p, q;
         int64_t dims;
         if (!as_tensor(a[0], x) || !as_tensor(a[1], y) || !as_offset(a[2], off) || !as_pair(a[3], p, q) || !as_int(a[4], dims)) return none();
-        return wrap(op_matmul(x, y, off, p, q, dims));
+        return wrapped([&] { return op_matmul(x, y, off, p, q, dims); });
     });
 }
 
@@ -927,7 +937,7 @@ PyObject* py_elementwise(PyObject*, PyObject* const* a, Py_ssize_t nargs) {   //
         if (!(as_number(a[0], nx) || (as_tensor(a[0], x) && x.defined())) || !(as_number(a[1], ny) || (as_tensor(a[1], y) && y.defined())))
             return none();
         if (!as_offset(a[2], off) || !as_pair(a[3], p, q)) return none();
-        return wrap(op_elementwise(OP, x, nx, y, ny, off, p, q));
+        return wrapped([&] { return op_elementwise(OP, x, nx, y, ny, off, p, q); });
     });
 }
 
@@ -942,7 +952,7 @@ PyObject* py_layer_norm(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
         if (!as_tensor(a[0], x) || !as_int(a[1], width) || !as_tensor(a[2], w) || !as_tensor(a[3], b) || !as_number(a[4], eps) ||
             !as_offset(a[5], off) || !as_pair(a[6], p, q) || p != q)
             return none();
-        return wrap(op_layer_norm(x, width, w, b, eps, off, p));
+        return wrapped([&] { return op_layer_norm(x, width, w, b, eps, off, p); });
     });
 }
 
@@ -954,7 +964,7 @@ PyObject* py_softmax(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
         double off;
         bool p, q;
         if (!as_tensor(a[0], x) || !as_offset(a[1], off) || !as_pair(a[2], p, q) || p != q) return none();
-        return wrap(op_softmax(x, off, p));
+        return wrapped([&] { return op_softmax(x, off, p); });
     });
 }
 
@@ -966,7 +976,7 @@ PyObject* py_attention_qkv(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
         int64_t heads;
         double scale, off;
         if (!as_tensor(a[0], x) || !as_int(a[1], heads) || !as_number(a[2], scale) || !as_offset(a[3], off)) return none();
-        return wrap(op_attention_qkv(x, heads, scale, off));
+        return wrapped([&] { return op_attention_qkv(x, heads, scale, off); });
     });
 }
 
@@ -980,7 +990,7 @@ PyObject* py_attention_heads(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
         if (!as_tensor(a[0], q) || !as_tensor(a[1], k) || !as_tensor(a[2], v) || !as_tensor(a[3], m) || !as_int(a[4], heads) ||
             !as_offset(a[5], off))
             return none();
-        return wrap(op_attention_heads(q, k, v, m, heads, off));
+        return wrapped([&] { return op_attention_heads(q, k, v, m, heads, off); });
     });
 }
 
@@ -1098,11 +1108,14 @@ PyObject* py_adam_apply(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
             s[i] = PyFloat_AsDouble(a[i + 1]);
             if (s[i] == -1.0 && PyErr_Occurred()) return nullptr;
         }
-        const Tensor& like = b->keep[0];
-        c10::cuda::CUDAGuard guard(like.device());
-        check(lib.pamk_adam_step(b->p.data(), b->g.data(), b->m.data(), b->v.data(), b->n.data(), (int)b->n.size(), (float)s[0], (float)s[1],
-                                 (float)s[2], (float)s[3], (float)s[4], (float)s[5], (float)s[6], 1.0f, stream_of(like)),
-              "pamk_adam_step");
+        {
+            pybind11::gil_scoped_release unlocked;
+            const Tensor& like = b->keep[0];
+            c10::cuda::CUDAGuard guard(like.device());
+            check(lib.pamk_adam_step(b->p.data(), b->g.data(), b->m.data(), b->v.data(), b->n.data(), (int)b->n.size(), (float)s[0], (float)s[1],
+                                     (float)s[2], (float)s[3], (float)s[4], (float)s[5], (float)s[6], 1.0f, stream_of(like)),
+                  "pamk_adam_step");
+        }
         for (PyObject* st : b->states)
             if (PyDict_SetItem(st, step_key(), b->step) < 0) return nullptr;
         return none();

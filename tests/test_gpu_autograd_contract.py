@@ -1,6 +1,9 @@
 """What torch.autograd.Function promises and the native host path has to keep: tracing records the operator, forward-mode
 AD and functorch transforms are refused, exceptions keep their type, missing gradients count as zeros, a compiled
 backward pass runs.  Each test failed on a host path that went past one of these."""
+import threading
+import time
+
 import numpy as np
 import pytest
 import torch
@@ -247,3 +250,61 @@ def test_adam_takes_a_parameter_listed_twice_in_turn():
     assert s["step"] == t["step"] == 2
     assert_bits_equal(got, want)
     assert_bits_equal(s["exp_avg"], t["exp_avg"])
+
+
+# ---- threads and streams ------------------------------------------------------------------------------------------
+
+def test_threads_and_streams_agree():
+    """The same block, forward and backward, from four threads on a stream each, repeatedly, against one thread's."""
+    def block(x, w, g):
+        y = pam.softmax(pam.layer_norm(pam.linear(x, w, g, approx_bwd=True), (64,), g, g, approx_bwd=True), dim=-1, approx_bwd=True)
+        return torch.autograd.grad(pam.mul(y, y, approx_bwd=True).sum(), [x, w, g])
+    data = [(randn(300, 128, seed=k).requires_grad_(), (randn(64, 128, seed=k + 10) * 0.1).requires_grad_(),
+             randn(64, seed=k + 20).requires_grad_()) for k in range(4)]
+    want = [block(*d) for d in data]
+    torch.cuda.synchronize()
+    got, errors = [None] * 4, []
+
+    def work(k):
+        try:
+            stream = torch.cuda.Stream()
+            with torch.cuda.stream(stream):
+                for _ in range(20):
+                    got[k] = block(*data[k])
+            stream.synchronize()
+        except Exception as e:                                # noqa: BLE001
+            errors.append(e)
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors
+    for g, w in zip(got, want):
+        for a, b in zip(g, w):
+            assert_bits_equal(a, b)
+
+
+def test_python_threads_go_on_while_a_launch_waits():
+    """Launches behind a busy stream: when the queue is full the launching thread waits, and only that thread may."""
+    x = randn(8)
+    pam.mul(x, 2.0)
+    ticks, stop = [], threading.Event()
+
+    def tick():
+        while not stop.wait(0.005):
+            ticks.append(time.perf_counter())
+    ticker = threading.Thread(target=tick)
+    ticker.start()
+    try:
+        torch.cuda._sleep(1_500_000_000)                      # (most of a second; a full queue is some 1000 launches)
+        begin = time.perf_counter()
+        for _ in range(3000):
+            pam.mul(x, 2.0)
+        waited = time.perf_counter() - begin
+        torch.cuda.synchronize()
+    finally:
+        stop.set()
+        ticker.join()
+    gaps = [b - a for a, b in zip(ticks, ticks[1:])]
+    assert waited > 0.3 and max(gaps) < 0.5 * waited, (waited, max(gaps))
