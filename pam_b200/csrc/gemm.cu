@@ -240,8 +240,13 @@ __device__ __forceinline__ int slab_line(int id, int c) {
     return KC ? (id % (T::BK / 4)) * 4 + c : id / (R / 4);
 }
 
-// k lines of this thread's staged elements that hold an out-of-band element (low 16 bits) and an
-// element above the band (bits 16..31).
+// A slab's word: bit k for a k line that holds an out-of-band element, and above bit 15 whether any lies above the band.
+// The kernels of the 64x64 tile keep kAbove for that and, in the bits from kUnasked on, how many slabs, this one
+// included, are not asked for zeros (see the loop).  Those of the other tiles have bit 16 + k: the count costs registers
+// that clean slabs of the 32x32 tile (1.4 %) and slabs with specials of the 128x128 tile (0.9 %) then miss.
+enum Word : unsigned { kAbove = 1u << 16, kUnasked = 1u << 17 };
+
+// The word's bits for this thread's staged elements.
 template <class T, int R, int NT, bool KC>
 __device__ __forceinline__ unsigned dirty_lines(const float (&r)[NT * 4], int tid) {
     unsigned lines = 0;
@@ -253,7 +258,7 @@ __device__ __forceinline__ unsigned dirty_lines(const float (&r)[NT * 4], int ti
             const uint32_t m2 = b + b;
             if (m2 - kBandLo2 >= kBandSpan2) {
                 const unsigned bit = 1u << slab_line<T, R, KC>(tid + t * T::kThreads, c);
-                lines |= bit | (m2 >= kBandHi2 ? bit << 16 : 0u);
+                lines |= bit | (m2 >= kBandHi2 ? (T::BM == 64 ? (unsigned)kAbove : bit << 16) : 0u);
             }
         }
     return lines;
@@ -262,6 +267,7 @@ __device__ __forceinline__ unsigned dirty_lines(const float (&r)[NT * 4], int ti
 // Sorts of out-of-band elements in four consecutive words of a staged slab row (`bias` undoes the A side's
 // pre-bias): `zero_kind` for zeros, kOther for the rest.
 enum Kind { kZerosA = 1, kZerosB = 2, kOther = 4 };
+constexpr unsigned kSlabsUnasked = 9;                          // after a slab with others than zeros, itself included
 
 __device__ __forceinline__ unsigned kinds_of(const int4& v, int bias, unsigned zero_kind) {
     unsigned kinds = 0;
@@ -278,13 +284,14 @@ template <int MODE, class T, bool A_KC, bool B_KC, bool VEC>
 __global__ void __launch_bounds__(T::kThreads, MODE == kPam || MODE == kStd ? T::kCtasPerSm : T::kCtasPerSm / 2)
 gemm_kernel(const GemmParams p) {
     constexpr int BM = T::BM, BN = T::BN, BK = T::BK, MT = T::MT;
+    constexpr unsigned kDirty = BM == 64 ? kUnasked - 1u : ~0u;      // of a slab's word: the slab is not clean
     // (the variant with both operands contiguous along their row index spills registers at 8)
     constexpr int kFastUnroll = (!A_KC && !B_KC) || 8 > BK ? BK : 8;
     __shared__ __align__(16) float As[2][BK * row_stride(BM)];
     __shared__ __align__(16) float Bs[2][BK * row_stride(BN)];
     __shared__ __align__(16) float weights[MODE == kPam ? BK * row_stride(BM) : 1];   // of the side that holds zeros
     __shared__ unsigned kinds[3];   // per slab: the sorts of out-of-band elements it holds (Kind), filled where a loop below asks
-    __shared__ unsigned lines[3];   // per slab: bit k = k line holds an out-of-band element, bit 16 + k = one above the band
+    __shared__ unsigned lines[3];   // per slab (Word)
     __shared__ unsigned overflow_lines;   // bit k = some product of k line may leave the pass range
 
     const int tid = threadIdx.x;
@@ -396,7 +403,7 @@ gemm_kernel(const GemmParams p) {
         const float4 w1 = MT == 8 ? *reinterpret_cast<const float4*>(weights + (kk) * row_stride(BM) + (at) * 4 + BM / 2) : w0; \
         const float w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
 
-        if (MODE == kPam && dirty == 0) {
+        if (MODE == kPam && (dirty & kDirty) == 0) {
 #pragma unroll kFastUnroll
             for (int kk = 0; kk < BK; ++kk) {
                 PAMK_FRAGMENTS(kk)
@@ -410,9 +417,11 @@ gemm_kernel(const GemmParams p) {
             // Is everything out of the band a zero?  Looked up here and not while staging, where the registers
             // for it spilled and every dirty slab slowed down by 3 to 7 %.  A slab with elements above the band need
             // not be asked, one with few dirty lines is better off in the runs below (0.1 % zeros: 261 us with
-            // them, 283 us when asked).  The zero-filled lines past the end of K count on both sides.
+            // them, 283 us when asked).  The zero-filled lines past the end of K count on both sides.  Where the
+            // answer was no, the next slabs are not asked (operands of which most values lie below the band:
+            // 4235x1152x67 on the 64x64 tile 85 -> 80 us; 78 us before there was the question).
             unsigned kind = kOther;
-            if (dirty >> 16 == 0 && __popc(dirty) * 4 >= BK * 3) {
+            if (dirty < kAbove && __popc(dirty) * 4 >= BK * 3) {
                 unsigned seen = 0;
 #pragma unroll
                 for (int t = 0; t < T::kTasksA; ++t) {
@@ -425,7 +434,9 @@ gemm_kernel(const GemmParams p) {
                 if ((tid & 31) == 0) atomicOr(&kinds[s % 3], seen);
                 __syncthreads();
                 kind = kinds[s % 3];
+                if (BM == 64 && kind >= kOther) dirty += kSlabsUnasked * kUnasked;
             }
+            if (BM == 64 && tid == 0 && dirty >= 2 * kUnasked) atomicOr(&lines[(s + 1) % 3], (dirty - kUnasked) & ~(kUnasked - 1u));
             if (kind < kOther) {                                // (not 0: the slab is dirty)
                 // Zeros, and everything else in the band (an operand that went through a ReLU).  A pass over one
                 // side's slab replaces each zero by a value that makes the product in-band and writes a weight beside
@@ -493,7 +504,7 @@ gemm_kernel(const GemmParams p) {
             } else {
                 // lines that hold an element above the band: can a product leave the pass range?
                 unsigned full = 0;
-                if (dirty >> 16) {                                  // (uniform: read from shared memory after a barrier)
+                if (dirty & (kDirty & ~all_lines)) {                // (uniform: read from shared memory after a barrier)
                     constexpr int kLanes = T::kThreads / BK;        // threads that share one k line
                     const int line = tid / kLanes, lane = tid % kLanes;
                     if (tid == 0) overflow_lines = 0;
@@ -514,10 +525,13 @@ gemm_kernel(const GemmParams p) {
                     __syncthreads();
                     full = overflow_lines;
                 }
-                if (__popc(dirty & all_lines) * 4 >= BK * 3 && full == 0) {
-                    // most lines dirty, none can overflow (e.g. an operand that is half zeros): "flush or add"
-                    // for the whole slab in one unrolled loop (it is exact for clean lines too)
-#pragma unroll 2
+                // Most lines dirty, none can overflow (e.g. gradients of which most lie below the band): "flush or add"
+                // for the whole slab, which is exact for clean lines too.  The 64x64 tile runs it in the loop for
+                // runs below: with a copy of its own, 512 instructions, its dirty slabs wait for instructions
+                // (2235x183x1152 with 1 % specials 148 -> 109 us; 140 us before the loops for zeros came).
+                const bool flush_all = __popc(dirty & all_lines) * 4 >= BK * 3 && full == 0;
+                if (BM != 64 && flush_all) {
+#pragma unroll (MT == 4 ? 4 : 2)
                     for (int kk = 0; kk < BK; ++kk) {
                         PAMK_FRAGMENTS(kk)
                         float araw[MT];          // a[] holds pre-biased patterns; the rule needs the values
@@ -534,7 +548,7 @@ gemm_kernel(const GemmParams p) {
                 } else {
                     // The lines are walked in runs of one kind, each run by a loop of its own with one copy of
                     // its body (with the three bodies side by side in one loop the schedule cost 12 %).
-                    const unsigned flush = dirty & ~full & all_lines;
+                    const unsigned flush = flush_all ? all_lines : dirty & ~full & all_lines;
                     int kk = 0;
                     while (kk < BK) {
                         const unsigned here = 1u << kk;

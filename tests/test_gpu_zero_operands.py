@@ -42,3 +42,29 @@ def test_zeros_in_an_operand(policy, M, K, N, a_share, b_share, offset, oracle):
     finally:
         pam.set_strict_k_order(False)
         _lib.lib().pamk_test_set_tile_policy(0)
+
+
+@pytest.mark.parametrize("policy", [1, 2, 3], ids=["tile128", "tile64", "tile32"])
+@pytest.mark.parametrize("every", [1, 3, 12])
+def test_slabs_of_zeros_among_slabs_that_hold_others(policy, every, oracle):
+    """After a slab whose many out-of-band elements are not all zeros the next ones are not asked whether theirs are: runs
+    of both sorts, of every length around that count (K is 40 slabs of 16)."""
+    import pam_b200 as pam
+    from pam_b200 import _lib
+    from pam_b200.cuda_bindings import cuda_kernels
+    g = torch.Generator().manual_seed(every)
+    M, K, N = 70, 640, 65
+    A, B = _with_zeros(0.5, g, M, K), _with_zeros(0.0, g, K, N)
+    for first in range(0, K, 16 * every):
+        A[::3, first:first + 16] *= 2.0 ** -64                   # below the band
+    B[::7, :] = torch.where(torch.rand(B[::7].shape, generator=g) < 0.5, 0.0, B[::7])
+    want = oracle.kernels().pam_matmul_fwd(A, B, True, True, 1.0)
+    _lib.check(_lib.lib().pamk_test_set_tile_policy(policy), "tile policy")
+    pam.set_strict_k_order(True)
+    try:
+        for x in (A.cuda(), A.cuda().t().contiguous().t()):
+            for y in (B.cuda(), B.cuda().t().contiguous().t()):
+                assert_bits_equal(cuda_kernels.pam_matmul_fwd(x, y, True, True, 1.0), want)
+    finally:
+        pam.set_strict_k_order(False)
+        _lib.lib().pamk_test_set_tile_policy(0)
