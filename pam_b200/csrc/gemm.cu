@@ -828,6 +828,12 @@ Plan plan_for(int mode, int64_t batch, int64_t M, int64_t N, int64_t K, int spli
     return pl;
 }
 
+// Whether an unsplit launch of `ctas` 32x32 tiles takes slabs of 8 (see TileTinyFine).
+bool fine_slabs(int64_t ctas, int64_t K) {
+    const int64_t tail = K % TileTiny::BK;
+    return ctas > 4 * (int64_t)sm_count() && tail > 0 && tail <= TileTinyFine::BK;
+}
+
 // 0: choose by cost; 1: always the large tile; 2: the 64x64 tile wherever it exists; 3: the 32x32
 // tile wherever it exists (PAM products), else the 64x64 tile.
 int g_tile_policy = 0;
@@ -848,7 +854,13 @@ Plan make_plan(int mode, int64_t batch, int64_t M, int64_t N, int64_t K, int spl
         const int64_t small_tiles = batch * ((M + TileSmall::BM - 1) / TileSmall::BM) * ((N + TileSmall::BN - 1) / TileSmall::BN);
         const bool throughput_bound = small_tiles >= 2 * (int64_t)sm_count() * TileSmall::kCtasPerSm;
         const double margin = throughput_bound || M <= TileTiny::BM || N <= TileTiny::BN ? 0.9 : 0.8;
-        const Plan tiny = plan_for<TileTiny>(mode, batch, M, N, K, split_request);
+        Plan tiny = plan_for<TileTiny>(mode, batch, M, N, K, split_request);
+        // (slabs of 8 are a form of the unsplit launch: planned with the work that they leave, 363 products 47x65x17 stay
+        // on this tile; taken for two slabs of 16 each, they went to the 64x64 tile, 18.5 -> 26.8 us)
+        if (split_request <= 1 && fine_slabs(batch * ((M + TileTiny::BM - 1) / TileTiny::BM) * ((N + TileTiny::BN - 1) / TileTiny::BN), K)) {
+            const Plan fine = plan_for<TileTinyFine>(mode, batch, M, N, K, 1);
+            if (fine.cost < tiny.cost) tiny = fine;
+        }
         if (g_tile_policy == 3 || tiny.cost < margin * best.cost) best = tiny;
     }
     return best;
@@ -883,8 +895,7 @@ int run(int mode, GemmParams p, bool a_kc, bool b_kc, int split_k, void* workspa
     const int bm = pl.tile == kTileTiny ? TileTiny::BM : (pl.tile == kTileSmall ? TileSmall::BM : TileLarge::BM);
     const int bn = pl.tile == kTileTiny ? TileTiny::BN : (pl.tile == kTileSmall ? TileSmall::BN : TileLarge::BN);
     const int64_t ctas = ((p.N + bn - 1) / bn) * (int64_t)((p.M + bm - 1) / bm) * p.batch * pl.splits;
-    const int k_tail = p.K % TileTiny::BK;
-    const bool fine = pl.tile == kTileTiny && pl.splits == 1 && ctas > 4 * (int64_t)sm_count() && k_tail > 0 && k_tail <= TileTinyFine::BK;
+    const bool fine = pl.tile == kTileTiny && pl.splits == 1 && fine_slabs(ctas, p.K);
     const int bk = fine ? TileTinyFine::BK : pl.tile == kTileTiny ? TileTiny::BK : (pl.tile == kTileSmall ? TileSmall::BK : TileLarge::BK);
     if (p.inner < 1) p.inner = 1;
     if (p.ldc == 0) {                                        // plain output: [batch][M][N]

@@ -68,3 +68,27 @@ def test_slabs_of_zeros_among_slabs_that_hold_others(policy, every, oracle):
     finally:
         pam.set_strict_k_order(False)
         _lib.lib().pamk_test_set_tile_policy(0)
+
+
+@pytest.mark.parametrize("K", [5, 8, 17, 24, 21])
+@pytest.mark.parametrize("share", [(0.5, 0.0), (0.0, 0.5), (0.5, 0.5), (0.0, 0.0)])
+def test_many_small_products_whose_k_ends_early_in_a_slab(K, share, oracle):
+    """More than four 32x32 tiles per SM and K just past a multiple of 16: the slabs of 8 of that tile, on zeros and on
+    other out-of-band values."""
+    import pam_b200 as pam
+    from pam_b200 import _lib
+    from pam_b200.cuda_bindings import cuda_kernels
+    g = torch.Generator().manual_seed(K)
+    batch, M, N = 1300, 30, 31
+    A, B = _with_zeros(share[0], g, batch, M, K), _with_zeros(share[1], g, batch, K, N)
+    A.view(-1)[::997], B.view(-1)[::1009] = 1e-30, 1e30
+    want = oracle.kernels().pam_bmm_fwd(A, B, True, True, 1.0552)
+    _lib.check(_lib.lib().pamk_test_set_tile_policy(3), "tile policy")
+    pam.set_strict_k_order(True)
+    try:
+        for x in (A.cuda(), A.cuda().mT.contiguous().mT):
+            for y in (B.cuda(), B.cuda().mT.contiguous().mT):
+                assert_bits_equal(cuda_kernels.pam_bmm_fwd(x, y, True, True, 1.0552), want)
+    finally:
+        pam.set_strict_k_order(False)
+        _lib.lib().pamk_test_set_tile_policy(0)

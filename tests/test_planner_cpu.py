@@ -41,6 +41,7 @@ def test_products_of_one_to_two_waves_are_split_to_shorten_the_last_wave(lib, M,
     (192, 197, 197, 64, 32),                                     # its score products: 224 x 224 instead of 256 x 256 padded
     (512, 32, 32, 128, 32),                                      # attention over 32 tokens
     (8, 160, 197, 64, 32),                                       # a launch that leaves most SMs empty (21.6 -> 9.4 us)
+    (363, 47, 65, 17, 32), (192, 197, 64, 197, 32),              # K just past a slab of 16: slabs of 8 (26.8 -> 18.5 us)
 ])
 def test_tile_choices_that_sweeps_measured_best(lib, batch, M, N, K, tile):
     assert lib.pamk_test_set_tile_policy(0) == 0
