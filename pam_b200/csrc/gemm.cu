@@ -690,10 +690,10 @@ struct OutArg {
 };
 
 // Adds the split-K partials in split order: C = ((P0 + P1) + P2) + ... (+ bias[column] last; then the
-// PAM product with post_scale, if asked for).  W consecutive outputs per thread: 4 where N and the output's
-// strides keep a group of four in one row and 16-byte aligned, else 1.  The partials of a launch sit in L2, so
-// the pass is bound by the latency of its loads: four splits are in flight at a time.  512x512 outputs
-// of 16 ranges 4.5 -> 3.4 us, against one output and one load at a time.
+// PAM product with post_scale, if asked for).  W consecutive outputs per thread, 4 or 1 (see the launch).  The
+// partials of a launch sit in L2 and the pass is bound by its loads: by their bytes for large outputs, where
+// four at a time are faster (2048x2048 of 4 ranges 20.2 -> 12.0 us, 512x512 of 16 4.3 -> 3.7 us), by their latency
+// for small ones, which need every thread.
 template <int W>
 __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restrict__ part, const OutArg o,
                                                             int64_t count, int splits,
@@ -703,7 +703,6 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restr
     const int64_t stride = (int64_t)gridDim.x * blockDim.x * W;
     for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * W; i < count; i += stride) {
         Pack v = *reinterpret_cast<const Pack*>(part + i);
-#pragma unroll 4
         for (int s = 1; s < splits; ++s) {
             const Pack u = *reinterpret_cast<const Pack*>(part + (int64_t)s * count + i);
 #pragma unroll
@@ -948,8 +947,11 @@ int run(int mode, GemmParams p, bool a_kc, bool b_kc, int split_k, void* workspa
             break;
     }
     if (rc != PAMK_OK || pl.splits == 1) return rc;
-    // (the partials are 256-byte aligned; count = batch * M * N is then a multiple of 4 too)
-    const bool wide = ((out.N | out.ldc | out.sCb | out.sCb2) & 3) == 0 && aligned16(out.C);
+    // Four outputs per thread where there are enough of them (400x512 of 20 ranges 3.8 us with one, 4.1 with four; 192x192
+    // of 64 ranges 4.9 and 7.4; for more see the kernel) and where N and the output's strides keep a group of
+    // four in one row and 16-byte aligned.  (The partials are 256-byte aligned; count = batch * M * N is then a
+    // multiple of 4 too.)
+    const bool wide = count >= 1536 * (int64_t)sm_count() && ((out.N | out.ldc | out.sCb | out.sCb2) & 3) == 0 && aligned16(out.C);
     const int threads = wide ? 128 : 256;
     const int64_t blocks = (count / (wide ? 4 : 1) + threads - 1) / threads;
     const int64_t cap = (int64_t)sm_count() * (2048 / threads);

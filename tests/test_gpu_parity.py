@@ -868,3 +868,21 @@ def test_layer_norm_backward_from_saved_row_scalars(pam, dev, width, affine):
         assert_close_nan(db1, db0, 1e-5, 1e-5 * float(db0.nan_to_num().abs().max()), "dbias")
         if affine:      # (without eps the constant row's NaN reaches every column of dweight, on both sides)
             assert_close_nan(dw1, dw0, 1e-5, 1e-5 * float(dw0.nan_to_num().abs().max()), "dweight")
+
+
+@pytest.mark.parametrize("M,N", [(443, 512), (444, 512), (512, 446), (3, 8), (2, 5)])
+@pytest.mark.parametrize("biased", [False, True])
+def test_split_k_partials_are_added_in_range_order(pam, dev, M, N, biased):
+    """Against the ranges' products added one after the other, bit for bit, around the size from which the reduction takes four
+    outputs per thread (1536 for each of 148 SMs)."""
+    from pam_b200 import _lib, cuda_bindings as cb
+    g = torch.Generator().manual_seed(M)
+    A, B, b = torch.randn(M, 96, generator=g).to(dev), torch.randn(96, N, generator=g).to(dev), torch.randn(N, generator=g).to(dev)
+    _lib.check(_lib.lib().pamk_test_set_tile_policy(1), "tile policy")
+    try:
+        got = cb._matmul(_lib.MUL_PAM, A, B, 1.0, 2, split_k=3, bias=b if biased else None)
+        parts = [cb._matmul(_lib.MUL_PAM, A[:, k:k + 32], B[k:k + 32], 1.0, 2, split_k=1) for k in (0, 32, 64)]
+    finally:
+        _lib.lib().pamk_test_set_tile_policy(0)
+    want = (parts[0] + parts[1]) + parts[2]
+    assert_bits_equal(got, want + b if biased else want)
