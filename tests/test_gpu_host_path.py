@@ -7,7 +7,7 @@ import torch
 
 import pam_b200 as pam
 from conftest import assert_bits_equal
-from pam_b200 import _lib, optim
+from pam_b200 import _lib, fused, optim
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -70,8 +70,9 @@ def test_elementwise_broadcasts(op, approx):
 @pytest.mark.parametrize("rows,fin,fout", [(1, 64, 64), (32, 130, 67), (197, 192, 96)])
 def test_linear_and_products(approx, rows, fin, fout):
     x, w, b = randn(rows, fin), randn(fout, fin, seed=2), randn(fout, seed=3)
-    pam.set_strict_k_order(True)          # (the weight gradient is formed as [out, in] here and as [in, out] there)
-    try:
+    # (the weight gradient is formed as [out, in] here and as [in, out] there: plans and sums are the same either way)
+    for strict in (False, True):
+        pam.set_strict_k_order(strict)
         both(lambda x, w, b: pam.linear(x, w, b, approx_bwd=approx), x, w, b)
         both(lambda x, w: pam.linear(x, w, approx_bwd=approx), x, w)
         both(lambda x, w, b: pam.linear(x[None].expand(3, -1, -1), w, b, approx_bwd=approx), x, w, b)
@@ -80,8 +81,12 @@ def test_linear_and_products(approx, rows, fin, fout):
         both(lambda x, w: pam.matmul(x, w, approx_bwd=(approx, not approx)), x, randn(fin, fout, seed=2))
         both(lambda x, y: pam.bmm(x, y.mT, approx_bwd=approx), randn(3, rows, fin), randn(3, fout, fin, seed=2))
         both(lambda x, y: pam.bmm(x, y, approx_bwd=approx), randn(3, rows, 9)[:, :, ::2], randn(3, 5, fout, seed=2))
-    finally:
-        pam.set_strict_k_order(False)
+
+
+@pytest.fixture(autouse=True)
+def default_k_order():
+    yield
+    pam.set_strict_k_order(False)
 
 
 @pytest.mark.parametrize("approx", [True, False])
@@ -93,6 +98,22 @@ def test_rows(approx):
     both(lambda x: pam.layer_norm(x.transpose(0, 1), (65,), approx_bwd=approx), x)
     both(lambda x: pam.softmax(x, dim=-1, approx_bwd=approx), x)
     both(lambda x: pam.softmax(x.transpose(0, 1), dim=2, approx_bwd=approx), x)
+
+
+@pytest.mark.parametrize("T,S,heads,hd", [(1, 1, 1, 1), (5, 7, 2, 3), (33, 17, 3, 8), (64, 130, 1, 64)])
+@pytest.mark.parametrize("offset", [None, 1.0552])
+def test_attention(T, S, heads, hd, offset):
+    d = heads * hd
+    for qkv in (randn(2, T, 3 * d, specials=False), randn(T, 2, 3 * d, specials=False).transpose(0, 1)):
+        both(lambda t: fused.attention_qkv(t, heads, hd ** -0.5, offset=offset), qkv)
+        with route(False):
+            y = fused.attention_qkv(qkv, heads, hd ** -0.5, offset=offset)        # (no gradient: nothing is kept)
+        with route(True):
+            assert_bits_equal(y, fused.attention_qkv(qkv, heads, hd ** -0.5, offset=offset))
+    causal = torch.full((T, S), float("-inf"), device=DEV).triu(1 + max(S - T, 0))
+    for mask in (None, causal, randn(2 * heads, T, S, seed=6, specials=False)):
+        both(lambda q, k, v: fused.attention_heads(q, k, v, heads, mask, offset=offset), randn(2, T, d, specials=False),
+             randn(2, S, d, seed=2, specials=False), randn(S, 2, d, seed=3, specials=False).transpose(0, 1))
 
 
 def test_adam_groups_and_fallbacks():
