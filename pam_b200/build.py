@@ -20,6 +20,7 @@ CSRC = PKG / "csrc"
 OBJ = PKG / "build"
 LIB = PKG / "libpam_b200.so"
 HOST = PKG / "_host.so"
+HOST_STAMP = OBJ / "host_platform.txt"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -38,13 +39,24 @@ def _stale(target, deps):
     return not target.exists() or any(d.stat().st_mtime > target.stat().st_mtime for d in deps)
 
 
+def _host_platform():
+    """What the host module's binary depends on beside its sources: torch's C++ ABI and Python's."""
+    import torch
+    return f"torch {torch.__version__}, Python {sys.version_info.major}.{sys.version_info.minor}"
+
+
+def host_stale():
+    return (_stale(HOST, [CSRC / "host.cpp", PKG.parent / "include" / "pam_b200.h", pathlib.Path(__file__)])
+            or not HOST_STAMP.exists() or HOST_STAMP.read_text() != _host_platform())
+
+
 def build_host(force=False, verbose=False):
     """The CPython module with the operators' host path: plain C++, no device code."""
     import sysconfig
 
     import torch
     src = CSRC / "host.cpp"
-    if not force and not _stale(HOST, [src, PKG.parent / "include" / "pam_b200.h", pathlib.Path(__file__)]):
+    if not force and not host_stale():
         return HOST
     root = pathlib.Path(torch.__file__).resolve().parent
     cuda = pathlib.Path(_nvcc()).resolve().parents[1] / "include"
@@ -57,6 +69,8 @@ def build_host(force=False, verbose=False):
         sys.stderr.write(res.stdout + res.stderr)
     if res.returncode:
         raise RuntimeError("g++ failed: " + " ".join(cmd))
+    OBJ.mkdir(exist_ok=True)
+    HOST_STAMP.write_text(_host_platform())
     return HOST
 
 

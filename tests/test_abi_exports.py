@@ -58,3 +58,14 @@ def test_nvtx_wrapper_marks_only_entry_points_that_launch():
     finally:
         _lib.set_nvtx(False)
     assert _lib.lib() is plain
+
+
+def test_host_module_is_rebuilt_for_another_torch(monkeypatch, tmp_path):
+    from pam_b200 import build
+    monkeypatch.setattr(build, "_stale", lambda target, deps: False)
+    monkeypatch.setattr(build, "HOST_STAMP", tmp_path / "stamp")
+    assert build.host_stale()
+    build.HOST_STAMP.write_text(build._host_platform())
+    assert not build.host_stale()
+    build.HOST_STAMP.write_text("torch 0.0, Python 3.0")
+    assert build.host_stale()
