@@ -194,6 +194,30 @@ def _ordinary_call(device):
                 or torch._C._len_torch_dispatch_stack() or (device.type == "cuda" and torch.cuda.is_current_stream_capturing()))
 
 
+def _kept(module, name, length, device, make, cut):
+    """A constant table for sequences of `length`: `cut` of the one that `module` keeps, on each device, for the longest
+    sequence so far (to the next power of two), made by `make`."""
+    if not _ordinary_call(device):
+        return cut(make(length, device), length)
+    tables = module.__dict__.setdefault("_kept_tables", {})
+    stream = torch._C._cuda_getCurrentRawStream(device.index) if device.type == "cuda" else None
+    entry = tables.get((name, device))                       # (stream that made it, table, last length, its cut)
+    if entry is None or entry[1].device != device:
+        entry = (stream, None, 0, None)
+    owner, table, last, view = entry
+    if table is not None and stream != owner:
+        table.record_stream(torch.cuda.current_stream(device))    # (a longer one may replace it while the stream still reads it)
+    if last != length:
+        with torch.inference_mode(False):
+            if table is None or table.shape[0] < length:
+                owner, table = stream, make(1 << (length - 1).bit_length(), device)
+                if stream is not None:
+                    torch.cuda.current_stream(device).synchronize()      # (other streams use it without waiting for this one)
+            view = cut(table, length)
+        tables[name, device] = (owner, table, length, view)
+    return view
+
+
 class _Stack(nn.Module):
     def __init__(self, cfg, layers, cross, linear_factory, norm_layer, op_dict):
         super().__init__()
@@ -203,20 +227,14 @@ class _Stack(nn.Module):
         self.layers = nn.ModuleList([TransformerLayer(cfg, cross, linear_factory, norm_layer, op_dict) for _ in range(layers)])
 
     def _positions(self, length, device):
-        """The first `length` rows of the sinusoidal table.  Making them takes the host and a copy that waits, so the
-        table is kept, on each device, for the longest sequence so far (to the next power of two)."""
-        if not _ordinary_call(device):
-            return sinusoidal_positions(length, self.cfg.dim, self.cfg.pad, device)
-        tables = self.__dict__.setdefault("_position_tables", {})
-        stream = torch.cuda.current_stream(device) if device.type == "cuda" else None
-        owner, table = tables.get(device, (None, None))
-        if table is None or table.shape[0] < length or table.device != device:
-            with torch.inference_mode(False):
-                table = sinusoidal_positions(1 << (length - 1).bit_length(), self.cfg.dim, self.cfg.pad, device)
-            tables[device] = (stream and stream.cuda_stream, table)
-        elif stream and stream.cuda_stream != owner:
-            table.record_stream(stream)          # (a longer table may replace this one while the stream still reads it)
-        return table[:length]
+        """The first rows of the sinusoidal table, which take the host and a copy that waits to make."""
+        return _kept(self, "positions", length, device, lambda n, d: sinusoidal_positions(n, self.cfg.dim, self.cfg.pad, d),
+                     lambda table, n: table[:n])
+
+    def _future(self, length, device):
+        """-inf above the diagonal."""
+        return _kept(self, "future", length, device, lambda n, d: torch.full((n, n), float("-inf"), device=d).triu(1),
+                     lambda table, n: table[:n, :n])
 
     def embed(self, tokens):
         x = self.op_dict["mul"](self.embed_scale, self.embed_tokens(tokens))
@@ -244,8 +262,7 @@ class Transformer(nn.Module):
         x = self.encoder.embed(src)
         for layer in self.encoder.layers:
             x = layer(x)
-        T = prev_out.shape[1]
-        future = torch.full((T, T), float("-inf"), device=src.device).triu(1)
+        future = self.decoder._future(prev_out.shape[1], src.device)
         y = self.decoder.embed(prev_out)
         for layer in self.decoder.layers:
             y = layer(y, x, future)

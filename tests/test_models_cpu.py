@@ -80,6 +80,7 @@ def test_kept_position_table(monkeypatch):
         got = stack._positions(length, cpu)
         assert not got.is_inference()
         assert_bits_equal(got, steps.sinusoidal_positions(length, TRANSFORMER.dim, TRANSFORMER.pad, cpu), str(length))
+        assert torch.equal(stack._future(length, cpu), torch.full((length, length), float("-inf")).triu(1))
     assert made == [4, 8, 16]
 
     torch.func.grad(lambda t: (t * stack._positions(20, cpu)[0, 0]).sum())(torch.ones(2))
@@ -87,5 +88,5 @@ def test_kept_position_table(monkeypatch):
         stack._positions(21, cpu)
     assert made == [4, 8, 16, 20, 21] and type(stack._positions(16, cpu)) is torch.Tensor and len(made) == 5
 
-    del stack.__dict__["_position_tables"]                        # a model that was saved before there was one
+    del stack.__dict__["_kept_tables"]                        # a model that was saved before there was one
     assert stack._positions(2, cpu).shape[0] == 2
