@@ -61,17 +61,18 @@ __device__ __forceinline__ bool field_in(int32_t bits) {
     return b + b - 2u * (LO << 23) < 2u * ((HI - LO) << 23);
 }
 
+// Whether the rule without its range rules (below) may be tried on these.
+__device__ __forceinline__ bool ordinary(float g, float m, float v) {
+    return field_in<66, 188>(f2i(g)) && field_in<27, 227>(f2i(m)) && field_in<27, 227>(f2i(v));
+}
+
 // The rule without its range rules, for values of ordinary magnitude; false (and nothing changed) where one of
-// them might apply.  A primitive is then one integer add: a product of factors in [2^-61, 2^61), or of one in
+// them might apply after all.  A primitive is one integer add: a product of factors in [2^-61, 2^61), or of one in
 // [2^-100, 2^100) and a scalar in [2^-20, 2^20], passes the range rule, and so does such a quotient.  floor(log2f(x))
 // is the exponent of x unless the mantissa lies so close to either end that log2f might round across
 // the power of two (it is off by a few ulp, at most 2^-15 for exponents up to 128; the ends taken are 2^-11 wide).
-//
-// The kernel is bound by its instructions, five or six per primitive with the range rule and more for the division
-// and log2f that only classify.  42 M parameters: 281 -> 260 us (4.5 TB/s).
 __device__ __forceinline__ bool adam_plain(float& p, float g, float& m, float& v, const AdamScalars& s) {
     const int32_t gb = f2i(g), mb = f2i(m), vb = f2i(v), bias = kBias - s.off;
-    if (!(field_in<66, 188>(gb) && field_in<27, 227>(mb) && field_in<27, 227>(vb))) return false;
     const int32_t gg = isub(iadd(gb, gb), bias);
     const float m1 = fadd(i2f(iadd(mb, isub(f2i(s.b1), bias))), i2f(iadd(gb, isub(f2i(s.one_minus_b1), bias))));
     const float v1 = fadd(i2f(iadd(vb, isub(f2i(s.b2), bias))), i2f(iadd(gg, isub(f2i(s.one_minus_b2), bias))));
@@ -88,18 +89,26 @@ __device__ __forceinline__ bool adam_plain(float& p, float g, float& m, float& v
                     (uint32_t)(mant - 0x1000) < 0x7fe000u && fabsf(x) > 0x1p-20f &&
                     field_in<66, 188>(f2i(m1)) && field_in<66, 188>(f2i(den)) && field_in<66, 188>(d);
     if (!ok) return false;
-    float q = p;
-    if (s.decay != 0.0f) q = fadd(q, -mul(q, s.decay, s.off));
-    p = fadd(q, -i2f(iadd(d, isub(f2i(s.step_size), bias))));
+    if (s.decay != 0.0f) p = fadd(p, -mul(p, s.decay, s.off));
+    p = fadd(p, -i2f(iadd(d, isub(f2i(s.step_size), bias))));
     m = m1;
     v = v1;
     return true;
 }
 
-__device__ __forceinline__ void adam_any(float& p, float g, float& m, float& v, const AdamScalars& s, float lb2) {
-    if (!(s.plain && adam_plain(p, g, m, v, s))) adam_one(p, g, m, v, s, lb2);
+// One element of each thread in `mask`, by one rule for all of them; the few whose values in between turn out not to be
+// ordinary take the full rule after the short one.
+__device__ __forceinline__ void adam_any(float& p, float g, float& m, float& v, const AdamScalars& s, float lb2, unsigned mask) {
+    bool done = s.plain && __all_sync(mask, ordinary(g, m, v));
+    if (done) done = adam_plain(p, g, m, v, s);
+    if (!done) adam_one(p, g, m, v, s, lb2);
 }
 
+// Four elements per thread.  With the full rule the kernel is bound by its instructions, five or six per primitive and more
+// for the division and log2f that only classify (2^25 elements 192 us); without the range rules by DRAM (150 us).
+// The 32 elements that a warp works on at a time take one of the two together, by a vote on the inputs: where each
+// thread chose for itself, zeros among the gradients (rows of an embedding that no token met, units behind
+// a ReLU) made the warp run both (one zero in ten: 365 us, now 198).
 __global__ void __launch_bounds__(kThreads) adam_kernel(const AdamTable t, const AdamScalars s) {
     int which = 0, hi = t.used;                    // largest k with first[k] <= blockIdx.x (the same for the whole CTA)
     while (hi - which > 1) {
@@ -117,24 +126,29 @@ __global__ void __launch_bounds__(kThreads) adam_kernel(const AdamTable t, const
     const bool vec = ((reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(g) |
                        reinterpret_cast<uintptr_t>(m) | reinterpret_cast<uintptr_t>(v)) & 15u) == 0;
     const int64_t i = base + threadIdx.x * 4;
-    if (vec && i + 3 < n) {
+    const bool four = vec && i + 3 < n;
+    const unsigned fours = __ballot_sync(0xffffffffu, four);          // (every thread of the CTA is here)
+    if (four) {
         float4 p4 = *reinterpret_cast<const float4*>(p + i);
         const float4 g4 = __ldg(reinterpret_cast<const float4*>(g + i));
         float4 m4 = *reinterpret_cast<const float4*>(m + i);
         float4 v4 = *reinterpret_cast<const float4*>(v + i);
-        adam_any(p4.x, g4.x, m4.x, v4.x, s, lb2);
-        adam_any(p4.y, g4.y, m4.y, v4.y, s, lb2);
-        adam_any(p4.z, g4.z, m4.z, v4.z, s, lb2);
-        adam_any(p4.w, g4.w, m4.w, v4.w, s, lb2);
+        adam_any(p4.x, g4.x, m4.x, v4.x, s, lb2, fours);
+        adam_any(p4.y, g4.y, m4.y, v4.y, s, lb2, fours);
+        adam_any(p4.z, g4.z, m4.z, v4.z, s, lb2, fours);
+        adam_any(p4.w, g4.w, m4.w, v4.w, s, lb2, fours);
         *reinterpret_cast<float4*>(p + i) = p4;
         *reinterpret_cast<float4*>(m + i) = m4;
         *reinterpret_cast<float4*>(v + i) = v4;
     } else {
-#pragma unroll
+#pragma unroll 1
         for (int c = 0; c < 4; ++c) {
-            if (i + c < n) {
+            const bool on = i + c < n;
+            const unsigned ons = __ballot_sync(~fours, on);
+            if (on) {
                 float pp = p[i + c], mm = m[i + c], vv = v[i + c];
-                adam_any(pp, g[i + c], mm, vv, s, lb2);
+                const float gg = g[i + c];
+                adam_any(pp, gg, mm, vv, s, lb2, ons);
                 p[i + c] = pp;
                 m[i + c] = mm;
                 v[i + c] = vv;

@@ -32,3 +32,30 @@ def test_adam_step_at_every_magnitude(lo, hi, lr, decay, betas, oracle):
     want = oracle.adam_step(p.clone(), grad, m.clone(), v.clone(), step=10, lr=lr, betas=betas, eps=1e-8, weight_decay=decay)
     for got, w, what in zip((param.detach(), opt.state[param]["exp_avg"], opt.state[param]["exp_avg_sq"]), want, "pmv"):
         assert_bits_equal(got, w, what)
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 127, 128, 129, 1024, 4099])
+@pytest.mark.parametrize("aligned", [True, False])
+@pytest.mark.parametrize("zeros", ["none", "one", "rows", "tenth", "all"])
+def test_adam_step_where_gradients_are_zero(n, aligned, zeros, oracle):
+    """A warp (128 elements) takes the rule without range rules or the full one as a whole: gradients without zeros, with one, with
+    blocks of zeros (and moments that were never touched), zeros everywhere between; edges of a warp and of a block."""
+    from pam_b200 import optim
+    g = torch.Generator().manual_seed(n)
+    p, grad, m, v = (torch.randn(n, generator=g) * s for s in (0.04, 1e-3, 1e-4, 1e-3))
+    v = v.square()
+    zero = {"none": torch.zeros(n), "one": torch.arange(n) == n // 2, "rows": torch.arange(n) // 512 % 2,
+            "tenth": torch.rand(n, generator=g) < 0.1, "all": torch.ones(n)}[zeros].bool()
+    grad[zero] = 0.0
+    if zeros == "rows":
+        m[zero], v[zero] = 0.0, 0.0
+    first = 0 if aligned else 1
+    own = lambda t: torch.cat([torch.zeros(first), t]).cuda()[first:]          # (a float past a 16-byte boundary)
+    param = torch.nn.Parameter(own(p))
+    param.grad = own(grad)
+    opt = optim.Adam([param], lr=5e-4, betas=(0.9, 0.98), eps=1e-8, weight_decay=0.05, opt_functional_cfg="pam")
+    opt.state[param] = {"step": 9, "exp_avg": own(m), "exp_avg_sq": own(v)}
+    opt.step()
+    want = oracle.adam_step(p.clone(), grad, m.clone(), v.clone(), step=10, lr=5e-4, betas=(0.9, 0.98), eps=1e-8, weight_decay=0.05)
+    for got, w, what in zip((param.detach(), opt.state[param]["exp_avg"], opt.state[param]["exp_avg_sq"]), want, "pmv"):
+        assert_bits_equal(got, w, what)
