@@ -280,6 +280,21 @@ __device__ __forceinline__ unsigned kinds_of(const int4& v, int bias, unsigned z
     return kinds;
 }
 
+// ---- two sums in one instruction ----------------------------------------------------------------------------------
+// acc0 += p0, acc1 += p1 and acc0 = p0 * w0 + acc0, acc1 = p1 * w1 + acc1, each with the one rounding of its scalar form.
+// The packed add does not double the adds per cycle (register-only: 16.7 T pairs of one integer and one packed half against
+// 16.3 T), but it halves the adds that the scheduler has to issue: 4096^3 4848 -> 4562 us, 4096x512x512 101.8 -> 96.7 us,
+// with zeros in one operand 133 -> 125 us; the 64x64 and 32x32 tiles, which issue more beside the adds, gain 0 to 2 %.
+__device__ __forceinline__ void add_pair(float& acc0, float& acc1, int p0, int p1) {
+    asm("{ .reg .b64 s, t;\n mov.b64 s, {%0, %1};\n mov.b64 t, {%2, %3};\n add.rn.f32x2 s, s, t;\n mov.b64 {%0, %1}, s; }"
+        : "+f"(acc0), "+f"(acc1) : "r"(p0), "r"(p1));
+}
+__device__ __forceinline__ void fma_pair(float& acc0, float& acc1, int p0, int p1, float w0, float w1) {
+    asm("{ .reg .b64 s, t, w;\n mov.b64 s, {%0, %1};\n mov.b64 t, {%2, %3};\n mov.b64 w, {%4, %5};\n"
+        " fma.rn.f32x2 s, t, w, s;\n mov.b64 {%0, %1}, s; }"
+        : "+f"(acc0), "+f"(acc1) : "r"(p0), "r"(p1), "f"(w0), "f"(w1));
+}
+
 template <int MODE, class T, bool A_KC, bool B_KC, bool VEC>
 __global__ void __launch_bounds__(T::kThreads, MODE == kPam || MODE == kStd ? T::kCtasPerSm : T::kCtasPerSm / 2)
 gemm_kernel(const GemmParams p) {
@@ -410,7 +425,7 @@ gemm_kernel(const GemmParams p) {
 #pragma unroll
                 for (int i = 0; i < MT; ++i)
 #pragma unroll
-                    for (int j = 0; j < MT; ++j) acc[i][j] = fadd(acc[i][j], i2f(iadd(a[i], b[j])));
+                    for (int j = 0; j < MT; j += 2) add_pair(acc[i][j], acc[i][j + 1], iadd(a[i], b[j]), iadd(a[i], b[j + 1]));
             }
         } else if constexpr (MODE == kPam) {
             constexpr unsigned all_lines = (1u << BK) - 1u;
@@ -488,7 +503,7 @@ gemm_kernel(const GemmParams p) {
 #pragma unroll
                         for (int i = 0; i < MT; ++i)
 #pragma unroll
-                            for (int j = 0; j < MT; ++j) acc[i][j] = __fmaf_rn(i2f(iadd(a[i], b[j])), w[i], acc[i][j]);
+                            for (int j = 0; j < MT; j += 2) fma_pair(acc[i][j], acc[i][j + 1], iadd(a[i], b[j]), iadd(a[i], b[j + 1]), w[i], w[i]);
                     }
                 } else {
 #pragma unroll 1
@@ -498,7 +513,7 @@ gemm_kernel(const GemmParams p) {
 #pragma unroll
                         for (int i = 0; i < MT; ++i)
 #pragma unroll
-                            for (int j = 0; j < MT; ++j) acc[i][j] = __fmaf_rn(i2f(iadd(a[i], b[j])), w[j], acc[i][j]);
+                            for (int j = 0; j < MT; j += 2) fma_pair(acc[i][j], acc[i][j + 1], iadd(a[i], b[j]), iadd(a[i], b[j + 1]), w[j], w[j + 1]);
                     }
                 }
             } else {
@@ -592,7 +607,7 @@ gemm_kernel(const GemmParams p) {
 #pragma unroll
                                 for (int i = 0; i < MT; ++i)
 #pragma unroll
-                                    for (int j = 0; j < MT; ++j) acc[i][j] = fadd(acc[i][j], i2f(iadd(a[i], b[j])));
+                                    for (int j = 0; j < MT; j += 2) add_pair(acc[i][j], acc[i][j + 1], iadd(a[i], b[j]), iadd(a[i], b[j + 1]));
                             }
                         }
                     }
