@@ -72,10 +72,12 @@ struct GemmParams {
 //   128x128x16, 256 threads, 2 CTAs/SM: least staging overhead, for large outputs;
 //   64x64x8,     64 threads, 8 CTAs/SM: four times as many CTAs, for outputs that would leave a
 //                                       large tile grid with a ragged last wave (e.g. 12608 x 192).
-template <int BM_, int BN_, int BK_, int CPS_, int MT_ = 8>
+template <int BM_, int BN_, int BK_, int CPS_, int MT_ = 8, int MR_ = MT_>
 struct Tile {
-    // every thread owns an MT x MT micro-tile (8, or 4 for the tile meant for very small outputs)
-    static constexpr int BM = BM_, BN = BN_, BK = BK_, MT = MT_, kCtasPerSm = CPS_;
+    // every thread owns an MR x MT micro-tile (8, or 4 for the tile meant for very small outputs; MR below MT leaves
+    // the last row slots of every thread empty)
+    static constexpr int BM = BM_, BN = BN_, BK = BK_, MT = MT_, MR = MR_, kCtasPerSm = CPS_;
+    static constexpr int kRows = BM_ / MT_ * MR_;      // rows of the output that a tile covers
     static constexpr int kThreads = (BM_ / MT_) * (BN_ / MT_);
     static constexpr int TX = BN_ / MT_;
     // float4 tasks per thread when staging one operand slab
@@ -84,6 +86,12 @@ struct Tile {
     static constexpr int kRowsPerWarp = 32 / (BK_ / 4);
 };
 using TileLarge = Tile<128, 128, 16, 2>;
+// 112x128x16: the large tile with seven rows per thread, for products of few large tiles per SM whose number then fits
+// the SMs better (4096 rows x 512: 128 tiles of 128 rows leave 20 of 148 SMs idle, 148 tiles of 112 none; one CTA of
+// this size already runs an SM at 95 % of what two do).  Row slot 7 of every thread is staged with a copy of a neighbouring row and
+// takes no part in the sums.  4096x512x512 96.6 us (two K ranges and their reduction) -> 83.3, 4096x1024x512 174.5 -> 153.4,
+// 2000x1024x512 96.7 -> 83.4; of 94 products of all sizes those that get it gain 4 to 14 %.
+using TileLarge7 = Tile<128, 128, 16, 2, 8, 7>;
 using TileSmall = Tile<64, 64, 8, 8>;
 // 32x32x16 with a 4x4 micro-tile, 64 threads: batched products whose matrices are a fraction of a
 // 64x64 tile (attention over 32 tokens) would otherwise spend three quarters of their adds on
@@ -101,6 +109,16 @@ using TileTiny = Tile<32, 32, 16, 12, 4>;
 // that the arithmetic loops carry no address computation (an XOR swizzle measured the same speed
 // with more instructions and a few spilled registers).
 __host__ __device__ constexpr int row_stride(int R) { return R + 4; }
+
+// Row of the tile that is staged in row slot `slot`: a thread's slots are ty * 4 + (0..3) and R / 2 + ty * 4 + (0..3), of
+// which the last MT - MR are empty.  Identity for MR = MT.
+template <class T, int R>
+__host__ __device__ constexpr int slot_row(int slot) {
+    constexpr int kSecond = T::MR - 4;                 // rows of a thread's second group of slots
+    if (T::MR == T::MT || slot < R / 2) return slot;
+    const int in = slot - R / 2;
+    return R / 2 + in / 4 * kSecond + (in % 4 < kSecond ? in % 4 : kSecond - 1);
+}
 
 // ---- loaders: global -> registers ---------------------------------------------------------------
 // A slab is R rows x BK k, staged as float4 "tasks"; thread t takes tasks t, t + kThreads, ...
@@ -156,13 +174,15 @@ struct SlabWalker {
     const float* ptr[NT];
     int64_t step;                                    // elements to advance per slab
 
+    template <bool MAPPED>
     __device__ __forceinline__ void init(const MatArg& m, const float* base, int row0, int rows, int k_begin, int tid) {
+        static_assert(KC || !MAPPED, "four consecutive rows have to lie in four consecutive slots");
         step = KC ? (int64_t)T::BK : (int64_t)T::BK * m.sk;
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
             const int id = tid + t * T::kThreads;
             if (KC) {
-                int row = row0 + id / (T::BK / 4);
+                int row = row0 + (MAPPED ? slot_row<T, R>(id / (T::BK / 4)) : id / (T::BK / 4));
                 row = row < rows ? row : rows - 1;
                 ptr[t] = base + (int64_t)row * m.sr + k_begin + (id % (T::BK / 4)) * 4;
             } else {
@@ -298,7 +318,8 @@ __device__ __forceinline__ void fma_pair(float& acc0, float& acc1, int p0, int p
 template <int MODE, class T, bool A_KC, bool B_KC, bool VEC>
 __global__ void __launch_bounds__(T::kThreads, MODE == kPam || MODE == kStd ? T::kCtasPerSm : T::kCtasPerSm / 2)
 gemm_kernel(const GemmParams p) {
-    constexpr int BM = T::BM, BN = T::BN, BK = T::BK, MT = T::MT;
+    constexpr int BM = T::BM, BN = T::BN, BK = T::BK, MT = T::MT, MR = T::MR;
+    static_assert(MR == MT || (MODE == kPam && A_KC && VEC), "fewer rows per thread: products with A contiguous along K alone");
     constexpr unsigned kDirty = BM == 64 ? kUnasked - 1u : ~0u;      // of a slab's word: the slab is not clean
     // (the variant with both operands contiguous along their row index spills registers at 8)
     constexpr int kFastUnroll = (!A_KC && !B_KC) || 8 > BK ? BK : 8;
@@ -311,7 +332,7 @@ gemm_kernel(const GemmParams p) {
 
     const int tid = threadIdx.x;
     const int tx = tid % T::TX, ty = tid / T::TX;
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    const int m0 = blockIdx.y * T::kRows, n0 = blockIdx.x * BN;
     const int z = blockIdx.z / p.splits, sp = blockIdx.z - z * p.splits;
     const int k_begin = sp * p.k_chunk;
     const int k_end = min(p.K, k_begin + p.k_chunk);
@@ -324,19 +345,19 @@ gemm_kernel(const GemmParams p) {
     const float* Ab = p.A.p + (int64_t)zo * p.A.sb + (int64_t)z * p.A.sb2;
     const float* Bb = p.B.p + (int64_t)zo * p.B.sb + (int64_t)z * p.B.sb2;
 
-    float acc[MT][MT];
+    float acc[MR][MT];
 #pragma unroll
-    for (int i = 0; i < MT; ++i)
+    for (int i = 0; i < MR; ++i)
 #pragma unroll
         for (int j = 0; j < MT; ++j) acc[i][j] = 0.0f;
 
     // exact-gradient product: per-output constant (mantissa of D + offset) that the slope adds to
     // the other operand's bits (pam_scalar.cuh mul_slope).
-    int32_t dm[MODE >= kBwdL ? MT : 1][MODE >= kBwdL ? MT : 1];
+    int32_t dm[MODE >= kBwdL ? MR : 1][MODE >= kBwdL ? MT : 1];
     if constexpr (MODE >= kBwdL) {
         const float* Db = p.D + (int64_t)z * p.sDb;
 #pragma unroll
-        for (int i = 0; i < MT; ++i) {
+        for (int i = 0; i < MR; ++i) {
             int row = m0 + ty * 4 + (i & 3) + (i >> 2) * (BM / 2);
             row = row < p.M ? row : p.M - 1;
 #pragma unroll
@@ -354,8 +375,8 @@ gemm_kernel(const GemmParams p) {
     SlabWalker<T, BM, T::kTasksA, A_KC> walk_a;
     SlabWalker<T, BN, T::kTasksB, B_KC> walk_b;
     if constexpr (VEC) {
-        walk_a.init(p.A, Ab, m0, p.M, k_begin, tid);
-        walk_b.init(p.B, Bb, n0, p.N, k_begin, tid);
+        walk_a.template init<T::MR != T::MT>(p.A, Ab, m0, p.M, k_begin, tid);
+        walk_b.template init<false>(p.B, Bb, n0, p.N, k_begin, tid);
     }
     auto stage_load = [&](int k0) {
         if constexpr (VEC) {
@@ -423,7 +444,7 @@ gemm_kernel(const GemmParams p) {
             for (int kk = 0; kk < BK; ++kk) {
                 PAMK_FRAGMENTS(kk)
 #pragma unroll
-                for (int i = 0; i < MT; ++i)
+                for (int i = 0; i < MR; ++i)
 #pragma unroll
                     for (int j = 0; j < MT; j += 2) add_pair(acc[i][j], acc[i][j + 1], iadd(a[i], b[j]), iadd(a[i], b[j + 1]));
             }
@@ -491,7 +512,7 @@ gemm_kernel(const GemmParams p) {
                         for (int j = 0; j < MT; ++j) {
                             const bool on = 2u * (uint32_t)b[j] != 0;
 #pragma unroll
-                            for (int i = 0; i < MT; ++i)
+                            for (int i = 0; i < MR; ++i)
                                 if (on) acc[i][j] = __fmaf_rn(i2f(iadd(a[i], b[j])), w[i], acc[i][j]);
                         }
                     }
@@ -501,7 +522,7 @@ gemm_kernel(const GemmParams p) {
                         PAMK_FRAGMENTS(kk)
                         PAMK_WEIGHTS(kk, ty)
 #pragma unroll
-                        for (int i = 0; i < MT; ++i)
+                        for (int i = 0; i < MR; ++i)
 #pragma unroll
                             for (int j = 0; j < MT; j += 2) fma_pair(acc[i][j], acc[i][j + 1], iadd(a[i], b[j]), iadd(a[i], b[j + 1]), w[i], w[i]);
                     }
@@ -511,7 +532,7 @@ gemm_kernel(const GemmParams p) {
                         PAMK_FRAGMENTS(kk)
                         PAMK_WEIGHTS(kk, tx)
 #pragma unroll
-                        for (int i = 0; i < MT; ++i)
+                        for (int i = 0; i < MR; ++i)
 #pragma unroll
                             for (int j = 0; j < MT; j += 2) fma_pair(acc[i][j], acc[i][j + 1], iadd(a[i], b[j]), iadd(a[i], b[j + 1]), w[j], w[j + 1]);
                     }
@@ -549,11 +570,11 @@ gemm_kernel(const GemmParams p) {
 #pragma unroll (MT == 4 ? 4 : 2)
                     for (int kk = 0; kk < BK; ++kk) {
                         PAMK_FRAGMENTS(kk)
-                        float araw[MT];          // a[] holds pre-biased patterns; the rule needs the values
+                        float araw[MR];          // a[] holds pre-biased patterns; the rule needs the values
 #pragma unroll
-                        for (int i = 0; i < MT; ++i) araw[i] = i2f(iadd(a[i], p.bias_sub));
+                        for (int i = 0; i < MR; ++i) araw[i] = i2f(iadd(a[i], p.bias_sub));
 #pragma unroll
-                        for (int i = 0; i < MT; ++i)
+                        for (int i = 0; i < MR; ++i)
 #pragma unroll
                             for (int j = 0; j < MT; ++j) {
                                 const float mag = fabsf(fmul(araw[i], i2f(b[j])));
@@ -569,11 +590,11 @@ gemm_kernel(const GemmParams p) {
                         const unsigned here = 1u << kk;
                         if (full & here) {
                             PAMK_FRAGMENTS(kk)
-                            float araw[MT];
+                            float araw[MR];
 #pragma unroll
-                            for (int i = 0; i < MT; ++i) araw[i] = i2f(iadd(a[i], p.bias_sub));
+                            for (int i = 0; i < MR; ++i) araw[i] = i2f(iadd(a[i], p.bias_sub));
 #pragma unroll
-                            for (int i = 0; i < MT; ++i)
+                            for (int i = 0; i < MR; ++i)
 #pragma unroll
                                 for (int j = 0; j < MT; ++j) {
                                     const float mag = fabsf(fmul(araw[i], i2f(b[j])));
@@ -587,11 +608,11 @@ gemm_kernel(const GemmParams p) {
 #pragma unroll 1
                             for (; kk < end; ++kk) {
                                 PAMK_FRAGMENTS(kk)
-                                float araw[MT];
+                                float araw[MR];
 #pragma unroll
-                                for (int i = 0; i < MT; ++i) araw[i] = i2f(iadd(a[i], p.bias_sub));
+                                for (int i = 0; i < MR; ++i) araw[i] = i2f(iadd(a[i], p.bias_sub));
 #pragma unroll
-                                for (int i = 0; i < MT; ++i)
+                                for (int i = 0; i < MR; ++i)
 #pragma unroll
                                     for (int j = 0; j < MT; ++j) {
                                         const float mag = fabsf(fmul(araw[i], i2f(b[j])));
@@ -605,7 +626,7 @@ gemm_kernel(const GemmParams p) {
                             for (; kk < end; ++kk) {
                                 PAMK_FRAGMENTS(kk)
 #pragma unroll
-                                for (int i = 0; i < MT; ++i)
+                                for (int i = 0; i < MR; ++i)
 #pragma unroll
                                     for (int j = 0; j < MT; j += 2) add_pair(acc[i][j], acc[i][j + 1], iadd(a[i], b[j]), iadd(a[i], b[j + 1]));
                             }
@@ -619,13 +640,13 @@ gemm_kernel(const GemmParams p) {
                 PAMK_FRAGMENTS(kk)
                 if constexpr (MODE == kStd) {
 #pragma unroll
-                    for (int i = 0; i < MT; ++i)
+                    for (int i = 0; i < MR; ++i)
 #pragma unroll
                         for (int j = 0; j < MT; ++j) acc[i][j] = __fmaf_rn(i2f(a[i]), i2f(b[j]), acc[i][j]);
                 } else {
                     // acc += delta * 2^slope, slope from the non-delta operand and D
 #pragma unroll
-                    for (int i = 0; i < MT; ++i)
+                    for (int i = 0; i < MR; ++i)
 #pragma unroll
                         for (int j = 0; j < MT; ++j) {
                             const int other = MODE == kBwdL ? b[j] : a[i];
@@ -657,7 +678,7 @@ gemm_kernel(const GemmParams p) {
         // slope's bit pattern is -inf and the term is NaN.
         if (p.K & 31) {
 #pragma unroll
-            for (int i = 0; i < MT; ++i)
+            for (int i = 0; i < MR; ++i)
 #pragma unroll
                 for (int j = 0; j < MT; ++j) {
                     if constexpr (MODE == kStd) acc[i][j] = fadd(acc[i][j], 0.0f);
@@ -666,8 +687,8 @@ gemm_kernel(const GemmParams p) {
         }
     }
 #pragma unroll
-    for (int i = 0; i < MT; ++i) {
-        const int row = m0 + ty * 4 + (i & 3) + (i >> 2) * (BM / 2);
+    for (int i = 0; i < MR; ++i) {
+        const int row = m0 + slot_row<T, BM>(ty * 4 + (i & 3) + (i >> 2) * (BM / 2));
         if (row >= p.M) continue;
         float* crow = Cz + (int64_t)row * p.ldc;
 #pragma unroll
@@ -758,6 +779,14 @@ int dispatch(const GemmParams& p, bool a_kc, bool b_kc, bool vec, dim3 grid, cud
     return check_launch();
 }
 
+// (the tiles with fewer rows per thread exist for A contiguous along K and 128-bit loads)
+template <class T>
+int dispatch_rows(const GemmParams& p, bool b_kc, dim3 grid, cudaStream_t st) {
+    if (b_kc) gemm_kernel<kPam, T, true, true, true><<<grid, T::kThreads, 0, st>>>(p);
+    else gemm_kernel<kPam, T, true, false, true><<<grid, T::kThreads, 0, st>>>(p);
+    return check_launch();
+}
+
 // An operand can use 128-bit loads when its base and both non-unit strides keep every group of
 // four elements 16-byte aligned and its contiguous extent is a multiple of four.
 bool vectorisable(const MatArg& m, bool kc, int rows, int K) {
@@ -769,7 +798,7 @@ bool vectorisable(const MatArg& m, bool kc, int rows, int K) {
 // The kernel is issue-bound, so the time of a launch is (the largest number of tiles any SM ends up
 // with) x (work per tile), inflated when an SM holds too few warps to keep its schedulers busy,
 // which is also the state of the SMs that run the last, partly filled wave of a larger launch.
-enum TileKind { kTileLarge = 0, kTileSmall = 1, kTileTiny = 2 };
+enum TileKind { kTileLarge = 0, kTileSmall = 1, kTileTiny = 2, kTileLarge7 = 3 };
 
 struct Plan {
     int tile;        // TileKind
@@ -783,7 +812,7 @@ Plan plan_for(int mode, int64_t batch, int64_t M, int64_t N, int64_t K, int spli
     // half as many of their CTAs fit on an SM
     const int ctas_per_sm = mode == kBwdL || mode == kBwdR ? T::kCtasPerSm / 2 : T::kCtasPerSm;
     const int64_t sms = sm_count();
-    const int64_t tiles = batch * ((M + T::BM - 1) / T::BM) * ((N + T::BN - 1) / T::BN);
+    const int64_t tiles = batch * ((M + T::kRows - 1) / T::kRows) * ((N + T::BN - 1) / T::BN);
     const int64_t slabs = (K + T::BK - 1) / T::BK;
     const int64_t slots = sms * ctas_per_sm;
     // cost of cutting K into s ranges, in multiply-accumulates per SM at full issue rate
@@ -796,12 +825,13 @@ Plan plan_for(int mode, int64_t batch, int64_t M, int64_t N, int64_t K, int spli
         // 8 about 74 %
         auto util = [](int64_t ctas) {
             const double warps = (double)ctas * (T::kThreads / 32);
+            if (T::MR < T::MT && warps >= 8.0) return warps >= 16.0 ? 1.0 : 0.94;      // (one 256-thread CTA: 2.75 us a slab, two: 5.23)
             return warps >= 16.0 ? 1.0 : (warps >= 8.0 ? 0.58 + 0.02 * warps : warps / 10.8);
         };
         // the smaller the tile, the more bytes are staged (and fragments loaded) per MAC
         const double staging = T::BM >= 128 ? 1.0 : (T::BM >= 64 ? 1.06 : 1.25);
         // every CTA also pays a prologue (first loads exposed) and an epilogue worth about 16 k-steps
-        const double per_cta = (double)T::BM * T::BN * ((double)(chunk_slabs * T::BK) + 16.0);
+        const double per_cta = (double)T::kRows * T::BN * ((double)(chunk_slabs * T::BK) + 16.0);
         const int64_t ctas = tiles * s;
         // CTAs spread evenly over the SMs ...
         const int64_t per_sm = (ctas + sms - 1) / sms;
@@ -818,7 +848,7 @@ Plan plan_for(int mode, int64_t batch, int64_t M, int64_t N, int64_t K, int spli
         return cost * staging + (s > 1 ? 1.1e6 : 0.0);        // the reduction pass and its launch (~12 us)
     };
     Plan pl;
-    pl.tile = T::BM >= 128 ? kTileLarge : (T::BM >= 64 ? kTileSmall : kTileTiny);
+    pl.tile = T::MR < T::MT ? kTileLarge7 : (T::BM >= 128 ? kTileLarge : (T::BM >= 64 ? kTileSmall : kTileTiny));
     int64_t s = split_request > 0 ? split_request : 1, actual = 1;
     pl.cost = cost_of(s, &actual);
     pl.splits = (int)actual;
@@ -849,12 +879,16 @@ bool fine_slabs(int64_t ctas, int64_t K) {
 }
 
 // 0: choose by cost; 1: always the large tile; 2: the 64x64 tile wherever it exists; 3: the 32x32
-// tile wherever it exists (PAM products), else the 64x64 tile.
+// tile wherever it exists (PAM products), else the 64x64 tile; 4: the large tile, with seven rows per thread wherever
+// that exists.
 int g_tile_policy = 0;
 
-Plan make_plan(int mode, int64_t batch, int64_t M, int64_t N, int64_t K, int split_request) {
+// seven_rows: the operands allow TileLarge7 (the callers that only ask for the split do not know, and get the split of
+// the other tiles).
+Plan make_plan(int mode, int64_t batch, int64_t M, int64_t N, int64_t K, int split_request, bool seven_rows = false) {
     const Plan large = plan_for<TileLarge>(mode, batch, M, N, K, split_request);
     if (mode == kStd || g_tile_policy == 1) return large;    // the true-multiply product uses the large tile
+    if (g_tile_policy == 4) return seven_rows && split_request <= 1 ? plan_for<TileLarge7>(mode, batch, M, N, K, 1) : large;
     const Plan small = plan_for<TileSmall>(mode, batch, M, N, K, split_request);
     if (g_tile_policy == 2 || (g_tile_policy == 3 && mode != kPam)) return small;
     Plan best = small.cost < large.cost ? small : large;
@@ -876,6 +910,10 @@ Plan make_plan(int mode, int64_t batch, int64_t M, int64_t N, int64_t K, int spl
             if (fine.cost < tiny.cost) tiny = fine;
         }
         if (g_tile_policy == 3 || tiny.cost < margin * best.cost) best = tiny;
+        if (seven_rows && split_request <= 1 && g_tile_policy == 0) {
+            const Plan seven = plan_for<TileLarge7>(mode, batch, M, N, K, 1);
+            if (seven.cost < 0.95 * best.cost) best = seven;
+        }
     }
     return best;
 }
@@ -894,19 +932,21 @@ int run(int mode, GemmParams p, bool a_kc, bool b_kc, int split_k, void* workspa
         return e == cudaSuccess ? PAMK_OK : record_cuda_error(e);
     }
     if (split_k < 0) return PAMK_ERR_ARG;
-    Plan pl = p.K == 0 ? Plan{kTileSmall, 1, 0.0} : make_plan(mode, p.batch, p.M, p.N, p.K, split_k);   // K = 0: rows of bias
+    const bool vec = vectorisable(p.A, a_kc, p.M, p.K) && vectorisable(p.B, b_kc, p.N, p.K);
+    const bool seven_rows = mode == kPam && p.batch == 1 && a_kc && vec;
+    Plan pl = p.K == 0 ? Plan{kTileSmall, 1, 0.0} : make_plan(mode, p.batch, p.M, p.N, p.K, split_k, seven_rows);   // K = 0: rows of bias
     if (pl.splits > 1 && !workspace_ok(workspace, workspace_bytes, pl.splits, count)) {
         if (split_k != 0) return PAMK_ERR_WORKSPACE;         // an explicit split needs its scratch
-        pl = make_plan(mode, p.batch, p.M, p.N, p.K, 1);     // automatic: fall back to no split
+        pl = make_plan(mode, p.batch, p.M, p.N, p.K, 1, seven_rows);     // automatic: fall back to no split
     }
     // the M tiles ride on grid.y (at most 65535): a very tall product planned with a small tile moves to
     // the 128x128 tile, which reaches 8.3 M rows
-    if (pl.tile != kTileLarge && (p.M + (pl.tile == kTileTiny ? TileTiny::BM : TileSmall::BM) - 1) /
+    if (pl.tile != kTileLarge && pl.tile != kTileLarge7 && (p.M + (pl.tile == kTileTiny ? TileTiny::BM : TileSmall::BM) - 1) /
                                          (pl.tile == kTileTiny ? TileTiny::BM : TileSmall::BM) > 65535) {
         const int splits = pl.splits;
         pl = plan_for<TileLarge>(mode, p.batch, p.M, p.N, p.K, splits);
     }
-    const int bm = pl.tile == kTileTiny ? TileTiny::BM : (pl.tile == kTileSmall ? TileSmall::BM : TileLarge::BM);
+    const int bm = pl.tile == kTileTiny ? TileTiny::BM : (pl.tile == kTileSmall ? TileSmall::BM : (pl.tile == kTileLarge7 ? TileLarge7::kRows : TileLarge::BM));
     const int bn = pl.tile == kTileTiny ? TileTiny::BN : (pl.tile == kTileSmall ? TileSmall::BN : TileLarge::BN);
     const int64_t ctas = ((p.N + bn - 1) / bn) * (int64_t)((p.M + bm - 1) / bm) * p.batch * pl.splits;
     const bool fine = pl.tile == kTileTiny && pl.splits == 1 && fine_slabs(ctas, p.K);
@@ -927,7 +967,6 @@ int run(int mode, GemmParams p, bool a_kc, bool b_kc, int split_k, void* workspa
         p.sCsplit = count;
     }
     // batch strides into the kernel's form (see MatArg)
-    const bool vec = vectorisable(p.A, a_kc, p.M, p.K) && vectorisable(p.B, b_kc, p.N, p.K);
     auto kernel_form = [&](int64_t& outer, int64_t& inner_stride) {
         if (p.inner == 1) { inner_stride = outer; outer = 0; }
         else outer -= (int64_t)p.inner * inner_stride;
@@ -949,6 +988,7 @@ int run(int mode, GemmParams p, bool a_kc, bool b_kc, int split_k, void* workspa
             rc = fine                    ? dispatch<kPam, TileTinyFine>(p, a_kc, b_kc, vec, grid, st)
                  : pl.tile == kTileTiny  ? dispatch<kPam, TileTiny>(p, a_kc, b_kc, vec, grid, st)
                  : pl.tile == kTileSmall ? dispatch<kPam, TileSmall>(p, a_kc, b_kc, vec, grid, st)
+                 : pl.tile == kTileLarge7 ? dispatch_rows<TileLarge7>(p, b_kc, grid, st)
                                          : dispatch<kPam, TileLarge>(p, a_kc, b_kc, vec, grid, st);
             break;
         case kStd: rc = dispatch<kStd, TileLarge>(p, a_kc, b_kc, vec, grid, st); break;
@@ -1028,7 +1068,7 @@ size_t pamk_matmul_workspace_bytes(int64_t batch, int64_t M, int64_t N, int spli
 }
 
 int pamk_test_set_tile_policy(int policy) {
-    if (policy < 0 || policy > 3) return PAMK_ERR_ARG;
+    if (policy < 0 || policy > 4) return PAMK_ERR_ARG;
     g_tile_policy = policy;
     return PAMK_OK;
 }
