@@ -18,12 +18,9 @@
 //     every element's exponent is tested against the safe band;
 //   * the reference's per-product range rule (flush below 1e-37, NaN above 1e37 or for
 //     inf/NaN; epfml/pam pam/cuda_kernels.cu:24-37) is hoisted.  A slab whose elements all have their
-//     exponent in a band that keeps every product in range runs the two-instruction loop, and so does one
-//     whose other elements are all zeros (their products get weight 0).  In any other
-//     slab the choice is made per k line: a line without out-of-band elements still costs two
-//     instructions per product; a line whose largest magnitudes cannot multiply beyond the pass range
-//     evaluates the true product only to decide "flush or add" (four instructions); only a line
-//     that could overflow, or holds an inf / NaN, applies the full three-way rule.  Either way every
+//     exponent in a band that keeps every product in range runs the two-instruction loop.  In any other
+//     slab the choice is made per k line, on the large tile per warp too: products that all pass are summed as they
+//     are, products that all flush are left out, and only what is left evaluates the true product.  Either way every
 //     product equals the reference's bit for bit;
 //   * each output is summed by one thread, strictly in k order, from +0.0f — the same order as
 //     the reference's kernel (cuda_kernels.cu:608-629), so without split-K the sums are
@@ -31,6 +28,8 @@
 //
 // The same skeleton serves true-multiply products (standard_matmul) and the exact-gradient
 // product (pam_matmul_bwd_kernel, cuda_kernels.cu:729-832).
+#include <type_traits>
+
 #include "common.cuh"
 #include "pam_scalar.cuh"
 
@@ -228,21 +227,21 @@ __device__ __forceinline__ void store_slab(float* s, const float (&r)[NT * 4], i
 // (cuda_kernels.cu:24-37) returns the integer sum.  The band test is one three-input add and one
 // unsigned max per element: 2 * bits drops the sign, minus twice the band's lower bound makes "below"
 // wrap around to huge values.
-//   * A slab whose elements are all in the band runs the two-instruction loop.
-//   * Otherwise the staging threads that hold out-of-band elements record, per k line, that the line
-//     is dirty and whether it holds an element above the band.  A clean line of a dirty slab still
-//     costs two instructions per product.
-//   * A slab whose out-of-band elements are all zeros gives them weight 0 in a fused multiply-add and stays
-//     at two instructions per product (see the loop).
-//   * Any other dirty line evaluates the true fp32 product.  It can skip the overflow test when the largest
+//   * A slab whose elements are all in the band runs the two-instruction loop.  Otherwise the staging threads that hold
+//     out-of-band elements record for which k lines, and of what sort they are.
+//   * Zeros alone, in most lines (an operand that went through a ReLU): a zero's products are left out of the sums by a
+//     predicate or a weight.
+//   * Anything else, large tile: the lines with out-of-band elements are looked through once and every warp takes, for each
+//     line, the cheapest loop that its own rows and columns allow (class_of, kind_of).
+//   * Anything else, smaller tiles, where that look costs more than it saves (12608x768x192 with 1 % specials 304 -> 475 us): a line
+//     without out-of-band elements costs two instructions per product, any other evaluates the true fp32 product.
+//     It can skip the overflow test when the largest
 //     magnitudes of its two operand lines cannot multiply beyond 1e37 and neither holds an inf / NaN
 //     (|a * b| rounded grows with |a| and |b|, so the two maxima bound every product of the line):
 //     four instructions per product, "flush or add".  Only the remaining lines apply the full rule.
-enum Path { kFast = 0, kFlush = 1, kFull = 2 };
-
-constexpr uint32_t kBandLo2 = 2u * (66u << 23);                // 2 * smallest in-band magnitude
-constexpr uint32_t kBandSpan2 = 2u * ((188u - 66u) << 23);     // in band iff 2*bits - kBandLo2 < span
-constexpr uint32_t kBandHi2 = 2u * (188u << 23);               // 2 * smallest magnitude above the band
+constexpr uint32_t kBandLo = 66u << 23, kBandHi = 188u << 23;  // smallest magnitude in the band, smallest above it
+constexpr uint32_t kBandLo2 = 2u * kBandLo, kBandHi2 = 2u * kBandHi;
+constexpr uint32_t kBandSpan2 = kBandHi2 - kBandLo2;           // in band iff 2*bits - kBandLo2 < span
 
 template <int N>
 __device__ __forceinline__ uint32_t band_excess(const float (&r)[N], uint32_t vmax) {
@@ -260,15 +259,12 @@ __device__ __forceinline__ int slab_line(int id, int c) {
     return KC ? (id % (T::BK / 4)) * 4 + c : id / (R / 4);
 }
 
-// A slab's word: bit k for a k line that holds an out-of-band element, and above bit 15 whether any lies above the band.
-// The kernels of the 64x64 tile keep kAbove for that and, in the bits from kUnasked on, how many slabs, this one
-// included, are not asked for zeros (see the loop).  Those of the other tiles have bit 16 + k: the count costs registers
-// that clean slabs of the 32x32 tile (1.4 %) and slabs with specials of the 128x128 tile (0.9 %) then miss.
-enum Word : unsigned { kAbove = 1u << 16, kUnasked = 1u << 17 };
+// A slab's word: bit k for a k line that holds an out-of-band element, and what such elements there are.
+enum Word : unsigned { kZerosA = 1u << 16, kZerosB = 1u << 17, kNonZero = 1u << 18, kAbove = 1u << 19 };
 
 // The word's bits for this thread's staged elements.
 template <class T, int R, int NT, bool KC>
-__device__ __forceinline__ unsigned dirty_lines(const float (&r)[NT * 4], int tid) {
+__device__ __forceinline__ unsigned dirty_lines(const float (&r)[NT * 4], int tid, unsigned zeros) {
     unsigned lines = 0;
 #pragma unroll
     for (int t = 0; t < NT; ++t)
@@ -276,28 +272,45 @@ __device__ __forceinline__ unsigned dirty_lines(const float (&r)[NT * 4], int ti
         for (int c = 0; c < 4; ++c) {
             const uint32_t b = (uint32_t)f2i(r[t * 4 + c]);
             const uint32_t m2 = b + b;
-            if (m2 - kBandLo2 >= kBandSpan2) {
-                const unsigned bit = 1u << slab_line<T, R, KC>(tid + t * T::kThreads, c);
-                lines |= bit | (m2 >= kBandHi2 ? (T::BM == 64 ? (unsigned)kAbove : bit << 16) : 0u);
-            }
+            if (m2 - kBandLo2 >= kBandSpan2)
+                lines |= (1u << slab_line<T, R, KC>(tid + t * T::kThreads, c)) |
+                         (m2 == 0 ? zeros : (m2 >= kBandHi2 ? kNonZero | kAbove : (unsigned)kNonZero));
         }
     return lines;
 }
 
-// Sorts of out-of-band elements in four consecutive words of a staged slab row (`bias` undoes the A side's
-// pre-bias): `zero_kind` for zeros, kOther for the rest.
-enum Kind { kZerosA = 1, kZerosB = 2, kOther = 4 };
-constexpr unsigned kSlabsUnasked = 9;                          // after a slab with others than zeros, itself included
+// ---- the large tile's look through a dirty slab ------------------------------------------------------------------------
+// What does the range rule do to the products of an out-of-band element with its line's partners that are not above the band?
+// The rounded product |a * b| grows with both factors, so the largest such partner and the smallest
+// partner inside the band answer that exactly:
+//   kMasked  every product flushes to +0 (zeros; small values against partners of ordinary size)
+//   kSmall   below the band, and every product with a partner inside the band passes
+//   kGreat   above the band, finite, and every product with a partner not above the band stays below the pass bound
+//            (with a partner inside the band it does not flush either: 2^61 * 2^-61 = 1)
+//   kOdd     anything else: inf, NaN, values whose products do not all behave alike
+// Only products of two out-of-band elements are left to sort out: two masked ones flush (each has the other among its
+// partners), and so do a masked and a small one; any other such pair among a warp's rows and columns, and anything odd,
+// sends the line to the loop that forms the true product of every pair.
+// Against "flush or add" for every dirty line, 4096^3: 1 % special values 10428 -> 9940 us, 0.1 % 6700 -> 6360, one operand
+// below the band 10240 -> 6830.  The look itself costs about 40 % of a clean slab; one warp per two lines, with redux and
+// ballots for the shuffles, measured 5 % slower.
+enum Class { kMasked = 1, kSmall = 2, kGreat = 4, kOdd = 8 };
+enum LineKind { kPlain = 0, kRowsOff = 1, kColsOff = 2, kBothOff = 3, kChecked = 4, kNothing = 5 };
 
-__device__ __forceinline__ unsigned kinds_of(const int4& v, int bias, unsigned zero_kind) {
-    unsigned kinds = 0;
-    const int e[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        const uint32_t b = (uint32_t)iadd(e[c], bias), m2 = b + b;
-        if (m2 - kBandLo2 >= kBandSpan2) kinds |= m2 == 0 ? zero_kind : (unsigned)kOther;
-    }
-    return kinds;
+__device__ __forceinline__ unsigned class_of(uint32_t magnitude, float smallest, float largest) {
+    const float m = i2f((int32_t)magnitude);
+    if (magnitude >= kBandHi) return fmul(m, largest) <= i2f(kPassBits) ? kGreat : kOdd;      // (not <=: inf and NaN)
+    if (fmul(m, largest) <= i2f(kFlushBits)) return kMasked;
+    return fmul(m, smallest) > i2f(kFlushBits) ? kSmall : kOdd;
+}
+
+// The loop for a line whose rows / columns of one warp hold elements of these classes; `flushes`: the line's largest
+// magnitudes that are not above the band flush each other.
+__device__ __forceinline__ unsigned kind_of(unsigned rows, unsigned cols, bool flushes) {
+    const unsigned both = rows | cols;
+    if ((both & kOdd) || ((rows & kGreat) && cols) || ((cols & kGreat) && rows) || (rows & cols & kSmall)) return kChecked;
+    if (flushes && !(both & kGreat)) return kNothing;
+    return (rows & kMasked ? kRowsOff : 0u) | (cols & kMasked ? kColsOff : 0u);
 }
 
 // ---- two sums in one instruction ----------------------------------------------------------------------------------
@@ -321,18 +334,21 @@ __global__ void __launch_bounds__(T::kThreads, MODE == kPam || MODE == kStd ? T:
 gemm_kernel(const GemmParams p) {
     constexpr int BM = T::BM, BN = T::BN, BK = T::BK, MT = T::MT, MR = T::MR;
     static_assert(MR == MT || (MODE == kPam && A_KC && VEC), "fewer rows per thread: products with A contiguous along K alone");
-    constexpr unsigned kDirty = BM == 64 ? kUnasked - 1u : ~0u;      // of a slab's word: the slab is not clean
+    constexpr bool kLook = MODE == kPam && BM == 128;      // dirty slabs are looked through (see class_of)
     // (the variant with both operands contiguous along their row index spills registers at 8)
     constexpr int kFastUnroll = (!A_KC && !B_KC) || 8 > BK ? BK : 8;
     __shared__ __align__(16) float As[2][BK * row_stride(BM)];
     __shared__ __align__(16) float Bs[2][BK * row_stride(BN)];
-    __shared__ __align__(16) float weights[MODE == kPam ? BK * row_stride(BM) : 1];   // of the side that holds zeros
-    __shared__ unsigned kinds[3];   // per slab: the sorts of out-of-band elements it holds (Kind), filled where a loop below asks
+    __shared__ __align__(16) float weights[MODE == kPam && MT == 4 ? BK * row_stride(BM) : 1];   // of the side that holds zeros (32x32 tile)
     __shared__ unsigned lines[3];   // per slab (Word)
     __shared__ unsigned overflow_lines;   // bit k = some product of k line may leave the pass range
+    // looked-through slabs: per line and thread row / column a bit for each masked element, per warp and line the LineKind
+    __shared__ unsigned char rows_off[kLook ? BK : 1][16], cols_off[kLook ? BK : 1][16], line_kinds[kLook ? 8 : 1][BK];
 
     const int tid = threadIdx.x;
-    const int tx = tid % T::TX, ty = tid / T::TX;
+    // a warp is 4 x 8 threads: the fewer rows and columns it has, the fewer of their lines hold out-of-band elements
+    const int tx = T::TX == 16 ? (tid >> 5 & 1) * 8 + (tid & 7) : tid % T::TX;
+    const int ty = T::TX == 16 ? (tid >> 6) * 4 + (tid >> 3 & 3) : tid / T::TX;
     const int m0 = blockIdx.y * T::kRows, n0 = blockIdx.x * BN;
     const int z = blockIdx.z / p.splits, sp = blockIdx.z - z * p.splits;
     const int k_begin = sp * p.k_chunk;
@@ -370,7 +386,7 @@ gemm_kernel(const GemmParams p) {
         }
     }
 
-    if (MODE == kPam && tid < 3) lines[tid] = kinds[tid] = 0;
+    if (MODE == kPam && tid < 3) lines[tid] = 0;
 
     float ra[T::kTasksA * 4], rb[T::kTasksB * 4];
     SlabWalker<T, BM, T::kTasksA, A_KC> walk_a;
@@ -394,7 +410,7 @@ gemm_kernel(const GemmParams p) {
             // an out-of-band element locates it and reports its k line to the slab's word
             const bool out = band_excess(rb, band_excess(ra, 0u)) >= kBandSpan2;
             if (__any_sync(0xffffffffu, out)) {
-                unsigned f = out ? (dirty_lines<T, BM, T::kTasksA, A_KC>(ra, tid) | dirty_lines<T, BN, T::kTasksB, B_KC>(rb, tid)) : 0u;
+                unsigned f = out ? (dirty_lines<T, BM, T::kTasksA, A_KC>(ra, tid, kZerosA) | dirty_lines<T, BN, T::kTasksB, B_KC>(rb, tid, kZerosB)) : 0u;
                 f = __reduce_or_sync(0xffffffffu, f);
                 if ((tid & 31) == 0) atomicOr(&lines[slot], f);
             }
@@ -421,8 +437,8 @@ gemm_kernel(const GemmParams p) {
         unsigned dirty = 0;
         if (MODE == kPam) {
             dirty = lines[s % 3];
-            // the words two slabs ahead were last read before the previous barrier: reset them now
-            if (tid == 0) lines[(s + 2) % 3] = kinds[(s + 2) % 3] = 0;
+            // the word two slabs ahead was last read before the previous barrier: reset it now
+            if (tid == 0) lines[(s + 2) % 3] = 0;
         }
         const float* as = As[buf];
         const float* bs = Bs[buf];
@@ -436,11 +452,10 @@ gemm_kernel(const GemmParams p) {
         const int b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
 
 #define PAMK_WEIGHTS(kk, at)                                                                            \
-        const float4 w0 = *reinterpret_cast<const float4*>(weights + (kk) * row_stride(BM) + (at) * 4); \
-        const float4 w1 = MT == 8 ? *reinterpret_cast<const float4*>(weights + (kk) * row_stride(BM) + (at) * 4 + BM / 2) : w0; \
-        const float w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+        const float4 w4 = *reinterpret_cast<const float4*>(weights + (kk) * row_stride(BM) + (at) * 4); \
+        const float w[4] = {w4.x, w4.y, w4.z, w4.w};
 
-        if (MODE == kPam && (dirty & kDirty) == 0) {
+        if (MODE == kPam && dirty == 0) {
 #pragma unroll kFastUnroll
             for (int kk = 0; kk < BK; ++kk) {
                 PAMK_FRAGMENTS(kk)
@@ -451,40 +466,205 @@ gemm_kernel(const GemmParams p) {
             }
         } else if constexpr (MODE == kPam) {
             constexpr unsigned all_lines = (1u << BK) - 1u;
-            // Is everything out of the band a zero?  Looked up here and not while staging, where the registers
-            // for it spilled and every dirty slab slowed down by 3 to 7 %.  A slab with elements above the band need
-            // not be asked, one with few dirty lines is better off in the runs below (0.1 % zeros: 261 us with
-            // them, 283 us when asked).  The zero-filled lines past the end of K count on both sides.  Where the
-            // answer was no, the next slabs are not asked (operands of which most values lie below the band:
-            // 4235x1152x67 on the 64x64 tile 85 -> 80 us; 78 us before there was the question).
-            unsigned kind = kOther;
-            if (dirty < kAbove && __popc(dirty) * 4 >= BK * 3) {
-                unsigned seen = 0;
+            const unsigned any = dirty & all_lines;
+            const bool mostly = __popc(any) * 4 >= BK * 3;              // most lines are dirty
+            // One line by the plain sum, by "flush or add", or by the full rule.
+            auto plain_line = [&](int kk) {
+                PAMK_FRAGMENTS(kk)
 #pragma unroll
-                for (int t = 0; t < T::kTasksA; ++t) {
-                    const int id = tid + t * T::kThreads;
-                    const int at = id / (BM / 4) * row_stride(BM) + id % (BM / 4) * 4;
-                    seen |= kinds_of(*reinterpret_cast<const int4*>(as + at), p.bias_sub, kZerosA);
-                    seen |= kinds_of(*reinterpret_cast<const int4*>(bs + at), 0, kZerosB);
+                for (int i = 0; i < MR; ++i)
+#pragma unroll
+                    for (int j = 0; j < MT; ++j) acc[i][j] = fadd(acc[i][j], i2f(iadd(a[i], b[j])));
+            };
+            auto checked_line = [&](int kk, auto full_rule) {
+                PAMK_FRAGMENTS(kk)
+                float araw[MR];                                         // a[] holds pre-biased patterns; the rule needs the values
+#pragma unroll
+                for (int i = 0; i < MR; ++i) araw[i] = i2f(iadd(a[i], p.bias_sub));
+#pragma unroll
+                for (int i = 0; i < MR; ++i)
+#pragma unroll
+                    for (int j = 0; j < MT; ++j) {
+                        const float mag = fabsf(fmul(araw[i], i2f(b[j])));
+                        if constexpr (decltype(full_rule)::value) {
+                            const float prod = mag <= i2f(kPassBits) ? i2f(iadd(a[i], b[j])) : quiet_nan();
+                            if (!(mag <= i2f(kFlushBits))) acc[i][j] = fadd(acc[i][j], prod);
+                        } else {
+                            if (mag > i2f(kFlushBits)) acc[i][j] = fadd(acc[i][j], i2f(iadd(a[i], b[j])));
+                        }
+                    }
+            };
+            int kk = 0;
+            auto run_end = [&](unsigned mask) { return min(BK, kk + __ffs((int)(~mask >> kk)) - 1); };
+            if (MT == 8 && !(dirty & kNonZero) && mostly) {
+                // Zeros, and everything else in the band: a zero's products are left out by a predicate.
+                // 4096^3 with one operand half zeros 6020 us (clean: 4565), both 7500; by
+                // weights of 0 and 1 in a fused multiply-add, prepared by a pass over the slab, 6040 and 9670.
+                if (!(dirty & kZerosA)) {
+#pragma unroll 1
+                    for (; kk < BK; ++kk) {
+                        PAMK_FRAGMENTS(kk)
+#pragma unroll
+                        for (int i = 0; i < MR; ++i)
+#pragma unroll
+                            for (int j = 0; j < MT; ++j)
+                                if (2u * (uint32_t)b[j] != 0u) acc[i][j] = fadd(acc[i][j], i2f(iadd(a[i], b[j])));
+                    }
+                } else if (!(dirty & kZerosB)) {
+#pragma unroll 1
+                    for (; kk < BK; ++kk) {
+                        PAMK_FRAGMENTS(kk)
+                        // (columns outside: with the rows outside the compiler makes a branch of each row's condition)
+#pragma unroll
+                        for (int j = 0; j < MT; ++j)
+#pragma unroll
+                            for (int i = 0; i < MR; ++i)
+                                if (2u * (uint32_t)iadd(a[i], p.bias_sub) != 0u) acc[i][j] = fadd(acc[i][j], i2f(iadd(a[i], b[j])));
+                    }
+                } else {
+                    // rows by a weight: a zero's products (made finite) get weight 0 in a fused multiply-add, which leaves a sum alone
+                    // (it is never -0)
+#pragma unroll 1
+                    for (; kk < BK; ++kk) {
+                        PAMK_FRAGMENTS(kk)
+#pragma unroll
+                        for (int i = 0; i < MR; ++i) {
+                            const bool zero = 2u * (uint32_t)iadd(a[i], p.bias_sub) == 0u;
+                            const float w = zero ? 0.0f : 1.0f;
+                            const int ai = zero ? 0 : a[i];
+#pragma unroll
+                            for (int j = 0; j < MT; ++j)
+                                if (2u * (uint32_t)b[j] != 0u) acc[i][j] = __fmaf_rn(i2f(iadd(ai, b[j])), w, acc[i][j]);
+                        }
+                    }
                 }
-                seen = __reduce_or_sync(0xffffffffu, seen);
-                if ((tid & 31) == 0) atomicOr(&kinds[s % 3], seen);
+            } else if constexpr (kLook) {
+                // sixteen threads look through one line, the two groups of four elements of either side that thread row / column
+                // `at` works on each
+                static_assert(!kLook || (BK == 16 && T::kThreads == 256 && BN == 128 && MT == 8), "a warp looks through two lines");
+                const int lane = tid & 31, warp = tid >> 5, line = tid >> 4, at = tid & 15;
+                if (any >> (2 * warp) & 3u) {                       // (the same for a warp)
+                    uint32_t ma[8], mb[8];
+                    // the smallest magnitude in the band and the largest that is not above it, as offsets in which what does not count
+                    // wraps around to the losing end
+                    uint32_t lo_a = ~0u, hi_a = 0u, lo_b = ~0u, hi_b = 0u;
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) {
+                        const int4 va = *reinterpret_cast<const int4*>(as + line * row_stride(BM) + q * (BM / 2) + at * 4);
+                        const int4 vb = *reinterpret_cast<const int4*>(bs + line * row_stride(BN) + q * (BN / 2) + at * 4);
+                        const int ea[4] = {va.x, va.y, va.z, va.w}, eb[4] = {vb.x, vb.y, vb.z, vb.w};
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) {
+                            const uint32_t xa = (uint32_t)iadd(ea[c], p.bias_sub) & 0x7fffffffu, xb = (uint32_t)eb[c] & 0x7fffffffu;
+                            ma[q * 4 + c] = xa;
+                            mb[q * 4 + c] = xb;
+                            lo_a = min(lo_a, xa - kBandLo); hi_a = max(hi_a, xa - kBandHi);
+                            lo_b = min(lo_b, xb - kBandLo); hi_b = max(hi_b, xb - kBandHi);
+                        }
+                    }
+#pragma unroll
+                    for (int d = 1; d < 16; d <<= 1) {
+                        lo_a = min(lo_a, __shfl_xor_sync(0xffffffffu, lo_a, d)); hi_a = max(hi_a, __shfl_xor_sync(0xffffffffu, hi_a, d));
+                        lo_b = min(lo_b, __shfl_xor_sync(0xffffffffu, lo_b, d)); hi_b = max(hi_b, __shfl_xor_sync(0xffffffffu, hi_b, d));
+                    }
+                    auto smallest = [](uint32_t lo) { return lo < kBandHi - kBandLo ? i2f((int32_t)(lo + kBandLo)) : INFINITY; };
+                    auto largest = [](uint32_t hi) { return hi >= 0u - kBandHi ? i2f((int32_t)(hi + kBandHi)) : 0.0f; };   // +0: all above
+                    const float small_a = smallest(lo_a), large_a = largest(hi_a), small_b = smallest(lo_b), large_b = largest(hi_b);
+                    const bool flushes = fmul(large_a, large_b) <= i2f(kFlushBits);
+                    unsigned off_a = 0, off_b = 0, classes = 0;          // masked elements; classes of the rows, and of the columns from bit 8 on
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) {
+                        if (ma[c] - kBandLo >= kBandHi - kBandLo) {
+                            const unsigned k = class_of(ma[c], small_b, large_b);
+                            off_a |= (k & kMasked) << c;
+                            classes |= k;
+                        }
+                        if (mb[c] - kBandLo >= kBandHi - kBandLo) {
+                            const unsigned k = class_of(mb[c], small_a, large_a);
+                            off_b |= (k & kMasked) << c;
+                            classes |= k << 8;
+                        }
+                    }
+                    rows_off[line][at] = (unsigned char)off_a;
+                    cols_off[line][at] = (unsigned char)off_b;
+                    // of the four thread rows, and the eight thread columns, of a warp
+                    classes |= __shfl_xor_sync(0xffffffffu, classes, 1);
+                    classes |= __shfl_xor_sync(0xffffffffu, classes, 2);
+                    const unsigned rows = classes & 15u, cols = (classes | __shfl_xor_sync(0xffffffffu, classes, 4)) >> 8;
+                    const unsigned other = __shfl_xor_sync(0xffffffffu, cols, 8);
+                    if (at % 4 == 0) {
+                        line_kinds[at / 4 * 2 + at / 8][line] = (unsigned char)kind_of(rows, cols, flushes);
+                        line_kinds[at / 4 * 2 + (at / 8 ^ 1)][line] = (unsigned char)kind_of(rows, other, flushes);
+                    }
+                } else if (at < 8) {
+                    line_kinds[at][line] = kPlain;
+                }
                 __syncthreads();
-                kind = kinds[s % 3];
-                if (BM == 64 && kind >= kOther) dirty += kSlabsUnasked * kUnasked;
-            }
-            if (BM == 64 && tid == 0 && dirty >= 2 * kUnasked) atomicOr(&lines[(s + 1) % 3], (dirty - kUnasked) & ~(kUnasked - 1u));
-            if (kind < kOther) {                                // (not 0: the slab is dirty)
-                // Zeros, and everything else in the band (an operand that went through a ReLU).  A pass over one
+                // This warp's lines, in runs of one kind, each kind with a loop of its own with one copy of its body (with three
+                // bodies side by side in one loop the schedule cost 12 %).
+                const unsigned kind = line_kinds[warp][lane % BK];
+                const unsigned plain = __ballot_sync(0xffffffffu, kind == kPlain) & all_lines;
+                const unsigned rows_only = __ballot_sync(0xffffffffu, kind == kRowsOff) & all_lines;
+                const unsigned cols_only = __ballot_sync(0xffffffffu, kind == kColsOff) & all_lines;
+                const unsigned checked = __ballot_sync(0xffffffffu, kind == kChecked) & all_lines;
+                const unsigned nothing = __ballot_sync(0xffffffffu, kind == kNothing) & all_lines;
+                while (kk < BK) {
+                    const unsigned here = 1u << kk;
+                    if (plain & here) {
+                        const int end = run_end(plain);
+#pragma unroll 1
+                        for (; kk < end; ++kk) plain_line(kk);
+                    } else if (cols_only & here) {
+                        const int end = run_end(cols_only);
+#pragma unroll 1
+                        for (; kk < end; ++kk) {
+                            PAMK_FRAGMENTS(kk)
+                            const unsigned off = cols_off[kk][tx];
+#pragma unroll
+                            for (int i = 0; i < MR; ++i)
+#pragma unroll
+                                for (int j = 0; j < MT; ++j)
+                                    if (!(off & (1u << j))) acc[i][j] = fadd(acc[i][j], i2f(iadd(a[i], b[j])));
+                        }
+                    } else if (rows_only & here) {
+                        const int end = run_end(rows_only);
+#pragma unroll 1
+                        for (; kk < end; ++kk) {
+                            PAMK_FRAGMENTS(kk)
+                            const unsigned off = rows_off[kk][ty];
+#pragma unroll
+                            for (int j = 0; j < MT; ++j)
+#pragma unroll
+                                for (int i = 0; i < MR; ++i)
+                                    if (!(off & (1u << i))) acc[i][j] = fadd(acc[i][j], i2f(iadd(a[i], b[j])));
+                        }
+                    } else if (checked & here) {
+                        const int end = run_end(checked);
+#pragma unroll 1
+                        for (; kk < end; ++kk) checked_line(kk, std::true_type{});
+                    } else if (nothing & here) {
+                        kk = run_end(nothing);
+                    } else {                                            // rows (by weights, as above) and columns
+                        PAMK_FRAGMENTS(kk)
+                        const unsigned off = cols_off[kk][tx], rows = rows_off[kk][ty];
+#pragma unroll
+                        for (int i = 0; i < MR; ++i) {
+                            const float w = rows & (1u << i) ? 0.0f : 1.0f;
+                            const int ai = rows & (1u << i) ? 0 : a[i];
+#pragma unroll
+                            for (int j = 0; j < MT; ++j)
+                                if (!(off & (1u << j))) acc[i][j] = __fmaf_rn(i2f(iadd(ai, b[j])), w, acc[i][j]);
+                        }
+                        ++kk;
+                    }
+                }
+            } else if (MT == 4 && !(dirty & kNonZero) && mostly) {
+                // Zeros on the 32x32 tile, whose launches are chains of slabs: a pass over one
                 // side's slab replaces each zero by a value that makes the product in-band and writes a weight beside
                 // it, 0 for a zero and 1 for anything else; the sum then is acc = fma(product, weight, acc), which
                 // is the plain sum for weight 1 and leaves acc alone for weight 0 (the products are finite, and a
-                // sum is never -0).  Two instructions per product, no compare and no predicate, against the four of
-                // "flush or add": 4096x1024x512 with one operand half zeros 387 -> 252 us (clean: 188),
-                // 1024x512x4096 359 -> 237 us, both operands half zeros 387 -> 346 us.  (Unrolling these loops by
-                // two spilled up to 160 bytes in the 128x128 kernels and cost clean slabs 7 %; predicated adds
-                // without weights took 249 and 294 us, and 376 us instead of 288 where an SM holds eight warps.)
-                const bool side_b = kind == kZerosB;
+                // sum is never -0).
+                const bool side_b = !(dirty & kZerosA);
                 float* side = side_b ? Bs[buf] : As[buf];
                 // (the stand-in makes the product the other operand's own pattern, whatever the offset)
                 const int zero_bits = side_b ? 0 : -p.bias_sub, stand_in = side_b ? p.bias_sub : 0;
@@ -503,45 +683,45 @@ gemm_kernel(const GemmParams p) {
                     *reinterpret_cast<float4*>(weights + at) = w;
                 }
                 __syncthreads();
-                if (kind == (kZerosA | kZerosB)) {
+                if ((dirty & (kZerosA | kZerosB)) == (kZerosA | kZerosB)) {
                     // (weights for A's zeros, a predicate for B's)
 #pragma unroll 1
-                    for (int kk = 0; kk < BK; ++kk) {
+                    for (; kk < BK; ++kk) {
                         PAMK_FRAGMENTS(kk)
                         PAMK_WEIGHTS(kk, ty)
 #pragma unroll
-                        for (int j = 0; j < MT; ++j) {
+                        for (int j = 0; j < 4; ++j) {
                             const bool on = 2u * (uint32_t)b[j] != 0;
 #pragma unroll
-                            for (int i = 0; i < MR; ++i)
-                                if (on) acc[i][j] = __fmaf_rn(i2f(iadd(a[i], b[j])), w[i], acc[i][j]);
+                            for (int i = 0; i < 4; ++i)
+                                if (on) acc[i % MR][j] = __fmaf_rn(i2f(iadd(a[i], b[j])), w[i], acc[i % MR][j]);
                         }
                     }
                 } else if (!side_b) {
 #pragma unroll 1
-                    for (int kk = 0; kk < BK; ++kk) {
+                    for (; kk < BK; ++kk) {
                         PAMK_FRAGMENTS(kk)
                         PAMK_WEIGHTS(kk, ty)
 #pragma unroll
-                        for (int i = 0; i < MR; ++i)
+                        for (int i = 0; i < 4; ++i)
 #pragma unroll
-                            for (int j = 0; j < MT; j += 2) fma_pair(acc[i][j], acc[i][j + 1], iadd(a[i], b[j]), iadd(a[i], b[j + 1]), w[i], w[i]);
+                            for (int j = 0; j < 4; j += 2) fma_pair(acc[i % MR][j], acc[i % MR][j + 1], iadd(a[i], b[j]), iadd(a[i], b[j + 1]), w[i], w[i]);
                     }
                 } else {
 #pragma unroll 1
-                    for (int kk = 0; kk < BK; ++kk) {
+                    for (; kk < BK; ++kk) {
                         PAMK_FRAGMENTS(kk)
                         PAMK_WEIGHTS(kk, tx)
 #pragma unroll
-                        for (int i = 0; i < MR; ++i)
+                        for (int i = 0; i < 4; ++i)
 #pragma unroll
-                            for (int j = 0; j < MT; j += 2) fma_pair(acc[i][j], acc[i][j + 1], iadd(a[i], b[j]), iadd(a[i], b[j + 1]), w[j], w[j + 1]);
+                            for (int j = 0; j < 4; j += 2) fma_pair(acc[i % MR][j], acc[i % MR][j + 1], iadd(a[i], b[j]), iadd(a[i], b[j + 1]), w[j], w[j + 1]);
                     }
                 }
             } else {
-                // lines that hold an element above the band: can a product leave the pass range?
+                // lines of a slab that holds an element above the band: can a product leave the pass range?
                 unsigned full = 0;
-                if (dirty & (kDirty & ~all_lines)) {                // (uniform: read from shared memory after a barrier)
+                if (dirty & kAbove) {                               // (uniform: read from shared memory after a barrier)
                     constexpr int kLanes = T::kThreads / BK;        // threads that share one k line
                     const int line = tid / kLanes, lane = tid % kLanes;
                     if (tid == 0) overflow_lines = 0;
@@ -562,75 +742,29 @@ gemm_kernel(const GemmParams p) {
                     __syncthreads();
                     full = overflow_lines;
                 }
-                // Most lines dirty, none can overflow (e.g. gradients of which most lie below the band): "flush or add"
-                // for the whole slab, which is exact for clean lines too.  The 64x64 tile runs it in the loop for
-                // runs below: with a copy of its own, 512 instructions, its dirty slabs wait for instructions
-                // (2235x183x1152 with 1 % specials 148 -> 109 us; 140 us before the loops for zeros came).
-                const bool flush_all = __popc(dirty & all_lines) * 4 >= BK * 3 && full == 0;
-                if (BM != 64 && flush_all) {
-#pragma unroll (MT == 4 ? 4 : 2)
-                    for (int kk = 0; kk < BK; ++kk) {
-                        PAMK_FRAGMENTS(kk)
-                        float araw[MR];          // a[] holds pre-biased patterns; the rule needs the values
-#pragma unroll
-                        for (int i = 0; i < MR; ++i) araw[i] = i2f(iadd(a[i], p.bias_sub));
-#pragma unroll
-                        for (int i = 0; i < MR; ++i)
-#pragma unroll
-                            for (int j = 0; j < MT; ++j) {
-                                const float mag = fabsf(fmul(araw[i], i2f(b[j])));
-                                if (mag > i2f(kFlushBits)) acc[i][j] = fadd(acc[i][j], i2f(iadd(a[i], b[j])));
-                            }
-                    }
+                // Most lines dirty, none can overflow (e.g. gradients of which most lie below the band): "flush or add" for the
+                // whole slab, which is exact for clean lines too.  The 64x64 tile runs it in the loop for runs below: with a copy
+                // of its own, 512 instructions, its dirty slabs wait for instructions (2235x183x1152 with 1 % specials 148 -> 109 us).
+                const bool flush_all = mostly && full == 0;
+                if (MT == 4 && flush_all) {
+#pragma unroll 4
+                    for (int k = 0; k < BK; ++k) checked_line(k, std::false_type{});
                 } else {
-                    // The lines are walked in runs of one kind, each run by a loop of its own with one copy of
-                    // its body (with the three bodies side by side in one loop the schedule cost 12 %).
-                    const unsigned flush = flush_all ? all_lines : dirty & ~full & all_lines;
-                    int kk = 0;
+                    const unsigned flush = flush_all ? all_lines : any & ~full;
                     while (kk < BK) {
                         const unsigned here = 1u << kk;
                         if (full & here) {
-                            PAMK_FRAGMENTS(kk)
-                            float araw[MR];
-#pragma unroll
-                            for (int i = 0; i < MR; ++i) araw[i] = i2f(iadd(a[i], p.bias_sub));
-#pragma unroll
-                            for (int i = 0; i < MR; ++i)
-#pragma unroll
-                                for (int j = 0; j < MT; ++j) {
-                                    const float mag = fabsf(fmul(araw[i], i2f(b[j])));
-                                    const float prod = mag <= i2f(kPassBits) ? i2f(iadd(a[i], b[j])) : quiet_nan();
-                                    if (!(mag <= i2f(kFlushBits))) acc[i][j] = fadd(acc[i][j], prod);
-                                }
+                            checked_line(kk, std::true_type{});
                             ++kk;
                         } else if (flush & here) {
-                            const unsigned others = ~flush >> kk;
-                            const int end = min(BK, kk + __ffs((int)others) - 1);
+                            const int end = run_end(flush);
 #pragma unroll 1
-                            for (; kk < end; ++kk) {
-                                PAMK_FRAGMENTS(kk)
-                                float araw[MR];
-#pragma unroll
-                                for (int i = 0; i < MR; ++i) araw[i] = i2f(iadd(a[i], p.bias_sub));
-#pragma unroll
-                                for (int i = 0; i < MR; ++i)
-#pragma unroll
-                                    for (int j = 0; j < MT; ++j) {
-                                        const float mag = fabsf(fmul(araw[i], i2f(b[j])));
-                                        if (mag > i2f(kFlushBits)) acc[i][j] = fadd(acc[i][j], i2f(iadd(a[i], b[j])));
-                                    }
-                            }
+                            for (; kk < end; ++kk) checked_line(kk, std::false_type{});
                         } else {
-                            const unsigned others = (dirty & all_lines) >> kk;
+                            const unsigned others = any >> kk;
                             const int end = others ? kk + __ffs((int)others) - 1 : BK;
 #pragma unroll 1
-                            for (; kk < end; ++kk) {
-                                PAMK_FRAGMENTS(kk)
-#pragma unroll
-                                for (int i = 0; i < MR; ++i)
-#pragma unroll
-                                    for (int j = 0; j < MT; j += 2) add_pair(acc[i][j], acc[i][j + 1], iadd(a[i], b[j]), iadd(a[i], b[j + 1]));
-                            }
+                            for (; kk < end; ++kk) plain_line(kk);
                         }
                     }
                 }
