@@ -28,6 +28,7 @@
 //
 // The same skeleton serves true-multiply products (standard_matmul) and the exact-gradient
 // product (pam_matmul_bwd_kernel, cuda_kernels.cu:729-832).
+#include <array>
 #include <type_traits>
 
 #include "common.cuh"
@@ -1019,12 +1020,10 @@ bool fine_slabs(int64_t ctas, int64_t K) {
 // that exists.
 int g_tile_policy = 0;
 
-// seven_rows: the operands allow TileLarge7 (the callers that only ask for the split do not know, and get the split of
-// the other tiles).
-Plan make_plan(int mode, int64_t batch, int64_t M, int64_t N, int64_t K, int split_request, bool seven_rows = false) {
+Plan search_plan(int mode, int64_t batch, int64_t M, int64_t N, int64_t K, int split_request) {
     const Plan large = plan_for<TileLarge>(mode, batch, M, N, K, split_request);
     if (mode == kStd || g_tile_policy == 1) return large;    // the true-multiply product uses the large tile
-    if (g_tile_policy == 4) return seven_rows && split_request <= 1 ? plan_for<TileLarge7>(mode, batch, M, N, K, 1) : large;
+    if (g_tile_policy == 4) return large;
     const Plan small = plan_for<TileSmall>(mode, batch, M, N, K, split_request);
     if (g_tile_policy == 2 || (g_tile_policy == 3 && mode != kPam)) return small;
     Plan best = small.cost < large.cost ? small : large;
@@ -1046,12 +1045,26 @@ Plan make_plan(int mode, int64_t batch, int64_t M, int64_t N, int64_t K, int spl
             if (fine.cost < tiny.cost) tiny = fine;
         }
         if (g_tile_policy == 3 || tiny.cost < margin * best.cost) best = tiny;
-        if (seven_rows && split_request <= 1 && g_tile_policy == 0) {
-            const Plan seven = plan_for<TileLarge7>(mode, batch, M, N, K, 1);
-            if (seven.cost < 0.95 * best.cost) best = seven;
-        }
     }
     return best;
+}
+
+// seven_rows: the operands allow TileLarge7 (the callers that only ask for the split do not know, and get the split of
+// the other tiles).  A caller asks for the split and then calls the product: the last search of a thread, a function of its
+// arguments alone, is kept, so that the second does not pay for it again.
+Plan make_plan(int mode, int64_t batch, int64_t M, int64_t N, int64_t K, int split_request, bool seven_rows = false) {
+    struct Search {
+        std::array<int64_t, 8> key;
+        Plan plan;
+    };
+    thread_local Search last{};                              // (all zero: the key of no search, which has at least one SM)
+    const std::array<int64_t, 8> key{mode, batch, M, N, K, split_request, g_tile_policy, sm_count()};
+    if (last.key != key) last = {key, search_plan(mode, batch, M, N, K, split_request)};
+    if (seven_rows && split_request <= 1 && (g_tile_policy == 0 || g_tile_policy == 4)) {
+        const Plan seven = plan_for<TileLarge7>(mode, batch, M, N, K, 1);
+        if (g_tile_policy == 4 || seven.cost < 0.95 * last.plan.cost) return seven;
+    }
+    return last.plan;
 }
 
 bool workspace_ok(const void* ws, size_t bytes, int splits, int64_t count) {
@@ -1069,7 +1082,7 @@ int run(int mode, GemmParams p, bool a_kc, bool b_kc, int split_k, void* workspa
     }
     if (split_k < 0) return PAMK_ERR_ARG;
     const bool vec = vectorisable(p.A, a_kc, p.M, p.K) && vectorisable(p.B, b_kc, p.N, p.K);
-    const bool seven_rows = mode == kPam && p.batch == 1 && a_kc && vec;
+    const bool seven_rows = mode == kPam && p.batch == 1 && a_kc && vec && p.M <= 65535 * TileLarge7::kRows;    // (grid.y, see below)
     Plan pl = p.K == 0 ? Plan{kTileSmall, 1, 0.0} : make_plan(mode, p.batch, p.M, p.N, p.K, split_k, seven_rows);   // K = 0: rows of bias
     if (pl.splits > 1 && !workspace_ok(workspace, workspace_bytes, pl.splits, count)) {
         if (split_k != 0) return PAMK_ERR_WORKSPACE;         // an explicit split needs its scratch

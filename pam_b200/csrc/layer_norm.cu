@@ -427,8 +427,22 @@ __global__ void __launch_bounds__(kGradWarps * 32) ln_param_grad_kernel(const fl
     const int col = blockIdx.x * 32 + lane;
     float sw = 0.0f, sb = 0.0f;
     if (col < width) {
-#pragma unroll 4
-        for (int k = wid; k < ctas; k += kGradWarps) {
+        // eight partials of each sum requested at a time: with a CTA per 32 columns there is little but the loads' latency
+        int k = wid;
+        for (; k + 7 * kGradWarps < ctas; k += 8 * kGradWarps) {
+            float w[8], b[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                w[u] = __ldg(partials + ((int64_t)(k + u * kGradWarps) * 2) * width + col);
+                b[u] = __ldg(partials + ((int64_t)(k + u * kGradWarps) * 2 + 1) * width + col);
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                sw = fadd(sw, w[u]);
+                sb = fadd(sb, b[u]);
+            }
+        }
+        for (; k < ctas; k += kGradWarps) {
             sw = fadd(sw, __ldg(partials + ((int64_t)k * 2) * width + col));
             sb = fadd(sb, __ldg(partials + ((int64_t)k * 2 + 1) * width + col));
         }
