@@ -107,9 +107,7 @@ int pamk_pa_log_bwd(const float* x, const float* dy, float* dx, int64_t n, float
  *          >1 = K is cut into that many contiguous ranges summed independently and then added in
  *               range order (deterministic, but a different association than the reference);
  *               needs `workspace` of pamk_matmul_workspace_bytes(...) bytes, 256-byte aligned.
- *          0  = let the library choose; it only splits when `workspace` is large enough
- *               (pamk_matmul_auto_split's ranges), and need not split where another tile shape
- *               fills the GPU without.
+ *          0  = let the library choose; it only splits when `workspace` is large enough.
  */
 #define PAMK_MUL_PAM 0
 #define PAMK_MUL_STANDARD 1
@@ -146,8 +144,7 @@ int pamk_matmul_strided(const float* A, const float* B, float* C,
                         int split_k, void* workspace, size_t workspace_bytes, void* stream);
 /* Scratch needed by pamk_matmul for a given split_k (0 for split_k <= 1). */
 size_t pamk_matmul_workspace_bytes(int64_t batch, int64_t M, int64_t N, int split_k);
-/* The split the library would choose for split_k = 0 given unlimited workspace (an upper bound: operands
- * that lie contiguous along K may get a tile shape that needs none). */
+/* The split the library would choose for split_k = 0 given unlimited workspace. */
 int pamk_matmul_auto_split(int64_t batch, int64_t M, int64_t N, int64_t K);
 
 /* Split-K PAM product for callers that cannot allocate.  It has no counterpart in the reference.

@@ -13,7 +13,7 @@ extern "C" {
  * same problem and check that results do not depend on the tile (the library normally picks a
  * 128x128, a 64x64 or, for small or ragged-edged products, a 32x32 tile per problem from a cost
  * model).  0 = by cost model (default), 1 = always 128x128, 2 = always 64x64, 3 = always
- * 32x32 (products that have no 32x32 kernel use 64x64), 4 = 112x128 for unsplit PAM products whose operands
+ * 32x32 (products that have no 32x32 kernel use 64x64), 4 = 112x128 for plain PAM products whose operands
  * allow it (A contiguous along K, 128-bit loads), else 128x128.  Process-wide and not thread-safe, which is
  * why it is kept out of pam_b200.h.  No counterpart in the reference. */
 int pamk_test_set_tile_policy(int policy);
@@ -22,6 +22,11 @@ int pamk_test_set_tile_policy(int policy);
  * current policy, with the automatic split: lets a test pin the measured-best choices without a GPU.
  * Negative (PAMK_ERR_ARG) for an empty problem.  No counterpart in the reference. */
 int pamk_test_planned_tile(int64_t batch, int64_t M, int64_t N, int64_t K);
+
+/* Rows per tile (128, 112, 64 or 32) of a plain PAM product of these dimensions and K ranges (0 = the library's choice)
+ * whose operands allow every tile: A contiguous along K, 128-bit loads.  Negative (PAMK_ERR_ARG) for an empty problem or a
+ * negative split.  No counterpart in the reference. */
+int pamk_test_planned_rows(int64_t M, int64_t N, int64_t K, int split_k);
 
 #ifdef __cplusplus
 }

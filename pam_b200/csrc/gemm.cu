@@ -28,7 +28,6 @@
 //
 // The same skeleton serves true-multiply products (standard_matmul) and the exact-gradient
 // product (pam_matmul_bwd_kernel, cuda_kernels.cu:729-832).
-#include <array>
 #include <type_traits>
 
 #include "common.cuh"
@@ -86,11 +85,13 @@ struct Tile {
     static constexpr int kRowsPerWarp = 32 / (BK_ / 4);
 };
 using TileLarge = Tile<128, 128, 16, 2>;
-// 112x128x16: the large tile with seven rows per thread, for products of few large tiles per SM whose number then fits
-// the SMs better (4096 rows x 512: 128 tiles of 128 rows leave 20 of 148 SMs idle, 148 tiles of 112 none; one CTA of
-// this size already runs an SM at 95 % of what two do).  Row slot 7 of every thread is staged with a copy of a neighbouring row and
-// takes no part in the sums.  4096x512x512 96.6 us (two K ranges and their reduction) -> 83.3, 4096x1024x512 174.5 -> 153.4,
-// 2000x1024x512 96.7 -> 83.4; of 94 products of all sizes those that get it gain 4 to 14 %.
+// 112x128x16: the large tile with seven rows per thread, for unsplit products of few large tiles per SM whose number then
+// fits the SMs better (4096 rows x 1024: 256 tiles of 128 rows leave 40 of the 148 SMs with one tile where the others have two, 296
+// tiles of 112 none; one CTA of this size already runs an SM at 95 % of what two do).  Row slot 7 of every thread is staged
+// with a copy of a neighbouring row and takes no part in the sums.  4096x1024x512 174.5 -> 153.4 us, 8192x512x512 the same.
+// Products that the plan cuts along K do not take it: unsplit they would run 14 % faster (4096x512x512 98.6 -> 83.5 us), but their sums
+// would depend on whether the operands' layout and alignment allow this tile; with the plan's ranges summed one
+// after another in one CTA they cost 5.5 to 6.5 us per range (89.9 us, 2304x768x256 of 4 ranges 46.6 -> 57.0).
 using TileLarge7 = Tile<128, 128, 16, 2, 8, 7>;
 using TileSmall = Tile<64, 64, 8, 8>;
 // 32x32x16 with a 4x4 micro-tile, 64 threads: batched products whose matrices are a fraction of a
@@ -1020,7 +1021,7 @@ bool fine_slabs(int64_t ctas, int64_t K) {
 // that exists.
 int g_tile_policy = 0;
 
-Plan search_plan(int mode, int64_t batch, int64_t M, int64_t N, int64_t K, int split_request) {
+Plan make_plan(int mode, int64_t batch, int64_t M, int64_t N, int64_t K, int split_request) {
     const Plan large = plan_for<TileLarge>(mode, batch, M, N, K, split_request);
     if (mode == kStd || g_tile_policy == 1) return large;    // the true-multiply product uses the large tile
     if (g_tile_policy == 4) return large;
@@ -1049,22 +1050,12 @@ Plan search_plan(int mode, int64_t batch, int64_t M, int64_t N, int64_t K, int s
     return best;
 }
 
-// seven_rows: the operands allow TileLarge7 (the callers that only ask for the split do not know, and get the split of
-// the other tiles).  A caller asks for the split and then calls the product: the last search of a thread, a function of its
-// arguments alone, is kept, so that the second does not pay for it again.
-Plan make_plan(int mode, int64_t batch, int64_t M, int64_t N, int64_t K, int split_request, bool seven_rows = false) {
-    struct Search {
-        std::array<int64_t, 8> key;
-        Plan plan;
-    };
-    thread_local Search last{};                              // (all zero: the key of no search, which has at least one SM)
-    const std::array<int64_t, 8> key{mode, batch, M, N, K, split_request, g_tile_policy, sm_count()};
-    if (last.key != key) last = {key, search_plan(mode, batch, M, N, K, split_request)};
-    if (seven_rows && split_request <= 1 && (g_tile_policy == 0 || g_tile_policy == 4)) {
-        const Plan seven = plan_for<TileLarge7>(mode, batch, M, N, K, 1);
-        if (g_tile_policy == 4 || seven.cost < 0.95 * last.plan.cost) return seven;
-    }
-    return last.plan;
+// Whether a plain PAM product planned as `pl` takes TileLarge7 where its operands allow that.  Only unsplit ones: the ranges of K, and
+// with them the order of the sums, follow from the shape alone, not from how the operands lie in memory.
+bool seven_rows_better(const Plan& pl, int64_t M, int64_t N, int64_t K) {
+    if (pl.splits > 1 || (g_tile_policy != 0 && g_tile_policy != 4)) return false;
+    if (M > (int64_t)65535 * TileLarge7::kRows) return false;                          // (grid.y)
+    return g_tile_policy == 4 || plan_for<TileLarge7>(kPam, 1, M, N, K, 1).cost < 0.95 * pl.cost;
 }
 
 bool workspace_ok(const void* ws, size_t bytes, int splits, int64_t count) {
@@ -1082,19 +1073,19 @@ int run(int mode, GemmParams p, bool a_kc, bool b_kc, int split_k, void* workspa
     }
     if (split_k < 0) return PAMK_ERR_ARG;
     const bool vec = vectorisable(p.A, a_kc, p.M, p.K) && vectorisable(p.B, b_kc, p.N, p.K);
-    const bool seven_rows = mode == kPam && p.batch == 1 && a_kc && vec && p.M <= 65535 * TileLarge7::kRows;    // (grid.y, see below)
-    Plan pl = p.K == 0 ? Plan{kTileSmall, 1, 0.0} : make_plan(mode, p.batch, p.M, p.N, p.K, split_k, seven_rows);   // K = 0: rows of bias
+    Plan pl = p.K == 0 ? Plan{kTileSmall, 1, 0.0} : make_plan(mode, p.batch, p.M, p.N, p.K, split_k);   // K = 0: rows of bias
     if (pl.splits > 1 && !workspace_ok(workspace, workspace_bytes, pl.splits, count)) {
         if (split_k != 0) return PAMK_ERR_WORKSPACE;         // an explicit split needs its scratch
-        pl = make_plan(mode, p.batch, p.M, p.N, p.K, 1, seven_rows);     // automatic: fall back to no split
+        pl = make_plan(mode, p.batch, p.M, p.N, p.K, 1);     // automatic: fall back to no split
     }
     // the M tiles ride on grid.y (at most 65535): a very tall product planned with a small tile moves to
     // the 128x128 tile, which reaches 8.3 M rows
-    if (pl.tile != kTileLarge && pl.tile != kTileLarge7 && (p.M + (pl.tile == kTileTiny ? TileTiny::BM : TileSmall::BM) - 1) /
+    if (pl.tile != kTileLarge && (p.M + (pl.tile == kTileTiny ? TileTiny::BM : TileSmall::BM) - 1) /
                                          (pl.tile == kTileTiny ? TileTiny::BM : TileSmall::BM) > 65535) {
         const int splits = pl.splits;
         pl = plan_for<TileLarge>(mode, p.batch, p.M, p.N, p.K, splits);
     }
+    if (mode == kPam && p.batch == 1 && p.K > 0 && a_kc && vec && seven_rows_better(pl, p.M, p.N, p.K)) pl.tile = kTileLarge7;
     const int bm = pl.tile == kTileTiny ? TileTiny::BM : (pl.tile == kTileSmall ? TileSmall::BM : (pl.tile == kTileLarge7 ? TileLarge7::kRows : TileLarge::BM));
     const int bn = pl.tile == kTileTiny ? TileTiny::BN : (pl.tile == kTileSmall ? TileSmall::BN : TileLarge::BN);
     const int64_t ctas = ((p.N + bn - 1) / bn) * (int64_t)((p.M + bm - 1) / bm) * p.batch * pl.splits;
@@ -1226,6 +1217,13 @@ int pamk_test_planned_tile(int64_t batch, int64_t M, int64_t N, int64_t K) {
     if (batch <= 0 || M <= 0 || N <= 0 || K <= 0) return PAMK_ERR_ARG;
     const int tile = make_plan(kPam, batch, M, N, K, 0).tile;
     return tile == kTileLarge ? 128 : (tile == kTileSmall ? 64 : 32);
+}
+
+int pamk_test_planned_rows(int64_t M, int64_t N, int64_t K, int split_k) {
+    if (M <= 0 || N <= 0 || K <= 0 || split_k < 0 || !dims_ok(1, M, N, K)) return PAMK_ERR_ARG;
+    const Plan pl = make_plan(kPam, 1, M, N, K, split_k);
+    if (seven_rows_better(pl, M, N, K)) return TileLarge7::kRows;
+    return pl.tile == kTileLarge ? TileLarge::BM : (pl.tile == kTileSmall ? TileSmall::BM : TileTiny::BM);
 }
 
 int pamk_matmul_auto_split(int64_t batch, int64_t M, int64_t N, int64_t K) {

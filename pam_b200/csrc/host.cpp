@@ -157,8 +157,7 @@ Mat matrix(Tensor& t) {
 Tensor product(const Mat& a, const Mat& b, const Tensor& bias, int64_t batch, int64_t M, int64_t N, int64_t K, double offset,
                at::IntArrayRef out_shape, const Tensor& like) {
     Tensor out = empty_on(out_shape, like);
-    const bool strict = g_strict.load(std::memory_order_relaxed);
-    const int split = strict ? 1 : lib.pamk_matmul_auto_split(batch, M, N, K);
+    const int split = g_strict.load(std::memory_order_relaxed) ? 1 : lib.pamk_matmul_auto_split(batch, M, N, K);
     Tensor ws;
     size_t bytes = 0;
     if (split > 1) {
@@ -166,7 +165,7 @@ Tensor product(const Mat& a, const Mat& b, const Tensor& bias, int64_t batch, in
         ws = scratch_bytes(bytes, like);
     }
     check(lib.pamk_matmul_bias(PAMK_MUL_PAM, a.p, b.p, ptr(bias), ptr(out), batch, M, N, K, a.sb, a.sr, a.sc, b.sb, b.sr, b.sc,
-                               (float)offset, strict ? 1 : 0, ws.defined() ? ws.data_ptr() : nullptr, bytes, stream_of(like)),
+                               (float)offset, split, ws.defined() ? ws.data_ptr() : nullptr, bytes, stream_of(like)),
           "pamk_matmul");
     return out;
 }
@@ -195,7 +194,7 @@ Tensor column_sum(const Tensor& x, int64_t rows, int64_t cols) {
     return out;
 }
 
-// One product of the attention path: the plan is the plain product's of the same shape.
+// One product of the attention path: the split is the plain product's of the same shape.
 void strided(const float* a, const float* b, float* c, int64_t outer, int64_t inner, int64_t M, int64_t N, int64_t K,
              const std::array<int64_t, 4>& sa, const std::array<int64_t, 4>& sb, const std::array<int64_t, 3>& sc,
              double offset, std::optional<double> post, const Tensor& like) {
@@ -207,7 +206,7 @@ void strided(const float* a, const float* b, float* c, int64_t outer, int64_t in
         ws = scratch_bytes(bytes, like);
     }
     check(lib.pamk_matmul_strided(a, b, c, outer, inner, M, N, K, sa[0], sa[1], sa[2], sa[3], sb[0], sb[1], sb[2], sb[3],
-                                  sc[0], sc[1], sc[2], (float)offset, post.has_value(), (float)post.value_or(0.0), 0,
+                                  sc[0], sc[1], sc[2], (float)offset, post.has_value(), (float)post.value_or(0.0), split,
                                   ws.defined() ? ws.data_ptr() : nullptr, bytes, stream_of(like)),
           "pamk_matmul_strided");
 }

@@ -169,14 +169,12 @@ def _matmul(kind, A, B, offset, dims, split_k=None, bias=None):
     M, K, N = A.shape[-2], A.shape[-1], B.shape[-1]
     out = torch.empty((batch, M, N) if dims == 3 else (M, N), dtype=torch.float32, device=device)
     handle = _lib.lib()
-    ranges = split_k
     if split_k is None:
         # (the true-multiply product has one tile shape and its own cost model: it is never split here)
-        split_k = 1 if _strict_k_order or kind != _lib.MUL_PAM else 0          # 0: the library's choice
-        ranges = split_k or handle.pamk_matmul_auto_split(batch, M, N, K)
+        split_k = 1 if _strict_k_order or kind != _lib.MUL_PAM else handle.pamk_matmul_auto_split(batch, M, N, K)
     ws_ptr, ws_bytes = None, 0
-    if ranges > 1:
-        ws_bytes = handle.pamk_matmul_workspace_bytes(batch, M, N, ranges)
+    if split_k > 1:
+        ws_bytes = handle.pamk_matmul_workspace_bytes(batch, M, N, split_k)
         ws_ptr = _workspace(device, ws_bytes).data_ptr()
     with _lib.device_guard(device):
         if bias is None:

@@ -232,7 +232,7 @@ def attention_supported(qkv, num_heads, approx_bwd=False):
 
 
 def _strided_product(dev, a_ptr, b_ptr, c_ptr, outer, inner, M, N, K, sa, sb, sc, offset, post_scale=None):
-    """One pamk_matmul_strided call with the plan that the plain product of the same shape would get."""
+    """One pamk_matmul_strided call with the split the plain product of the same shape would get."""
     handle = _lib.lib()
     split = handle.pamk_matmul_auto_split(outer * inner, M, N, K)
     ws_ptr, ws_bytes = None, 0
@@ -241,7 +241,7 @@ def _strided_product(dev, a_ptr, b_ptr, c_ptr, outer, inner, M, N, K, sa, sb, sc
         ws_ptr = _workspace(dev, ws_bytes).data_ptr()
     with _lib.device_guard(dev):
         status = handle.pamk_matmul_strided(a_ptr, b_ptr, c_ptr, outer, inner, M, N, K, *sa, *sb, *sc, offset,
-                                            int(post_scale is not None), float(post_scale or 0.0), 0,
+                                            int(post_scale is not None), float(post_scale or 0.0), split,
                                             ws_ptr, ws_bytes, _lib.stream_ptr(dev))
     _lib.check(status, "pamk_matmul_strided")
 

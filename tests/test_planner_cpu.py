@@ -48,6 +48,19 @@ def test_tile_choices_that_sweeps_measured_best(lib, batch, M, N, K, tile):
     assert lib.pamk_test_planned_tile(batch, M, N, K) == tile
 
 
+@pytest.mark.parametrize("M,N,K,rows", [
+    (4096, 1024, 512, 112), (4096, 1024, 1024, 112), (8192, 512, 512, 112), (2000, 2048, 512, 112),   # one or two per SM, none left over
+    (4096, 512, 512, 128), (4096, 512, 1024, 128), (4096, 512, 10000, 128),     # cut along K: the order of the sums is the shape's
+    (4096, 4096, 4096, 128), (4096, 10000, 512, 128), (TOKENS, 192, 192, 64), (32, 512, 512, 32),
+])
+def test_rows_per_tile_of_aligned_products(lib, M, N, K, rows):
+    """What runs where A lies contiguous along K and both operands allow 128-bit loads."""
+    assert lib.pamk_test_set_tile_policy(0) == 0
+    split = lib.pamk_matmul_auto_split(1, M, N, K)
+    assert lib.pamk_test_planned_rows(M, N, K, split) == rows
+    assert rows != 112 or split == 1
+
+
 def test_planner_basic_properties(lib):
     # large outputs fill the GPU without a split; tiny K is never split; empty problems do not divide by zero
     assert lib.pamk_matmul_auto_split(1, 4096, 4096, 4096) == 1
