@@ -194,11 +194,11 @@ Tensor column_sum(const Tensor& x, int64_t rows, int64_t cols) {
     return out;
 }
 
-// One product of the attention path: the split is the plain product's of the same shape.
+// One product of the attention path: the split is the plain product's of the same shape (none in strict k order).
 void strided(const float* a, const float* b, float* c, int64_t outer, int64_t inner, int64_t M, int64_t N, int64_t K,
              const std::array<int64_t, 4>& sa, const std::array<int64_t, 4>& sb, const std::array<int64_t, 3>& sc,
              double offset, std::optional<double> post, const Tensor& like) {
-    const int split = lib.pamk_matmul_auto_split(outer * inner, M, N, K);
+    const int split = g_strict.load(std::memory_order_relaxed) ? 1 : lib.pamk_matmul_auto_split(outer * inner, M, N, K);
     Tensor ws;
     size_t bytes = 0;
     if (split > 1) {

@@ -232,9 +232,10 @@ def attention_supported(qkv, num_heads, approx_bwd=False):
 
 
 def _strided_product(dev, a_ptr, b_ptr, c_ptr, outer, inner, M, N, K, sa, sb, sc, offset, post_scale=None):
-    """One pamk_matmul_strided call with the split the plain product of the same shape would get."""
+    """One pamk_matmul_strided call with the split the plain product of the same shape would get (none in strict k order)."""
+    from .cuda_bindings import strict_k_order
     handle = _lib.lib()
-    split = handle.pamk_matmul_auto_split(outer * inner, M, N, K)
+    split = 1 if strict_k_order() else handle.pamk_matmul_auto_split(outer * inner, M, N, K)
     ws_ptr, ws_bytes = None, 0
     if split > 1:
         ws_bytes = handle.pamk_matmul_workspace_bytes(outer * inner, M, N, split)

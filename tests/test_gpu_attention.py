@@ -70,6 +70,51 @@ def test_strided_attention_against_the_oracle(oracle):
     assert_close_nan(a.grad, b.grad, 1e-4, 1e-4 * float(b.grad.abs().max()), "d qkv")
 
 
+@pytest.mark.parametrize("native", [True, False], ids=["native", "python"])
+def test_strict_k_order_holds_for_the_attention_products(native, monkeypatch, oracle):
+    """3 x 256 x 64 x 256 is split by default (8 ranges): in strict k order both attention forms equal the strict chain, and the
+    products inside it the oracle, which sums one range."""
+    import pam_b200 as pam
+    from pam_b200 import _lib, fused
+    dev = torch.device("cuda", 0)
+    B, N, heads, hd = 1, 256, 3, 64
+    assert _lib.lib().pamk_matmul_auto_split(B * heads, N, hd, N) > 1
+    g = torch.Generator().manual_seed(11)
+    qkv0 = torch.randn(B, N, 3 * heads * hd, generator=g).to(dev)
+    q0, k0, v0 = (t.contiguous() for t in qkv0.chunk(3, dim=-1))
+    dout = torch.randn(B, N, heads * hd, generator=g).to(dev)
+    probs, v = torch.rand(3, N, N, generator=g), torch.randn(3, N, hd, generator=g)
+    if not native:
+        monkeypatch.setattr(_lib, "host", lambda: None)
+
+    def both():
+        a = qkv0.clone().requires_grad_()
+        ya = fused.attention_qkv(a, heads, hd ** -0.5)
+        ya.backward(dout)
+        q, k, w = (t.clone().requires_grad_() for t in (q0, k0, v0))
+        yb = fused.attention_heads(q, k, w, heads)
+        yb.backward(dout)
+        return [ya.detach(), a.grad, yb.detach(), q.grad, k.grad, w.grad]
+
+    default = both()
+    pam.set_strict_k_order(True)
+    try:
+        got = both()
+        b = qkv0.clone().requires_grad_()
+        yb = chain(pam, b, heads, hd ** -0.5, KW)
+        yb.backward(dout)
+        q, k, w = (t.clone().requires_grad_() for t in (q0, k0, v0))
+        yc = heads_chain(pam, q, k, w, heads, None, KW)
+        yc.backward(dout)
+        assert_bits_equal(pam.bmm(probs.to(dev), v.to(dev)), oracle.kernels().pam_bmm_fwd(probs, v, True, True, 1.0))
+    finally:
+        pam.set_strict_k_order(False)
+    for name, a, c in zip(("context", "d qkv", "context of separate projections", "d q", "d k", "d v"), got,
+                          (yb.detach(), b.grad, yc.detach(), q.grad, k.grad, w.grad)):
+        assert_bits_equal(a, c, name)
+    assert not torch.equal(default[0], got[0])
+
+
 def test_unsupported_calls_are_refused():
     from pam_b200 import fused
     dev = torch.device("cuda", 0)
