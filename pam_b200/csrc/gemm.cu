@@ -261,12 +261,15 @@ __device__ __forceinline__ int slab_line(int id, int c) {
     return KC ? (id % (T::BK / 4)) * 4 + c : id / (R / 4);
 }
 
-// A slab's word: bit k for a k line that holds an out-of-band element, and what such elements there are.
-enum Word : unsigned { kZerosA = 1u << 16, kZerosB = 1u << 17, kNonZero = 1u << 18, kAbove = 1u << 19 };
+// A slab's word: bit k for a k line that holds an out-of-band element, which operand such elements are in, and whether any is
+// not zero, or above the band.
+enum Word : unsigned { kInA = 1u << 16, kInB = 1u << 17, kNonZero = 1u << 18, kAbove = 1u << 19 };
 
-// The word's bits for this thread's staged elements.
+// The k lines of this thread's staged elements that are out of the band; `bits` collects the magnitudes of those elements, `top` the
+// largest magnitude (twice the pattern, both).  No branch per element: with one, few such elements in a slab cost
+// more than many, 4096^3 with 2 % specials 1.5 %.
 template <class T, int R, int NT, bool KC>
-__device__ __forceinline__ unsigned dirty_lines(const float (&r)[NT * 4], int tid, unsigned zeros) {
+__device__ __forceinline__ unsigned dirty_lines(const float (&r)[NT * 4], int tid, uint32_t& bits, uint32_t& top) {
     unsigned lines = 0;
 #pragma unroll
     for (int t = 0; t < NT; ++t)
@@ -274,9 +277,10 @@ __device__ __forceinline__ unsigned dirty_lines(const float (&r)[NT * 4], int ti
         for (int c = 0; c < 4; ++c) {
             const uint32_t b = (uint32_t)f2i(r[t * 4 + c]);
             const uint32_t m2 = b + b;
-            if (m2 - kBandLo2 >= kBandSpan2)
-                lines |= (1u << slab_line<T, R, KC>(tid + t * T::kThreads, c)) |
-                         (m2 == 0 ? zeros : (m2 >= kBandHi2 ? kNonZero | kAbove : (unsigned)kNonZero));
+            const bool off = m2 - kBandLo2 >= kBandSpan2;
+            lines |= off ? 1u << slab_line<T, R, KC>(tid + t * T::kThreads, c) : 0u;
+            bits |= off ? m2 : 0u;
+            top = max(top, m2);
         }
     return lines;
 }
@@ -412,9 +416,21 @@ gemm_kernel(const GemmParams p) {
             // an out-of-band element locates it and reports its k line to the slab's word
             const bool out = band_excess(rb, band_excess(ra, 0u)) >= kBandSpan2;
             if (__any_sync(0xffffffffu, out)) {
-                unsigned f = out ? (dirty_lines<T, BM, T::kTasksA, A_KC>(ra, tid, kZerosA) | dirty_lines<T, BN, T::kTasksB, B_KC>(rb, tid, kZerosB)) : 0u;
-                f = __reduce_or_sync(0xffffffffu, f);
-                if ((tid & 31) == 0) atomicOr(&lines[slot], f);
+                unsigned f = 0;
+                if (out) {
+                    uint32_t bits = 0, top = 0;
+                    const unsigned in_a = dirty_lines<T, BM, T::kTasksA, A_KC>(ra, tid, bits, top);
+                    const unsigned in_b = dirty_lines<T, BN, T::kTasksB, B_KC>(rb, tid, bits, top);
+                    f = in_a | in_b | (in_a ? (unsigned)kInA : 0u) | (in_b ? (unsigned)kInB : 0u) | (bits ? (unsigned)kNonZero : 0u) |
+                        (top >= kBandHi2 ? (unsigned)kAbove : 0u);
+                }
+                if constexpr (MT == 4) {
+                    // (the 32x32 tile's launches are chains of slabs: atomics of two warps cost less than the wait for a reduction)
+                    if (f) atomicOr(&lines[slot], f);
+                } else {
+                    f = __reduce_or_sync(0xffffffffu, f);
+                    if ((tid & 31) == 0) atomicOr(&lines[slot], f);
+                }
             }
             // the A side is pre-biased (bits - (0x3f800000 - offset)) so that a product is a two-input add
 #pragma unroll
@@ -464,7 +480,14 @@ gemm_kernel(const GemmParams p) {
 #pragma unroll
                 for (int i = 0; i < MR; ++i)
 #pragma unroll
-                    for (int j = 0; j < MT; j += 2) add_pair(acc[i][j], acc[i][j + 1], iadd(a[i], b[j]), iadd(a[i], b[j + 1]));
+                    for (int j = 0; j < MT; j += 2) {
+                        if constexpr (MT == 8 || VEC) {
+                            add_pair(acc[i][j], acc[i][j + 1], iadd(a[i], b[j]), iadd(a[i], b[j + 1]));
+                        } else {                                        // (the pairs made the 32x32 tile's scalar-load kernels spill)
+                            acc[i][j] = fadd(acc[i][j], i2f(iadd(a[i], b[j])));
+                            acc[i][j + 1] = fadd(acc[i][j + 1], i2f(iadd(a[i], b[j + 1])));
+                        }
+                    }
             }
         } else if constexpr (MODE == kPam) {
             constexpr unsigned all_lines = (1u << BK) - 1u;
@@ -502,7 +525,7 @@ gemm_kernel(const GemmParams p) {
                 // Zeros, and everything else in the band: a zero's products are left out by a predicate.
                 // 4096^3 with one operand half zeros 6020 us (clean: 4565), both 7500; by
                 // weights of 0 and 1 in a fused multiply-add, prepared by a pass over the slab, 6040 and 9670.
-                if (!(dirty & kZerosA)) {
+                if (!(dirty & kInA)) {
 #pragma unroll 1
                     for (; kk < BK; ++kk) {
                         PAMK_FRAGMENTS(kk)
@@ -512,7 +535,7 @@ gemm_kernel(const GemmParams p) {
                             for (int j = 0; j < MT; ++j)
                                 if (2u * (uint32_t)b[j] != 0u) acc[i][j] = fadd(acc[i][j], i2f(iadd(a[i], b[j])));
                     }
-                } else if (!(dirty & kZerosB)) {
+                } else if (!(dirty & kInB)) {
 #pragma unroll 1
                     for (; kk < BK; ++kk) {
                         PAMK_FRAGMENTS(kk)
@@ -666,7 +689,7 @@ gemm_kernel(const GemmParams p) {
                 // it, 0 for a zero and 1 for anything else; the sum then is acc = fma(product, weight, acc), which
                 // is the plain sum for weight 1 and leaves acc alone for weight 0 (the products are finite, and a
                 // sum is never -0).
-                const bool side_b = !(dirty & kZerosA);
+                const bool side_b = !(dirty & kInA);
                 float* side = side_b ? Bs[buf] : As[buf];
                 // (the stand-in makes the product the other operand's own pattern, whatever the offset)
                 const int zero_bits = side_b ? 0 : -p.bias_sub, stand_in = side_b ? p.bias_sub : 0;
@@ -685,7 +708,7 @@ gemm_kernel(const GemmParams p) {
                     *reinterpret_cast<float4*>(weights + at) = w;
                 }
                 __syncthreads();
-                if ((dirty & (kZerosA | kZerosB)) == (kZerosA | kZerosB)) {
+                if ((dirty & (kInA | kInB)) == (kInA | kInB)) {
                     // (weights for A's zeros, a predicate for B's)
 #pragma unroll 1
                     for (; kk < BK; ++kk) {
@@ -707,7 +730,7 @@ gemm_kernel(const GemmParams p) {
 #pragma unroll
                         for (int i = 0; i < 4; ++i)
 #pragma unroll
-                            for (int j = 0; j < 4; j += 2) fma_pair(acc[i % MR][j], acc[i % MR][j + 1], iadd(a[i], b[j]), iadd(a[i], b[j + 1]), w[i], w[i]);
+                            for (int j = 0; j < 4; ++j) acc[i % MR][j] = __fmaf_rn(i2f(iadd(a[i], b[j])), w[i], acc[i % MR][j]);
                     }
                 } else {
 #pragma unroll 1
@@ -717,7 +740,7 @@ gemm_kernel(const GemmParams p) {
 #pragma unroll
                         for (int i = 0; i < 4; ++i)
 #pragma unroll
-                            for (int j = 0; j < 4; j += 2) fma_pair(acc[i % MR][j], acc[i % MR][j + 1], iadd(a[i], b[j]), iadd(a[i], b[j + 1]), w[j], w[j + 1]);
+                            for (int j = 0; j < 4; ++j) acc[i % MR][j] = __fmaf_rn(i2f(iadd(a[i], b[j])), w[j], acc[i % MR][j]);
                     }
                 }
             } else {
