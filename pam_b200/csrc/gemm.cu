@@ -67,7 +67,7 @@ struct GemmParams {
     int32_t off;              // offset_bits
 };
 
-// Tile shapes.  Every thread owns a square register micro-tile (8x8 unless said otherwise).
+// Tile shapes.  Every thread owns an 8x8 register micro-tile unless said otherwise.
 //   128x128x16, 256 threads, 2 CTAs/SM: least staging overhead, for large outputs;
 //   64x64x8,     64 threads, 8 CTAs/SM: four times as many CTAs, for outputs that would leave a
 //                                       large tile grid with a ragged last wave (e.g. 12608 x 192).
@@ -297,11 +297,22 @@ __device__ __forceinline__ unsigned dirty_lines(const float (&r)[NT * 4], int ti
 // Only products of two out-of-band elements are left to sort out: two masked ones flush (each has the other among its
 // partners), and so do a masked and a small one; any other such pair among a warp's rows and columns, and anything odd,
 // sends the line to the loop that forms the true product of every pair.
-// Against "flush or add" for every dirty line, 4096^3: 1 % special values 10428 -> 9940 us, 0.1 % 6700 -> 6360, one operand
-// below the band 10240 -> 6830.  The look itself costs about 40 % of a clean slab; one warp per two lines, with redux and
-// ballots for the shuffles, measured 5 % slower.
+// When the look is taken.  A slab without it takes the loops of the smaller tiles: "flush or add" for every dirty line, the full
+// rule for those that can overflow.  (Figures: 4096^3, with a look in every dirty slab -> now.)
+//   * Not for one or two dirty lines (one in a slab with elements above the band): the look costs about 40 % of a clean slab, a
+//     dirty line 8 % (0.01 % zeros 5130 -> 5010 us).
+//   * Not while it finds too much to check.  A checked line takes the full rule (a second loop here, for lines that cannot overflow,
+//     cost 2 % specials 24 %: the loops compete for the instruction cache), and warps with many of them keep the others waiting.
+//     Each look weighs 2 * (lines to check, of 16 in each of 8 warps) against 3 * (dirty lines) - 4, or against 200 in a slab
+//     with elements above the band, where a slab without the look has to search for overflows; the sum forgets
+//     a quarter with each look, and above kAgainst the next slabs of the tile go without (one slab's count is too coarse:
+//     where looks and slabs without alternate among the tiles of an SM, both are slower).
+//     One operand around the flush bound 16700 -> 9560 us (with "flush or add" alone 10490), 3 % values below the
+//     band 13410 -> 9530 (10530), 10 % specials 16920 -> 15830 (16300); 1 % specials keep their looks: 9880 (10650).
 enum Class { kMasked = 1, kSmall = 2, kGreat = 4, kOdd = 8 };
 enum LineKind { kPlain = 0, kRowsOff = 1, kColsOff = 2, kBothOff = 3, kChecked = 4, kNothing = 5 };
+
+constexpr int kFewBelow = 2, kFewAbove = 1, kCheckedAbove = 200, kAgainst = 16, kSlabsWithout = 64;
 
 __device__ __forceinline__ unsigned class_of(uint32_t magnitude, float smallest, float largest) {
     const float m = i2f((int32_t)magnitude);
@@ -347,6 +358,7 @@ gemm_kernel(const GemmParams p) {
     __shared__ __align__(16) float Bs[2][BK * row_stride(BN)];
     __shared__ __align__(16) float weights[MODE == kPam && MT == 4 ? BK * row_stride(BM) : 1];   // of the side that holds zeros (32x32 tile)
     __shared__ unsigned lines[3];   // per slab (Word)
+    __shared__ int look_from, against;    // looks: from which slab on, and what speaks against them (see class_of)
     __shared__ unsigned overflow_lines;   // bit k = some product of k line may leave the pass range
     // looked-through slabs: per line and thread row / column a bit for each masked element, per warp and line the LineKind
     __shared__ unsigned char rows_off[kLook ? BK : 1][16], cols_off[kLook ? BK : 1][16], line_kinds[kLook ? 8 : 1][BK];
@@ -393,6 +405,7 @@ gemm_kernel(const GemmParams p) {
     }
 
     if (MODE == kPam && tid < 3) lines[tid] = 0;
+    if (kLook && tid == 0) look_from = against = 0;
 
     float ra[T::kTasksA * 4], rb[T::kTasksB * 4];
     SlabWalker<T, BM, T::kTasksA, A_KC> walk_a;
@@ -563,11 +576,14 @@ gemm_kernel(const GemmParams p) {
                         }
                     }
                 }
-            } else if constexpr (kLook) {
+            } else if (kLook && __popc(any) > (dirty & kAbove ? kFewAbove : kFewBelow) && s >= look_from) {
+                // (the same for all threads: look_from is read after the barrier that ends a slab and written after the one below)
+                if constexpr (kLook) {
                 // sixteen threads look through one line, the two groups of four elements of either side that thread row / column
                 // `at` works on each
                 static_assert(!kLook || (BK == 16 && T::kThreads == 256 && BN == 128 && MT == 8), "a warp looks through two lines");
                 const int lane = tid & 31, warp = tid >> 5, line = tid >> 4, at = tid & 15;
+                bool vote = false;
                 if (any >> (2 * warp) & 3u) {                       // (the same for a warp)
                     uint32_t ma[8], mb[8];
                     // the smallest magnitude in the band and the largest that is not above it, as offsets in which what does not count
@@ -617,30 +633,31 @@ gemm_kernel(const GemmParams p) {
                     classes |= __shfl_xor_sync(0xffffffffu, classes, 2);
                     const unsigned rows = classes & 15u, cols = (classes | __shfl_xor_sync(0xffffffffu, classes, 4)) >> 8;
                     const unsigned other = __shfl_xor_sync(0xffffffffu, cols, 8);
+                    const unsigned kind = kind_of(rows, cols, flushes), other_kind = kind_of(rows, other, flushes);
                     if (at % 4 == 0) {
-                        line_kinds[at / 4 * 2 + at / 8][line] = (unsigned char)kind_of(rows, cols, flushes);
-                        line_kinds[at / 4 * 2 + (at / 8 ^ 1)][line] = (unsigned char)kind_of(rows, other, flushes);
+                        line_kinds[at / 4 * 2 + at / 8][line] = (unsigned char)kind;
+                        line_kinds[at / 4 * 2 + (at / 8 ^ 1)][line] = (unsigned char)other_kind;
                     }
+                    vote = at % 4 == 0 ? kind == kChecked : (at % 4 == 1 && other_kind == kChecked);    // (four threads hold the same)
                 } else if (at < 8) {
                     line_kinds[at][line] = kPlain;
                 }
-                __syncthreads();
+                const int votes = __syncthreads_count(vote);        // lines to be checked, of eight warps
+                if (tid == 0) {
+                    against += 2 * votes - (dirty & kAbove ? kCheckedAbove : 3 * __popc(any) - 4) - against / 4;
+                    if (against > kAgainst) look_from = s + kSlabsWithout;
+                }
                 // This warp's lines, in runs of one kind, each kind with a loop of its own with one copy of its body (with three
-                // bodies side by side in one loop the schedule cost 12 %).
-                const unsigned kind = line_kinds[warp][lane % BK];
-                const unsigned plain = __ballot_sync(0xffffffffu, kind == kPlain) & all_lines;
-                const unsigned rows_only = __ballot_sync(0xffffffffu, kind == kRowsOff) & all_lines;
-                const unsigned cols_only = __ballot_sync(0xffffffffu, kind == kColsOff) & all_lines;
-                const unsigned checked = __ballot_sync(0xffffffffu, kind == kChecked) & all_lines;
-                const unsigned nothing = __ballot_sync(0xffffffffu, kind == kNothing) & all_lines;
+                // bodies side by side in one loop the schedule cost 12 %).  Lane k holds the kind of line k: a mask per kind, kept in
+                // registers, was 3 % faster with 0.1 % specials and 12 to 32 % slower with 1.5 to 3 %.
+                const unsigned mine = line_kinds[warp][lane % BK];
                 while (kk < BK) {
-                    const unsigned here = 1u << kk;
-                    if (plain & here) {
-                        const int end = run_end(plain);
+                    const unsigned kind = __shfl_sync(0xffffffffu, mine, kk);
+                    const int end = run_end(__ballot_sync(0xffffffffu, mine == kind) & all_lines);
+                    if (kind == kPlain) {
 #pragma unroll 1
                         for (; kk < end; ++kk) plain_line(kk);
-                    } else if (cols_only & here) {
-                        const int end = run_end(cols_only);
+                    } else if (kind == kColsOff) {
 #pragma unroll 1
                         for (; kk < end; ++kk) {
                             PAMK_FRAGMENTS(kk)
@@ -651,8 +668,7 @@ gemm_kernel(const GemmParams p) {
                                 for (int j = 0; j < MT; ++j)
                                     if (!(off & (1u << j))) acc[i][j] = fadd(acc[i][j], i2f(iadd(a[i], b[j])));
                         }
-                    } else if (rows_only & here) {
-                        const int end = run_end(rows_only);
+                    } else if (kind == kRowsOff) {
 #pragma unroll 1
                         for (; kk < end; ++kk) {
                             PAMK_FRAGMENTS(kk)
@@ -663,25 +679,26 @@ gemm_kernel(const GemmParams p) {
                                 for (int i = 0; i < MR; ++i)
                                     if (!(off & (1u << i))) acc[i][j] = fadd(acc[i][j], i2f(iadd(a[i], b[j])));
                         }
-                    } else if (checked & here) {
-                        const int end = run_end(checked);
+                    } else if (kind == kChecked) {
 #pragma unroll 1
                         for (; kk < end; ++kk) checked_line(kk, std::true_type{});
-                    } else if (nothing & here) {
-                        kk = run_end(nothing);
-                    } else {                                            // rows (by weights, as above) and columns
-                        PAMK_FRAGMENTS(kk)
-                        const unsigned off = cols_off[kk][tx], rows = rows_off[kk][ty];
+                    } else if (kind == kBothOff) {                      // rows by weights, as above
+#pragma unroll 1
+                        for (; kk < end; ++kk) {
+                            PAMK_FRAGMENTS(kk)
+                            const unsigned off = cols_off[kk][tx], rows = rows_off[kk][ty];
 #pragma unroll
-                        for (int i = 0; i < MR; ++i) {
-                            const float w = rows & (1u << i) ? 0.0f : 1.0f;
-                            const int ai = rows & (1u << i) ? 0 : a[i];
+                            for (int i = 0; i < MR; ++i) {
+                                const float w = rows & (1u << i) ? 0.0f : 1.0f;
+                                const int ai = rows & (1u << i) ? 0 : a[i];
 #pragma unroll
-                            for (int j = 0; j < MT; ++j)
-                                if (!(off & (1u << j))) acc[i][j] = __fmaf_rn(i2f(iadd(ai, b[j])), w, acc[i][j]);
+                                for (int j = 0; j < MT; ++j)
+                                    if (!(off & (1u << j))) acc[i][j] = __fmaf_rn(i2f(iadd(ai, b[j])), w, acc[i][j]);
+                            }
                         }
-                        ++kk;
                     }
+                    kk = end;                                           // (kNothing: there is nothing to add)
+                }
                 }
             } else if (MT == 4 && !(dirty & kNonZero) && mostly) {
                 // Zeros on the 32x32 tile, whose launches are chains of slabs: a pass over one

@@ -47,8 +47,8 @@ def test_zeros_in_an_operand(policy, M, K, N, a_share, b_share, offset, oracle):
 @pytest.mark.parametrize("policy", [1, 2, 3], ids=["tile128", "tile64", "tile32"])
 @pytest.mark.parametrize("every", [1, 3, 12])
 def test_slabs_of_zeros_among_slabs_that_hold_others(policy, every, oracle):
-    """After a slab whose many out-of-band elements are not all zeros the next ones are not asked whether theirs are: runs
-    of both sorts, of every length around that count (K is 40 slabs of 16)."""
+    """Slabs whose many out-of-band elements are all zeros among slabs where they are not: runs of both sorts, of several
+    lengths (K is 40 slabs of 16)."""
     import pam_b200 as pam
     from pam_b200 import _lib
     from pam_b200.cuda_bindings import cuda_kernels
