@@ -37,17 +37,7 @@ __global__ void __launch_bounds__(256) scaled_max_kernel(const float* __restrict
     const bool vec = aligned16(x);
     if (vec) {
         const int64_t n4 = n >> 2;
-        int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
-        for (; i + 2 * stride < n4; i += 3 * stride) {          // three vectors requested at a time
-            float4 w[3];
-#pragma unroll
-            for (int u = 0; u < 3; ++u) w[u] = __ldg(reinterpret_cast<const float4*>(x) + i + u * stride);
-#pragma unroll
-            for (int u = 0; u < 3; ++u)
-                m = nan_max(m, nan_max(nan_max(scaled_of(w[u].x, off), scaled_of(w[u].y, off)),
-                                       nan_max(scaled_of(w[u].z, off), scaled_of(w[u].w, off))));
-        }
-        for (; i < n4; i += stride) {
+        for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n4; i += stride) {
             const float4 v = __ldg(reinterpret_cast<const float4*>(x) + i);
             m = nan_max(m, nan_max(nan_max(scaled_of(v.x, off), scaled_of(v.y, off)),
                                    nan_max(scaled_of(v.z, off), scaled_of(v.w, off))));
