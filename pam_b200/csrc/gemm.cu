@@ -28,6 +28,7 @@
 //
 // The same skeleton serves true-multiply products (standard_matmul) and the exact-gradient
 // product (pam_matmul_bwd_kernel, cuda_kernels.cu:729-832).
+#include <array>
 #include <type_traits>
 
 #include "common.cuh"
@@ -1061,7 +1062,7 @@ bool fine_slabs(int64_t ctas, int64_t K) {
 // that exists.
 int g_tile_policy = 0;
 
-Plan make_plan(int mode, int64_t batch, int64_t M, int64_t N, int64_t K, int split_request) {
+Plan search_plan(int mode, int64_t batch, int64_t M, int64_t N, int64_t K, int split_request) {
     const Plan large = plan_for<TileLarge>(mode, batch, M, N, K, split_request);
     if (mode == kStd || g_tile_policy == 1) return large;    // the true-multiply product uses the large tile
     if (g_tile_policy == 4) return large;
@@ -1088,6 +1089,20 @@ Plan make_plan(int mode, int64_t batch, int64_t M, int64_t N, int64_t K, int spl
         if (g_tile_policy == 3 || tiny.cost < margin * best.cost) best = tiny;
     }
     return best;
+}
+
+// A thread's last automatic search is kept, a function of its arguments alone: a layer that is called again and again does not pay for
+// it each time (a call of one 32-row projection 11.5 -> 11.0 us; a given split takes a fraction of that search).
+Plan make_plan(int mode, int64_t batch, int64_t M, int64_t N, int64_t K, int split_request) {
+    if (split_request != 0) return search_plan(mode, batch, M, N, K, split_request);
+    struct Search {
+        std::array<int64_t, 7> key;
+        Plan plan;
+    };
+    thread_local Search last{};                              // (all zero: the key of no search, which has at least one SM)
+    const std::array<int64_t, 7> key{mode, batch, M, N, K, g_tile_policy, sm_count()};
+    if (last.key != key) last = {key, search_plan(mode, batch, M, N, K, 0)};
+    return last.plan;
 }
 
 // Whether a plain PAM product planned as `pl` takes TileLarge7 where its operands allow that.  Only unsplit ones: the ranges of K, and
