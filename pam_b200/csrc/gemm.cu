@@ -129,8 +129,8 @@ __host__ __device__ constexpr int slot_row(int slot) {
 //   otherwise (contiguous along the row index): task id -> k = id / (R/4), four rows (id % (R/4))*4:
 //       a warp reads 512 contiguous bytes of one k.
 // Rows beyond the matrix are clamped to the last valid row (their products land in outputs that
-// are never stored); k beyond the range reads as 0.0f, which the range rule turns into +0.
-template <class T, int R, int NT, bool KC, bool VEC>
+// are never stored); k beyond the range reads as 0.0f, which the range rule turns into +0.  This is the scalar form.
+template <class T, int R, int NT, bool KC>
 __device__ __forceinline__ void load_slab(float (&r)[NT * 4], const MatArg& m, const float* base,
                                           int row0, int rows, int k0, int k_end, int tid) {
 #pragma unroll
@@ -141,28 +141,17 @@ __device__ __forceinline__ void load_slab(float (&r)[NT * 4], const MatArg& m, c
             row = row < rows ? row : rows - 1;
             const int k = k0 + (id % (T::BK / 4)) * 4;
             const float* src = base + (int64_t)row * m.sr + k;
-            if (VEC) {   // K and the split ranges are multiples of 4, pointers 16-byte aligned
-                const float4 v = k < k_end ? __ldg(reinterpret_cast<const float4*>(src)) : make_float4(0.f, 0.f, 0.f, 0.f);
-                r[t * 4] = v.x; r[t * 4 + 1] = v.y; r[t * 4 + 2] = v.z; r[t * 4 + 3] = v.w;
-            } else {
 #pragma unroll
-                for (int c = 0; c < 4; ++c) r[t * 4 + c] = k + c < k_end ? __ldg(src + c) : 0.0f;
-            }
+            for (int c = 0; c < 4; ++c) r[t * 4 + c] = k + c < k_end ? __ldg(src + c) : 0.0f;
         } else {
             const int k = k0 + id / (R / 4);
             const int c0 = row0 + (id % (R / 4)) * 4;
             const bool on = k < k_end;
             const float* src = base + (int64_t)k * m.sk;
-            if (VEC) {   // rows % 4 == 0: a group of four is entirely inside or entirely outside
-                const int g = c0 < rows ? c0 : rows - 4;
-                const float4 v = on ? __ldg(reinterpret_cast<const float4*>(src + g)) : make_float4(0.f, 0.f, 0.f, 0.f);
-                r[t * 4] = v.x; r[t * 4 + 1] = v.y; r[t * 4 + 2] = v.z; r[t * 4 + 3] = v.w;
-            } else {
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const int col = c0 + c < rows ? c0 + c : rows - 1;
-                    r[t * 4 + c] = on ? __ldg(src + col) : 0.0f;
-                }
+            for (int c = 0; c < 4; ++c) {
+                const int col = c0 + c < rows ? c0 + c : rows - 1;
+                r[t * 4 + c] = on ? __ldg(src + col) : 0.0f;
             }
         }
     }
@@ -234,14 +223,14 @@ __device__ __forceinline__ void store_slab(float* s, const float (&r)[NT * 4], i
 //     out-of-band elements record for which k lines, and of what sort they are.
 //   * Zeros alone, in most lines (an operand that went through a ReLU): a zero's products are left out of the sums by a
 //     predicate or a weight.
-//   * Anything else, large tile: the lines with out-of-band elements are looked through once and every warp takes, for each
-//     line, the cheapest loop that its own rows and columns allow (class_of, kind_of).
-//   * Anything else, smaller tiles, where that look costs more than it saves (12608x768x192 with 1 % specials 304 -> 475 us): a line
-//     without out-of-band elements costs two instructions per product, any other evaluates the true fp32 product.
-//     It can skip the overflow test when the largest
+//   * Anything else, large tile, where it pays (class_of): the lines with out-of-band elements are looked through once and every
+//     warp takes, for each line, the cheapest loop that its own rows and columns allow (kind_of).
+//   * Anything else: a line without out-of-band elements costs two instructions per product, any other evaluates the true fp32
+//     product.  It can skip the overflow test when the largest
 //     magnitudes of its two operand lines cannot multiply beyond 1e37 and neither holds an inf / NaN
 //     (|a * b| rounded grows with |a| and |b|, so the two maxima bound every product of the line):
-//     four instructions per product, "flush or add".  Only the remaining lines apply the full rule.
+//     four instructions per product, "flush or add".  Only the remaining lines apply the full rule.  (On the smaller tiles a look
+//     costs more than it saves: 12608x768x192 with 1 % specials 304 -> 475 us.)
 constexpr uint32_t kBandLo = 66u << 23, kBandHi = 188u << 23;  // smallest magnitude in the band, smallest above it
 constexpr uint32_t kBandLo2 = 2u * kBandLo, kBandHi2 = 2u * kBandHi;
 constexpr uint32_t kBandSpan2 = kBandHi2 - kBandLo2;           // in band iff 2*bits - kBandLo2 < span
@@ -334,8 +323,9 @@ __device__ __forceinline__ unsigned kind_of(unsigned rows, unsigned cols, bool f
 // ---- two sums in one instruction ----------------------------------------------------------------------------------
 // acc0 += p0, acc1 += p1 and acc0 = p0 * w0 + acc0, acc1 = p1 * w1 + acc1, each with the one rounding of its scalar form.
 // The packed add does not double the adds per cycle (register-only: 16.7 T pairs of one integer and one packed half against
-// 16.3 T), but it halves the adds that the scheduler has to issue: 4096^3 4848 -> 4562 us, 4096x512x512 101.8 -> 96.7 us,
-// with zeros in one operand 133 -> 125 us; the 64x64 and 32x32 tiles, which issue more beside the adds, gain 0 to 2 %.
+// 16.3 T), but it halves the adds that the scheduler has to issue: clean loops 4096^3 4848 -> 4562 us, 4096x512x512 (two K ranges)
+// 98.4 -> 94.4; the 64x64 and 32x32 tiles, which issue more beside the adds, gain 0 to 5 %.  In a rolled loop (the lines of dirty
+// slabs) it is slower than the scalar one, 11.6 against 16.4 T.
 // The exact-gradient products, which take three instructions per product, gain 3 to 10 % (12608x192x768 211 -> 200 us).
 __device__ __forceinline__ void add_pair(float& acc0, float& acc1, int p0, int p1) {
     asm("{ .reg .b64 s, t;\n mov.b64 s, {%0, %1};\n mov.b64 t, {%2, %3};\n add.rn.f32x2 s, s, t;\n mov.b64 {%0, %1}, s; }"
@@ -420,8 +410,8 @@ gemm_kernel(const GemmParams p) {
             walk_a.load(ra, k0, k_end, tid);
             walk_b.load(rb, k0, k_end, tid);
         } else {
-            load_slab<T, BM, T::kTasksA, A_KC, false>(ra, p.A, Ab, m0, p.M, k0, k_end, tid);
-            load_slab<T, BN, T::kTasksB, B_KC, false>(rb, p.B, Bb, n0, p.N, k0, k_end, tid);
+            load_slab<T, BM, T::kTasksA, A_KC>(ra, p.A, Ab, m0, p.M, k0, k_end, tid);
+            load_slab<T, BN, T::kTasksB, B_KC>(rb, p.B, Bb, n0, p.N, k0, k_end, tid);
         }
     };
     auto stage_store = [&](int buf, int slot) {
@@ -537,8 +527,8 @@ gemm_kernel(const GemmParams p) {
             auto run_end = [&](unsigned mask) { return min(BK, kk + __ffs((int)(~mask >> kk)) - 1); };
             if (MT == 8 && !(dirty & kNonZero) && mostly) {
                 // Zeros, and everything else in the band: a zero's products are left out by a predicate.
-                // 4096^3 with one operand half zeros 6020 us (clean: 4565), both 7500; by
-                // weights of 0 and 1 in a fused multiply-add, prepared by a pass over the slab, 6040 and 9670.
+                // 4096^3 with one operand half zeros 5720 us (clean: 4580), both 7280; by weights of 0 and 1 in a fused
+                // multiply-add, prepared by a pass over the slab, 6020 and 9660 (before dirty lines were found without a branch).
                 if (!(dirty & kInA)) {
 #pragma unroll 1
                     for (; kk < BK; ++kk) {

@@ -428,6 +428,7 @@ __global__ void __launch_bounds__(kGradWarps * 32) ln_param_grad_kernel(const fl
     float sw = 0.0f, sb = 0.0f;
     if (col < width) {
         // eight partials of each sum requested at a time: with a CTA per 32 columns there is little but the loads' latency
+        // (from four: 4096 rows of 512 6.4 -> 5.5 us, 12608 of 192 9.4 -> 8.8, 65536 of 1024 13.1 -> 11.7, 300 of 768 unchanged)
         int k = wid;
         for (; k + 7 * kGradWarps < ctas; k += 8 * kGradWarps) {
             float w[8], b[8];
