@@ -66,6 +66,7 @@ struct GemmParams {
     int splits, k_chunk;      // K is cut into `splits` ranges of k_chunk (a multiple of the slab)
     int32_t bias_sub;         // 0x3f800000 - offset_bits
     int32_t off;              // offset_bits
+    int32_t one, least;       // 1 and INT32_MIN, as values that the compiler does not know (see sum_on_alu)
 };
 
 // Tile shapes.  Every thread owns an 8x8 register micro-tile unless said otherwise.
@@ -337,6 +338,63 @@ __device__ __forceinline__ void fma_pair(float& acc0, float& acc1, int p0, int p
         : "+f"(acc0), "+f"(acc1) : "r"(p0), "r"(p1), "f"(w0), "f"(w1));
 }
 
+// ---- which pipe an integer add runs on -------------------------------------------------------------------------------
+// An SM partition dispatches one 32-lane instruction per cycle (a packed one counts twice) to three pipes of 16 lanes:
+// integer / logic, and two for floating point, of which the first also takes integer multiply-adds.  Per pair of products
+// the packed add occupies both floating-point pipes, so of the two integer adds three quarters belong on the integer pipe.
+// Left to choose, the compiler forms so many as multiply-adds that the first floating-point pipe becomes the bound
+// (4096^3: busy 84 %, the integer pipe 48 %, dispatch 93 %).  Here the source chooses: the larger of
+// x + y and INT32_MIN is one instruction of the integer pipe, x * 1 + y one of the floating-point pipe, and both are
+// x + y for all values.  (A constant bound or factor would be folded away.  A three-operand add is slower, 4096^3 4950
+// to 5240 us: one more register read.)
+// Products (i, j) of a thread's micro-tile that multiply_add_product names go to the floating-point pipe, 26 % of 64: 4096^3
+// 4555 -> 4387 us, 12608x768x192 139.3 -> 131.5, 4096x512x512 96.3 -> 92.2.  The share and the places were found by trial:
+// 0 % 4735, 19 % 4497, 25 % 4367 to 4550 by place, 31 % 4372, 38 % 4430, 50 % 4582.
+__device__ __forceinline__ int sum_on_alu(int x, int y, int least) { return __viaddmax_s32(x, y, least); }
+__device__ __forceinline__ int sum_on_fma(int x, int y, int one) {
+    int d;
+    asm("mad.lo.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(x), "r"(one), "r"(y));
+    return d;
+}
+__host__ __device__ constexpr bool multiply_add_product(int i, int j) { return j == 3 || j == 5 || (i == 7 && j == 1); }
+
+// ---- eight sums at once, or none of them ----------------------------------------------------------------------------
+// c += p where x is not zero (either sign of it), and where pattern x is not `zero`: one compare for eight adds.  Written as conditions
+// around each add, the compiler makes branches of them once the products' adds are no longer plain ones.
+#define PAMK_EIGHT(c0, c1, c2, c3, c4, c5, c6, c7) "+f"(c0), "+f"(c1), "+f"(c2), "+f"(c3), "+f"(c4), "+f"(c5), "+f"(c6), "+f"(c7)
+#define PAMK_PRODUCTS "f"(i2f(q[0])), "f"(i2f(q[1])), "f"(i2f(q[2])), "f"(i2f(q[3])), "f"(i2f(q[4])), "f"(i2f(q[5])), "f"(i2f(q[6])), "f"(i2f(q[7]))
+#define PAMK_ADD_EIGHT                                                                                            \
+    "@on add.rn.f32 %0, %0, %8;\n @on add.rn.f32 %1, %1, %9;\n @on add.rn.f32 %2, %2, %10;\n @on add.rn.f32 %3, %3, %11;\n"   \
+    "@on add.rn.f32 %4, %4, %12;\n @on add.rn.f32 %5, %5, %13;\n @on add.rn.f32 %6, %6, %14;\n @on add.rn.f32 %7, %7, %15; }"
+template <int MR, int MT>
+__device__ __forceinline__ void add_column_unless_zero(int x, float (&acc)[MR][MT], int j, const int (&q)[8]) {
+    float spare = 0.0f;
+    float& last = MR == 8 ? acc[7 % MR][j] : spare;
+    asm("{ .reg .pred on;\n setp.neu.f32 on, %16, 0f00000000;\n" PAMK_ADD_EIGHT
+        : PAMK_EIGHT(acc[0][j], acc[1][j], acc[2][j], acc[3][j], acc[4 % MR][j], acc[5 % MR][j], acc[6 % MR][j], last)
+        : PAMK_PRODUCTS, "f"(i2f(x)));
+}
+template <int MT>
+__device__ __forceinline__ void add_row_unless(int x, int zero, float (&acc)[MT], const int (&q)[8]) {
+    asm("{ .reg .pred on;\n setp.ne.s32 on, %16, %17;\n" PAMK_ADD_EIGHT
+        : PAMK_EIGHT(acc[0], acc[1], acc[2], acc[3], acc[4 % MT], acc[5 % MT], acc[6 % MT], acc[7 % MT])
+        : PAMK_PRODUCTS, "r"(x), "r"(zero));
+}
+// c = fma(p, w, c) where x is not zero
+template <int MR, int MT>
+__device__ __forceinline__ void fma_column_unless_zero(int x, float (&acc)[MR][MT], int j, const int (&q)[8], const float (&w)[8]) {
+    float spare = 0.0f;
+    float& last = MR == 8 ? acc[7 % MR][j] : spare;
+    asm("{ .reg .pred on;\n setp.neu.f32 on, %24, 0f00000000;\n"
+        "@on fma.rn.f32 %0, %8, %16, %0;\n @on fma.rn.f32 %1, %9, %17, %1;\n @on fma.rn.f32 %2, %10, %18, %2;\n @on fma.rn.f32 %3, %11, %19, %3;\n"
+        "@on fma.rn.f32 %4, %12, %20, %4;\n @on fma.rn.f32 %5, %13, %21, %5;\n @on fma.rn.f32 %6, %14, %22, %6;\n @on fma.rn.f32 %7, %15, %23, %7; }"
+        : PAMK_EIGHT(acc[0][j], acc[1][j], acc[2][j], acc[3][j], acc[4 % MR][j], acc[5 % MR][j], acc[6 % MR][j], last)
+        : PAMK_PRODUCTS, "f"(w[0]), "f"(w[1]), "f"(w[2]), "f"(w[3]), "f"(w[4]), "f"(w[5]), "f"(w[6]), "f"(w[7]), "f"(i2f(x)));
+}
+#undef PAMK_ADD_EIGHT
+#undef PAMK_PRODUCTS
+#undef PAMK_EIGHT
+
 template <int MODE, class T, bool A_KC, bool B_KC, bool VEC>
 __global__ void __launch_bounds__(T::kThreads, MODE == kPam || MODE == kStd ? T::kCtasPerSm : T::kCtasPerSm / 2)
 gemm_kernel(const GemmParams p) {
@@ -427,6 +485,10 @@ gemm_kernel(const GemmParams p) {
                     const unsigned in_b = dirty_lines<T, BN, T::kTasksB, B_KC>(rb, tid, bits, top);
                     f = in_a | in_b | (in_a ? (unsigned)kInA : 0u) | (in_b ? (unsigned)kInB : 0u) | (bits ? (unsigned)kNonZero : 0u) |
                         (top >= kBandHi2 ? (unsigned)kAbove : 0u);
+                    if (MT == 8) {                     // one pattern for A's zeros, of either sign: the loops for zeros look for it
+#pragma unroll
+                        for (int c = 0; c < T::kTasksA * 4; ++c) ra[c] = fadd(ra[c], 0.0f);
+                    }
                 }
                 if constexpr (MT == 4) {
                     // (the 32x32 tile's launches are chains of slabs: atomics of two warps cost less than the wait for a reduction)
@@ -486,7 +548,10 @@ gemm_kernel(const GemmParams p) {
 #pragma unroll
                     for (int j = 0; j < MT; j += 2) {
                         if constexpr (MT == 8 || VEC) {
-                            add_pair(acc[i][j], acc[i][j + 1], iadd(a[i], b[j]), iadd(a[i], b[j + 1]));
+                            auto product = [&](int c) {
+                                return multiply_add_product(i, c) ? sum_on_fma(a[i], b[c], p.one) : sum_on_alu(a[i], b[c], p.least);
+                            };
+                            add_pair(acc[i][j], acc[i][j + 1], product(j), product(j + 1));
                         } else {                                        // (the pairs made the 32x32 tile's scalar-load kernels spill)
                             acc[i][j] = fadd(acc[i][j], i2f(iadd(a[i], b[j])));
                             acc[i][j + 1] = fadd(acc[i][j + 1], i2f(iadd(a[i], b[j + 1])));
@@ -527,28 +592,32 @@ gemm_kernel(const GemmParams p) {
             auto run_end = [&](unsigned mask) { return min(BK, kk + __ffs((int)(~mask >> kk)) - 1); };
             if (MT == 8 && !(dirty & kNonZero) && mostly) {
                 // Zeros, and everything else in the band: a zero's products are left out by a predicate.
-                // 4096^3 with one operand half zeros 5720 us (clean: 4580), both 7280; by weights of 0 and 1 in a fused
-                // multiply-add, prepared by a pass over the slab, 6020 and 9660 (before dirty lines were found without a branch).
+                // 4096^3 with one operand half zeros 5500 us (clean: 4387), both 7070 (a condition around each add: 5840 and 7420, of
+                // which a compare per row or column, and for A's rows the removal of the bias, took 16 instructions a line).
+                if constexpr (MT == 8) {
                 if (!(dirty & kInA)) {
 #pragma unroll 1
                     for (; kk < BK; ++kk) {
                         PAMK_FRAGMENTS(kk)
 #pragma unroll
-                        for (int i = 0; i < MR; ++i)
+                        for (int j = 0; j < MT; ++j) {
+                            int q[8];
 #pragma unroll
-                            for (int j = 0; j < MT; ++j)
-                                if (2u * (uint32_t)b[j] != 0u) acc[i][j] = fadd(acc[i][j], i2f(iadd(a[i], b[j])));
+                            for (int i = 0; i < 8; ++i) q[i] = iadd(a[i], b[j]);
+                            add_column_unless_zero(b[j], acc, j, q);
+                        }
                     }
                 } else if (!(dirty & kInB)) {
 #pragma unroll 1
                     for (; kk < BK; ++kk) {
                         PAMK_FRAGMENTS(kk)
-                        // (columns outside: with the rows outside the compiler makes a branch of each row's condition)
 #pragma unroll
-                        for (int j = 0; j < MT; ++j)
+                        for (int i = 0; i < MR; ++i) {
+                            int q[8];
 #pragma unroll
-                            for (int i = 0; i < MR; ++i)
-                                if (2u * (uint32_t)iadd(a[i], p.bias_sub) != 0u) acc[i][j] = fadd(acc[i][j], i2f(iadd(a[i], b[j])));
+                            for (int j = 0; j < 8; ++j) q[j] = iadd(a[i], b[j]);
+                            add_row_unless(a[i], -p.bias_sub, acc[i], q);
+                        }
                     }
                 } else {
                     // rows by a weight: a zero's products (made finite) get weight 0 in a fused multiply-add, which leaves a sum alone
@@ -556,16 +625,23 @@ gemm_kernel(const GemmParams p) {
 #pragma unroll 1
                     for (; kk < BK; ++kk) {
                         PAMK_FRAGMENTS(kk)
+                        float w[8];
+                        int ai[8];
 #pragma unroll
-                        for (int i = 0; i < MR; ++i) {
-                            const bool zero = 2u * (uint32_t)iadd(a[i], p.bias_sub) == 0u;
-                            const float w = zero ? 0.0f : 1.0f;
-                            const int ai = zero ? 0 : a[i];
+                        for (int i = 0; i < 8; ++i) {
+                            const bool zero = a[i] == -p.bias_sub;
+                            w[i] = zero ? 0.0f : 1.0f;
+                            ai[i] = zero ? 0 : a[i];
+                        }
 #pragma unroll
-                            for (int j = 0; j < MT; ++j)
-                                if (2u * (uint32_t)b[j] != 0u) acc[i][j] = __fmaf_rn(i2f(iadd(ai, b[j])), w, acc[i][j]);
+                        for (int j = 0; j < MT; ++j) {
+                            int q[8];
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) q[i] = iadd(ai[i], b[j]);
+                            fma_column_unless_zero(b[j], acc, j, q, w);
                         }
                     }
+                }
                 }
             } else if (kLook && __popc(any) > (dirty & kAbove ? kFewAbove : kFewBelow) && s >= look_from) {
                 // (the same for all threads: look_from is read after the barrier that ends a slab and written after the one below)
@@ -1138,6 +1214,8 @@ int run(int mode, GemmParams p, bool a_kc, bool b_kc, int split_k, void* workspa
     const bool fine = pl.tile == kTileTiny && pl.splits == 1 && fine_slabs(ctas, p.K);
     const int bk = fine ? TileTinyFine::BK : pl.tile == kTileTiny ? TileTiny::BK : (pl.tile == kTileSmall ? TileSmall::BK : TileLarge::BK);
     if (p.inner < 1) p.inner = 1;
+    p.one = 1;
+    p.least = INT32_MIN;
     if (p.ldc == 0) {                                        // plain output: [batch][M][N]
         p.ldc = p.N;
         p.sCb = (int64_t)p.inner * p.M * p.N;
