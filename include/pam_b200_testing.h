@@ -24,9 +24,13 @@ int pamk_test_set_tile_policy(int policy);
 int pamk_test_planned_tile(int64_t batch, int64_t M, int64_t N, int64_t K);
 
 /* Rows per tile (128, 112, 64 or 32) of a plain PAM product of these dimensions and K ranges (0 = the library's choice)
- * whose operands allow every tile: A contiguous along K, 128-bit loads.  Negative (PAMK_ERR_ARG) for an empty problem or a
+ * whose operands allow every tile, as planned: A contiguous along K, 128-bit loads.  Negative (PAMK_ERR_ARG) for an empty problem or a
  * negative split.  No counterpart in the reference. */
 int pamk_test_planned_rows(int64_t M, int64_t N, int64_t K, int split_k);
+
+/* The same for a product in several K ranges as it is launched: ranges planned for 128 rows may run on tiles of 112, with
+ * the same bounds.  No counterpart in the reference. */
+int pamk_test_split_rows(int64_t M, int64_t N, int64_t K, int split_k);
 
 #ifdef __cplusplus
 }

@@ -87,13 +87,13 @@ struct Tile {
     static constexpr int kRowsPerWarp = 32 / (BK_ / 4);
 };
 using TileLarge = Tile<128, 128, 16, 2>;
-// 112x128x16: the large tile with seven rows per thread, for unsplit products of few large tiles per SM whose number then
+// 112x128x16: the large tile with seven rows per thread, for products of few large tiles per SM whose number then
 // fits the SMs better (4096 rows x 1024: 256 tiles of 128 rows leave 40 of the 148 SMs with one tile where the others have two, 296
 // tiles of 112 none; one CTA of this size already runs an SM at 95 % of what two do).  Row slot 7 of every thread is staged
 // with a copy of a neighbouring row and takes no part in the sums.  4096x1024x512 174.5 -> 153.4 us, 8192x512x512 the same.
-// Products that the plan cuts along K do not take it: unsplit they would run 14 % faster (4096x512x512 98.6 -> 83.5 us), but their sums
-// would depend on whether the operands' layout and alignment allow this tile; with the plan's ranges summed one
-// after another in one CTA they cost 5.5 to 6.5 us per range (89.9 us, 2304x768x256 of 4 ranges 46.6 -> 57.0).
+// Products that the plan cuts along K keep their ranges on it: 4096x512x512 in two ranges is 256 tiles of 128 rows on 296 slots, and
+// exactly 296 of 112, 92.2 -> 84.0 us (1 % special values 187.7 -> 166.0).  (Unsplit it ran 83.5 us, but the order of the sums would
+// depend on whether the operands' layout and alignment allow this tile.)
 using TileLarge7 = Tile<128, 128, 16, 2, 8, 7>;
 using TileSmall = Tile<64, 64, 8, 8>;
 // 32x32x16 with a 4x4 micro-tile, 64 threads: batched products whose matrices are a fraction of a
@@ -1177,12 +1177,20 @@ Plan make_plan(int mode, int64_t batch, int64_t M, int64_t N, int64_t K, int spl
     return last.plan;
 }
 
-// Whether a plain PAM product planned as `pl` takes TileLarge7 where its operands allow that.  Only unsplit ones: the ranges of K, and
-// with them the order of the sums, follow from the shape alone, not from how the operands lie in memory.
+// Whether a plain PAM product planned as `pl` takes TileLarge7 where its operands allow that.  The ranges of K, and with them the order of
+// the sums, follow from the shape alone, not from how the operands lie in memory: unsplit products stay unsplit, and ranges keep their
+// number and their bounds (both tiles have slabs of 16).
 bool seven_rows_better(const Plan& pl, int64_t M, int64_t N, int64_t K) {
     if (pl.splits > 1 || (g_tile_policy != 0 && g_tile_policy != 4)) return false;
     if (M > (int64_t)65535 * TileLarge7::kRows) return false;                          // (grid.y)
     return g_tile_policy == 4 || plan_for<TileLarge7>(kPam, 1, M, N, K, 1).cost < 0.95 * pl.cost;
+}
+
+bool seven_rows_better_in_ranges(const Plan& pl, int64_t M, int64_t N, int64_t K) {
+    if (pl.splits == 1 || pl.tile != kTileLarge || (g_tile_policy != 0 && g_tile_policy != 4)) return false;
+    if (M > (int64_t)65535 * TileLarge7::kRows) return false;
+    const Plan seven = plan_for<TileLarge7>(kPam, 1, M, N, K, pl.splits);
+    return seven.splits == pl.splits && (g_tile_policy == 4 || seven.cost < 0.95 * pl.cost);
 }
 
 bool workspace_ok(const void* ws, size_t bytes, int splits, int64_t count) {
@@ -1212,7 +1220,9 @@ int run(int mode, GemmParams p, bool a_kc, bool b_kc, int split_k, void* workspa
         const int splits = pl.splits;
         pl = plan_for<TileLarge>(mode, p.batch, p.M, p.N, p.K, splits);
     }
-    if (mode == kPam && p.batch == 1 && p.K > 0 && a_kc && vec && seven_rows_better(pl, p.M, p.N, p.K)) pl.tile = kTileLarge7;
+    if (mode == kPam && p.batch == 1 && p.K > 0 && a_kc && vec &&
+        (seven_rows_better(pl, p.M, p.N, p.K) || seven_rows_better_in_ranges(pl, p.M, p.N, p.K)))
+        pl.tile = kTileLarge7;
     const int bm = pl.tile == kTileTiny ? TileTiny::BM : (pl.tile == kTileSmall ? TileSmall::BM : (pl.tile == kTileLarge7 ? TileLarge7::kRows : TileLarge::BM));
     const int bn = pl.tile == kTileTiny ? TileTiny::BN : (pl.tile == kTileSmall ? TileSmall::BN : TileLarge::BN);
     const int64_t ctas = ((p.N + bn - 1) / bn) * (int64_t)((p.M + bm - 1) / bm) * p.batch * pl.splits;
@@ -1353,6 +1363,12 @@ int pamk_test_planned_rows(int64_t M, int64_t N, int64_t K, int split_k) {
     const Plan pl = make_plan(kPam, 1, M, N, K, split_k);
     if (seven_rows_better(pl, M, N, K)) return TileLarge7::kRows;
     return pl.tile == kTileLarge ? TileLarge::BM : (pl.tile == kTileSmall ? TileSmall::BM : TileTiny::BM);
+}
+
+int pamk_test_split_rows(int64_t M, int64_t N, int64_t K, int split_k) {
+    if (M <= 0 || N <= 0 || K <= 0 || split_k < 0 || !dims_ok(1, M, N, K)) return PAMK_ERR_ARG;
+    const Plan pl = make_plan(kPam, 1, M, N, K, split_k);
+    return seven_rows_better_in_ranges(pl, M, N, K) ? TileLarge7::kRows : pamk_test_planned_rows(M, N, K, split_k);
 }
 
 int pamk_matmul_auto_split(int64_t batch, int64_t M, int64_t N, int64_t K) {
