@@ -144,6 +144,12 @@ int pamk_matmul_strided(const float* A, const float* B, float* C,
                         int split_k, void* workspace, size_t workspace_bytes, void* stream);
 /* Scratch needed by pamk_matmul for a given split_k (0 for split_k <= 1). */
 size_t pamk_matmul_workspace_bytes(int64_t batch, int64_t M, int64_t N, int split_k);
+/* Scratch with which pamk_matmul, pamk_matmul_bias and pamk_matmul_strided form a PAM product fastest: that of the split (0: the
+ * library's choice) and, for large products, room for both operands in the form that the kernel reads (about the
+ * operands' size again).  With less, down to pamk_matmul_workspace_bytes, the results are the same bits.  Products of at most
+ * PAMK_PACKED_PRODUCTS multiply-accumulates never use more than pamk_matmul_workspace_bytes (rounded up to 256). */
+#define PAMK_PACKED_PRODUCTS 3.0e9
+size_t pamk_matmul_scratch_bytes(int64_t batch, int64_t M, int64_t N, int64_t K, int split_k);
 /* The split the library would choose for split_k = 0 given unlimited workspace. */
 int pamk_matmul_auto_split(int64_t batch, int64_t M, int64_t N, int64_t K);
 

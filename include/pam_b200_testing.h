@@ -32,6 +32,14 @@ int pamk_test_planned_rows(int64_t M, int64_t N, int64_t K, int split_k);
  * the same bounds.  No counterpart in the reference. */
 int pamk_test_split_rows(int64_t M, int64_t N, int64_t K, int split_k);
 
+/* Whether PAM products of large tiles run on packed operands: 0 = where it pays (default), 1 = wherever the scratch suffices,
+ * 2 = never.  Process-wide and not thread-safe.  No counterpart in the reference. */
+int pamk_test_set_packing_policy(int policy);
+
+/* How many waits inside kernels have run out on the current device since the library was loaded (a product whose wait ran out holds
+ * NaN): 0 unless something is wrong.  Synchronises.  No counterpart in the reference. */
+int pamk_test_expired_waits(unsigned* count);
+
 #ifdef __cplusplus
 }
 #endif

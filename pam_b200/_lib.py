@@ -46,6 +46,9 @@ _SIGNATURES = {
     "pamk_test_planned_tile": (_i, [_i64] * 4),
     "pamk_test_planned_rows": (_i, [_i64] * 3 + [_i]),
     "pamk_test_split_rows": (_i, [_i64] * 3 + [_i]),
+    "pamk_test_set_packing_policy": (_i, [_i]),
+    "pamk_test_expired_waits": (_i, [ctypes.POINTER(ctypes.c_uint)]),
+    "pamk_matmul_scratch_bytes": (_sz, [_i64] * 4 + [_i]),
     "pamk_matmul_static_scratch_bytes": (_sz, []),
     "pamk_matmul_static_scratch": (_i, [_p, _p, _p] + [_i64] * 10 + [_f, _i, _p]),
     "pamk_matmul_bwd": (_i, [_p] * 4 + [_i64] * 13 + [_i, _f, _i, _p, ctypes.c_size_t, _p]),

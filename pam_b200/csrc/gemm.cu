@@ -369,6 +369,10 @@ __host__ __device__ constexpr bool multiply_add_slope(int i, int j) { return (i 
 #define PAMK_ADD_EIGHT                                                                                            \
     "@on add.rn.f32 %0, %0, %8;\n @on add.rn.f32 %1, %1, %9;\n @on add.rn.f32 %2, %2, %10;\n @on add.rn.f32 %3, %3, %11;\n"   \
     "@on add.rn.f32 %4, %4, %12;\n @on add.rn.f32 %5, %5, %13;\n @on add.rn.f32 %6, %6, %14;\n @on add.rn.f32 %7, %7, %15; }"
+#define PAMK_WEIGHTS_EIGHT "f"(w[0]), "f"(w[1]), "f"(w[2]), "f"(w[3]), "f"(w[4]), "f"(w[5]), "f"(w[6]), "f"(w[7])
+#define PAMK_FMA_EIGHT                                                                                                                     \
+    "@on fma.rn.f32 %0, %8, %16, %0;\n @on fma.rn.f32 %1, %9, %17, %1;\n @on fma.rn.f32 %2, %10, %18, %2;\n @on fma.rn.f32 %3, %11, %19, %3;\n" \
+    "@on fma.rn.f32 %4, %12, %20, %4;\n @on fma.rn.f32 %5, %13, %21, %5;\n @on fma.rn.f32 %6, %14, %22, %6;\n @on fma.rn.f32 %7, %15, %23, %7; }"
 template <int MR, int MT>
 __device__ __forceinline__ void add_column_unless_zero(int x, float (&acc)[MR][MT], int j, const int (&q)[8]) {
     float spare = 0.0f;
@@ -377,8 +381,23 @@ __device__ __forceinline__ void add_column_unless_zero(int x, float (&acc)[MR][M
         : PAMK_EIGHT(acc[0][j], acc[1][j], acc[2][j], acc[3][j], acc[4 % MR][j], acc[5 % MR][j], acc[6 % MR][j], last)
         : PAMK_PRODUCTS, "f"(i2f(x)));
 }
+// the same where `off` is zero
+template <int MR, int MT>
+__device__ __forceinline__ void add_column_unless(unsigned off, float (&acc)[MR][MT], int j, const int (&q)[8]) {
+    float spare = 0.0f;
+    float& last = MR == 8 ? acc[7 % MR][j] : spare;
+    asm("{ .reg .pred on;\n setp.eq.s32 on, %16, 0;\n" PAMK_ADD_EIGHT
+        : PAMK_EIGHT(acc[0][j], acc[1][j], acc[2][j], acc[3][j], acc[4 % MR][j], acc[5 % MR][j], acc[6 % MR][j], last)
+        : PAMK_PRODUCTS, "r"(off));
+}
 template <int MT>
-__device__ __forceinline__ void add_row_unless(int x, int zero, float (&acc)[MT], const int (&q)[8]) {
+__device__ __forceinline__ void add_row_unless(unsigned off, float (&acc)[MT], const int (&q)[8]) {
+    asm("{ .reg .pred on;\n setp.eq.s32 on, %16, 0;\n" PAMK_ADD_EIGHT
+        : PAMK_EIGHT(acc[0], acc[1], acc[2], acc[3], acc[4 % MT], acc[5 % MT], acc[6 % MT], acc[7 % MT])
+        : PAMK_PRODUCTS, "r"(off));
+}
+template <int MT>
+__device__ __forceinline__ void add_row_unless_zero(int x, int zero, float (&acc)[MT], const int (&q)[8]) {
     asm("{ .reg .pred on;\n setp.ne.s32 on, %16, %17;\n" PAMK_ADD_EIGHT
         : PAMK_EIGHT(acc[0], acc[1], acc[2], acc[3], acc[4 % MT], acc[5 % MT], acc[6 % MT], acc[7 % MT])
         : PAMK_PRODUCTS, "r"(x), "r"(zero));
@@ -388,12 +407,20 @@ template <int MR, int MT>
 __device__ __forceinline__ void fma_column_unless_zero(int x, float (&acc)[MR][MT], int j, const int (&q)[8], const float (&w)[8]) {
     float spare = 0.0f;
     float& last = MR == 8 ? acc[7 % MR][j] : spare;
-    asm("{ .reg .pred on;\n setp.neu.f32 on, %24, 0f00000000;\n"
-        "@on fma.rn.f32 %0, %8, %16, %0;\n @on fma.rn.f32 %1, %9, %17, %1;\n @on fma.rn.f32 %2, %10, %18, %2;\n @on fma.rn.f32 %3, %11, %19, %3;\n"
-        "@on fma.rn.f32 %4, %12, %20, %4;\n @on fma.rn.f32 %5, %13, %21, %5;\n @on fma.rn.f32 %6, %14, %22, %6;\n @on fma.rn.f32 %7, %15, %23, %7; }"
+    asm("{ .reg .pred on;\n setp.neu.f32 on, %24, 0f00000000;\n" PAMK_FMA_EIGHT
         : PAMK_EIGHT(acc[0][j], acc[1][j], acc[2][j], acc[3][j], acc[4 % MR][j], acc[5 % MR][j], acc[6 % MR][j], last)
-        : PAMK_PRODUCTS, "f"(w[0]), "f"(w[1]), "f"(w[2]), "f"(w[3]), "f"(w[4]), "f"(w[5]), "f"(w[6]), "f"(w[7]), "f"(i2f(x)));
+        : PAMK_PRODUCTS, PAMK_WEIGHTS_EIGHT, "f"(i2f(x)));
 }
+template <int MR, int MT>
+__device__ __forceinline__ void fma_column_unless(unsigned off, float (&acc)[MR][MT], int j, const int (&q)[8], const float (&w)[8]) {
+    float spare = 0.0f;
+    float& last = MR == 8 ? acc[7 % MR][j] : spare;
+    asm("{ .reg .pred on;\n setp.eq.s32 on, %24, 0;\n" PAMK_FMA_EIGHT
+        : PAMK_EIGHT(acc[0][j], acc[1][j], acc[2][j], acc[3][j], acc[4 % MR][j], acc[5 % MR][j], acc[6 % MR][j], last)
+        : PAMK_PRODUCTS, PAMK_WEIGHTS_EIGHT, "r"(off));
+}
+#undef PAMK_FMA_EIGHT
+#undef PAMK_WEIGHTS_EIGHT
 #undef PAMK_ADD_EIGHT
 #undef PAMK_PRODUCTS
 #undef PAMK_EIGHT
@@ -619,7 +646,7 @@ gemm_kernel(const GemmParams p) {
                             int q[8];
 #pragma unroll
                             for (int j = 0; j < 8; ++j) q[j] = iadd(a[i], b[j]);
-                            add_row_unless(a[i], -p.bias_sub, acc[i], q);
+                            add_row_unless_zero(a[i], -p.bias_sub, acc[i], q);
                         }
                     }
                 } else {
@@ -966,6 +993,8 @@ gemm_kernel(const GemmParams p) {
     }
 }
 
+#include "gemm_packed.cuh"
+
 // Where the finished sums of a split-K product go: a plain [batch][M][N] array, or the strided output
 // of the call (row stride and two batch strides).
 struct OutArg {
@@ -1193,6 +1222,18 @@ bool seven_rows_better_in_ranges(const Plan& pl, int64_t M, int64_t N, int64_t K
     return seven.splits == pl.splits && (g_tile_policy == 4 || seven.cost < 0.95 * pl.cost);
 }
 
+// Whether a PAM product planned as `pl` runs on packed operands, given the scratch, and its rows per tile then (whatever the operands'
+// layout: packing brings them into one).
+bool runs_packed(const Plan& pl, int64_t batch, int64_t M, int64_t N, int64_t K, int* tile_rows) {
+    if (pl.tile != kTileLarge || K == 0 || !packing_pays(batch, M, N, K)) return false;
+    const bool seven = batch == 1 && (seven_rows_better(pl, M, N, K) || seven_rows_better_in_ranges(pl, M, N, K));
+    *tile_rows = seven ? TileLarge7::kRows : TileLarge::kRows;
+    return true;
+}
+
+// Bytes of the partials of a product, a multiple of 256.
+size_t partial_bytes(int splits, int64_t count) { return splits > 1 ? ((size_t)splits * (size_t)count * sizeof(float) + 255) / 256 * 256 : 0; }
+
 bool workspace_ok(const void* ws, size_t bytes, int splits, int64_t count) {
     return ws != nullptr && (reinterpret_cast<uintptr_t>(ws) & 255u) == 0 &&
            bytes >= (size_t)splits * (size_t)count * sizeof(float);
@@ -1220,10 +1261,18 @@ int run(int mode, GemmParams p, bool a_kc, bool b_kc, int split_k, void* workspa
         const int splits = pl.splits;
         pl = plan_for<TileLarge>(mode, p.batch, p.M, p.N, p.K, splits);
     }
-    if (mode == kPam && p.batch == 1 && p.K > 0 && a_kc && vec &&
+    int tile_rows = 0;
+    PackLayout layout{};
+    bool packed = mode == kPam && workspace != nullptr && (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0 &&
+                  runs_packed(pl, p.batch, p.M, p.N, p.K, &tile_rows);
+    if (packed) {
+        layout = pack_layout(p.batch, p.M, p.N, p.K, tile_rows);
+        packed = workspace_bytes >= partial_bytes(pl.splits, count) && workspace_bytes - partial_bytes(pl.splits, count) >= layout.bytes;
+    }
+    if (!packed && mode == kPam && p.batch == 1 && p.K > 0 && a_kc && vec &&
         (seven_rows_better(pl, p.M, p.N, p.K) || seven_rows_better_in_ranges(pl, p.M, p.N, p.K)))
         pl.tile = kTileLarge7;
-    const int bm = pl.tile == kTileTiny ? TileTiny::BM : (pl.tile == kTileSmall ? TileSmall::BM : (pl.tile == kTileLarge7 ? TileLarge7::kRows : TileLarge::BM));
+    const int bm = packed ? tile_rows : pl.tile == kTileTiny ? TileTiny::BM : (pl.tile == kTileSmall ? TileSmall::BM : (pl.tile == kTileLarge7 ? TileLarge7::kRows : TileLarge::BM));
     const int bn = pl.tile == kTileTiny ? TileTiny::BN : (pl.tile == kTileSmall ? TileSmall::BN : TileLarge::BN);
     const int64_t ctas = ((p.N + bn - 1) / bn) * (int64_t)((p.M + bm - 1) / bm) * p.batch * pl.splits;
     const bool fine = pl.tile == kTileTiny && pl.splits == 1 && fine_slabs(ctas, p.K);
@@ -1264,7 +1313,9 @@ int run(int mode, GemmParams p, bool a_kc, bool b_kc, int split_k, void* workspa
     int rc;
     switch (mode) {
         case kPam:
-            rc = fine                    ? dispatch<kPam, TileTinyFine>(p, a_kc, b_kc, vec, grid, st)
+            rc = packed                  ? run_packed(p, layout, a_kc, b_kc, vectorisable(p.A, a_kc, p.M, p.K), vectorisable(p.B, b_kc, p.N, p.K),
+                                                      static_cast<unsigned char*>(workspace) + partial_bytes(pl.splits, count), st)
+                 : fine                  ? dispatch<kPam, TileTinyFine>(p, a_kc, b_kc, vec, grid, st)
                  : pl.tile == kTileTiny  ? dispatch<kPam, TileTiny>(p, a_kc, b_kc, vec, grid, st)
                  : pl.tile == kTileSmall ? dispatch<kPam, TileSmall>(p, a_kc, b_kc, vec, grid, st)
                  : pl.tile == kTileLarge7 ? dispatch_rows<TileLarge7>(p, b_kc, grid, st)
@@ -1344,6 +1395,26 @@ extern "C" {
 size_t pamk_matmul_workspace_bytes(int64_t batch, int64_t M, int64_t N, int split_k) {
     if (split_k <= 1 || batch <= 0 || M <= 0 || N <= 0) return 0;
     return (size_t)split_k * (size_t)batch * (size_t)M * (size_t)N * sizeof(float);
+}
+
+size_t pamk_matmul_scratch_bytes(int64_t batch, int64_t M, int64_t N, int64_t K, int split_k) {
+    if (batch <= 0 || M <= 0 || N <= 0 || K <= 0 || split_k < 0 || !dims_ok(batch, M, N, K)) return 0;
+    const Plan pl = make_plan(kPam, batch, M, N, K, split_k);
+    const size_t partials = partial_bytes(pl.splits, batch * M * N);
+    int tile_rows = 0;
+    return partials + (runs_packed(pl, batch, M, N, K, &tile_rows) ? pack_layout(batch, M, N, K, tile_rows).bytes : 0);
+}
+
+int pamk_test_set_packing_policy(int policy) {
+    if (policy < 0 || policy > 2) return PAMK_ERR_ARG;
+    g_packing_policy = policy;
+    return PAMK_OK;
+}
+
+int pamk_test_expired_waits(unsigned* count) {
+    if (count == nullptr) return PAMK_ERR_ARG;
+    const cudaError_t e = cudaMemcpyFromSymbol(count, g_expired_waits, sizeof(unsigned));
+    return e == cudaSuccess ? PAMK_OK : record_cuda_error(e);
 }
 
 int pamk_test_set_tile_policy(int policy) {

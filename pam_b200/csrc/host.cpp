@@ -56,7 +56,7 @@ using torch::autograd::variable_list;
 // those that launch.
 #define PAMK_QUERIES(X)                                                                                   \
     X(pamk_status_string) X(pamk_last_cuda_error) X(pamk_matmul_auto_split) X(pamk_matmul_bwd_auto_split) \
-    X(pamk_column_sum_workspace_bytes) X(pamk_layer_norm_max_width) X(pamk_layer_norm_stats_per_row)      \
+    X(pamk_matmul_scratch_bytes) X(pamk_column_sum_workspace_bytes) X(pamk_layer_norm_max_width) X(pamk_layer_norm_stats_per_row)      \
     X(pamk_layer_norm_bwd_workspace_bytes) X(pamk_softmax_max_len) X(pamk_softmax_workspace_bytes)
 #define PAMK_LAUNCHES(X)                                                                                  \
     X(pamk_pam_fwd) X(pamk_pad_fwd) X(pamk_pam_grad) X(pamk_pad_grad) X(pamk_matmul_bias)                 \
@@ -159,11 +159,19 @@ Tensor product(const Mat& a, const Mat& b, const Tensor& bias, int64_t batch, in
     Tensor out = empty_on(out_shape, like);
     const int split = g_strict.load(std::memory_order_relaxed) ? 1 : lib.pamk_matmul_auto_split(batch, M, N, K);
     Tensor ws;
-    size_t bytes = 0;
-    if (split > 1) {
-        bytes = (size_t)split * batch * M * N * sizeof(float);
-        ws = scratch_bytes(bytes, like);
+    size_t bytes = split > 1 ? (size_t)split * batch * M * N * sizeof(float) : 0;
+    if ((double)batch * (double)M * (double)N * (double)K > PAMK_PACKED_PRODUCTS) {
+        // scratch for packed operands too; a product that cannot have it runs without
+        const size_t packed = lib.pamk_matmul_scratch_bytes(batch, M, N, K, split);
+        if (packed > bytes) {
+            try {
+                ws = scratch_bytes(packed, like);
+                bytes = packed;
+            } catch (const c10::OutOfMemoryError&) {
+            }
+        }
     }
+    if (!ws.defined() && bytes != 0) ws = scratch_bytes(bytes, like);
     check(lib.pamk_matmul_bias(PAMK_MUL_PAM, a.p, b.p, ptr(bias), ptr(out), batch, M, N, K, a.sb, a.sr, a.sc, b.sb, b.sr, b.sc,
                                (float)offset, split, ws.defined() ? ws.data_ptr() : nullptr, bytes, stream_of(like)),
           "pamk_matmul");

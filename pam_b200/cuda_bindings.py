@@ -157,6 +157,20 @@ def _workspace(device, nbytes):
     return buf
 
 
+_PACKED_PRODUCTS = 3e9                                       # PAMK_PACKED_PRODUCTS
+
+
+def _packed_scratch(device, nbytes, partials):
+    """Scratch for a product on packed operands, given back after the call; None where the product takes no more than its
+    partial sums, or where there is no room (it then runs on the operands as they are)."""
+    if nbytes <= (partials + 255) // 256 * 256:
+        return None
+    try:
+        return torch.empty(nbytes, dtype=torch.uint8, device=device)
+    except torch.cuda.OutOfMemoryError:
+        return None
+
+
 def _matmul(kind, A, B, offset, dims, split_k=None, bias=None):
     device = _lib.require_cuda(A, B)
     A, sa = _matrix(A, dims)
@@ -172,8 +186,13 @@ def _matmul(kind, A, B, offset, dims, split_k=None, bias=None):
     if split_k is None:
         # (the true-multiply product has one tile shape and its own cost model: it is never split here)
         split_k = 1 if _strict_k_order or kind != _lib.MUL_PAM else handle.pamk_matmul_auto_split(batch, M, N, K)
-    ws_ptr, ws_bytes = None, 0
-    if split_k > 1:
+    ws_ptr, ws_bytes, packed = None, 0, None
+    if kind == _lib.MUL_PAM and batch * M * N * K > _PACKED_PRODUCTS:
+        packed = _packed_scratch(device, handle.pamk_matmul_scratch_bytes(batch, M, N, K, split_k),
+                                 handle.pamk_matmul_workspace_bytes(batch, M, N, split_k))
+    if packed is not None:
+        ws_ptr, ws_bytes = packed.data_ptr(), packed.numel()
+    elif split_k > 1:
         ws_bytes = handle.pamk_matmul_workspace_bytes(batch, M, N, split_k)
         ws_ptr = _workspace(device, ws_bytes).data_ptr()
     with _lib.device_guard(device):
