@@ -14,7 +14,8 @@ extern "C" {
  * 128x128, a 64x64 or, for small or ragged-edged products, a 32x32 tile per problem from a cost
  * model).  0 = by cost model (default), 1 = always 128x128, 2 = always 64x64, 3 = always
  * 32x32 (products that have no 32x32 kernel use 64x64), 4 = 112x128 for plain PAM products whose operands
- * allow it (A contiguous along K, 128-bit loads), else 128x128.  Process-wide and not thread-safe, which is
+ * allow it (A contiguous along K, 128-bit loads), else 128x128, 5 = 56x64 for unsplit PAM products whose operands
+ * allow it (A contiguous along K, or no 128-bit loads), else 64x64.  Process-wide and not thread-safe, which is
  * why it is kept out of pam_b200.h.  No counterpart in the reference. */
 int pamk_test_set_tile_policy(int policy);
 

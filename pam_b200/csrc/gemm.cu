@@ -96,6 +96,10 @@ using TileLarge = Tile<128, 128, 16, 2>;
 // depend on whether the operands' layout and alignment allow this tile.)
 using TileLarge7 = Tile<128, 128, 16, 2, 8, 7>;
 using TileSmall = Tile<64, 64, 8, 8>;
+// 56x64x8: the 64x64 tile with seven rows per thread, for unsplit products whose rows fill tiles of 56 better (attention over 197 tokens:
+// four tiles of 56 pad 14 % of the rows, of 64 30 %).  192 products 197x64x197 69.7 -> 57.4 us, with A contiguous along its rows 75.4 -> 59.4,
+// 500 products 100x100x64 43.5 -> 40.1 (small7_better).
+using TileSmall7 = Tile<64, 64, 8, 8, 8, 7>;
 // 32x32x16 with a 4x4 micro-tile, 64 threads: batched products whose matrices are a fraction of a
 // 64x64 tile (attention over 32 tokens) would otherwise spend three quarters of their adds on
 // rows and columns that do not exist.  A launch of few such CTAs is a chain of slabs, each as long as a
@@ -130,7 +134,8 @@ __host__ __device__ constexpr int slot_row(int slot) {
 //   otherwise (contiguous along the row index): task id -> k = id / (R/4), four rows (id % (R/4))*4:
 //       a warp reads 512 contiguous bytes of one k.
 // Rows beyond the matrix are clamped to the last valid row (their products land in outputs that
-// are never stored); k beyond the range reads as 0.0f, which the range rule turns into +0.  This is the scalar form.
+// are never stored); k beyond the range reads as 0.0f, which the range rule turns into +0.  This is the scalar form of the 32x32x16 tile, whose
+// launches are chains of slabs: all addresses follow from k0, no slab waits for the last one's.
 template <class T, int R, int NT, bool KC>
 __device__ __forceinline__ void load_slab(float (&r)[NT * 4], const MatArg& m, const float* base,
                                           int row0, int rows, int k0, int k_end, int tid) {
@@ -157,6 +162,47 @@ __device__ __forceinline__ void load_slab(float (&r)[NT * 4], const MatArg& m, c
         }
     }
 }
+
+// The scalar form of the other tiles: one pointer per task that walks along K, and where the operand is contiguous along its rows the four
+// clamped rows.  192 products 64x197x197 on 32x32x8 tiles 75.8 -> 69.6 us, 3001x1501x777 275 -> 265; on the 32x32x16 tile it is
+// slower (12 products 197x64x197 14.4 -> 16.4).
+template <class T, int R, int NT, bool KC>
+struct ScalarWalker {
+    const float* ptr[NT];
+    int rows_of[KC ? 1 : NT][4];
+    int64_t step;
+
+    template <bool MAPPED>
+    __device__ __forceinline__ void init(const MatArg& m, const float* base, int row0, int rows, int k_begin, int tid) {
+        step = KC ? (int64_t)T::BK : (int64_t)T::BK * m.sk;
+        auto row_at = [&](int slot) {
+            const int row = row0 + (MAPPED ? slot_row<T, R>(slot) : slot);
+            return row < rows ? row : rows - 1;
+        };
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+            const int id = tid + t * T::kThreads;
+            if (KC) {
+                ptr[t] = base + (int64_t)row_at(id / (T::BK / 4)) * m.sr + k_begin + (id % (T::BK / 4)) * 4;
+            } else {
+                ptr[t] = base + (int64_t)(k_begin + id / (R / 4)) * m.sk;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) rows_of[KC ? 0 : t][c] = row_at((id % (R / 4)) * 4 + c);
+            }
+        }
+    }
+
+    __device__ __forceinline__ void load(float (&r)[NT * 4], int k0, int k_end, int tid) {
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+            const int id = tid + t * T::kThreads;
+            const int k = KC ? k0 + (id % (T::BK / 4)) * 4 : k0 + id / (R / 4);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) r[t * 4 + c] = (KC ? k + c : k) < k_end ? __ldg(ptr[t] + (KC ? c : rows_of[KC ? 0 : t][c])) : 0.0f;
+            ptr[t] += step;
+        }
+    }
+};
 
 // Vectorised loads keep one pointer per task that walks along K, so the per-slab work is the load,
 // the range predicate and one pointer increment; the row clamp and the 64-bit address arithmetic
@@ -429,7 +475,7 @@ template <int MODE, class T, bool A_KC, bool B_KC, bool VEC>
 __global__ void __launch_bounds__(T::kThreads, MODE == kPam || MODE == kStd ? T::kCtasPerSm : T::kCtasPerSm / 2)
 gemm_kernel(const GemmParams p) {
     constexpr int BM = T::BM, BN = T::BN, BK = T::BK, MT = T::MT, MR = T::MR;
-    static_assert(MR == MT || (MODE == kPam && A_KC && VEC), "fewer rows per thread: products with A contiguous along K alone");
+    static_assert(MR == MT || (MODE == kPam && (A_KC || !VEC)), "fewer rows per thread: no 128-bit loads along A's rows");
     constexpr bool kLook = MODE == kPam && BM == 128;      // dirty slabs are looked through (see class_of)
     // (the variant with both operands contiguous along their row index spills registers at 8)
     constexpr int kFastUnroll = (!A_KC && !B_KC) || 8 > BK ? BK : 8;
@@ -487,14 +533,16 @@ gemm_kernel(const GemmParams p) {
     if (kLook && tid == 0) look_from = against = 0;
 
     float ra[T::kTasksA * 4], rb[T::kTasksB * 4];
-    SlabWalker<T, BM, T::kTasksA, A_KC> walk_a;
-    SlabWalker<T, BN, T::kTasksB, B_KC> walk_b;
-    if constexpr (VEC) {
+    // (not the scalar form of the 32x32x16 tile, nor of the 32x32x8 tile with both operands along K: 200 products 151x150x150 98.6 -> 100.3 us)
+    constexpr bool kWalks = VEC || T::MT == 8 || (T::BK == 8 && !(A_KC && B_KC));
+    std::conditional_t<VEC, SlabWalker<T, BM, T::kTasksA, A_KC>, ScalarWalker<T, BM, T::kTasksA, A_KC>> walk_a;
+    std::conditional_t<VEC, SlabWalker<T, BN, T::kTasksB, B_KC>, ScalarWalker<T, BN, T::kTasksB, B_KC>> walk_b;
+    if constexpr (kWalks) {
         walk_a.template init<T::MR != T::MT>(p.A, Ab, m0, p.M, k_begin, tid);
         walk_b.template init<false>(p.B, Bb, n0, p.N, k_begin, tid);
     }
     auto stage_load = [&](int k0) {
-        if constexpr (VEC) {
+        if constexpr (kWalks) {
             walk_a.load(ra, k0, k_end, tid);
             walk_b.load(rb, k0, k_end, tid);
         } else {
@@ -1058,11 +1106,20 @@ int dispatch(const GemmParams& p, bool a_kc, bool b_kc, bool vec, dim3 grid, cud
     return check_launch();
 }
 
-// (the tiles with fewer rows per thread exist for A contiguous along K and 128-bit loads)
+// (with fewer rows per thread there are no 128-bit loads along A's rows, and of the large tile only 128-bit loads)
 template <class T>
 int dispatch_rows(const GemmParams& p, bool b_kc, dim3 grid, cudaStream_t st) {
     if (b_kc) gemm_kernel<kPam, T, true, true, true><<<grid, T::kThreads, 0, st>>>(p);
     else gemm_kernel<kPam, T, true, false, true><<<grid, T::kThreads, 0, st>>>(p);
+    return check_launch();
+}
+
+template <class T>
+int dispatch_rows_scalar(const GemmParams& p, bool a_kc, bool b_kc, dim3 grid, cudaStream_t st) {
+    if (a_kc && b_kc) gemm_kernel<kPam, T, true, true, false><<<grid, T::kThreads, 0, st>>>(p);
+    else if (a_kc) gemm_kernel<kPam, T, true, false, false><<<grid, T::kThreads, 0, st>>>(p);
+    else if (b_kc) gemm_kernel<kPam, T, false, true, false><<<grid, T::kThreads, 0, st>>>(p);
+    else gemm_kernel<kPam, T, false, false, false><<<grid, T::kThreads, 0, st>>>(p);
     return check_launch();
 }
 
@@ -1077,7 +1134,7 @@ bool vectorisable(const MatArg& m, bool kc, int rows, int K) {
 // The kernel is issue-bound, so the time of a launch is (the largest number of tiles any SM ends up
 // with) x (work per tile), inflated when an SM holds too few warps to keep its schedulers busy,
 // which is also the state of the SMs that run the last, partly filled wave of a larger launch.
-enum TileKind { kTileLarge = 0, kTileSmall = 1, kTileTiny = 2, kTileLarge7 = 3 };
+enum TileKind { kTileLarge = 0, kTileSmall = 1, kTileTiny = 2, kTileLarge7 = 3, kTileSmall7 = 4 };
 
 struct Plan {
     int tile;        // TileKind
@@ -1104,7 +1161,7 @@ Plan plan_for(int mode, int64_t batch, int64_t M, int64_t N, int64_t K, int spli
         // 8 about 74 %
         auto util = [](int64_t ctas) {
             const double warps = (double)ctas * (T::kThreads / 32);
-            if (T::MR < T::MT && warps >= 8.0) return warps >= 16.0 ? 1.0 : 0.94;      // (one 256-thread CTA: 2.75 us a slab, two: 5.23)
+            if (T::BM >= 128 && T::MR < T::MT && warps >= 8.0) return warps >= 16.0 ? 1.0 : 0.94;      // (one 256-thread CTA: 2.75 us a slab, two: 5.23)
             return warps >= 16.0 ? 1.0 : (warps >= 8.0 ? 0.58 + 0.02 * warps : warps / 10.8);
         };
         // the smaller the tile, the more bytes are staged (and fragments loaded) per MAC
@@ -1127,7 +1184,7 @@ Plan plan_for(int mode, int64_t batch, int64_t M, int64_t N, int64_t K, int spli
         return cost * staging + (s > 1 ? 1.1e6 : 0.0);        // the reduction pass and its launch (~12 us)
     };
     Plan pl;
-    pl.tile = T::MR < T::MT ? kTileLarge7 : (T::BM >= 128 ? kTileLarge : (T::BM >= 64 ? kTileSmall : kTileTiny));
+    pl.tile = T::MR < T::MT ? (T::BM >= 128 ? kTileLarge7 : kTileSmall7) : (T::BM >= 128 ? kTileLarge : (T::BM >= 64 ? kTileSmall : kTileTiny));
     int64_t s = split_request > 0 ? split_request : 1, actual = 1;
     pl.cost = cost_of(s, &actual);
     pl.splits = (int)actual;
@@ -1167,7 +1224,7 @@ Plan search_plan(int mode, int64_t batch, int64_t M, int64_t N, int64_t K, int s
     if (mode == kStd || g_tile_policy == 1) return large;    // the true-multiply product uses the large tile
     if (g_tile_policy == 4) return large;
     const Plan small = plan_for<TileSmall>(mode, batch, M, N, K, split_request);
-    if (g_tile_policy == 2 || (g_tile_policy == 3 && mode != kPam)) return small;
+    if (g_tile_policy == 2 || g_tile_policy == 5 || (g_tile_policy == 3 && mode != kPam)) return small;
     Plan best = small.cost < large.cost ? small : large;
     // The 32x32 tile wins where the 64x64 tile pads much (192 x 197x197x64: 256x256 against 224x224
     // outputs) or leaves most SMs empty.  Its modelled cost has to be lower by a margin that sweeps of
@@ -1222,6 +1279,17 @@ bool seven_rows_better_in_ranges(const Plan& pl, int64_t M, int64_t N, int64_t K
     return seven.splits == pl.splits && (g_tile_policy == 4 || seven.cost < 0.95 * pl.cost);
 }
 
+// Whether an unsplit PAM product planned for the 64x64 or the 32x32 tile takes TileSmall7 (the sums of one range are the same on any tile).
+// By the model: 5 % cheaper; with scalar loads up to 15 % dearer than the 32x32 tile, whose cost with those it does not know (20 batched
+// products: modelled 0.88 x, measured 0.85 to 0.92; scalar 1.12 x, 0.79 and 0.82; 1.18 x, 0.98 and 1.05; 1.6 x, 1.04; aligned 0.99 x,
+// 1.02; 1.1 x, 0.88 to 1.09).
+bool small7_better(const Plan& pl, int64_t batch, int64_t M, int64_t N, int64_t K, bool a_kc, bool vec) {
+    if (pl.splits > 1 || (pl.tile != kTileSmall && pl.tile != kTileTiny) || (vec && !a_kc) || K == 0) return false;
+    if (M > (int64_t)65535 * TileSmall7::kRows) return false;                          // (grid.y)
+    if (g_tile_policy != 0) return g_tile_policy == 5;
+    return plan_for<TileSmall7>(kPam, batch, M, N, K, 1).cost < (vec || pl.tile == kTileSmall ? 0.95 : 1.15) * pl.cost;
+}
+
 // Whether a PAM product planned as `pl` runs on packed operands, given the scratch, and its rows per tile then (whatever the operands'
 // layout: packing brings them into one).
 bool runs_packed(const Plan& pl, int64_t batch, int64_t M, int64_t N, int64_t K, int* tile_rows) {
@@ -1272,11 +1340,12 @@ int run(int mode, GemmParams p, bool a_kc, bool b_kc, int split_k, void* workspa
     if (!packed && mode == kPam && p.batch == 1 && p.K > 0 && a_kc && vec &&
         (seven_rows_better(pl, p.M, p.N, p.K) || seven_rows_better_in_ranges(pl, p.M, p.N, p.K)))
         pl.tile = kTileLarge7;
-    const int bm = packed ? tile_rows : pl.tile == kTileTiny ? TileTiny::BM : (pl.tile == kTileSmall ? TileSmall::BM : (pl.tile == kTileLarge7 ? TileLarge7::kRows : TileLarge::BM));
-    const int bn = pl.tile == kTileTiny ? TileTiny::BN : (pl.tile == kTileSmall ? TileSmall::BN : TileLarge::BN);
+    if (mode == kPam && small7_better(pl, p.batch, p.M, p.N, p.K, a_kc, vec)) pl.tile = kTileSmall7;
+    const int bm = packed ? tile_rows : pl.tile == kTileSmall7 ? TileSmall7::kRows : pl.tile == kTileTiny ? TileTiny::BM : (pl.tile == kTileSmall ? TileSmall::BM : (pl.tile == kTileLarge7 ? TileLarge7::kRows : TileLarge::BM));
+    const int bn = pl.tile == kTileTiny ? TileTiny::BN : (pl.tile == kTileSmall || pl.tile == kTileSmall7 ? TileSmall::BN : TileLarge::BN);
     const int64_t ctas = ((p.N + bn - 1) / bn) * (int64_t)((p.M + bm - 1) / bm) * p.batch * pl.splits;
     const bool fine = pl.tile == kTileTiny && pl.splits == 1 && fine_slabs(ctas, p.K);
-    const int bk = fine ? TileTinyFine::BK : pl.tile == kTileTiny ? TileTiny::BK : (pl.tile == kTileSmall ? TileSmall::BK : TileLarge::BK);
+    const int bk = fine ? TileTinyFine::BK : pl.tile == kTileTiny ? TileTiny::BK : (pl.tile == kTileSmall || pl.tile == kTileSmall7 ? TileSmall::BK : TileLarge::BK);
     if (p.inner < 1) p.inner = 1;
     p.one = 1;
     p.least = INT32_MIN;
@@ -1319,6 +1388,7 @@ int run(int mode, GemmParams p, bool a_kc, bool b_kc, int split_k, void* workspa
                  : pl.tile == kTileTiny  ? dispatch<kPam, TileTiny>(p, a_kc, b_kc, vec, grid, st)
                  : pl.tile == kTileSmall ? dispatch<kPam, TileSmall>(p, a_kc, b_kc, vec, grid, st)
                  : pl.tile == kTileLarge7 ? dispatch_rows<TileLarge7>(p, b_kc, grid, st)
+                 : pl.tile == kTileSmall7 ? (vec ? dispatch_rows<TileSmall7>(p, b_kc, grid, st) : dispatch_rows_scalar<TileSmall7>(p, a_kc, b_kc, grid, st))
                                          : dispatch<kPam, TileLarge>(p, a_kc, b_kc, vec, grid, st);
             break;
         case kStd: rc = dispatch<kStd, TileLarge>(p, a_kc, b_kc, vec, grid, st); break;
@@ -1418,7 +1488,7 @@ int pamk_test_expired_waits(unsigned* count) {
 }
 
 int pamk_test_set_tile_policy(int policy) {
-    if (policy < 0 || policy > 4) return PAMK_ERR_ARG;
+    if (policy < 0 || policy > 5) return PAMK_ERR_ARG;
     g_tile_policy = policy;
     return PAMK_OK;
 }
