@@ -1092,6 +1092,130 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restr
     }
 }
 
+// ---- small products in ranges of K, in one launch ---------------------------------------------------------------------------
+// The 32x32 tile's products in ranges are latencies: a launch that forms the partials, one that adds them, and the host's
+// work for both.  Here one CTA forms all partials of a 16x16 tile, half a warp per range, and adds them from shared
+// memory: same ranges, same order, same bits.  Kernel times, two launches and one: 32x512x512 in 16 ranges 6.6 + a gap and 5.9 us, 8x1024x512 7.2
+// and 6.0, 100x300x700 9.2 and 8.2; a call of 32x512x512 through the operators 11.6 and 8.8, most of it the host.
+// Bound by latencies: the launch, two loads from the L2, the sum of the partials.  (A cluster of eight CTAs per tile with the partials in
+// distributed shared memory: 6.9 us.)
+struct TileRange : Tile<16, 16, 16, 1, 4> {};
+struct RangeShared {                                          // of one range
+    union {
+        struct { float a[TileRange::BK * row_stride(16)], b[TileRange::BK * row_stride(16)]; };
+        float partial[16 * 16];
+    };
+};
+constexpr int kMaxRanges = 16;                                // 256 threads: two CTAs per SM, 40 KB of shared memory each
+
+// Whether a product planned as ranges on the 32x32 tile takes this form: all of its CTAs resident at once, and no more ranges than
+// above (197x192x768 in 24 ranges 9.3 us in two launches, 13.3 in one; 32x512x1024 in 32 7.8 and 9.2).
+bool ranges_in_one_launch(int64_t batch, int64_t M, int64_t N, int splits) {
+    return splits > 1 && splits <= kMaxRanges && batch <= 65535 && M <= (int64_t)65535 * 16 &&
+           batch * ((M + 15) / 16) * ((N + 15) / 16) * splits * 16 <= (int64_t)sm_count() * 512;
+}
+
+template <bool A_KC, bool B_KC, bool VEC>
+__global__ void __launch_bounds__(16 * kMaxRanges) ranges_kernel(const GemmParams p) {
+    using T = TileRange;
+    constexpr int BK = T::BK;
+    static_assert(T::kThreads == 16 && T::kTasksA == 4, "half a warp per range");
+    extern __shared__ __align__(16) unsigned char shared_bytes[];
+    RangeShared* ranges = reinterpret_cast<RangeShared*>(shared_bytes);
+    const int range = threadIdx.x / 16, tid = threadIdx.x % 16, z = blockIdx.z;
+    const unsigned half = 0xffffu << (threadIdx.x & 16);
+    const int m0 = blockIdx.y * 16, n0 = blockIdx.x * 16, tx = tid % 4, ty = tid / 4;
+    RangeShared& sh = ranges[range];
+    const unsigned zo = __umulhi((unsigned)z, p.inner_magic);
+    const float* Ab = p.A.p + (int64_t)zo * p.A.sb + (int64_t)z * p.A.sb2;
+    const float* Bb = p.B.p + (int64_t)zo * p.B.sb + (int64_t)z * p.B.sb2;
+    const int k_begin = range * p.k_chunk, k_end = min(p.K, k_begin + p.k_chunk);
+    float acc[4][4] = {};
+    // two slabs on their way: a range is seldom longer, and each wait is one for the L2
+    float ra[2][T::kTasksA * 4], rb[2][T::kTasksB * 4];
+    SlabWalker<T, 16, T::kTasksA, A_KC> walk_a;
+    SlabWalker<T, 16, T::kTasksB, B_KC> walk_b;
+    if constexpr (VEC) {
+        walk_a.template init<false>(p.A, Ab, m0, p.M, k_begin, tid);
+        walk_b.template init<false>(p.B, Bb, n0, p.N, k_begin, tid);
+    }
+    auto load = [&](float (&a)[T::kTasksA * 4], float (&b)[T::kTasksB * 4], int k0) {
+        if (k0 >= k_end) return;
+        if constexpr (VEC) {
+            walk_a.load(a, k0, k_end, tid);
+            walk_b.load(b, k0, k_end, tid);
+        } else {
+            load_slab<T, 16, T::kTasksA, A_KC>(a, p.A, Ab, m0, p.M, k0, k_end, tid);
+            load_slab<T, 16, T::kTasksB, B_KC>(b, p.B, Bb, n0, p.N, k0, k_end, tid);
+        }
+    };
+    auto slab = [&](float (&a_in)[T::kTasksA * 4], float (&b_in)[T::kTasksB * 4], int k0) {
+        if (k0 >= k_end) return;
+        const bool out = band_excess(b_in, band_excess(a_in, 0u)) >= kBandSpan2;
+        const bool dirty = __any_sync(half, out);
+#pragma unroll
+        for (int c = 0; c < T::kTasksA * 4; ++c) a_in[c] = i2f(isub(f2i(a_in[c]), p.bias_sub));
+        __syncwarp(half);                                     // the last slab has been read
+        store_slab<T, 16, T::kTasksA, A_KC>(sh.a, a_in, tid);
+        store_slab<T, 16, T::kTasksB, B_KC>(sh.b, b_in, tid);
+        load(a_in, b_in, k0 + 2 * BK);
+        __syncwarp(half);
+        auto line = [&](int kk, auto checked) {
+            const int4 a4 = *reinterpret_cast<const int4*>(sh.a + kk * row_stride(16) + ty * 4);
+            const int4 b4 = *reinterpret_cast<const int4*>(sh.b + kk * row_stride(16) + tx * 4);
+            const int a[4] = {a4.x, a4.y, a4.z, a4.w}, b[4] = {b4.x, b4.y, b4.z, b4.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int sum = iadd(a[i], b[j]);
+                    if constexpr (decltype(checked)::value) acc[i][j] = fadd(acc[i][j], range_rule(fmul(i2f(iadd(a[i], p.bias_sub)), i2f(b[j])), sum));
+                    else acc[i][j] = fadd(acc[i][j], i2f(sum));
+                }
+        };
+        if (!dirty) {
+#pragma unroll 4
+            for (int kk = 0; kk < BK; ++kk) line(kk, std::false_type{});
+        } else {                                              // the full rule for every product: a flushed one is +0, and a sum is never -0
+#pragma unroll 1
+            for (int kk = 0; kk < BK; ++kk) line(kk, std::true_type{});
+        }
+    };
+    load(ra[0], rb[0], k_begin);
+    load(ra[1], rb[1], k_begin + BK);
+    for (int k0 = k_begin; k0 < k_end; k0 += 2 * BK) {
+        slab(ra[0], rb[0], k0);
+        slab(ra[1], rb[1], k0 + BK);
+    }
+    __syncwarp(half);                                         // the partial takes the slab's place
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        *reinterpret_cast<float4*>(sh.partial + (ty * 4 + i) * 16 + tx * 4) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+    __syncthreads();
+
+    float* Cz = p.C + (int64_t)zo * p.sCb + (int64_t)z * p.sCb2;
+    for (int o = threadIdx.x; o < 16 * 16; o += blockDim.x) {
+        const int row = m0 + o / 16, col = n0 + o % 16;
+        if (row >= p.M || col >= p.N) continue;
+        float v = ranges[0].partial[o];
+        for (int r = 1; r < p.splits; ++r) v = fadd(v, ranges[r].partial[o]);
+        if (p.bias != nullptr) v = fadd(v, __ldg(p.bias + col));
+        if (p.post) v = mul(v, p.post_scale, p.off);
+        Cz[(int64_t)row * p.ldc + col] = v;
+    }
+}
+
+template <bool VEC>
+int dispatch_ranges(const GemmParams& p, bool a_kc, bool b_kc, cudaStream_t st) {
+    const dim3 grid((unsigned)((p.N + 15) / 16), (unsigned)((p.M + 15) / 16), (unsigned)p.batch);
+    const auto kernel = a_kc ? (b_kc ? ranges_kernel<true, true, VEC> : ranges_kernel<true, false, VEC>)
+                             : (b_kc ? ranges_kernel<false, true, VEC> : ranges_kernel<false, false, VEC>);
+    const size_t shared = p.splits * sizeof(RangeShared);
+    static_assert(kMaxRanges * sizeof(RangeShared) <= 48 * 1024, "what a launch may use unasked");
+    kernel<<<grid, (unsigned)(16 * p.splits), shared, st>>>(p);
+    return check_launch();
+}
+
 template <int MODE, class T>
 int dispatch(const GemmParams& p, bool a_kc, bool b_kc, bool vec, dim3 grid, cudaStream_t st) {
 #define PAMK_LAUNCH(AK, BKC, V) gemm_kernel<MODE, T, AK, BKC, V><<<grid, T::kThreads, 0, st>>>(p)
@@ -1356,7 +1480,8 @@ int run(int mode, GemmParams p, bool a_kc, bool b_kc, int split_k, void* workspa
     }
     OutArg out{p.C, p.ldc, p.sCb, p.sCb2, p.M, p.N, p.inner,
                p.ldc == p.N && p.sCb2 == (int64_t)p.M * p.N && p.sCb == (int64_t)p.inner * p.M * p.N};
-    if (pl.splits > 1) {                                     // partials: [split][batch][M][N] in the scratch
+    const bool one_launch = mode == kPam && pl.tile == kTileTiny && ranges_in_one_launch(p.batch, p.M, p.N, pl.splits);
+    if (pl.splits > 1 && !one_launch) {                      // partials: [split][batch][M][N] in the scratch
         p.C = static_cast<float*>(workspace);
         p.ldc = p.N;
         p.sCb = (int64_t)p.inner * p.M * p.N;
@@ -1382,7 +1507,8 @@ int run(int mode, GemmParams p, bool a_kc, bool b_kc, int split_k, void* workspa
     int rc;
     switch (mode) {
         case kPam:
-            rc = packed                  ? run_packed(p, layout, a_kc, b_kc, vectorisable(p.A, a_kc, p.M, p.K), vectorisable(p.B, b_kc, p.N, p.K),
+            rc = one_launch              ? (vec ? dispatch_ranges<true>(p, a_kc, b_kc, st) : dispatch_ranges<false>(p, a_kc, b_kc, st))
+                 : packed                ? run_packed(p, layout, a_kc, b_kc, vectorisable(p.A, a_kc, p.M, p.K), vectorisable(p.B, b_kc, p.N, p.K),
                                                       static_cast<unsigned char*>(workspace) + partial_bytes(pl.splits, count), st)
                  : fine                  ? dispatch<kPam, TileTinyFine>(p, a_kc, b_kc, vec, grid, st)
                  : pl.tile == kTileTiny  ? dispatch<kPam, TileTiny>(p, a_kc, b_kc, vec, grid, st)
@@ -1401,7 +1527,7 @@ int run(int mode, GemmParams p, bool a_kc, bool b_kc, int split_k, void* workspa
                                        : dispatch<kBwdR, TileLarge>(p, a_kc, b_kc, vec, grid, st);
             break;
     }
-    if (rc != PAMK_OK || pl.splits == 1) return rc;
+    if (rc != PAMK_OK || pl.splits == 1 || one_launch) return rc;
     // Four outputs per thread where there are enough of them (400x512 of 20 ranges 3.8 us with one, 4.1 with four; 192x192
     // of 64 ranges 4.9 and 7.4; for more see the kernel) and where N and the output's strides keep a group of
     // four in one row and 16-byte aligned.  (The partials are 256-byte aligned; count = batch * M * N is then a
