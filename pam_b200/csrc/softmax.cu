@@ -58,14 +58,29 @@ __global__ void __launch_bounds__(256) scaled_max_kernel(const float* __restrict
     }
 }
 
-// shift = floor(max over the per-CTA maxima); every thread of the row kernel computes it itself
-__device__ __forceinline__ float load_shift(const float* __restrict__ partials, int count) {
+// shift = floor(max over the per-CTA maxima), by all threads of the CTA: a warp alone would wait for 37 loads, one after the other
+template <int THREADS>
+__device__ __forceinline__ float load_shift(const float* __restrict__ partials, int count, float* scratch) {
     float m = -INFINITY;
-    for (int k = threadIdx.x & 31; k < count; k += 32) m = nan_max(m, __ldg(partials + k));
+#pragma unroll 5
+    for (int k = threadIdx.x; k < count; k += THREADS) m = nan_max(m, __ldg(partials + k));
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) m = nan_max(m, __shfl_xor_sync(0xffffffffu, m, d));
+    if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = m;
+    __syncthreads();
+    m = scratch[0];
+#pragma unroll
+    for (int w = 1; w < THREADS / 32; ++w) m = nan_max(m, scratch[w]);
+    __syncthreads();                                          // (the sums of a row use the same words)
     return floorf(m);
 }
+
+// ---- values far inside the range rules' bounds ---------------------------------------------------
+__host__ __device__ constexpr uint32_t exponent_bits(int e) { return (uint32_t)(127 + e) << 23; }
+constexpr uint32_t kPlainLo = exponent_bits(-60), kPlainHi = exponent_bits(60), kPlainExp = exponent_bits(6);
+// Below 2 * (hi - lo) where |x| lies in [lo, hi); what lies below wraps around.
+__device__ __forceinline__ uint32_t above(float x, uint32_t lo) { return 2u * (uint32_t)f2i(x) - 2u * lo; }
+__device__ __forceinline__ int exponent_of(uint32_t magnitude) { return (int)(magnitude >> 23) - 127; }
 
 // ---- rows in registers ---------------------------------------------------------------------------
 struct RowArgs {
@@ -155,14 +170,45 @@ row_kernel(const RowArgs a) {
     constexpr int kRowsPerCta = WARPS == 1 ? 4 : 1;
     const int t = WARPS == 1 ? (threadIdx.x & 31) : threadIdx.x;
     const int sub = WARPS == 1 ? (threadIdx.x >> 5) : 0;
-    const float shift = OP == kSoftmaxBwdSaved ? 0.0f : load_shift(a.partials, a.partial_count);
+    const float shift = OP == kSoftmaxBwdSaved ? 0.0f : load_shift<WARPS == 1 ? 128 : WARPS * 32>(a.partials, a.partial_count, scratch);
     const float lb2 = log2f(2.0f);
     const int32_t off = a.off;
     using R = Row<VEC, NCH, WARPS>;
 
-    for (int64_t row = (int64_t)blockIdx.x * kRowsPerCta + sub; row < a.rows; row += (int64_t)gridDim.x * kRowsPerCta) {
-        R x, e;
-        if constexpr (OP == kSoftmaxBwdSaved) {
+    // Short rows: the next row is on its way to registers while this one is worked on (a row is one chain of loads, two sums over the warp
+    // and a divisor, and 32 warps per SM alone leave half of the issue slots empty).
+    constexpr bool kAhead = WARPS == 1 && NCH * VEC <= 8 && (OP == kSoftmaxFwd || OP == kSoftmaxBwdSaved);
+    const int64_t step = (int64_t)gridDim.x * kRowsPerCta;
+    // Rows whose values lie far inside the range rules' bounds, by a look at them all, skip the rules: a product or quotient is
+    // one integer add instead of six instructions, chains of them without another operation between are one.  37824 rows of 197: forward
+    // 25.4 -> 17.0 us, backward 31.2 -> 18.9; 4096 rows of 1024 14.4 -> 10.0 and 15.8 -> 12.4.  What is left is memory (13.7 us backward) and the sums.
+    constexpr bool kPlain = WARPS == 1 && (OP == kSoftmaxFwd || OP == kSoftmaxBwdSaved);
+    // (an offset beyond an eighth of an exponent, or a post scale far from one, could carry results out of those bounds)
+    const bool plain_call = off > -(1 << 20) && off < (1 << 20) && lb2 == 1.0f && (!a.post || (fabsf(a.post_scale) >= 0x1p-8f && fabsf(a.post_scale) <= 0x1p8f));
+    // (after a row that failed the next three go without the look: it costs a fifth of a row)
+    constexpr int kWithout = 3;
+    int without = plain_call ? 0 : INT32_MAX;
+    // masked entries count as an input whose exponent is -1 or -2
+    const int32_t by_log2e = isub(f2i(kLog2e), kBias - off);
+    const float stand_in = i2f(isub(f2i(shift == 1.0f ? -1.0f : fadd(shift, -1.0f)), by_log2e));
+    R ahead, ahead_g;
+    if constexpr (kAhead) {
+        const int64_t row = (int64_t)blockIdx.x * kRowsPerCta + sub;
+        if (row < a.rows) {
+            ahead.load(a.x + row * a.len, a.len, t, OP == kSoftmaxFwd ? -INFINITY : -0.0f);
+            if (OP == kSoftmaxBwdSaved) ahead_g.load(a.g + row * a.len, a.len, t, 0.0f);
+        }
+    }
+    for (int64_t row = (int64_t)blockIdx.x * kRowsPerCta + sub; row < a.rows; row += step) {
+        R x, e, g;
+        if constexpr (kAhead) {
+            if (OP == kSoftmaxFwd) x = ahead;
+            else { e = ahead; g = ahead_g; }
+            if (row + step < a.rows) {
+                ahead.load(a.x + (row + step) * a.len, a.len, t, OP == kSoftmaxFwd ? -INFINITY : -0.0f);
+                if (OP == kSoftmaxBwdSaved) ahead_g.load(a.g + (row + step) * a.len, a.len, t, 0.0f);
+            }
+        } else if constexpr (OP == kSoftmaxBwdSaved) {
             // the saved exponentials; -0.0f marks a masked entry (and the padding) and acts as +0 in every
             // step below: flushed products and quotients are +0, and x + (-0) = x
             e.load(a.x + row * a.len, a.len, t, -0.0f);
@@ -177,16 +223,38 @@ row_kernel(const RowArgs a) {
         // forward kernels: this group's next row towards the L2 while the current one is computed (measured
         // on 1024-long rows: forward 169 -> 156 us per 2^26 elements; the backward kernels, which hold three
         // rows in registers at 12 warps per SM, lose a little with it)
-        if (OP == kSoftmaxFwd || OP == kLseFwd || OP == kLossFwd) {
+        if (!kAhead && (OP == kSoftmaxFwd || OP == kLseFwd || OP == kLossFwd)) {
             const int64_t next = row + (int64_t)gridDim.x * kRowsPerCta;
             if (next < a.rows) prefetch_row_l2(a.x + next * a.len, a.len, t, WARPS * 32);
         }
         float part = 0.0f;
+        bool plain = false;                                    // every value of this row is far inside the rules' bounds (see kPlain)
+        if (kPlain && OP == kSoftmaxFwd && without > 0) --without;
+        else if (kPlain && OP == kSoftmaxFwd) {
+            uint32_t far_x = 0u, far_y = 0u;
+#pragma unroll
+            for (int i = 0; i < NCH * VEC; ++i) {
+                const bool masked = x.v[i] == -INFINITY;
+                const float xi = masked ? stand_in : x.v[i];
+                const float y = i2f(iadd(f2i(fadd(i2f(iadd(f2i(xi), by_log2e)), -shift)), off));
+                far_x = max(far_x, above(xi, kPlainLo));
+                far_y = max(far_y, above(y, kPlainLo));
+                const float fl = floorf(y);
+                const float big = fmul(fadd(1.0f, fadd(y, -fl)), i2f((int32_t)(((uint32_t)(int32_t)fl << 23) + (uint32_t)kBias)));
+                e.v[i] = masked ? 0.0f : big;
+                part = fadd(part, e.v[i]);                     // (padding adds +0)
+            }
+            plain = __all_sync(0xffffffffu, far_x < 2u * (kPlainHi - kPlainLo) && far_y < 2u * (kPlainExp - kPlainLo));
+            if (!plain) {
+                part = 0.0f;
+                without = kWithout;
+            }
+        }
         if constexpr (OP == kSoftmaxBwdSaved) {
 #pragma unroll
             for (int i = 0; i < NCH * VEC; ++i)
                 if (R::col(i, t) < a.len) part = fadd(part, e.v[i]);
-        } else
+        } else if (!plain)
 #pragma unroll
         for (int i = 0; i < NCH * VEC; ++i) {
             const bool masked = x.v[i] == -INFINITY;
@@ -207,9 +275,16 @@ row_kernel(const RowArgs a) {
                 for (int i = 0; i < NCH * VEC; ++i) keep.v[i] = x.v[i] == -INFINITY ? -0.0f : e.v[i];
                 keep.store(a.aux + row * a.len, a.len, t);
             }
-            const Divisor by_total = make_divisor(total, off);
+            if (kPlain && plain && total > 0x1p-40f && total < 0x1p40f) {
+                // (exponentials between 2^-64 and 2^64: their quotients pass)
+                const int32_t sub = isub(f2i(total), kBias - off);
 #pragma unroll
-            for (int i = 0; i < NCH * VEC; ++i) e.v[i] = div_by(e.v[i], by_total);
+                for (int i = 0; i < NCH * VEC; ++i) e.v[i] = e.v[i] == 0.0f ? 0.0f : i2f(isub(f2i(e.v[i]), sub));
+            } else {
+                const Divisor by_total = make_divisor(total, off);
+#pragma unroll
+                for (int i = 0; i < NCH * VEC; ++i) e.v[i] = div_by(e.v[i], by_total);
+            }
             e.store(a.out + row * a.len, a.len, t);
         } else if (OP == kCeBwd) {
             // pam/pam_opt.py:27-51: (softmax(x) - target distribution), PAM-scaled by the class weight,
@@ -284,8 +359,64 @@ row_kernel(const RowArgs a) {
             const float res = div(fadd(shift, log_base(total, lb2, 0)), kLog2e, off);
             if (t == 0) a.out[row] = res;
         } else if (OP == kSoftmaxBwd || OP == kSoftmaxBwdSaved) {
-            R g;
-            g.load(a.g + row * a.len, a.len, t, 0.0f);
+            if (!kAhead) g.load(a.g + row * a.len, a.len, t, 0.0f);
+            if (kPlain && OP == kSoftmaxBwdSaved && without > 0) --without;
+            else if (kPlain && OP == kSoftmaxBwdSaved) {
+                // The magnitudes of the row's exponentials and gradients: with these bounds no product or quotient below leaves the
+                // pass range, so that each is a sum of patterns, and chains of them one sum.
+                uint32_t least_e = ~0u, most_e = 0u, least_g = ~0u, most_g = 0u;
+#pragma unroll
+                for (int i = 0; i < NCH * VEC; ++i) {
+                    const uint32_t be = (uint32_t)f2i(e.v[i]), bg = (uint32_t)f2i(g.v[i]) & 0x7fffffffu;
+                    const bool masked = be == 0x80000000u;      // (an entry that counts for nothing, like the padding)
+                    least_e = min(least_e, masked ? ~0u : be); most_e = max(most_e, masked ? 0u : be);
+                    least_g = min(least_g, masked ? ~0u : bg); most_g = max(most_g, bg);       // (a masked entry's inf or NaN counts)
+                }
+                least_e = __reduce_min_sync(0xffffffffu, least_e); most_e = __reduce_max_sync(0xffffffffu, most_e);
+                least_g = __reduce_min_sync(0xffffffffu, least_g); most_g = __reduce_max_sync(0xffffffffu, most_g);
+                const int e0 = exponent_of(least_e), e1 = exponent_of(most_e), g0 = exponent_of(least_g), g1 = exponent_of(most_g);
+                const int t0 = exponent_of((uint32_t)f2i(total));          // (a negative total has a huge one)
+                // the exponents of e / total, e / total / total, their product with g, and g / total, with one to spare for each step;
+                // e * (g / total + d_total) is looked at below
+                bool ok = e0 >= -60 && e1 <= 60 && g0 >= -60 && g1 <= 60 && t0 >= -40 && t0 <= 40 &&
+                          min(e0 - t0, e0 - 2 * t0) >= -100 && max(e1 - t0, e1 - 2 * t0) <= 100 && e0 - 2 * t0 + g0 >= -108 && e1 - 2 * t0 + g1 <= 108;
+                if (ok) {                                       // (the same for a warp)
+                    const int32_t sub = isub(f2i(total), kBias - off);
+                    const int32_t by_den = isub(isub(isub(0, sub), sub), kBias - off), by_recip = isub(isub(kBias, sub), kBias - off);
+                    float dsum = 0.0f;
+                    R d;
+#pragma unroll
+                    for (int i = 0; i < NCH * VEC; ++i) {
+                        const bool masked = f2i(e.v[i]) == (int32_t)0x80000000;
+                        const float dden = -i2f(iadd3(f2i(e.v[i]), f2i(g.v[i]), by_den));
+                        dsum = fadd(dsum, masked ? -0.0f : dden);
+                        d.v[i] = i2f(iadd(f2i(g.v[i]), by_recip));
+                    }
+                    const float d_total = group_sum<WARPS>(dsum, scratch);
+                    // ((e * ln 2) * d) * log2 e (* post): the constants of the four products in one
+                    const int32_t by_one = kBias - off, by_all = iadd(isub(isub(isub(iadd(f2i(kLn2), f2i(kLog2e)), by_one), by_one), by_one), a.post ? isub(f2i(a.post_scale), by_one) : 0);
+                    constexpr uint32_t kProductLo = 2u * (uint32_t)kBias - (104u << 23), kProductSpan = 204u << 23;   // e * d in [2^-104, 2^100)
+                    uint32_t far = 0u;
+#pragma unroll
+                    for (int i = 0; i < NCH * VEC; ++i) {
+                        const bool masked = f2i(e.v[i]) == (int32_t)0x80000000;
+                        d.v[i] = fadd(d.v[i], d_total);
+                        const uint32_t sum = (uint32_t)f2i(e.v[i]) + ((uint32_t)f2i(d.v[i]) & 0x7fffffffu);
+                        far = max(far, masked ? 0u : sum - kProductLo);
+                    }
+                    ok = __all_sync(0xffffffffu, far < kProductSpan);
+                    if (ok) {
+#pragma unroll
+                        for (int i = 0; i < NCH * VEC; ++i) {
+                            const bool masked = f2i(e.v[i]) == (int32_t)0x80000000;
+                            d.v[i] = masked ? 0.0f : i2f(iadd3(f2i(e.v[i]), f2i(d.v[i]), by_all));
+                        }
+                        d.store(a.out + row * a.len, a.len, t);
+                        continue;
+                    }
+                }
+                without = kWithout;
+            }
             const Divisor by_total = make_divisor(total, off);
             const float recip = div_by(1.0f, by_total);
             float dsum = 0.0f;
