@@ -20,7 +20,8 @@ namespace {
 
 constexpr int kTensorsPerLaunch = 256;     // (an 11 KB kernel argument: within the 32 KB that sm_70 and later take)
 constexpr int kThreads = 256;
-constexpr int kPerBlock = kThreads * 4;
+constexpr int kVectors = 2;                 // vectors of four elements per operand and thread
+constexpr int kPerBlock = kThreads * 4 * kVectors;
 
 struct AdamTable {
     float* p[kTensorsPerLaunch];
@@ -70,14 +71,21 @@ __device__ __forceinline__ bool ordinary(float g, float m, float v) {
 // them might apply after all.  A primitive is one integer add: a product of factors in [2^-61, 2^61), or of one in
 // [2^-100, 2^100) and a scalar in [2^-20, 2^20], passes the range rule, and so does such a quotient.  floor(log2f(x))
 // is the exponent of x unless the mantissa lies so close to either end that log2f might round across
-// the power of two (it is off by a few ulp, at most 2^-15 for exponents up to 128; the ends taken are 2^-11 wide).
+// the power of two (it is off by a few ulp, at most 2^-15 for exponents up to 128; the ends taken are 2^-11 wide): there it is
+// called.  (Sent to the full rule instead, the one in a hundred values of a run with steady gradients that lies there made a third of the
+// warps pay for both: 6+6 transformer 287 us after 3000 steps.)
 __device__ __forceinline__ bool adam_plain(float& p, float g, float& m, float& v, const AdamScalars& s) {
     const int32_t gb = f2i(g), mb = f2i(m), vb = f2i(v), bias = kBias - s.off;
     const int32_t gg = isub(iadd(gb, gb), bias);
     const float m1 = fadd(i2f(iadd(mb, isub(f2i(s.b1), bias))), i2f(iadd(gb, isub(f2i(s.one_minus_b1), bias))));
     const float v1 = fadd(i2f(iadd(vb, isub(f2i(s.b2), bias))), i2f(iadd(gg, isub(f2i(s.one_minus_b2), bias))));
     const int32_t v1b = f2i(v1), mant = v1b & kMant;
-    const float x = fadd((float)((v1b >> 23) - 127), fadd(i2f(mant | kBias), -1.0f));        // log2(v1)
+    float x = fadd((float)((v1b >> 23) - 127), fadd(i2f(mant | kBias), -1.0f));              // log2(v1)
+    if ((uint32_t)(mant - 0x1000) >= 0x7fe000u) {                                             // (log2's own form, see pam_scalar.cuh)
+        const float e = floorf(log2f(v1));
+        const int32_t ei = (int32_t)e;
+        x = fadd(e, fmul(fadd(v1, -i2f((ei + 127) << 23)), i2f((127 - ei) << 23)));
+    }
     // div by log2f(2) = 1, the product with 0.5, the product with log2f(2): one shift of the pattern
     const float h = i2f(iadd(f2i(x), s.off - 0x00800000));
     const float fl = floorf(h);
@@ -86,7 +94,7 @@ __device__ __forceinline__ bool adam_plain(float& p, float g, float& m, float& v
     const int32_t d = iadd(isub(f2i(m1), f2i(den)), bias);
     // (v1 is positive: its field is read without the sign's bit; log2(v1) near 0 would be flushed)
     const bool ok = field_in<27, 227>(gg) && (uint32_t)(v1b - (27 << 23)) < (uint32_t)(200 << 23) &&
-                    (uint32_t)(mant - 0x1000) < 0x7fe000u && fabsf(x) > 0x1p-20f &&
+                    fabsf(x) > 0x1p-20f &&
                     field_in<66, 188>(f2i(m1)) && field_in<66, 188>(f2i(den)) && field_in<66, 188>(d);
     if (!ok) return false;
     if (s.decay != 0.0f) p = fadd(p, -mul(p, s.decay, s.off));
@@ -104,7 +112,8 @@ __device__ __forceinline__ void adam_any(float& p, float g, float& m, float& v, 
     if (!done) adam_one(p, g, m, v, s, lb2);
 }
 
-// Four elements per thread.  With the full rule the kernel is bound by its instructions, five or six per primitive and more
+// Eight elements per thread, all of their loads on the way at once, which also halves the blocks that look for their tensor: the 254 tensors of
+// a 6+6 transformer (42 million parameters) 211 -> 193 us, one tensor of 2^25 154 -> 146.  With the full rule the kernel is bound by its instructions, five or six per primitive and more
 // for the division and log2f that only classify (2^25 elements 192 us); without the range rules by DRAM (150 us).
 // The 32 elements that a warp works on at a time take one of the two together, by a vote on the inputs: where each
 // thread chose for itself, zeros among the gradients (rows of an embedding that no token met, units behind
@@ -125,33 +134,61 @@ __global__ void __launch_bounds__(kThreads) adam_kernel(const AdamTable t, const
     const float lb2 = log2f(2.0f);
     const bool vec = ((reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(g) |
                        reinterpret_cast<uintptr_t>(m) | reinterpret_cast<uintptr_t>(v)) & 15u) == 0;
-    const int64_t i = base + threadIdx.x * 4;
-    const bool four = vec && i + 3 < n;
-    const unsigned fours = __ballot_sync(0xffffffffu, four);          // (every thread of the CTA is here)
-    if (four) {
-        float4 p4 = *reinterpret_cast<const float4*>(p + i);
-        const float4 g4 = __ldg(reinterpret_cast<const float4*>(g + i));
-        float4 m4 = *reinterpret_cast<const float4*>(m + i);
-        float4 v4 = *reinterpret_cast<const float4*>(v + i);
-        adam_any(p4.x, g4.x, m4.x, v4.x, s, lb2, fours);
-        adam_any(p4.y, g4.y, m4.y, v4.y, s, lb2, fours);
-        adam_any(p4.z, g4.z, m4.z, v4.z, s, lb2, fours);
-        adam_any(p4.w, g4.w, m4.w, v4.w, s, lb2, fours);
-        *reinterpret_cast<float4*>(p + i) = p4;
-        *reinterpret_cast<float4*>(m + i) = m4;
-        *reinterpret_cast<float4*>(v + i) = v4;
-    } else {
+    // whole blocks of aligned tensors: two vectors per operand and thread, all on their way before the first is worked on
+    if (vec && base + kPerBlock <= n) {
+        const int64_t i = base + threadIdx.x * 4;
+        float4 p4[kVectors], g4[kVectors], m4[kVectors], v4[kVectors];
+#pragma unroll
+        for (int q = 0; q < kVectors; ++q) {
+            const int64_t at = i + q * kThreads * 4;
+            p4[q] = *reinterpret_cast<const float4*>(p + at);
+            g4[q] = __ldg(reinterpret_cast<const float4*>(g + at));
+            m4[q] = *reinterpret_cast<const float4*>(m + at);
+            v4[q] = *reinterpret_cast<const float4*>(v + at);
+        }
+#pragma unroll
+        for (int q = 0; q < kVectors; ++q) {
+            const int64_t at = i + q * kThreads * 4;
+            adam_any(p4[q].x, g4[q].x, m4[q].x, v4[q].x, s, lb2, 0xffffffffu);
+            adam_any(p4[q].y, g4[q].y, m4[q].y, v4[q].y, s, lb2, 0xffffffffu);
+            adam_any(p4[q].z, g4[q].z, m4[q].z, v4[q].z, s, lb2, 0xffffffffu);
+            adam_any(p4[q].w, g4[q].w, m4[q].w, v4[q].w, s, lb2, 0xffffffffu);
+            *reinterpret_cast<float4*>(p + at) = p4[q];
+            *reinterpret_cast<float4*>(m + at) = m4[q];
+            *reinterpret_cast<float4*>(v + at) = v4[q];
+        }
+        return;
+    }
 #pragma unroll 1
-        for (int c = 0; c < 4; ++c) {
-            const bool on = i + c < n;
-            const unsigned ons = __ballot_sync(~fours, on);
-            if (on) {
-                float pp = p[i + c], mm = m[i + c], vv = v[i + c];
-                const float gg = g[i + c];
-                adam_any(pp, gg, mm, vv, s, lb2, ons);
-                p[i + c] = pp;
-                m[i + c] = mm;
-                v[i + c] = vv;
+    for (int q = 0; q < kVectors; ++q) {
+        const int64_t i = base + q * kThreads * 4 + threadIdx.x * 4;
+        const bool four = vec && i + 3 < n;
+        const unsigned fours = __ballot_sync(0xffffffffu, four);          // (every thread of the CTA is here)
+        if (four) {
+            float4 p4 = *reinterpret_cast<const float4*>(p + i);
+            const float4 g4 = __ldg(reinterpret_cast<const float4*>(g + i));
+            float4 m4 = *reinterpret_cast<const float4*>(m + i);
+            float4 v4 = *reinterpret_cast<const float4*>(v + i);
+            adam_any(p4.x, g4.x, m4.x, v4.x, s, lb2, fours);
+            adam_any(p4.y, g4.y, m4.y, v4.y, s, lb2, fours);
+            adam_any(p4.z, g4.z, m4.z, v4.z, s, lb2, fours);
+            adam_any(p4.w, g4.w, m4.w, v4.w, s, lb2, fours);
+            *reinterpret_cast<float4*>(p + i) = p4;
+            *reinterpret_cast<float4*>(m + i) = m4;
+            *reinterpret_cast<float4*>(v + i) = v4;
+        } else {
+#pragma unroll 1
+            for (int c = 0; c < 4; ++c) {
+                const bool on = i + c < n;
+                const unsigned ons = __ballot_sync(~fours, on);
+                if (on) {
+                    float pp = p[i + c], mm = m[i + c], vv = v[i + c];
+                    const float gg = g[i + c];
+                    adam_any(pp, gg, mm, vv, s, lb2, ons);
+                    p[i + c] = pp;
+                    m[i + c] = mm;
+                    v[i + c] = vv;
+                }
             }
         }
     }
