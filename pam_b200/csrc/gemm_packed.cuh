@@ -403,6 +403,7 @@ __global__ void __launch_bounds__(256, 2) packed_kernel(const PackedParams p) {
             for (int j = 0; j < MT; ++j) acc[i][j] = quiet_nan();
     }
 
+    next_may_start();                                           // (the reduction pass)
     const int m0 = blockIdx.y * (MR * 16), n0 = blockIdx.x * 128;
     float* Cz = p.C + (int64_t)sp * p.sCsplit + (int64_t)__umulhi((unsigned)z, p.inner_magic) * p.sCb + (int64_t)z * p.sCb2;
     const bool vec_out = ((p.N | p.ldc | p.sCb | p.sCb2 | p.sCsplit) & 3) == 0 && aligned16(p.C);

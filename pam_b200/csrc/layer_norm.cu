@@ -393,6 +393,7 @@ __global__ void __launch_bounds__(kThreads, VEC * NCH <= 16 ? (SAVED ? 5 : 3) : 
     }
 
     // per-CTA column sums for dw / db: warps are added in warp order, CTAs by the second kernel
+    next_may_start();
     if (a.partials) {
         float* slot = a.partials + (int64_t)blockIdx.x * 2 * a.width;
 #pragma unroll
@@ -419,13 +420,13 @@ __global__ void __launch_bounds__(kThreads, VEC * NCH <= 16 ? (SAVED ? 5 : 3) : 
 // the partials of CTAs j, j + 32, j + 64, ... in that order, then the 32 warp sums are added in
 // warp order.
 constexpr int kGradWarps = 32;
-__global__ void __launch_bounds__(kGradWarps * 32) ln_param_grad_kernel(const float* __restrict__ partials,
-                                                                       float* __restrict__ dw, float* __restrict__ db,
+__global__ void __launch_bounds__(kGradWarps * 32) ln_param_grad_kernel(const float* partials, float* __restrict__ dw, float* __restrict__ db,
                                                                        int ctas, int width) {
     __shared__ float stage[2][kGradWarps][32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int col = blockIdx.x * 32 + lane;
     float sw = 0.0f, sb = 0.0f;
+    after_previous();
     if (col < width) {
         // eight partials of each sum requested at a time: with a CTA per 32 columns there is little but the loads' latency
         // (from four: 4096 rows of 512 6.4 -> 5.5 us, 12608 of 192 9.4 -> 8.8, 65536 of 1024 13.1 -> 11.7, 300 of 768 unchanged)
@@ -434,8 +435,8 @@ __global__ void __launch_bounds__(kGradWarps * 32) ln_param_grad_kernel(const fl
             float w[8], b[8];
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
-                w[u] = __ldg(partials + ((int64_t)(k + u * kGradWarps) * 2) * width + col);
-                b[u] = __ldg(partials + ((int64_t)(k + u * kGradWarps) * 2 + 1) * width + col);
+                w[u] = __ldcg(partials + ((int64_t)(k + u * kGradWarps) * 2) * width + col);
+                b[u] = __ldcg(partials + ((int64_t)(k + u * kGradWarps) * 2 + 1) * width + col);
             }
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
@@ -444,8 +445,8 @@ __global__ void __launch_bounds__(kGradWarps * 32) ln_param_grad_kernel(const fl
             }
         }
         for (; k < ctas; k += kGradWarps) {
-            sw = fadd(sw, __ldg(partials + ((int64_t)k * 2) * width + col));
-            sb = fadd(sb, __ldg(partials + ((int64_t)k * 2 + 1) * width + col));
+            sw = fadd(sw, __ldcg(partials + ((int64_t)k * 2) * width + col));
+            sb = fadd(sb, __ldcg(partials + ((int64_t)k * 2 + 1) * width + col));
         }
     }
     stage[0][wid][lane] = sw;
@@ -557,9 +558,8 @@ int pamk_layer_norm_bwd_saved(const float* x, const float* weight, const float* 
              rows, (int)width, (float)width, 0.0f, offset_bits(offset), const_cast<float*>(stats)};
     const int rc = launch<true, true, true>(a, grid, st);
     if (rc != PAMK_OK || !params) return rc;
-    ln_param_grad_kernel<<<(unsigned)((width + 31) / 32), kGradWarps * 32, 0, st>>>(
-        static_cast<const float*>(workspace), dweight, dbias, grid, (int)width);
-    return check_launch();
+    return launch_behind(ln_param_grad_kernel, dim3((unsigned)((width + 31) / 32)), kGradWarps * 32, st, static_cast<const float*>(workspace), dweight,
+                         dbias, grid, (int)width);
 }
 
 size_t pamk_layer_norm_bwd_workspace_bytes(int64_t rows, int64_t width) {
@@ -589,9 +589,8 @@ int pamk_layer_norm_bwd(const float* x, const float* weight, const float* dy, fl
              rows, (int)width, (float)width, eps, offset_bits(offset)};
     const int rc = approx_bwd ? launch<true, true>(a, grid, st) : launch<true, false>(a, grid, st);
     if (rc != PAMK_OK || !params) return rc;
-    ln_param_grad_kernel<<<(unsigned)((width + 31) / 32), kGradWarps * 32, 0, st>>>(
-        static_cast<const float*>(workspace), dweight, dbias, grid, (int)width);
-    return check_launch();
+    return launch_behind(ln_param_grad_kernel, dim3((unsigned)((width + 31) / 32)), kGradWarps * 32, st, static_cast<const float*>(workspace), dweight,
+                         dbias, grid, (int)width);
 }
 
 }

@@ -38,6 +38,7 @@ __global__ void __launch_bounds__(kColWarps * 32) column_partial_kernel(const fl
                 if (c0 + j < cols) s[j] = fadd(s[j], __ldg(p + j));
         }
     }
+    next_may_start();
 #pragma unroll
     for (int j = 0; j < 4; ++j) stage[wid][lane * 4 + j] = s[j];
     __syncthreads();
@@ -53,15 +54,16 @@ __global__ void __launch_bounds__(kColWarps * 32) column_partial_kernel(const fl
 // out[c] = sum over chunks of partial[chunk][c].  One CTA per 32 columns; warp j adds the chunks
 // j, j + 32, j + 64, ... in that order, then the 32 warp sums are added in warp order.
 constexpr int kFinalWarps = 32;
-__global__ void __launch_bounds__(kFinalWarps * 32) column_final_kernel(const float* __restrict__ partial,
+__global__ void __launch_bounds__(kFinalWarps * 32) column_final_kernel(const float* partial,
                                                                         float* __restrict__ out, int chunks, int cols) {
     __shared__ float stage[kFinalWarps][32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int c = blockIdx.x * 32 + lane;
     float t = 0.0f;
+    after_previous();
     if (c < cols) {
 #pragma unroll 4
-        for (int k = wid; k < chunks; k += kFinalWarps) t = fadd(t, __ldg(partial + (int64_t)k * cols + c));
+        for (int k = wid; k < chunks; k += kFinalWarps) t = fadd(t, __ldcg(partial + (int64_t)k * cols + c));
     }
     stage[wid][lane] = t;
     __syncthreads();
@@ -119,8 +121,8 @@ int pamk_column_sum(const float* X, float* out, int64_t rows, int64_t cols, void
         column_partial_kernel<false><<<grid, kColWarps * 32, 0, st>>>(X, partial, rows, (int)cols, rows_per_chunk);
     int rc = check_launch();
     if (rc != PAMK_OK) return rc;
-    column_final_kernel<<<(unsigned)((cols + 31) / 32), kFinalWarps * 32, 0, st>>>(partial, out, chunks, (int)cols);
-    return check_launch();
+    return launch_behind(column_final_kernel, dim3((unsigned)((cols + 31) / 32)), kFinalWarps * 32, st, static_cast<const float*>(partial), out, chunks,
+                         (int)cols);
 }
 
 }

@@ -48,6 +48,8 @@ __global__ void __launch_bounds__(256) scaled_max_kernel(const float* __restrict
         for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += stride)
             m = nan_max(m, scaled_of(__ldg(x + i), off));
     }
+    // (not earlier: CTAs of the row pass would gather on the SMs that have room first, and keep their rows there)
+    next_may_start();
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) m = nan_max(m, __shfl_xor_sync(0xffffffffu, m, d));
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
@@ -60,10 +62,11 @@ __global__ void __launch_bounds__(256) scaled_max_kernel(const float* __restrict
 
 // shift = floor(max over the per-CTA maxima), by all threads of the CTA: a warp alone would wait for 37 loads, one after the other
 template <int THREADS>
-__device__ __forceinline__ float load_shift(const float* __restrict__ partials, int count, float* scratch) {
+__device__ __forceinline__ float load_shift(const float* partials, int count, float* scratch) {
+    after_previous();
     float m = -INFINITY;
 #pragma unroll 5
-    for (int k = threadIdx.x; k < count; k += THREADS) m = nan_max(m, __ldg(partials + k));
+    for (int k = threadIdx.x; k < count; k += THREADS) m = nan_max(m, __ldcg(partials + k));
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) m = nan_max(m, __shfl_xor_sync(0xffffffffu, m, d));
     if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = m;
@@ -170,15 +173,22 @@ row_kernel(const RowArgs a) {
     constexpr int kRowsPerCta = WARPS == 1 ? 4 : 1;
     const int t = WARPS == 1 ? (threadIdx.x & 31) : threadIdx.x;
     const int sub = WARPS == 1 ? (threadIdx.x >> 5) : 0;
-    const float shift = OP == kSoftmaxBwdSaved ? 0.0f : load_shift<WARPS == 1 ? 128 : WARPS * 32>(a.partials, a.partial_count, scratch);
-    const float lb2 = log2f(2.0f);
-    const int32_t off = a.off;
     using R = Row<VEC, NCH, WARPS>;
-
     // Short rows: the next row is on its way to registers while this one is worked on (a row is one chain of loads, two sums over the warp
     // and a divisor, and 32 warps per SM alone leave half of the issue slots empty).
     constexpr bool kAhead = WARPS == 1 && NCH * VEC <= 8 && (OP == kSoftmaxFwd || OP == kSoftmaxBwdSaved);
     const int64_t step = (int64_t)gridDim.x * kRowsPerCta;
+    R ahead, ahead_g;
+    if constexpr (kAhead) {                                    // (not written by the maximum pass, which may still run)
+        const int64_t row = (int64_t)blockIdx.x * kRowsPerCta + sub;
+        if (row < a.rows) {
+            ahead.load(a.x + row * a.len, a.len, t, OP == kSoftmaxFwd ? -INFINITY : -0.0f);
+            if (OP == kSoftmaxBwdSaved) ahead_g.load(a.g + row * a.len, a.len, t, 0.0f);
+        }
+    }
+    const float shift = OP == kSoftmaxBwdSaved ? 0.0f : load_shift<WARPS == 1 ? 128 : WARPS * 32>(a.partials, a.partial_count, scratch);
+    const float lb2 = log2f(2.0f);
+    const int32_t off = a.off;
     // Rows whose values lie far inside the range rules' bounds, by a look at them all, skip the rules: a product or quotient is
     // one integer add instead of six instructions, chains of them without another operation between are one.  37824 rows of 197: forward
     // 25.4 -> 17.0 us, backward 31.2 -> 18.9; 4096 rows of 1024 14.4 -> 10.0 and 15.8 -> 12.4.  What is left is memory (13.7 us backward) and the sums.
@@ -191,14 +201,6 @@ row_kernel(const RowArgs a) {
     // masked entries count as an input whose exponent is -1 or -2
     const int32_t by_log2e = isub(f2i(kLog2e), kBias - off);
     const float stand_in = i2f(isub(f2i(shift == 1.0f ? -1.0f : fadd(shift, -1.0f)), by_log2e));
-    R ahead, ahead_g;
-    if constexpr (kAhead) {
-        const int64_t row = (int64_t)blockIdx.x * kRowsPerCta + sub;
-        if (row < a.rows) {
-            ahead.load(a.x + row * a.len, a.len, t, OP == kSoftmaxFwd ? -INFINITY : -0.0f);
-            if (OP == kSoftmaxBwdSaved) ahead_g.load(a.g + row * a.len, a.len, t, 0.0f);
-        }
-    }
     for (int64_t row = (int64_t)blockIdx.x * kRowsPerCta + sub; row < a.rows; row += step) {
         R x, e, g;
         if constexpr (kAhead) {
@@ -465,11 +467,17 @@ int launch_rows(const RowArgs& a, cudaStream_t st) {
     const bool vec = (a.len & 3) == 0 && aligned16(a.x) && (OP == kLseFwd || OP == kLossFwd || aligned16(a.out)) &&
                      ((OP != kSoftmaxBwd && OP != kSoftmaxBwdSaved) || aligned16(a.g)) && (a.aux == nullptr || aligned16(a.aux));
     const int64_t sms = sm_count();
+    // Behind the maximum pass where there is one (2 us: 591 rows of 197 8.2 -> 6.5, 37824 26.7 -> 24.6).  Not the recomputing backward passes of
+    // several rows per warp, which are long enough for an uneven start to cost more: 65536 rows of 197 91 -> 96.
+    constexpr bool kForward = OP == kSoftmaxFwd || OP == kLseFwd || OP == kLossFwd;
+    const bool behind = OP != kSoftmaxBwdSaved;
 #define PAMK_ROWS(V, N, W)                                                                              \
     do {                                                                                                \
         const int64_t per = (W) == 1 ? 4 : 1;                                                           \
         const int64_t want = (a.rows + per - 1) / per, cap = sms * ((W) == 1 ? 8 : 4);                  \
-        row_kernel<OP, APPROX, V, N, W><<<(unsigned)(want < cap ? want : cap), (W) == 1 ? 128 : (W) * 32, 0, st>>>(a); \
+        const dim3 grid((unsigned)(want < cap ? want : cap));                                            \
+        if (behind && (kForward || want <= cap)) return launch_behind(row_kernel<OP, APPROX, V, N, W>, grid, (W) == 1 ? 128 : (W) * 32, st, a); \
+        row_kernel<OP, APPROX, V, N, W><<<grid, (W) == 1 ? 128 : (W) * 32, 0, st>>>(a);                  \
         return check_launch();                                                                          \
     } while (0)
     // (the number of chunks per thread only sets how many register slots a row may fill: a shorter layout
