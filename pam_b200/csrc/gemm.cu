@@ -128,6 +128,7 @@ __host__ __device__ constexpr int slot_row(int slot) {
 }
 
 // ---- loaders: global -> registers ---------------------------------------------------------------
+// (Plain loads: the compiler may move loads of constant memory, __ldg, in front of the wait for the kernel before, see after_previous.)
 // A slab is R rows x BK k, staged as float4 "tasks"; thread t takes tasks t, t + kThreads, ...
 //   KC (operand contiguous along k: row-major A, or B given as W[N,K]):
 //       task id -> row id / (BK/4), k-group id % (BK/4): a warp reads kRowsPerWarp rows x 4*BK bytes;
@@ -148,7 +149,7 @@ __device__ __forceinline__ void load_slab(float (&r)[NT * 4], const MatArg& m, c
             const int k = k0 + (id % (T::BK / 4)) * 4;
             const float* src = base + (int64_t)row * m.sr + k;
 #pragma unroll
-            for (int c = 0; c < 4; ++c) r[t * 4 + c] = k + c < k_end ? __ldg(src + c) : 0.0f;
+            for (int c = 0; c < 4; ++c) r[t * 4 + c] = k + c < k_end ? src[c] : 0.0f;
         } else {
             const int k = k0 + id / (R / 4);
             const int c0 = row0 + (id % (R / 4)) * 4;
@@ -157,7 +158,7 @@ __device__ __forceinline__ void load_slab(float (&r)[NT * 4], const MatArg& m, c
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 const int col = c0 + c < rows ? c0 + c : rows - 1;
-                r[t * 4 + c] = on ? __ldg(src + col) : 0.0f;
+                r[t * 4 + c] = on ? src[col] : 0.0f;
             }
         }
     }
@@ -198,7 +199,7 @@ struct ScalarWalker {
             const int id = tid + t * T::kThreads;
             const int k = KC ? k0 + (id % (T::BK / 4)) * 4 : k0 + id / (R / 4);
 #pragma unroll
-            for (int c = 0; c < 4; ++c) r[t * 4 + c] = (KC ? k + c : k) < k_end ? __ldg(ptr[t] + (KC ? c : rows_of[KC ? 0 : t][c])) : 0.0f;
+            for (int c = 0; c < 4; ++c) r[t * 4 + c] = (KC ? k + c : k) < k_end ? ptr[t][KC ? c : rows_of[KC ? 0 : t][c]] : 0.0f;
             ptr[t] += step;
         }
     }
@@ -235,7 +236,7 @@ struct SlabWalker {
         for (int t = 0; t < NT; ++t) {
             const int id = tid + t * T::kThreads;
             const int k = KC ? k0 + (id % (T::BK / 4)) * 4 : k0 + id / (R / 4);
-            const float4 v = k < k_end ? __ldg(reinterpret_cast<const float4*>(ptr[t])) : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float4 v = k < k_end ? *reinterpret_cast<const float4*>(ptr[t]) : make_float4(0.f, 0.f, 0.f, 0.f);
             r[t * 4] = v.x; r[t * 4 + 1] = v.y; r[t * 4 + 2] = v.z; r[t * 4 + 3] = v.w;
             ptr[t] += step;
         }
@@ -511,6 +512,7 @@ gemm_kernel(const GemmParams p) {
 #pragma unroll
         for (int j = 0; j < MT; ++j) acc[i][j] = 0.0f;
 
+    after_previous();
     // exact-gradient product: per-output constant (mantissa of D + offset) that the slope adds to
     // the other operand's bits (pam_scalar.cuh mul_slope).
     int32_t dm[MODE >= kBwdL ? MR : 1][MODE >= kBwdL ? MT : 1];
@@ -524,7 +526,7 @@ gemm_kernel(const GemmParams p) {
             for (int j = 0; j < MT; ++j) {
                 int col = n0 + tx * 4 + (j & 3) + (j >> 2) * (BN / 2);
                 col = col < p.N ? col : p.N - 1;
-                dm[i][j] = iadd(kMant & f2i(__ldg(Db + (int64_t)row * p.sDm + (int64_t)col * p.sDn)), p.off);
+                dm[i][j] = iadd(kMant & f2i(Db[(int64_t)row * p.sDm + (int64_t)col * p.sDn]), p.off);
             }
         }
     }
@@ -1023,7 +1025,7 @@ gemm_kernel(const GemmParams p) {
             if (add_bias) {                            // the bias row is re-read per output row (it stays in L1)
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
-                    if (col + j < p.N) acc[i][h * 4 + j] = fadd(acc[i][h * 4 + j], __ldg(p.bias + col + j));
+                    if (col + j < p.N) acc[i][h * 4 + j] = fadd(acc[i][h * 4 + j], p.bias[col + j]);
             }
             if (post) {
 #pragma unroll
@@ -1229,9 +1231,21 @@ int dispatch_ranges(const GemmParams& p, bool a_kc, bool b_kc, cudaStream_t st) 
     return check_launch();
 }
 
+// Launches a product's kernel, behind the kernel before it (512x512x1024 29.8 -> 27.6 us with its reduction, 12608x768x192 131.2 -> 129.7) where
+// some SM gets as many of its CTAs as it holds anyway.  A launch of fewer would gather on the SMs that have room first: the 591 tiles
+// of a product of 12608x192 are four per SM when all are free.
+template <class T>
+int launch_tiles(void (*kernel)(const GemmParams), const GemmParams& p, dim3 grid, int ctas_per_sm, cudaStream_t st) {
+    const int64_t ctas = (int64_t)grid.x * grid.y * grid.z, sms = sm_count();
+    if ((ctas + sms - 1) / sms >= ctas_per_sm) return launch_behind(kernel, grid, T::kThreads, st, p);
+    kernel<<<grid, T::kThreads, 0, st>>>(p);
+    return check_launch();
+}
+
 template <int MODE, class T>
 int dispatch(const GemmParams& p, bool a_kc, bool b_kc, bool vec, dim3 grid, cudaStream_t st) {
-#define PAMK_LAUNCH(AK, BKC, V) gemm_kernel<MODE, T, AK, BKC, V><<<grid, T::kThreads, 0, st>>>(p)
+    constexpr int kPerSm = MODE == kPam || MODE == kStd ? T::kCtasPerSm : T::kCtasPerSm / 2;
+#define PAMK_LAUNCH(AK, BKC, V) return launch_tiles<T>(gemm_kernel<MODE, T, AK, BKC, V>, p, grid, kPerSm, st)
     if (vec) {
         if (a_kc) { if (b_kc) PAMK_LAUNCH(true, true, true); else PAMK_LAUNCH(true, false, true); }
         else      { if (b_kc) PAMK_LAUNCH(false, true, true); else PAMK_LAUNCH(false, false, true); }
@@ -1240,24 +1254,21 @@ int dispatch(const GemmParams& p, bool a_kc, bool b_kc, bool vec, dim3 grid, cud
         else      { if (b_kc) PAMK_LAUNCH(false, true, false); else PAMK_LAUNCH(false, false, false); }
     }
 #undef PAMK_LAUNCH
-    return check_launch();
 }
 
 // (with fewer rows per thread there are no 128-bit loads along A's rows, and of the large tile only 128-bit loads)
 template <class T>
 int dispatch_rows(const GemmParams& p, bool b_kc, dim3 grid, cudaStream_t st) {
-    if (b_kc) gemm_kernel<kPam, T, true, true, true><<<grid, T::kThreads, 0, st>>>(p);
-    else gemm_kernel<kPam, T, true, false, true><<<grid, T::kThreads, 0, st>>>(p);
-    return check_launch();
+    if (b_kc) return launch_tiles<T>(gemm_kernel<kPam, T, true, true, true>, p, grid, T::kCtasPerSm, st);
+    else return launch_tiles<T>(gemm_kernel<kPam, T, true, false, true>, p, grid, T::kCtasPerSm, st);
 }
 
 template <class T>
 int dispatch_rows_scalar(const GemmParams& p, bool a_kc, bool b_kc, dim3 grid, cudaStream_t st) {
-    if (a_kc && b_kc) gemm_kernel<kPam, T, true, true, false><<<grid, T::kThreads, 0, st>>>(p);
-    else if (a_kc) gemm_kernel<kPam, T, true, false, false><<<grid, T::kThreads, 0, st>>>(p);
-    else if (b_kc) gemm_kernel<kPam, T, false, true, false><<<grid, T::kThreads, 0, st>>>(p);
-    else gemm_kernel<kPam, T, false, false, false><<<grid, T::kThreads, 0, st>>>(p);
-    return check_launch();
+    if (a_kc && b_kc) return launch_tiles<T>(gemm_kernel<kPam, T, true, true, false>, p, grid, T::kCtasPerSm, st);
+    else if (a_kc) return launch_tiles<T>(gemm_kernel<kPam, T, true, false, false>, p, grid, T::kCtasPerSm, st);
+    else if (b_kc) return launch_tiles<T>(gemm_kernel<kPam, T, false, true, false>, p, grid, T::kCtasPerSm, st);
+    else return launch_tiles<T>(gemm_kernel<kPam, T, false, false, false>, p, grid, T::kCtasPerSm, st);
 }
 
 // An operand can use 128-bit loads when its base and both non-unit strides keep every group of
