@@ -26,6 +26,8 @@
 //     the reference's kernel (cuda_kernels.cu:608-629), so without split-K the sums are
 //     bit-identical too.
 //
+// Products that are large in both dimensions run on operands packed by a pass over them (gemm_packed.cuh), small ones in ranges of K
+// in one launch (ranges_kernel).
 // The same skeleton serves true-multiply products (standard_matmul) and the exact-gradient
 // product (pam_matmul_bwd_kernel, cuda_kernels.cu:729-832).
 #include <array>

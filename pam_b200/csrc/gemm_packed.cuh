@@ -484,8 +484,12 @@ int run_packed(const GemmParams& p, const PackLayout& l, bool a_kc, bool b_kc, b
     const int64_t a_ctas = (int64_t)p.batch * groups * l.a_tiles, b_ctas = (int64_t)p.batch * groups * l.b_tiles;
     if (a_ctas + b_ctas > 0x7fffffff) return PAMK_ERR_SIZE;
     pack_kernel<<<(unsigned)(a_ctas + b_ctas), 256, 0, st>>>(A, B, groups, (int)a_ctas);
+    int rc = check_launch();
+    if (rc != PAMK_OK) return rc;
     const int64_t blocks = l.a_blocks + l.b_blocks, resident = (int64_t)sm_count() * 8;
     classify_kernel<<<(unsigned)(blocks < resident ? blocks : resident), 256, 0, st>>>(A, B, l.a_blocks, blocks);
+    rc = check_launch();
+    if (rc != PAMK_OK) return rc;
     const PackedParams g{A.out, B.out, p.C, p.ldc, p.sCb, p.sCb2, p.sCsplit, p.bias, p.post, p.post_scale, p.inner_magic,
                          p.M, p.N, p.K, p.splits, p.k_chunk / 16, l.slabs, l.a_tiles, l.b_tiles, p.bias_sub, p.off, p.one, p.least};
     const auto kernel = l.tile_rows == 128 ? packed_kernel<8> : packed_kernel<7>;

@@ -191,7 +191,7 @@ row_kernel(const RowArgs a) {
     const int32_t off = a.off;
     // Rows whose values lie far inside the range rules' bounds, by a look at them all, skip the rules: a product or quotient is
     // one integer add instead of six instructions, chains of them without another operation between are one.  37824 rows of 197: forward
-    // 25.4 -> 17.0 us, backward 31.2 -> 18.9; 4096 rows of 1024 14.4 -> 10.0 and 15.8 -> 12.4.  What is left is memory (13.7 us backward) and the sums.
+    // 25.4 -> 17.0 us, backward 31.2 -> 18.9; 4096 rows of 1024 14.4 -> 10.7 and 15.8 -> 11.7.  What is left is memory (13.7 us backward) and the sums.
     constexpr bool kPlain = WARPS == 1 && (OP == kSoftmaxFwd || OP == kSoftmaxBwdSaved);
     // (an offset beyond an eighth of an exponent, or a post scale far from one, could carry results out of those bounds)
     const bool plain_call = off > -(1 << 20) && off < (1 << 20) && lb2 == 1.0f && (!a.post || (fabsf(a.post_scale) >= 0x1p-8f && fabsf(a.post_scale) <= 0x1p8f));
