@@ -83,6 +83,7 @@ __host__ __device__ constexpr uint32_t exponent_bits(int e) { return (uint32_t)(
 constexpr uint32_t kPlainLo = exponent_bits(-60), kPlainHi = exponent_bits(60), kPlainExp = exponent_bits(6);
 // Below 2 * (hi - lo) where |x| lies in [lo, hi); what lies below wraps around.
 __device__ __forceinline__ uint32_t above(float x, uint32_t lo) { return 2u * (uint32_t)f2i(x) - 2u * lo; }
+constexpr int kMostE = 20;          // exponents of the exponentials that the short backward form takes
 __device__ __forceinline__ int exponent_of(uint32_t magnitude) { return (int)(magnitude >> 23) - 127; }
 
 // ---- rows in registers ---------------------------------------------------------------------------
@@ -379,8 +380,9 @@ row_kernel(const RowArgs a) {
                 const int e0 = exponent_of(least_e), e1 = exponent_of(most_e), g0 = exponent_of(least_g), g1 = exponent_of(most_g);
                 const int t0 = exponent_of((uint32_t)f2i(total));          // (a negative total has a huge one)
                 // the exponents of e / total, e / total / total, their product with g, and g / total, with one to spare for each step;
-                // e * (g / total + d_total) is looked at below
-                bool ok = e0 >= -60 && e1 <= 60 && g0 >= -60 && g1 <= 60 && t0 >= -40 && t0 <= 40 &&
+                // e * (g / total + d_total) is looked at below, by a sum of patterns that a second factor of zero (or a subnormal one) only brings
+                // below kProductLo where e < 2^22 (the forward pass saves none above 4)
+                bool ok = e0 >= -60 && e1 <= kMostE && g0 >= -60 && g1 <= 60 && t0 >= -40 && t0 <= 40 &&
                           min(e0 - t0, e0 - 2 * t0) >= -100 && max(e1 - t0, e1 - 2 * t0) <= 100 && e0 - 2 * t0 + g0 >= -108 && e1 - 2 * t0 + g1 <= 108;
                 if (ok) {                                       // (the same for a warp)
                     const int32_t sub = isub(f2i(total), kBias - off);
@@ -398,6 +400,7 @@ row_kernel(const RowArgs a) {
                     // ((e * ln 2) * d) * log2 e (* post): the constants of the four products in one
                     const int32_t by_one = kBias - off, by_all = iadd(isub(isub(isub(iadd(f2i(kLn2), f2i(kLog2e)), by_one), by_one), by_one), a.post ? isub(f2i(a.post_scale), by_one) : 0);
                     constexpr uint32_t kProductLo = 2u * (uint32_t)kBias - (104u << 23), kProductSpan = 204u << 23;   // e * d in [2^-104, 2^100)
+                    static_assert(exponent_bits(kMostE + 1) + (1u << 23) < kProductLo, "no e and subnormal d reach the bound");
                     uint32_t far = 0u;
 #pragma unroll
                     for (int i = 0; i < NCH * VEC; ++i) {

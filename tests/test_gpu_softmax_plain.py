@@ -108,3 +108,17 @@ def test_many_rows_per_warp():
     want, want_e = _forward(x, 1.0)
     assert_bits_equal(e, want_e), assert_bits_equal(y, want)
     assert_bits_equal(dx, _backward(e, dy, 1.0, None))
+
+
+@pytest.mark.parametrize("n", [1, 2])
+@pytest.mark.parametrize("offset", [1.0, 1.0552])
+def test_great_exponentials_whose_gradient_cancels(n, offset):
+    """Exponentials of a caller's own, far above those that the forward pass saves, with gradients that cancel: e * 0 is +0."""
+    from pam_b200 import _lib
+    k = torch.arange(-60, 61, dtype=torch.float32)
+    e, dy = torch.exp2(k)[:, None].expand(-1, n).contiguous().cuda(), torch.ones(121, n, device="cuda")
+    e, dy = torch.cat([e, e * 1.5, e]), torch.cat([dy, dy, dy * 2.0 ** -20])
+    dx = torch.full_like(e, -7.0)
+    _lib.check(_lib.lib().pamk_softmax_bwd_saved(e.data_ptr(), dy.data_ptr(), dx.data_ptr(), e.shape[0], n, offset, 0, 0.0,
+                                                 torch.cuda.current_stream().cuda_stream), "bwd")
+    assert_bits_equal(dx, _backward(e, dy, offset, None))
