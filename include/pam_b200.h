@@ -147,7 +147,10 @@ size_t pamk_matmul_workspace_bytes(int64_t batch, int64_t M, int64_t N, int spli
 /* Scratch with which pamk_matmul, pamk_matmul_bias and pamk_matmul_strided form a PAM product fastest: that of the split (0: the
  * library's choice) and, for large products, room for both operands in the form that the kernel reads (about the
  * operands' size again).  With less, down to pamk_matmul_workspace_bytes, the results are the same bits.  Products of at most
- * PAMK_PACKED_PRODUCTS multiply-accumulates never use more than pamk_matmul_workspace_bytes (rounded up to 256). */
+ * PAMK_PACKED_PRODUCTS multiply-accumulates never use more than pamk_matmul_workspace_bytes (rounded up to 256).
+ * The kernel with that room waits for its copies to shared memory, for at most two seconds each: should one not land (a fault of
+ * the GPU), the kernel ends and the outputs that lacked it are NaN.  The call has returned PAMK_OK by then, as calls do that queue work; NaN
+ * is the only sign in the results, and pamk_test_expired_waits (pam_b200_testing.h) counts such events. */
 #define PAMK_PACKED_PRODUCTS 3.0e9
 size_t pamk_matmul_scratch_bytes(int64_t batch, int64_t M, int64_t N, int64_t K, int split_k);
 /* The split the library would choose for split_k = 0 given unlimited workspace. */

@@ -37,9 +37,14 @@ int pamk_test_split_rows(int64_t M, int64_t N, int64_t K, int split_k);
  * 2 = never.  Process-wide and not thread-safe.  No counterpart in the reference. */
 int pamk_test_set_packing_policy(int policy);
 
-/* How many waits inside kernels have run out on the current device since the library was loaded (a product whose wait ran out holds
- * NaN): 0 unless something is wrong.  Synchronises.  No counterpart in the reference. */
+/* In how many CTAs a wait has run out on the current device since the library was loaded (see pamk_matmul_scratch_bytes):
+ * 0 unless something is wrong.  Synchronises.  No counterpart in the reference. */
 int pamk_test_expired_waits(unsigned* count);
+
+/* Lets a wait of those kernels run out after `ms` (at most 1000): one CTA of eight warps whose barriers nothing arrives at, the first with that
+ * limit.  out, ten values on the device: whether each warp's barrier was reached, the milliseconds until all warps had left, and
+ * how many ran out by themselves.  Not counted by pamk_test_expired_waits.  No counterpart in the reference. */
+int pamk_test_run_out(unsigned ms, unsigned* out, void* stream);
 
 #ifdef __cplusplus
 }

@@ -48,6 +48,7 @@ _SIGNATURES = {
     "pamk_test_split_rows": (_i, [_i64] * 3 + [_i]),
     "pamk_test_set_packing_policy": (_i, [_i]),
     "pamk_test_expired_waits": (_i, [ctypes.POINTER(ctypes.c_uint)]),
+    "pamk_test_run_out": (_i, [ctypes.c_uint, _p, _p]),
     "pamk_matmul_scratch_bytes": (_sz, [_i64] * 4 + [_i]),
     "pamk_matmul_static_scratch_bytes": (_sz, []),
     "pamk_matmul_static_scratch": (_i, [_p, _p, _p] + [_i64] * 10 + [_f, _i, _p]),

@@ -1638,6 +1638,12 @@ int pamk_test_expired_waits(unsigned* count) {
     return e == cudaSuccess ? PAMK_OK : record_cuda_error(e);
 }
 
+int pamk_test_run_out(unsigned ms, unsigned* out, void* stream) {
+    if (ms > 1000 || out == nullptr) return PAMK_ERR_ARG;
+    run_out_kernel<<<1, 256, 0, static_cast<cudaStream_t>(stream)>>>(ms, out);
+    return check_launch();
+}
+
 int pamk_test_set_tile_policy(int policy) {
     if (policy < 0 || policy > 5) return PAMK_ERR_ARG;
     g_tile_policy = policy;

@@ -200,18 +200,37 @@ __device__ __forceinline__ void barrier_arrive(uint64_t* b) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(shared_address(b)) : "memory");
 }
 
-// Waits that ran out.  A wait gives up after two million tries (seconds; a slab takes microseconds), counts itself here, and its warp
-// writes NaN for its outputs.
+// Waits that ran out: how many CTAs met one on this device.  The outputs of such a CTA's warps are NaN.
 __device__ unsigned g_expired_waits;
 
-__device__ __forceinline__ bool barrier_wait(uint64_t* b, unsigned parity) {
-    for (int i = 0; i < (1 << 21); ++i) {
-        unsigned done;
-        asm volatile("{ .reg .pred q;\n mbarrier.try_wait.parity.shared::cta.b64 q, [%1], %2;\n selp.u32 %0, 1, 0, q; }"
-                     : "=r"(done) : "r"(shared_address(b)), "r"(parity) : "memory");
-        if (done) return true;
+constexpr unsigned kWaitMs = 2000;          // (a slab takes microseconds; less than the clock's word below holds)
+
+// (the clock's low word goes round every four seconds)
+__device__ __forceinline__ unsigned clock_ns() {
+    unsigned t;
+    asm volatile("mov.u32 %0, %globaltimer_lo;" : "=r"(t));
+    return t;
+}
+__device__ __forceinline__ bool barrier_done(uint64_t* b, unsigned parity) {
+    unsigned done;
+    asm volatile("{ .reg .pred q;\n mbarrier.try_wait.parity.shared::cta.b64 q, [%1], %2;\n selp.u32 %0, 1, 0, q; }"
+                 : "=r"(done) : "r"(shared_address(b)), "r"(parity) : "memory");
+    return done != 0;
+}
+
+// A wait ends when `ms` have passed since its first tries failed, or when another wait of the CTA has ended so (`gave_up`, in shared
+// memory; null: regardless of others), and then returns false.  A try sleeps for a time that the hardware chooses, so tries alone
+// are no bound.  The first wait of a CTA to run out adds one to `expired`.
+__device__ __forceinline__ bool barrier_wait(uint64_t* b, unsigned parity, unsigned* gave_up, unsigned* expired, unsigned ms = kWaitMs) {
+    unsigned start = 0;
+    for (int i = 0; i < (1 << 30); ++i) {
+        if (barrier_done(b, parity)) return true;
+        if (i < 64) continue;
+        if (i == 64) start = clock_ns();
+        if (gave_up != nullptr && *(volatile unsigned*)gave_up != 0) return false;
+        if (clock_ns() - start > ms * 1000000u) break;
     }
-    atomicAdd(&g_expired_waits, 1u);
+    if (gave_up != nullptr && atomicExch(gave_up, 1u) == 0) atomicAdd(expired, 1u);
     return false;
 }
 
@@ -227,7 +246,29 @@ __device__ __forceinline__ void request_slab(PackBlock* stage, const PackBlock* 
 struct Ring {
     PackBlock stages[kStages][2];
     uint64_t full[kStages], empty[kStages];
+    unsigned gave_up;
 };
+
+// Test: eight warps at barriers that nothing arrives at, the first with a limit of `ms`, the others with the usual one.  out: what each
+// warp's wait returned, the milliseconds until all had, and how many were counted.
+__global__ void __launch_bounds__(256) run_out_kernel(unsigned ms, unsigned* out) {
+    __shared__ uint64_t never[8];
+    __shared__ unsigned gave_up, expired;
+    const int warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) {
+        gave_up = expired = 0;
+        for (int i = 0; i < 8; ++i) barrier_init(never + i, 1);
+    }
+    const unsigned start = clock_ns();
+    __syncthreads();
+    const bool arrived = __any_sync(0xffffffffu, barrier_wait(never + warp, 0, &gave_up, &expired, warp == 0 ? ms : kWaitMs));
+    if ((threadIdx.x & 31) == 0) out[warp] = arrived;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        out[8] = (clock_ns() - start) / 1000000u;
+        out[9] = expired;
+    }
+}
 
 // MR rows per thread: 8, or 7 for tiles of 112 rows.  A warp is 4 x 8 threads, as in gemm.cu.
 template <int MR>
@@ -247,6 +288,7 @@ __global__ void __launch_bounds__(256, 2) packed_kernel(const PackedParams p) {
             barrier_init(ring.full + i, 1);
             barrier_init(ring.empty + i, 8);
         }
+        ring.gave_up = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         for (int s = 0; s < kAhead && s < count; ++s) request_slab(ring.stages[s], a_src + s, b_src + s, ring.full + s);
@@ -273,7 +315,7 @@ __global__ void __launch_bounds__(256, 2) packed_kernel(const PackedParams p) {
     bool ok = true;
     for (int s = 0; s < count; ++s) {
         if (tid == 0 && s + kAhead < count) {
-            if (s + kAhead >= kStages) ok = barrier_wait(ring.empty + ahead, ahead_parity ^ 1);
+            if (s + kAhead >= kStages) ok = barrier_wait(ring.empty + ahead, ahead_parity ^ 1, &ring.gave_up, &g_expired_waits);
             if (ok) {
                 request_slab(ring.stages[ahead], a_src + s + kAhead, b_src + s + kAhead, ring.full + ahead);
                 ++requested;
@@ -281,7 +323,7 @@ __global__ void __launch_bounds__(256, 2) packed_kernel(const PackedParams p) {
         }
         if (++ahead == kStages) { ahead = 0; ahead_parity ^= 1; }
         __syncwarp();
-        ok = __all_sync(0xffffffffu, ok && barrier_wait(ring.full + stage, parity));
+        ok = __all_sync(0xffffffffu, ok && barrier_wait(ring.full + stage, parity, &ring.gave_up, &g_expired_waits));
         if (!ok) break;
         ++landed;
         const PackBlock &block_a = ring.stages[stage][0], &block_b = ring.stages[stage][1];
@@ -395,8 +437,9 @@ __global__ void __launch_bounds__(256, 2) packed_kernel(const PackedParams p) {
     }
 #undef PAMK_FRAGMENTS
     if (!ok) {
-        // no copy may be in flight when the CTA leaves
-        for (int s = landed; tid == 0 && s < requested; ++s) barrier_wait(ring.full + s % kStages, (unsigned)(s / kStages) & 1u);
+        // no copy may be in flight when the CTA leaves (at most kAhead are; one that does not land in time is the last waited for)
+        for (int s = landed; tid == 0 && s < requested; ++s)
+            if (!barrier_wait(ring.full + s % kStages, (unsigned)(s / kStages) & 1u, nullptr, nullptr)) break;
 #pragma unroll
         for (int i = 0; i < MR; ++i)
 #pragma unroll

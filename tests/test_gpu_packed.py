@@ -131,3 +131,16 @@ def test_a_large_product_through_the_operators():
         out = pam.matmul(A, B)
     graph.replay()
     assert_bits_equal(out, want)
+
+
+@pytest.mark.parametrize("ms", [0, 40, 300])
+def test_a_wait_ends_by_the_clock(ms):
+    """Barriers that nothing arrives at: the first warp leaves after its limit, the others, whose own is two seconds, with it, and
+    one of them is counted."""
+    from pam_b200 import _lib
+    out = torch.full((10,), 7, dtype=torch.int32, device="cuda")
+    _lib.check(_lib.lib().pamk_test_run_out(ms, out.data_ptr(), torch.cuda.current_stream().cuda_stream), "run out")
+    have = out.tolist()
+    assert have[:8] == [0] * 8 and have[9] == 1
+    assert ms <= have[8] < ms + 200                         # (a try sleeps for some microseconds)
+    assert _lib.lib().pamk_test_run_out(1001, out.data_ptr(), None) == -1
