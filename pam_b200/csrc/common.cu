@@ -11,6 +11,7 @@ void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 
 int record_cuda_error(cudaError_t err) {
     g_last_cuda_error = (int)err;
+    cudaGetLastError();                  // (the runtime keeps a failed call's status until it is asked for: the next launch's check would find it)
     return PAMK_ERR_CUDA;
 }
 
