@@ -138,6 +138,23 @@ bool usable(const Tensor& t) {
 
 bool wants_grad(const Tensor& t) { return t.defined() && t.requires_grad(); }
 
+// Whether scratch that a call can do without is there to be had, in a cached block or from the device: asked for in vain, it would make torch's
+// allocator give its whole cache back first, on every call.  (A cached block may turn out to be another stream's.)  A capture does
+// not touch the cache and may not ask.
+bool room_for(size_t bytes, c10::DeviceIndex device) {
+    c10::cuda::CUDAGuard guard(device);
+    if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return true;
+    auto* allocator = c10::cuda::CUDACachingAllocator::get();
+    size_t largest = 1;                   // (zero would stand for the device's free memory)
+    allocator->cacheInfo(device, &largest);
+    if (largest >= bytes) return true;
+    constexpr size_t kUnit = size_t(2) << 20;                 // of the allocator's requests
+    const size_t request = (bytes + kUnit - 1) / kUnit * kUnit;
+    const auto [free, total] = allocator->getMemoryInfo(device);
+    const auto reserved = allocator->getDeviceStats(device).reserved_bytes[0].current;
+    return free >= request && (double)reserved + (double)request <= allocator->getMemoryFraction(device) * (double)total;
+}
+
 // ---- matrix products ----------------------------------------------------------------------------------
 
 struct Mat {                              // element strides of one operand: batch, row, column
@@ -163,7 +180,7 @@ Tensor product(const Mat& a, const Mat& b, const Tensor& bias, int64_t batch, in
     if ((double)batch * (double)M * (double)N * (double)K > PAMK_PACKED_PRODUCTS) {
         // scratch for packed operands too; a product that cannot have it runs without
         const size_t packed = lib.pamk_matmul_scratch_bytes(batch, M, N, K, split);
-        if (packed > bytes) {
+        if (packed > bytes && room_for(packed, like.device().index())) {
             try {
                 ws = scratch_bytes(packed, like);
                 bytes = packed;
@@ -1161,6 +1178,18 @@ PyObject* py_set_nvtx(PyObject*, PyObject* flag) {
     return none();
 }
 
+// room_for(bytes, device index)
+PyObject* py_room_for(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+    PAMK_ARGS(2)
+    return guarded([&]() -> PyObject* {
+        const size_t bytes = PyLong_AsSize_t(a[0]);
+        if (bytes == (size_t)-1 && PyErr_Occurred()) return nullptr;
+        const long device = PyLong_AsLong(a[1]);
+        if (device == -1 && PyErr_Occurred()) return nullptr;
+        return PyBool_FromLong(room_for(bytes, (c10::DeviceIndex)device));
+    });
+}
+
 // setup(library path, error class)
 PyObject* py_setup(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     PAMK_ARGS(2)
@@ -1195,6 +1224,7 @@ PyMethodDef methods[] = {
     PAMK_FAST("setup", py_setup),
     {"set_strict", py_set_strict, METH_O, nullptr},
     {"set_nvtx", py_set_nvtx, METH_O, nullptr},
+    PAMK_FAST("room_for", py_room_for),
     PAMK_FAST("linear", py_linear),
     PAMK_FAST("matmul", py_matmul),
     PAMK_FAST("mul", py_elementwise<Ew::kMul>),

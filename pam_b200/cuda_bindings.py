@@ -163,7 +163,7 @@ _PACKED_PRODUCTS = 3e9                                       # PAMK_PACKED_PRODU
 def _packed_scratch(device, nbytes, partials):
     """Scratch for a product on packed operands, given back after the call; None where the product takes no more than its
     partial sums, or where there is no room (it then runs on the operands as they are)."""
-    if nbytes <= (partials + 255) // 256 * 256:
+    if nbytes <= (partials + 255) // 256 * 256 or not _lib.host().room_for(nbytes, device.index):
         return None
     try:
         return torch.empty(nbytes, dtype=torch.uint8, device=device)
