@@ -20,8 +20,7 @@ namespace {
 
 constexpr int kTensorsPerLaunch = 256;     // (an 11 KB kernel argument: within the 32 KB that sm_70 and later take)
 constexpr int kThreads = 256;
-constexpr int kVectors = 2;                 // vectors of four elements per operand and thread
-constexpr int kPerBlock = kThreads * 4 * kVectors;
+constexpr int kPerBlock = kThreads * 4;
 
 struct AdamTable {
     float* p[kTensorsPerLaunch];
@@ -112,13 +111,29 @@ __device__ __forceinline__ void adam_any(float& p, float g, float& m, float& v, 
     if (!done) adam_one(p, g, m, v, s, lb2);
 }
 
-// Eight elements per thread, all of their loads on the way at once, which also halves the blocks that look for their tensor: the 254 tensors of
-// a 6+6 transformer (42 million parameters) 211 -> 193 us, one tensor of 2^25 154 -> 146.  With the full rule the kernel is bound by its instructions, five or six per primitive and more
-// for the division and log2f that only classify (2^25 elements 192 us); without the range rules by DRAM (150 us).
+__device__ __forceinline__ void four_elements(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
+                                              const AdamScalars& s, float lb2, unsigned mask) {
+    float4 p4 = *reinterpret_cast<const float4*>(p);
+    const float4 g4 = __ldg(reinterpret_cast<const float4*>(g));
+    float4 m4 = *reinterpret_cast<const float4*>(m);
+    float4 v4 = *reinterpret_cast<const float4*>(v);
+    adam_any(p4.x, g4.x, m4.x, v4.x, s, lb2, mask);
+    adam_any(p4.y, g4.y, m4.y, v4.y, s, lb2, mask);
+    adam_any(p4.z, g4.z, m4.z, v4.z, s, lb2, mask);
+    adam_any(p4.w, g4.w, m4.w, v4.w, s, lb2, mask);
+    *reinterpret_cast<float4*>(p) = p4;
+    *reinterpret_cast<float4*>(m) = m4;
+    *reinterpret_cast<float4*>(v) = v4;
+}
+
+// Four elements per thread, in at most 48 registers for five CTAs per SM: bound by DRAM with the short rule (the 254 tensors of a 6+6 transformer,
+// 42 million parameters, 189 us; one tensor of 2^25 143), by its instructions with the full one, five or six per primitive and more
+// for the division and log2f that only classify (2^25 elements with 30 % zeros among the gradients 233 us).  Eight elements per
+// thread took 198, 155 and 300 us, and 6.8 us instead of 4.1 for 30000 elements with zeros: twice the code, fewer warps.
 // The 32 elements that a warp works on at a time take one of the two together, by a vote on the inputs: where each
 // thread chose for itself, zeros among the gradients (rows of an embedding that no token met, units behind
-// a ReLU) made the warp run both (one zero in ten: 365 us, now 198).
-__global__ void __launch_bounds__(kThreads) adam_kernel(const AdamTable t, const AdamScalars s) {
+// a ReLU) made the warp run both (2^25 elements, one zero in ten: 365 us, with the vote 198).
+__global__ void __launch_bounds__(kThreads, 5) adam_kernel(const AdamTable t, const AdamScalars s) {
     int which = 0, hi = t.used;                    // largest k with first[k] <= blockIdx.x (the same for the whole CTA)
     while (hi - which > 1) {
         const int mid = (which + hi) >> 1;
@@ -134,61 +149,28 @@ __global__ void __launch_bounds__(kThreads) adam_kernel(const AdamTable t, const
     const float lb2 = log2f(2.0f);
     const bool vec = ((reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(g) |
                        reinterpret_cast<uintptr_t>(m) | reinterpret_cast<uintptr_t>(v)) & 15u) == 0;
-    // whole blocks of aligned tensors: two vectors per operand and thread, all on their way before the first is worked on
+    const int64_t i = base + threadIdx.x * 4;
+    // (whole blocks of aligned tensors: no look at the tensor's end)
     if (vec && base + kPerBlock <= n) {
-        const int64_t i = base + threadIdx.x * 4;
-        float4 p4[kVectors], g4[kVectors], m4[kVectors], v4[kVectors];
-#pragma unroll
-        for (int q = 0; q < kVectors; ++q) {
-            const int64_t at = i + q * kThreads * 4;
-            p4[q] = *reinterpret_cast<const float4*>(p + at);
-            g4[q] = __ldg(reinterpret_cast<const float4*>(g + at));
-            m4[q] = *reinterpret_cast<const float4*>(m + at);
-            v4[q] = *reinterpret_cast<const float4*>(v + at);
-        }
-#pragma unroll
-        for (int q = 0; q < kVectors; ++q) {
-            const int64_t at = i + q * kThreads * 4;
-            adam_any(p4[q].x, g4[q].x, m4[q].x, v4[q].x, s, lb2, 0xffffffffu);
-            adam_any(p4[q].y, g4[q].y, m4[q].y, v4[q].y, s, lb2, 0xffffffffu);
-            adam_any(p4[q].z, g4[q].z, m4[q].z, v4[q].z, s, lb2, 0xffffffffu);
-            adam_any(p4[q].w, g4[q].w, m4[q].w, v4[q].w, s, lb2, 0xffffffffu);
-            *reinterpret_cast<float4*>(p + at) = p4[q];
-            *reinterpret_cast<float4*>(m + at) = m4[q];
-            *reinterpret_cast<float4*>(v + at) = v4[q];
-        }
+        four_elements(p + i, g + i, m + i, v + i, s, lb2, 0xffffffffu);
         return;
     }
+    const bool four = vec && i + 3 < n;
+    const unsigned fours = __ballot_sync(0xffffffffu, four);          // (every thread of the CTA is here)
+    if (four) {
+        four_elements(p + i, g + i, m + i, v + i, s, lb2, fours);
+    } else {
 #pragma unroll 1
-    for (int q = 0; q < kVectors; ++q) {
-        const int64_t i = base + q * kThreads * 4 + threadIdx.x * 4;
-        const bool four = vec && i + 3 < n;
-        const unsigned fours = __ballot_sync(0xffffffffu, four);          // (every thread of the CTA is here)
-        if (four) {
-            float4 p4 = *reinterpret_cast<const float4*>(p + i);
-            const float4 g4 = __ldg(reinterpret_cast<const float4*>(g + i));
-            float4 m4 = *reinterpret_cast<const float4*>(m + i);
-            float4 v4 = *reinterpret_cast<const float4*>(v + i);
-            adam_any(p4.x, g4.x, m4.x, v4.x, s, lb2, fours);
-            adam_any(p4.y, g4.y, m4.y, v4.y, s, lb2, fours);
-            adam_any(p4.z, g4.z, m4.z, v4.z, s, lb2, fours);
-            adam_any(p4.w, g4.w, m4.w, v4.w, s, lb2, fours);
-            *reinterpret_cast<float4*>(p + i) = p4;
-            *reinterpret_cast<float4*>(m + i) = m4;
-            *reinterpret_cast<float4*>(v + i) = v4;
-        } else {
-#pragma unroll 1
-            for (int c = 0; c < 4; ++c) {
-                const bool on = i + c < n;
-                const unsigned ons = __ballot_sync(~fours, on);
-                if (on) {
-                    float pp = p[i + c], mm = m[i + c], vv = v[i + c];
-                    const float gg = g[i + c];
-                    adam_any(pp, gg, mm, vv, s, lb2, ons);
-                    p[i + c] = pp;
-                    m[i + c] = mm;
-                    v[i + c] = vv;
-                }
+        for (int c = 0; c < 4; ++c) {
+            const bool on = i + c < n;
+            const unsigned ons = __ballot_sync(~fours, on);
+            if (on) {
+                float pp = p[i + c], mm = m[i + c], vv = v[i + c];
+                const float gg = g[i + c];
+                adam_any(pp, gg, mm, vv, s, lb2, ons);
+                p[i + c] = pp;
+                m[i + c] = mm;
+                v[i + c] = vv;
             }
         }
     }

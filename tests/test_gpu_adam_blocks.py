@@ -1,4 +1,4 @@
-"""The fused Adam kernel's whole blocks (2048 elements, two vectors per thread) and their ends: tensors around multiples of a block and of the
+"""The fused Adam kernel's whole blocks (1024 elements) and their ends: tensors around multiples of a block and of the
 parts that a thread takes, aligned and one float off, ordinary values beside zeros, bit for bit against the oracle's step."""
 import pytest
 import torch
