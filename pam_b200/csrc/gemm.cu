@@ -30,6 +30,7 @@
 // in one launch (ranges_kernel).
 // The same skeleton serves true-multiply products (standard_matmul) and the exact-gradient
 // product (pam_matmul_bwd_kernel, cuda_kernels.cu:729-832).
+#include <algorithm>
 #include <array>
 #include <type_traits>
 
@@ -1112,10 +1113,14 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* part, c
 // ---- small products in ranges of K, in one launch ---------------------------------------------------------------------------
 // The 32x32 tile's products in ranges are latencies: a launch that forms the partials, one that adds them, and the host's
 // work for both.  Here one CTA forms all partials of a 16x16 tile, half a warp per range, and adds them from shared
-// memory: same ranges, same order, same bits.  Kernel times, two launches and one: 32x512x512 in 16 ranges 6.6 + a gap and 5.9 us, 8x1024x512 7.2
-// and 6.0, 100x300x700 9.2 and 8.2; a call of 32x512x512 through the operators 11.6 and 8.8, most of it the host.
+// memory: same ranges, same order, same bits.  A call of 32x512x512 through the operators 11.6 and 8.8 us, most of it the host; kernel
+// times, two launches and one:
+//                               clean          half zeros in A   0.1 / 1 % specials
+//   32x512x512 in 16 ranges     6.8 and 5.4    7.3 and 6.8        8.1 / 9.5 and 6.7 / 8.9
+//   8x1024x512                  6.8 and 5.3    8.3 and 6.7        7.4 / 8.8 and 5.9 / 7.5
+//   100x300x700 in 15           9.3 and 7.4   11.5 and 9.3       10.7 / 14.0 and 9.5 / 12.1
 // Bound by latencies: the launch, two loads from the L2, the sum of the partials.  (A cluster of eight CTAs per tile with the partials in
-// distributed shared memory: 6.9 us.)
+// distributed shared memory: 6.9 us for the first.)
 struct TileRange : Tile<16, 16, 16, 1, 4> {};
 struct RangeShared {                                          // of one range
     union {
@@ -1125,6 +1130,8 @@ struct RangeShared {                                          // of one range
 };
 constexpr int kMaxRanges = 16;                                // 256 threads: two CTAs per SM, 40 KB of shared memory each
 
+constexpr int kWarpsOfAny = 12;                               // what the registers of every layout's kernel allow (see its launch bounds)
+
 // Whether a product planned as ranges on the 32x32 tile takes this form: all of its CTAs resident at once, and no more ranges than
 // above (197x192x768 in 24 ranges 9.3 us in two launches, 13.3 in one; 32x512x1024 in 32 7.8 and 9.2).
 bool ranges_in_one_launch(int64_t batch, int64_t M, int64_t N, int splits) {
@@ -1132,8 +1139,8 @@ bool ranges_in_one_launch(int64_t batch, int64_t M, int64_t N, int splits) {
            batch * ((M + 15) / 16) * ((N + 15) / 16) * splits * 16 <= (int64_t)sm_count() * 512;
 }
 
-template <bool A_KC, bool B_KC, bool VEC>
-__global__ void __launch_bounds__(16 * kMaxRanges) ranges_kernel(const GemmParams p) {
+template <bool A_KC, bool B_KC, bool VEC, int PER_SM = 1>
+__global__ void __launch_bounds__(PER_SM > 1 ? 16 * kMaxRanges : 32 * kWarpsOfAny, PER_SM) ranges_kernel(const GemmParams p) {
     using T = TileRange;
     constexpr int BK = T::BK;
     static_assert(T::kThreads == 16 && T::kTasksA == 4, "half a warp per range");
@@ -1166,10 +1173,26 @@ __global__ void __launch_bounds__(16 * kMaxRanges) ranges_kernel(const GemmParam
             load_slab<T, 16, T::kTasksB, B_KC>(b, p.B, Bb, n0, p.N, k0, k_end, tid);
         }
     };
+    // (the two ranges of a warp take the same loops, where both have a slab left: apart they would run one after the other)
+    const int other_begin = (range ^ 1) * p.k_chunk, other_end = (range ^ 1) < p.splits ? min(p.K, other_begin + p.k_chunk) : other_begin;
     auto slab = [&](float (&a_in)[T::kTasksA * 4], float (&b_in)[T::kTasksB * 4], int k0) {
         if (k0 >= k_end) return;
+        const unsigned both = k0 - k_begin + other_begin < other_end ? 0xffffffffu : half;
         const bool out = band_excess(b_in, band_excess(a_in, 0u)) >= kBandSpan2;
-        const bool dirty = __any_sync(half, out);
+        // The lines with out-of-band elements and of what sort these are, as the slab's word of gemm_kernel: by the threads that hold
+        // them, or, where registers are short, by a thread per line after the slab is stored.
+        const bool dirty = __any_sync(both, out);
+        unsigned f = 0;
+        if (dirty) {
+            if constexpr (PER_SM == 1) {
+                uint32_t bits = 0, top = 0;
+                f = dirty_lines<T, 16, T::kTasksA, A_KC>(a_in, tid, bits, top) | dirty_lines<T, 16, T::kTasksB, B_KC>(b_in, tid, bits, top);
+                f |= (bits ? (unsigned)kNonZero : 0u) | (top >= kBandHi2 ? (unsigned)kAbove : 0u);
+                f = __reduce_or_sync(both, f);
+            }
+#pragma unroll
+            for (int c = 0; c < T::kTasksA * 4; ++c) a_in[c] = fadd(a_in[c], 0.0f);          // (one pattern for A's zeros)
+        }
 #pragma unroll
         for (int c = 0; c < T::kTasksA * 4; ++c) a_in[c] = i2f(isub(f2i(a_in[c]), p.bias_sub));
         __syncwarp(half);                                     // the last slab has been read
@@ -1177,26 +1200,103 @@ __global__ void __launch_bounds__(16 * kMaxRanges) ranges_kernel(const GemmParam
         store_slab<T, 16, T::kTasksB, B_KC>(sh.b, b_in, tid);
         load(a_in, b_in, k0 + 2 * BK);
         __syncwarp(half);
-        auto line = [&](int kk, auto checked) {
-            const int4 a4 = *reinterpret_cast<const int4*>(sh.a + kk * row_stride(16) + ty * 4);
-            const int4 b4 = *reinterpret_cast<const int4*>(sh.b + kk * row_stride(16) + tx * 4);
-            const int a[4] = {a4.x, a4.y, a4.z, a4.w}, b[4] = {b4.x, b4.y, b4.z, b4.w};
+        if (PER_SM > 1 && dirty) {
+            uint32_t bits = 0, top = 0;
+            bool off = false;
+            auto see = [&](int x) {
+                const uint32_t m2 = 2u * (uint32_t)x;
+                if (m2 - kBandLo2 >= kBandSpan2) { off = true; bits |= m2; }
+                top = max(top, m2);
+            };
+#pragma unroll 1
+            for (int q = 0; q < 4; ++q) {
+                const int4 va = *reinterpret_cast<const int4*>(sh.a + tid * row_stride(16) + q * 4);
+                const int4 vb = *reinterpret_cast<const int4*>(sh.b + tid * row_stride(16) + q * 4);
+                see(iadd(va.x, p.bias_sub)); see(iadd(va.y, p.bias_sub)); see(iadd(va.z, p.bias_sub)); see(iadd(va.w, p.bias_sub));
+                see(vb.x); see(vb.y); see(vb.z); see(vb.w);
+            }
+            f = __ballot_sync(both, off);
+            f = (f | f >> 16) & 0xffffu;                      // (bits of absent threads are zero)
+            if (__any_sync(both, bits != 0)) f |= kNonZero;
+            if (__any_sync(both, top >= kBandHi2)) f |= kAbove;
+        }
+#define PAMK_RANGE_FRAGMENTS(kk)                                                                     \
+        const int4 a4 = *reinterpret_cast<const int4*>(sh.a + (kk) * row_stride(16) + ty * 4);       \
+        const int4 b4 = *reinterpret_cast<const int4*>(sh.b + (kk) * row_stride(16) + tx * 4);       \
+        const int a[4] = {a4.x, a4.y, a4.z, a4.w}, b[4] = {b4.x, b4.y, b4.z, b4.w};
+        auto plain_line = [&](int kk) {
+            PAMK_RANGE_FRAGMENTS(kk)
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = fadd(acc[i][j], i2f(iadd(a[i], b[j])));
+        };
+        auto checked_line = [&](int kk, auto full_rule) {
+            PAMK_RANGE_FRAGMENTS(kk)
+            float araw[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) araw[i] = i2f(iadd(a[i], p.bias_sub));
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    const int sum = iadd(a[i], b[j]);
-                    if constexpr (decltype(checked)::value) acc[i][j] = fadd(acc[i][j], range_rule(fmul(i2f(iadd(a[i], p.bias_sub)), i2f(b[j])), sum));
-                    else acc[i][j] = fadd(acc[i][j], i2f(sum));
+                    const float mag = fabsf(fmul(araw[i], i2f(b[j])));
+                    if constexpr (decltype(full_rule)::value) {
+                        const float prod = mag <= i2f(kPassBits) ? i2f(iadd(a[i], b[j])) : quiet_nan();
+                        if (!(mag <= i2f(kFlushBits))) acc[i][j] = fadd(acc[i][j], prod);
+                    } else {
+                        if (mag > i2f(kFlushBits)) acc[i][j] = fadd(acc[i][j], i2f(iadd(a[i], b[j])));
+                    }
                 }
         };
-        if (!dirty) {
+        auto zeros_line = [&](int kk) {                       // rows by weights, columns by predicates, as in gemm_kernel
+            PAMK_RANGE_FRAGMENTS(kk)
+            float w[4];
+            int ai[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const bool zero = a[i] == -p.bias_sub;
+                w[i] = zero ? 0.0f : 1.0f;
+                ai[i] = zero ? 0 : a[i];
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const bool on = 2u * (uint32_t)b[j] != 0;
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (on) acc[i][j] = __fmaf_rn(i2f(iadd(ai[i], b[j])), w[i], acc[i][j]);
+            }
+        };
+        // Zeros alone: all lines by weights.  Anything else: a few dirty lines one by one, many with the whole slab.  (The full rule for
+        // every line of a dirty slab: 32x512x512 with half zeros 9.4 us, 0.1 % specials 10.9.)
+        if (f == 0) {
 #pragma unroll 4
-            for (int kk = 0; kk < BK; ++kk) line(kk, std::false_type{});
-        } else {                                              // the full rule for every product: a flushed one is +0, and a sum is never -0
+            for (int kk = 0; kk < BK; ++kk) plain_line(kk);
+        } else if (!(f & kNonZero)) {
+#pragma unroll 4
+            for (int kk = 0; kk < BK; ++kk) zeros_line(kk);
+        } else if (__popc(f & 0xffffu) > 5) {
+            if (f & kAbove) {
+#pragma unroll 2
+                for (int kk = 0; kk < BK; ++kk) checked_line(kk, std::true_type{});
+            } else {                                          // "flush or add", exact for clean lines too
+#pragma unroll 2
+                for (int kk = 0; kk < BK; ++kk) checked_line(kk, std::false_type{});
+            }
+        } else {
+            int kk = 0;
+            while (kk < BK) {
+                const unsigned left = (f & 0xffffu) >> kk;
+                const int end = left ? kk + __ffs((int)left) - 1 : BK;
 #pragma unroll 1
-            for (int kk = 0; kk < BK; ++kk) line(kk, std::true_type{});
+                for (; kk < end; ++kk) plain_line(kk);
+                if (kk == BK) break;
+                if (f & kAbove) checked_line(kk, std::true_type{});
+                else checked_line(kk, std::false_type{});
+                ++kk;
+            }
         }
+#undef PAMK_RANGE_FRAGMENTS
     };
     load(ra[0], rb[0], k_begin);
     load(ra[1], rb[1], k_begin + BK);
@@ -1226,7 +1326,7 @@ template <bool VEC>
 int dispatch_ranges(const GemmParams& p, bool a_kc, bool b_kc, cudaStream_t st) {
     const dim3 grid((unsigned)((p.N + 15) / 16), (unsigned)((p.M + 15) / 16), (unsigned)p.batch);
     const auto kernel = a_kc ? (b_kc ? ranges_kernel<true, true, VEC> : ranges_kernel<true, false, VEC>)
-                             : (b_kc ? ranges_kernel<false, true, VEC> : ranges_kernel<false, false, VEC>);
+                       : (b_kc ? ranges_kernel<false, true, VEC> : ranges_kernel<false, false, VEC>);
     const size_t shared = p.splits * sizeof(RangeShared);
     static_assert(kMaxRanges * sizeof(RangeShared) <= 48 * 1024, "what a launch may use unasked");
     kernel<<<grid, (unsigned)(16 * p.splits), shared, st>>>(p);

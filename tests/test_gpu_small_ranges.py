@@ -1,14 +1,26 @@
 """Small products in ranges of K that run in one launch: each range summed in k order and the ranges added in theirs, which the oracle
 does range by range; rows, columns and K around the edges of tiles and slabs, every layout and alignment, a batch, a bias, a
 strided output with a PAM multiplication, special values."""
+import contextlib
+
 import pytest
 import torch
 
 from conftest import assert_bits_equal
 from test_gpu_packed import _layout, _product
-from test_gpu_special_lines import _values
+from test_gpu_special_lines import GREAT, MASKED, ODD, SMALL, STRADDLE, _values
 
 pytestmark = pytest.mark.gpu
+
+ZEROS = (0.0, -0.0)
+
+
+@contextlib.contextmanager
+def _launches(lib, count):
+    """The kernels launched inside are this many: which form a product took, as all forms give the same bits."""
+    before = lib.pamk_launch_count()
+    yield
+    assert lib.pamk_launch_count() - before == count
 
 
 @pytest.fixture
@@ -39,7 +51,35 @@ def test_ranges_in_one_launch(lib, M, N, K, split, pool, share, oracle):
     A, B, bias = _values(pool, share, g, 1, M, K), _values(pool, share, g, 1, K, N), torch.randn(N, generator=g)
     want = _in_ranges(oracle, A, B, split, 1.0552) + bias
     for lay in ("nn", "nt", "tn", "Tt"):
-        assert_bits_equal(_product(lib, _layout(A.cuda(), lay[0]), _layout(B.cuda(), lay[1]), split, bias.cuda()), want, lay)
+        x, y, b = _layout(A.cuda(), lay[0]), _layout(B.cuda(), lay[1]), bias.cuda()
+        with _launches(lib, 1):
+            have = _product(lib, x, y, split, b)
+        assert_bits_equal(have, want, lay)
+
+
+@pytest.mark.parametrize("M,N,K,split", [(33, 47, 100, 4), (20, 300, 50, 3), (208, 192, 512, 16)])
+@pytest.mark.parametrize("a_pool,b_pool,share", [(ZEROS, (), 0.5), ((), ZEROS, 0.5), (ZEROS, ZEROS, 0.3), (ZEROS, ZEROS, 0.01), (STRADDLE, (), 0.01),
+                                                 (SMALL, STRADDLE, 0.3), (GREAT, MASKED, 0.01), (ODD, GREAT, 0.01), (GREAT, ODD, 0.3)])
+def test_slabs_of_every_kind(lib, M, N, K, split, a_pool, b_pool, share, oracle):
+    """Each loop for dirty slabs, in all slabs and in some of them: a warp's two ranges see different kinds, and the last may be alone."""
+    g = torch.Generator().manual_seed(M + len(a_pool) * 10 + int(share * 1000))
+    def values(pool, *shape):
+        t = torch.randn(*shape, generator=g)
+        if pool:
+            pick = torch.tensor(pool)[torch.randint(0, len(pool), shape, generator=g)]
+            t = torch.where(torch.rand(*shape, generator=g) < share, pick, t)
+        return t
+    A, B = values(a_pool, 1, M, K), values(b_pool, 1, K, N)
+    for some in (False, True):
+        if some:                                             # every third slab as it is, the others clean
+            clean = (torch.arange(K) // 16 % 3 != 0)
+            A[..., clean], B[:, clean] = torch.randn(1, M, int(clean.sum()), generator=g), torch.randn(1, int(clean.sum()), N, generator=g)
+        want = _in_ranges(oracle, A, B, split, 1.0552)
+        for lay in ("nn", "nt", "tn", "Nt"):
+            x, y = _layout(A.cuda(), lay[0]), _layout(B.cuda(), lay[1])
+            with _launches(lib, 1):
+                have = _product(lib, x, y, split)
+            assert_bits_equal(have, want, lay)
 
 
 def test_a_batch_and_a_strided_output(lib, oracle):
@@ -48,8 +88,11 @@ def test_a_batch_and_a_strided_output(lib, oracle):
     g = torch.Generator().manual_seed(2)
     A, B = _values("all", 0.01, g, batch, M, K), _values("below", 0.01, g, batch, K, N)
     want = _in_ranges(oracle, A, B, split, 1.0)
-    assert_bits_equal(_product(lib, A.cuda(), B.cuda(), split, offset=1.0), want)
-    out, x, y = torch.full((batch, M, ld), -7.0, device="cuda"), A.cuda(), B.cuda()
+    x, y = A.cuda(), B.cuda()
+    with _launches(lib, 1):
+        have = _product(lib, x, y, split, offset=1.0)
+    assert_bits_equal(have, want)
+    out = torch.full((batch, M, ld), -7.0, device="cuda")
     ws = torch.empty(split * batch * M * N, device="cuda")
     _lib.check(lib.pamk_matmul_strided(x.data_ptr(), y.data_ptr(), out.data_ptr(), 1, batch, M, N, K, 0, M * K, K, 1, 0, K * N, N, 1, 0, M * ld, ld,
                                        1.0, 1, 0.125, split, ws.data_ptr(), 4 * ws.numel(), torch.cuda.current_stream().cuda_stream), "strided")
