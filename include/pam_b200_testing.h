@@ -33,6 +33,10 @@ int pamk_test_planned_rows(int64_t M, int64_t N, int64_t K, int split_k);
  * the same bounds.  No counterpart in the reference. */
 int pamk_test_split_rows(int64_t M, int64_t N, int64_t K, int split_k);
 
+/* Rows per tile (128, 64, 56 or 32) of an unsplit PAM product as planned, in place, whose A lies contiguous along K or not and whose operands allow
+ * 128-bit loads or not.  Negative (PAMK_ERR_ARG) for an empty problem.  No counterpart in the reference. */
+int pamk_test_small_rows(int64_t batch, int64_t M, int64_t N, int64_t K, int a_along_k, int wide_loads);
+
 /* Whether PAM products of large tiles run on packed operands: 0 = where it pays (default), 1 = wherever the scratch suffices,
  * 2 = never.  Process-wide and not thread-safe.  No counterpart in the reference. */
 int pamk_test_set_packing_policy(int policy);

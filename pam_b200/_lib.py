@@ -46,6 +46,7 @@ _SIGNATURES = {
     "pamk_test_planned_tile": (_i, [_i64] * 4),
     "pamk_test_planned_rows": (_i, [_i64] * 3 + [_i]),
     "pamk_test_split_rows": (_i, [_i64] * 3 + [_i]),
+    "pamk_test_small_rows": (_i, [_i64] * 4 + [_i] * 2),
     "pamk_test_set_packing_policy": (_i, [_i]),
     "pamk_test_expired_waits": (_i, [ctypes.POINTER(ctypes.c_uint)]),
     "pamk_test_run_out": (_i, [ctypes.c_uint, _p, _p]),

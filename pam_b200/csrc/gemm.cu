@@ -1544,14 +1544,19 @@ bool seven_rows_better_in_ranges(const Plan& pl, int64_t M, int64_t N, int64_t K
 }
 
 // Whether an unsplit PAM product planned for the 64x64 or the 32x32 tile takes TileSmall7 (the sums of one range are the same on any tile).
-// By the model: 5 % cheaper; with scalar loads up to 15 % dearer than the 32x32 tile, whose cost with those it does not know (20 batched
-// products: modelled 0.88 x, measured 0.85 to 0.92; scalar 1.12 x, 0.79 and 0.82; 1.18 x, 0.98 and 1.05; 1.6 x, 1.04; aligned 0.99 x,
-// 1.02; 1.1 x, 0.88 to 1.09).
+// By the model: 5 % cheaper; with scalar loads up to 15 % dearer than the 32x32 tile, whose cost with those it does not know, as long as the
+// tiles cover at most a fifth more outputs.  Measured against the other tile, clean operands (1 % special values): 64x64, 26 products
+// modelled 0.88 x 0.83 to 0.98 (0.80 to 0.95), 0.97 x and more 1.02 and up; 32x32, scalar loads, up to 1.2 x the outputs 0.85 to 0.99 (0.91
+// to 1.11), 237 products 146x146x128, 1.26 x, 1.03 to 1.05 (1.09 to 1.11), 394 products 329x90x32, 1.27 x, 1.01 to 1.05 (1.15 to 1.18), modelled
+// 1.18 x and more 0.97 to 1.15.
 bool small7_better(const Plan& pl, int64_t batch, int64_t M, int64_t N, int64_t K, bool a_kc, bool vec) {
     if (pl.splits > 1 || (pl.tile != kTileSmall && pl.tile != kTileTiny) || (vec && !a_kc) || K == 0) return false;
     if (M > (int64_t)65535 * TileSmall7::kRows) return false;                          // (grid.y)
     if (g_tile_policy != 0) return g_tile_policy == 5;
-    return plan_for<TileSmall7>(kPam, batch, M, N, K, 1).cost < (vec || pl.tile == kTileSmall ? 0.95 : 1.15) * pl.cost;
+    const bool lenient = !vec && pl.tile == kTileTiny;
+    auto padded = [&](int64_t rows, int64_t cols) { return (M + rows - 1) / rows * rows * ((N + cols - 1) / cols * cols); };
+    if (lenient && 5 * padded(TileSmall7::kRows, TileSmall7::BN) > 6 * padded(TileTiny::BM, TileTiny::BN)) return false;
+    return plan_for<TileSmall7>(kPam, batch, M, N, K, 1).cost < (lenient ? 1.15 : 0.95) * pl.cost;
 }
 
 // Whether a PAM product planned as `pl` runs on packed operands, given the scratch, and its rows per tile then (whatever the operands'
@@ -1781,6 +1786,13 @@ int pamk_test_split_rows(int64_t M, int64_t N, int64_t K, int split_k) {
     if (M <= 0 || N <= 0 || K <= 0 || split_k < 0 || !dims_ok(1, M, N, K)) return PAMK_ERR_ARG;
     const Plan pl = make_plan(kPam, 1, M, N, K, split_k);
     return seven_rows_better_in_ranges(pl, M, N, K) ? TileLarge7::kRows : pamk_test_planned_rows(M, N, K, split_k);
+}
+
+int pamk_test_small_rows(int64_t batch, int64_t M, int64_t N, int64_t K, int a_along_k, int wide_loads) {
+    if (batch <= 0 || M <= 0 || N <= 0 || K <= 0 || !dims_ok(batch, M, N, K)) return PAMK_ERR_ARG;
+    const Plan pl = make_plan(kPam, batch, M, N, K, 1);
+    if (small7_better(pl, batch, M, N, K, a_along_k != 0, wide_loads != 0)) return TileSmall7::kRows;
+    return pl.tile == kTileLarge ? TileLarge::BM : (pl.tile == kTileSmall ? TileSmall::BM : TileTiny::BM);
 }
 
 int pamk_matmul_auto_split(int64_t batch, int64_t M, int64_t N, int64_t K) {
