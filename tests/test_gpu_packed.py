@@ -36,22 +36,25 @@ def _layout(t, kind):
     return view if kind in ("n", "N") else view.transpose(-1, -2)
 
 
-def _product(lib, x, y, split=1, bias=None, offset=1.0552, scratch=None):
+def _product(lib, x, y, split=1, bias=None, offset=1.0552, scratch=None, launches=None):
     from pam_b200 import _lib
     batch, (M, K), N = x.shape[0], x.shape[1:], y.shape[2]
     nbytes = lib.pamk_matmul_scratch_bytes(batch, M, N, K, split)
     ws = torch.full((max(nbytes if scratch is None else scratch, 1),), 0x5a, dtype=torch.uint8, device="cuda")
     out = torch.full((batch, M, N), -7.0, device="cuda")
+    before = lib.pamk_launch_count()
     _lib.check(lib.pamk_matmul_bias(0, x.data_ptr(), y.data_ptr(), None if bias is None else bias.data_ptr(), out.data_ptr(), batch, M, N, K,
                                     *x.stride(), *y.stride(), offset, split, ws.data_ptr(), ws.numel(),
                                     torch.cuda.current_stream().cuda_stream), "product")
+    # (which form it took, as all forms give the same bits: three launches on packed operands, one in place, and the sum of the ranges)
+    assert launches is None or lib.pamk_launch_count() - before == launches + (1 if split > 1 else 0)
     return out
 
 
 def _in_place(lib, *args, **kw):
     lib.pamk_test_set_packing_policy(2)
     try:
-        return _product(lib, *args, **kw)
+        return _product(lib, *args, launches=1, **kw)
     finally:
         lib.pamk_test_set_packing_policy(1)
 
@@ -66,7 +69,7 @@ def test_lines_of_every_kind(packed, a_pool, b_pool, share, M, K, N, oracle):
     if a_pool != "none": A[5] = 0.0
     want = oracle.kernels().pam_matmul_fwd(A, B, True, True, 1.0552)
     for lay in ("nn", "nt", "tn", "tt", "Nt", "tN"):
-        assert_bits_equal(_product(packed, _layout(A[None].cuda(), lay[0]), _layout(B[None].cuda(), lay[1]))[0], want, lay)
+        assert_bits_equal(_product(packed, _layout(A[None].cuda(), lay[0]), _layout(B[None].cuda(), lay[1]), launches=3)[0], want, lay)
 
 
 @pytest.mark.parametrize("M,N", [(1, 1), (1, 300), (64, 64), (67, 127), (112, 128), (113, 129), (225, 4), (260, 256)])
@@ -76,7 +79,7 @@ def test_edges(packed, M, N, K, oracle):
     A, B, bias = _values("all", 0.002, g, M, K), _values("all", 0.002, g, K, N), torch.randn(N, generator=g)
     want = oracle.kernels().pam_matmul_fwd(A, B, True, True, 1.0552) + bias
     for lay in ("nt", "tn"):
-        assert_bits_equal(_product(packed, _layout(A[None].cuda(), lay[0]), _layout(B[None].cuda(), lay[1]), bias=bias.cuda())[0], want, lay)
+        assert_bits_equal(_product(packed, _layout(A[None].cuda(), lay[0]), _layout(B[None].cuda(), lay[1]), bias=bias.cuda(), launches=3)[0], want, lay)
 
 
 @pytest.mark.parametrize("batch,M,N,K,split", [(3, 130, 70, 100, 1), (2, 113, 132, 200, 3), (1, 300, 260, 1000, 5), (1, 260, 512, 2000, 1)])
@@ -86,9 +89,10 @@ def test_batches_ranges_and_scratch(packed, batch, M, N, K, split):
     for lay in ("nn", "nt", "tn", "Tt"):
         x, y = _layout(A.cuda(), lay[0]), _layout(B.cuda(), lay[1])
         want = _in_place(packed, x, y, split, bias)
-        assert_bits_equal(_product(packed, x, y, split, bias), want, lay)
+        assert_bits_equal(_product(packed, x, y, split, bias, launches=3), want, lay)
         # one byte too little for the packed operands: the product runs on them as they are
-        assert_bits_equal(_product(packed, x, y, split, bias, scratch=packed.pamk_matmul_scratch_bytes(batch, M, N, K, split) - 1), want, lay)
+        assert_bits_equal(_product(packed, x, y, split, bias, scratch=packed.pamk_matmul_scratch_bytes(batch, M, N, K, split) - 1,
+                                   launches=1), want, lay)
 
 
 def test_heads_of_a_fused_projection(packed):
@@ -124,8 +128,11 @@ def test_a_large_product_through_the_operators():
         want = cb._matmul(_lib.MUL_PAM, A, B, 1.0, 2)
     finally:
         lib.pamk_test_set_packing_policy(0)
+    launches = lib.pamk_launch_count()
     assert_bits_equal(cb._matmul(_lib.MUL_PAM, A, B, 1.0, 2), want)
     assert_bits_equal(pam.matmul(A, B), want)
+    reduction = lib.pamk_matmul_auto_split(1, M, N, K) > 1
+    assert lib.pamk_launch_count() - launches == 2 * (3 + reduction)
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph):
         out = pam.matmul(A, B)
