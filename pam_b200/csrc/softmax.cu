@@ -11,6 +11,8 @@
 // A row is owned by one warp (up to 1024 columns) or by a CTA of eight warps (up to 12288 columns,
 // e.g. a 10000-word vocabulary).  -inf inputs (attention masks) get probability 0 as in the
 // reference; NaN or +inf anywhere makes the shift, and with it every output, NaN as there.
+#include <type_traits>
+
 #include "common.cuh"
 #include "pam_scalar.cuh"
 
@@ -81,6 +83,7 @@ __device__ __forceinline__ float load_shift(const float* partials, int count, fl
 // ---- values far inside the range rules' bounds ---------------------------------------------------
 __host__ __device__ constexpr uint32_t exponent_bits(int e) { return (uint32_t)(127 + e) << 23; }
 constexpr uint32_t kPlainLo = exponent_bits(-60), kPlainHi = exponent_bits(60), kPlainExp = exponent_bits(6);
+constexpr uint32_t kNormalExp = 0x42fc0000u;      // 126: powers of two to less than this are normal numbers
 // Below 2 * (hi - lo) where |x| lies in [lo, hi); what lies below wraps around.
 __device__ __forceinline__ uint32_t above(float x, uint32_t lo) { return 2u * (uint32_t)f2i(x) - 2u * lo; }
 constexpr int kMostE = 20;          // exponents of the exponentials that the short backward form takes
@@ -191,8 +194,13 @@ row_kernel(const RowArgs a) {
     const float lb2 = log2f(2.0f);
     const int32_t off = a.off;
     // Rows whose values lie far inside the range rules' bounds, by a look at them all, skip the rules: a product or quotient is
-    // one integer add instead of six instructions, chains of them without another operation between are one.  37824 rows of 197: forward
-    // 25.4 -> 17.0 us, backward 31.2 -> 18.9; 4096 rows of 1024 14.4 -> 10.7 and 15.8 -> 11.7.  What is left is memory (13.7 us backward) and the sums.
+    // one integer add instead of six instructions, chains of them without another operation between are one.  Zeros among the gradients
+    // (attention dropout, targets that do not count) have a form of their own.  Without the look -> rows that skip the rules / with 10 %
+    // zeros / that never do (us, forward with the maximum pass):
+    //   37824 rows of 197   forward 32.6 -> 24.0 / 31.8 / 31.8    backward 28.6 -> 16.5 / 20.2 / 26.8
+    //   8192 of 512                 17.3 -> 14.9 / 16.0 / 19.3             12.6 ->  8.3 / 10.1 / 13.0
+    //   4096 of 1024                19.0 -> 16.2 / 17.2 / 23.1             14.4 ->  8.7 / 10.7 / 16.1
+    // What is left is memory (13.7 us backward for the first) and the sums.
     constexpr bool kPlain = WARPS == 1 && (OP == kSoftmaxFwd || OP == kSoftmaxBwdSaved);
     // (an offset beyond an eighth of an exponent, or a post scale far from one, could carry results out of those bounds)
     const bool plain_call = off > -(1 << 20) && off < (1 << 20) && lb2 == 1.0f && (!a.post || (fabsf(a.post_scale) >= 0x1p-8f && fabsf(a.post_scale) <= 0x1p8f));
@@ -231,7 +239,7 @@ row_kernel(const RowArgs a) {
             if (next < a.rows) prefetch_row_l2(a.x + next * a.len, a.len, t, WARPS * 32);
         }
         float part = 0.0f;
-        bool plain = false;                                    // every value of this row is far inside the rules' bounds (see kPlain)
+        bool plain = false, near = false;                      // every value of this row is far inside the rules' bounds (see kPlain), and every quotient
         if (kPlain && OP == kSoftmaxFwd && without > 0) --without;
         else if (kPlain && OP == kSoftmaxFwd) {
             uint32_t far_x = 0u, far_y = 0u;
@@ -247,7 +255,15 @@ row_kernel(const RowArgs a) {
                 e.v[i] = masked ? 0.0f : big;
                 part = fadd(part, e.v[i]);                     // (padding adds +0)
             }
-            plain = __all_sync(0xffffffffu, far_x < 2u * (kPlainHi - kPlainLo) && far_y < 2u * (kPlainExp - kPlainLo));
+            plain = near = __all_sync(0xffffffffu, far_x < 2u * (kPlainHi - kPlainLo) && far_y < 2u * (kPlainExp - kPlainLo));
+            if (NCH * VEC > 8 && !plain) {
+                // What also passes (looked at in long rows, where the first look costs a tenth and more): zeros, whose scaled pattern is a subnormal one and vanishes beside a shift that is not zero (with a shift of
+                // zero it fails as y), and exponentials down to the least normal number, whose quotients need the rule.
+                far_x = 0u;
+#pragma unroll
+                for (int i = 0; i < NCH * VEC; ++i) far_x = max(far_x, x.v[i] == 0.0f || x.v[i] == -INFINITY ? 0u : above(x.v[i], kPlainLo));
+                plain = __all_sync(0xffffffffu, far_x < 2u * (kPlainHi - kPlainLo) && far_y < 2u * (kNormalExp - kPlainLo));
+            }
             if (!plain) {
                 part = 0.0f;
                 without = kWithout;
@@ -278,7 +294,7 @@ row_kernel(const RowArgs a) {
                 for (int i = 0; i < NCH * VEC; ++i) keep.v[i] = x.v[i] == -INFINITY ? -0.0f : e.v[i];
                 keep.store(a.aux + row * a.len, a.len, t);
             }
-            if (kPlain && plain && total > 0x1p-40f && total < 0x1p40f) {
+            if (kPlain && plain && near && total > 0x1p-40f && total < 0x1p40f) {
                 // (exponentials between 2^-64 and 2^64: their quotients pass)
                 const int32_t sub = isub(f2i(total), kBias - off);
 #pragma unroll
@@ -371,30 +387,42 @@ row_kernel(const RowArgs a) {
 #pragma unroll
                 for (int i = 0; i < NCH * VEC; ++i) {
                     const uint32_t be = (uint32_t)f2i(e.v[i]), bg = (uint32_t)f2i(g.v[i]) & 0x7fffffffu;
-                    const bool masked = be == 0x80000000u;      // (an entry that counts for nothing, like the padding)
+                    const bool masked = e.v[i] == 0.0f;         // (an entry that counts for nothing, like the padding; an exponential that underflowed)
                     least_e = min(least_e, masked ? ~0u : be); most_e = max(most_e, masked ? 0u : be);
                     least_g = min(least_g, masked ? ~0u : bg); most_g = max(most_g, bg);       // (a masked entry's inf or NaN counts)
                 }
                 least_e = __reduce_min_sync(0xffffffffu, least_e); most_e = __reduce_max_sync(0xffffffffu, most_e);
                 least_g = __reduce_min_sync(0xffffffffu, least_g); most_g = __reduce_max_sync(0xffffffffu, most_g);
+                const bool zeros = least_g == 0u;
+                if (zeros) {                                    // the least of the others
+                    least_g = ~0u;
+#pragma unroll
+                    for (int i = 0; i < NCH * VEC; ++i) {
+                        const uint32_t bg = (uint32_t)f2i(g.v[i]) & 0x7fffffffu;
+                        least_g = min(least_g, e.v[i] == 0.0f || bg == 0u ? ~0u : bg);
+                    }
+                    least_g = __reduce_min_sync(0xffffffffu, least_g);
+                }
                 const int e0 = exponent_of(least_e), e1 = exponent_of(most_e), g0 = exponent_of(least_g), g1 = exponent_of(most_g);
                 const int t0 = exponent_of((uint32_t)f2i(total));          // (a negative total has a huge one)
                 // the exponents of e / total, e / total / total, their product with g, and g / total, with one to spare for each step;
                 // e * (g / total + d_total) is looked at below, by a sum of patterns that a second factor of zero (or a subnormal one) only brings
                 // below kProductLo where e < 2^22 (the forward pass saves none above 4)
-                bool ok = e0 >= -60 && e1 <= kMostE && g0 >= -60 && g1 <= 60 && t0 >= -40 && t0 <= 40 &&
-                          min(e0 - t0, e0 - 2 * t0) >= -100 && max(e1 - t0, e1 - 2 * t0) <= 100 && e0 - 2 * t0 + g0 >= -108 && e1 - 2 * t0 + g1 <= 108;
-                if (ok) {                                       // (the same for a warp)
+                const bool ok = e0 >= -60 && e1 <= kMostE && g0 >= -60 && g1 <= 60 && t0 >= -40 && t0 <= 40 &&
+                                min(e0 - t0, e0 - 2 * t0) >= -100 && max(e1 - t0, e1 - 2 * t0) <= 100 && e0 - 2 * t0 + g0 >= -108 && e1 - 2 * t0 + g1 <= 108;
+                // with_zeros: gradients of zero, and second factors of zero, whose products flush to +0
+                auto short_form = [&](auto with_zeros) {
+                    constexpr bool kZeros = decltype(with_zeros)::value;
                     const int32_t sub = isub(f2i(total), kBias - off);
                     const int32_t by_den = isub(isub(isub(0, sub), sub), kBias - off), by_recip = isub(isub(kBias, sub), kBias - off);
                     float dsum = 0.0f;
                     R d;
 #pragma unroll
                     for (int i = 0; i < NCH * VEC; ++i) {
-                        const bool masked = f2i(e.v[i]) == (int32_t)0x80000000;
+                        const bool masked = e.v[i] == 0.0f, zero = kZeros && g.v[i] == 0.0f;
                         const float dden = -i2f(iadd3(f2i(e.v[i]), f2i(g.v[i]), by_den));
-                        dsum = fadd(dsum, masked ? -0.0f : dden);
-                        d.v[i] = i2f(iadd(f2i(g.v[i]), by_recip));
+                        dsum = fadd(dsum, masked || zero ? -0.0f : dden);
+                        d.v[i] = zero ? 0.0f : i2f(iadd(f2i(g.v[i]), by_recip));
                     }
                     const float d_total = group_sum<WARPS>(dsum, scratch);
                     // ((e * ln 2) * d) * log2 e (* post): the constants of the four products in one
@@ -404,22 +432,21 @@ row_kernel(const RowArgs a) {
                     uint32_t far = 0u;
 #pragma unroll
                     for (int i = 0; i < NCH * VEC; ++i) {
-                        const bool masked = f2i(e.v[i]) == (int32_t)0x80000000;
                         d.v[i] = fadd(d.v[i], d_total);
+                        const bool flushed = e.v[i] == 0.0f || (kZeros && d.v[i] == 0.0f);
                         const uint32_t sum = (uint32_t)f2i(e.v[i]) + ((uint32_t)f2i(d.v[i]) & 0x7fffffffu);
-                        far = max(far, masked ? 0u : sum - kProductLo);
+                        far = max(far, flushed ? 0u : sum - kProductLo);
                     }
-                    ok = __all_sync(0xffffffffu, far < kProductSpan);
-                    if (ok) {
+                    if (!__all_sync(0xffffffffu, far < kProductSpan)) return false;
 #pragma unroll
-                        for (int i = 0; i < NCH * VEC; ++i) {
-                            const bool masked = f2i(e.v[i]) == (int32_t)0x80000000;
-                            d.v[i] = masked ? 0.0f : i2f(iadd3(f2i(e.v[i]), f2i(d.v[i]), by_all));
-                        }
-                        d.store(a.out + row * a.len, a.len, t);
-                        continue;
+                    for (int i = 0; i < NCH * VEC; ++i) {
+                        const bool flushed = e.v[i] == 0.0f || (kZeros && d.v[i] == 0.0f);
+                        d.v[i] = flushed ? 0.0f : i2f(iadd3(f2i(e.v[i]), f2i(d.v[i]), by_all));
                     }
-                }
+                    d.store(a.out + row * a.len, a.len, t);
+                    return true;
+                };
+                if (ok && (zeros ? short_form(std::true_type{}) : short_form(std::false_type{}))) continue;      // (the same for a warp)
                 without = kWithout;
             }
             const Divisor by_total = make_divisor(total, off);

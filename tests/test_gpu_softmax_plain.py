@@ -72,11 +72,15 @@ def _inputs(kind, rows, n, g):
         dy[torch.rand(rows, n, generator=g) < 0.01] = float("nan")
         dy[torch.rand(rows, n, generator=g) < 0.01] = float("inf")
     if kind == "equal": x[:], dy[:] = 1.0, 0.25
+    if kind == "some zeros":                                 # of either sign, among inputs and gradients, and rows of gradients that are all zeros
+        x, dy = (torch.where(torch.rand(rows, n, generator=g) < 0.1, torch.tensor([0.0, -0.0])[torch.randint(0, 2, (rows, n), generator=g)], t) for t in (x, dy))
+        x[1::4], dy[::5] = x[1::4] + 3.0, 0.0                # (shifts of zero and of more)
+    if kind == "deep": x[:, n // 2] -= torch.arange(rows) * 2.0          # exponentials from one down to beyond the least normal number
     return x.cuda(), dy.cuda()
 
 
 @pytest.mark.parametrize("n", [1, 31, 33, 64, 65, 128, 197, 224, 225, 252, 255, 256, 500, 512, 700, 768, 1001, 1024])
-@pytest.mark.parametrize("kind", ["plain", "masked", "zeros", "mixed", "wide", "odd", "equal"])
+@pytest.mark.parametrize("kind", ["plain", "masked", "zeros", "mixed", "wide", "odd", "equal", "some zeros", "deep"])
 @pytest.mark.parametrize("offset,post", [(1.0, None), (1.0552, 0.125), (0.97, 1e-3), (1.5, -2.0)])
 def test_rows_in_both_forms(n, kind, offset, post):
     from pam_b200 import _lib
