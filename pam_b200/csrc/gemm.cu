@@ -407,9 +407,17 @@ __device__ __forceinline__ int sum_on_fma(int x, int y, int one) {
     return d;
 }
 __host__ __device__ constexpr bool multiply_add_product(int i, int j) { return j == 3 || j == 5 || (i == 7 && j == 1); }
-// The exact-gradient products mask every sum on the integer pipe, which leaves more of the sums to the other: 88 %.
-// 12608x192x768 199 -> 184.5 us, 768x192x12608 213 -> 201, 2048x2048x1024 480 -> 453 (75 % 187 / 202 / 465, all 199 / 213 / 475).
+// The exact-gradient products mask every sum on the integer pipe, which leaves more of the sums to the other: 81 %.
+// 12608x192x768 198 -> 182 us, 768x192x12608 209 -> 195, 2048x2048x1024 474 -> 446 (75 % 185 / 195 / 455, 88 % 185 / 197 / 450, all
+// 195 / 208 / 469).
 __host__ __device__ constexpr bool multiply_add_slope(int i, int j) { return (i + j) % 4 != 0 || i % 4 == 2; }
+template <bool (*ON)(int, int)>
+constexpr int products_on_fma() {
+    int n = 0;
+    for (int i = 0; i < 64; ++i) n += ON(i / 8, i % 8);
+    return n;
+}
+static_assert(products_on_fma<multiply_add_product>() == 17 && products_on_fma<multiply_add_slope>() == 52, "the shares stated above, of 64");
 
 // ---- eight sums at once, or none of them ----------------------------------------------------------------------------
 // c += p where x is not zero (either sign of it), and where pattern x is not `zero`: one compare for eight adds.  Written as conditions
