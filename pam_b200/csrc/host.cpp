@@ -140,11 +140,13 @@ bool wants_grad(const Tensor& t) { return t.defined() && t.requires_grad(); }
 
 // Whether scratch that a call can do without is there to be had, in a cached block or from the device: asked for in vain, it would make torch's
 // allocator give its whole cache back first, on every call.  (A cached block may turn out to be another stream's.)  A capture does
-// not touch the cache and may not ask.
+// not touch the cache and may not ask.  Other allocators than torch's own keep no such cache, and some refuse the questions (pluggable ones)
+// or answer them by taking all memory that is free (cudaMallocAsync): they are just asked for the scratch.
 bool room_for(size_t bytes, c10::DeviceIndex device) {
     c10::cuda::CUDAGuard guard(device);
     if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return true;
     auto* allocator = c10::cuda::CUDACachingAllocator::get();
+    if (allocator->name() != "native") return true;
     size_t largest = 1;                   // (zero would stand for the device's free memory)
     allocator->cacheInfo(device, &largest);
     if (largest >= bytes) return true;
