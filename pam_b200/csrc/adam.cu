@@ -127,12 +127,12 @@ __device__ __forceinline__ void four_elements(float* __restrict__ p, const float
 }
 
 // Four elements per thread, in at most 48 registers for five CTAs per SM: bound by DRAM with the short rule (the 254 tensors of a 6+6 transformer,
-// 42 million parameters, 189 us; one tensor of 2^25 143), by its instructions with the full one, five or six per primitive and more
-// for the division and log2f that only classify (2^25 elements with 30 % zeros among the gradients 233 us).  Eight elements per
-// thread took 198, 155 and 300 us, and 6.8 us instead of 4.1 for 30000 elements with zeros: twice the code, fewer warps.
+// 42 million parameters, 189 us; one tensor of 2^25 145), by its instructions with the full one, five or six per primitive and more
+// for the division and log2f that only classify (2^25 elements with 30 % zeros among the gradients 210 us).  Eight elements per
+// thread took 198, 152 and 257 us, and 6.8 us instead of 4.1 for 30000 elements with zeros: twice the code, fewer warps.
 // The 32 elements that a warp works on at a time take one of the two together, by a vote on the inputs: where each
 // thread chose for itself, zeros among the gradients (rows of an embedding that no token met, units behind
-// a ReLU) made the warp run both (2^25 elements, one zero in ten: 365 us, with the vote 198).
+// a ReLU) made the warp run both (2^25 elements, one zero in ten: 365 us, with the vote 201 to 207).
 __global__ void __launch_bounds__(kThreads, 5) adam_kernel(const AdamTable t, const AdamScalars s) {
     int which = 0, hi = t.used;                    // largest k with first[k] <= blockIdx.x (the same for the whole CTA)
     while (hi - which > 1) {

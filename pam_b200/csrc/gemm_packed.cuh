@@ -10,8 +10,8 @@
 // memory; warps move through the ring on their own, up to three slabs apart.
 // The sums are those of gemm.cu bit for bit: one thread per output, strictly in k order, the same ranges of K.
 //   4096^3 (us)   clean  0.1 % zeros  0.1 / 1 / 3 / 10 % specials  half zeros in A / in both
-//   in place      4387   6659         6659 / 9854 / 12712 / 15857  5500 / 7072
-//   packed        4196   5234         5234 / 6131 /  8824 / 13715  5255 / 6577
+//   in place      4375   6842         6765 / 9783 / 12558 / 15106  5534 / 7178
+//   packed        4231   5246         5233 / 6152 /  8952 / 13525  5264 / 6691
 // of which the passes take 68 (and 41 more where blocks have to be classified).  What bounds it: dispatch, 98 % on clean operands
 // (a packed add counts as two); on others the instructions beside the products and the lines to check.
 
@@ -481,11 +481,12 @@ __global__ void __launch_bounds__(256, 2) packed_kernel(const PackedParams p) {
 }
 
 // ---- where the operands are packed, and the scratch that it takes --------------------------------------------------------------
-// On clean operands the packed kernel saves at least 1.76 us per 1e9 products (4096^3: 4138 us, in place 4260 with both operands contiguous
-// along their rows, 4390 to 4420 in the other layouts); the passes cost 1.83 us per million elements and 12 us of launches and
-// flags.  Below that line the operands are used in place, also where they hold special values, which nothing knows
-// beforehand.  Clean, row-contiguous operands: 4096x4096x512 in place 543 us, packed 578; 2048^3 557 and 603; 3000x1500x2000 608 and
-// 625; with 1 % specials 1500x1500x4096 1411 and 946.
+// The line lies where clean operands break even: 1.76 us saved per 1e9 products, 1.83 us per million elements and 12 us for the passes, their launches
+// and flags.  Below it the operands are used in place, also where they hold special values, which nothing knows beforehand.  Clean operands,
+// in place with both contiguous along their rows / in the other layouts / packed: 8192x8192x4096 16780 / 17350 to 17400 / 16510, 4096^3 4237 / 4377 to
+// 4399 / 4230, and right above the line, where the layout that has least to gain loses 1 %, 3000^3 1795 / 1858 to 1871 / 1816 (1 % specials in place a
+// half slower than packed); below it 4096x4096x512 543 us in place, 578 packed, 2048^3 557 and 603, 3000x1500x2000 608 and 625; with 1 % specials
+// 1500x1500x4096 1411 and 946.
 int g_packing_policy = 0;            // tests: 0 by the rule, 1 wherever it exists, 2 nowhere
 
 bool packing_pays(int64_t batch, int64_t M, int64_t N, int64_t K) {
